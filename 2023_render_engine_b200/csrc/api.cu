@@ -144,7 +144,7 @@ rtb::SceneView rt_scene::view() const
 uint64_t rt_scene::device_bytes() const
 {
     return d_nodes.bytes + d_tris.bytes + d_leafpos.bytes + d_ref_boxes.bytes + d_ref_sorted.bytes + d_ref_pos.bytes +
-           d_spheres.bytes + scratch.queue.bytes + scratch.counters.bytes + d_tri_transp.bytes + d_mat_transp.bytes;
+           d_spheres.bytes + scratch.counters.bytes + d_tri_transp.bytes + d_mat_transp.bytes;
 }
 
 extern "C" {
@@ -227,8 +227,8 @@ int rt_scene_destroy(rt_scene *s)
     cudaSetDevice(s->ctx->device);
     cudaStreamSynchronize(s->ctx->stream);
     for (DevBuf *b : {&s->d_nodes, &s->d_tris, &s->d_leafpos, &s->d_ref_boxes, &s->d_ref_sorted, &s->d_ref_pos,
-                      &s->d_spheres, &s->scratch.queue, &s->scratch.counters, &s->h2d_rays, &s->d2h_hits, &s->d_mats,
-                      &s->d_tri_mat, &s->d_tri_shape, &s->d_tri_nidx, &s->d_normals, &s->d_emit_tri, &s->d_emit_cdf, &s->d_plights})
+                      &s->d_spheres, &s->scratch.counters, &s->h2d_rays, &s->d2h_hits, &s->d_mats,
+                      &s->d_tri_mat, &s->d_tri_shape, &s->d_tri_nidx, &s->d_normals, &s->d_emit_tri, &s->d_emit_cdf, &s->d_plights, &s->d_rec_mat})
         b->release();
     s->rscratch.release();
     delete s;
@@ -415,9 +415,8 @@ static int trace_common(rt_scene *s, const rt_ray *rays, uint64_t n, rt_hit *hit
     if ((reinterpret_cast<uintptr_t>(rays) | reinterpret_cast<uintptr_t>(hits)) & 15u)
         return fail(RT_ERR_INVALID, "rt_trace_closest: buffers must be 16-byte aligned");
     RTB_CUDA(cudaSetDevice(s->ctx->device));
-    RTB_CHECK(s->scratch.queue.reserve(std::max<uint64_t>(n, 1) * 4));
-    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, s->scratch.queue.as<uint32_t>(), (uint32_t)n,
-                                   s->scratch.counters.as<uint32_t>(), s->ctx->stream));
+    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, s->scratch.counters.as<uint32_t>(),
+                                   s->ctx->stream));
     return RT_OK;
 }
 
@@ -469,15 +468,14 @@ static int trace_any_common(rt_scene *s, const rt_ray *rays, uint64_t n, void *o
     RTB_CUDA(cudaSetDevice(s->ctx->device));
     cudaStream_t st = s->ctx->stream;
     if (flags & RT_TRACE_FAST) {
-        RTB_CHECK(launch_trace_any(s->view(), rays, n, out, bits, flags, s->scratch.counters.as<uint32_t>(), st));
+        if (bits) RTB_CHECK(s->any_hits.reserve(n));
+        RTB_CHECK(launch_trace_any(s->view(), rays, n, bits ? s->any_hits.as<uint8_t>() : static_cast<uint8_t *>(out),
+                                   out, bits, flags, s->scratch.counters.as<uint32_t>(), st));
     } else {
         // the reference's decision: its closest hit along the unbounded ray, then t <= tmax
-        RTB_CHECK(s->scratch.queue.reserve(n * 4));
         RTB_CHECK(s->any_hits.reserve(n * sizeof(rt_hit)));
-        RTB_CHECK(launch_trace_closest(s->view(), rays, n, s->any_hits.as<rt_hit>(),
-                                       (flags & RT_TRACE_SHADOW) | kTraceUnbounded, s->scratch.queue.as<uint32_t>(),
-                                       (uint32_t)n, s->scratch.counters.as<uint32_t>(), st));
-        RTB_CHECK(launch_occlusion_from_hits(rays, n, s->any_hits.as<rt_hit>(), out, bits, st));
+        RTB_CHECK(launch_trace_visible(s->view(), rays, n, s->any_hits.as<rt_hit>(), flags, out, bits,
+                                       s->scratch.counters.as<uint32_t>(), st));
     }
     uint32_t c[4] = {0, 0, 0, 0};
     RTB_CUDA(cudaMemcpyAsync(c, s->scratch.counters.ptr, sizeof(c), cudaMemcpyDeviceToHost, s->ctx->stream));

@@ -496,15 +496,17 @@ int build_scene_device(rt_scene *s, float margin_out[1])
 namespace {
 
 // Shadow-ray transparency of every record (bit 0 of v2.w): the triangle's own flag or its
-// material's RT_MATF_TRANSPARENT (Triangle.cu:439-440).
+// material's RT_MATF_TRANSPARENT (Triangle.cu:439-440); and its material id in record order, which
+// the renderer reads right after a hit.
 __global__ void k_record_flags(TriRecord *__restrict__ recs, uint32_t n, const uint8_t *__restrict__ tri_transparent,
                                const uint32_t *__restrict__ tri_mat, const uint8_t *__restrict__ mat_transparent,
-                               uint32_t nmat)
+                               uint32_t nmat, uint32_t *__restrict__ rec_mat)
 {
     const uint32_t r = blockIdx.x * kT + threadIdx.x;
     if (r >= n) return;
     const uint32_t id = __float_as_uint(recs[r].v1.w);
     const uint32_t m = tri_mat[id];
+    rec_mat[r] = m;
     recs[r].v2.w = __uint_as_float((tri_transparent[id] || (m < nmat && mat_transparent[m])) ? 1u : 0u);
 }
 
@@ -520,9 +522,10 @@ int refresh_record_flags(rt_scene *s)
     RTB_CHECK(s->d_tri_transp.upload(s->tri_transparent.data(), n, st));
     RTB_CHECK(s->d_tri_mat.upload(s->tri_material.data(), 4ull * n, st));
     RTB_CHECK(s->d_mat_transp.upload(mt.data(), mt.size(), st));
+    RTB_CHECK(s->d_rec_mat.reserve(4ull * n));
     k_record_flags<<<blocks_for(n), kT, 0, st>>>(s->d_tris.as<TriRecord>(), n, s->d_tri_transp.as<uint8_t>(),
                                                  s->d_tri_mat.as<uint32_t>(), s->d_mat_transp.as<uint8_t>(),
-                                                 (uint32_t)s->materials.size());
+                                                 (uint32_t)s->materials.size(), s->d_rec_mat.as<uint32_t>());
     RTB_CUDA(cudaGetLastError());
     return RT_OK;
 }

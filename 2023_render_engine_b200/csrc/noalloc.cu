@@ -4,12 +4,11 @@
 // thread with a frame-time budget (an allocation can synchronise the device), hosts that
 // hand all device memory to their own pool allocator and forbid allocations from
 // libraries, and applications that have already claimed nearly all device memory. For
-// them this entry point takes its scratch — the queue of rays that need the
-// reference-order replay and the queue/status counters — from a fixed array compiled into
-// this library instead of from the scene's on-demand buffers.
+// them this entry point takes its scratch — the status and work counters — from a fixed array
+// compiled into this library instead of from the scene's on-demand buffers.
 //
 // The array is a file-scope __device__ array, so every GPU that loads the library holds
-// it (a little over 4 MiB) until the process exits. Host code cannot use the array's name
+// it until the process exits. Host code cannot use the array's name
 // as a device address; its address is looked up once per device with
 // cudaGetSymbolAddress, with that device current, and kept for the life of the process.
 // A cudaDeviceReset by the application destroys the module that holds the array, so the
@@ -24,7 +23,7 @@ namespace {
 constexpr uint64_t kNoAllocMaxRays = 1ull << 20;  // rays per call
 constexpr uint64_t kCounterWords = 16;
 
-static __device__ __align__(256) uint32_t g_noalloc_scratch[kCounterWords + kNoAllocMaxRays];
+static __device__ __align__(256) uint32_t g_noalloc_scratch[kCounterWords];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
@@ -67,12 +66,10 @@ extern "C" int rt_trace_closest_noalloc(rt_scene *s, const rt_ray *rays, uint64_
         return RT_OK;
     }
     RTB_CUDA(cudaSetDevice(s->ctx->device));
-    uint32_t *scratch = nullptr;
-    RTB_CHECK(scratch_for(s->ctx->device, &scratch));
-    uint32_t *counters = scratch;               // cleared by the launch before the kernels run
-    uint32_t *queue = scratch + kCounterWords;  // written before it is read within the call
+    uint32_t *counters = nullptr;  // cleared by the launch before the kernels run
+    RTB_CHECK(scratch_for(s->ctx->device, &counters));
     cudaStream_t st = s->ctx->stream;
-    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, queue, (uint32_t)n, counters, st));
+    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, counters, st));
     uint32_t c[4] = {0, 0, 0, 0};
     RTB_CUDA(cudaMemcpyAsync(c, counters, sizeof(c), cudaMemcpyDeviceToHost, st));
     RTB_CUDA(cudaStreamSynchronize(st));

@@ -522,7 +522,7 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
     }
     if (!(total > 0)) return fail(RT_ERR_STATE, "rt_photons_trace: lights have no power");
     const uint32_t cap = (uint32_t)n;
-    DevBuf rays[2], beta[2], carry[2], rng[2], hits, sel, perl, dpow, cnt, queue;  // freed on return
+    DevBuf rays[2], beta[2], carry[2], rng[2], hits, sel, perl, dpow, cnt;  // freed on return
     for (int b = 0; b < 2; b++) {
         RTB_CHECK(rays[b].reserve(32ull * cap));
         RTB_CHECK(beta[b].reserve(16ull * cap));
@@ -534,7 +534,6 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
     RTB_CHECK(perl.reserve(8ull * nl));
     RTB_CHECK(dpow.upload(power.data(), 4ull * nl, st));
     RTB_CHECK(cnt.reserve(64));
-    RTB_CHECK(queue.reserve(4ull * cap));
     RTB_CHECK(s->scratch.counters.reserve(64));
     uint64_t store_cap = std::max<uint64_t>(4 * n, 1024);
     rt_photon_map *m = nullptr;
@@ -574,7 +573,7 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
         rays_traced = 0;
         for (uint32_t depth = 0; depth < max_depth; depth++) {
             RTB_CHECK(launch_trace_closest_dev(rv.sv, pb.rays[cur], pb.cnt + cur, cap, pb.hits, RT_TRACE_FAST,
-                                               queue.as<uint32_t>(), s->scratch.counters.as<uint32_t>(), st));
+                                               s->scratch.counters.as<uint32_t>(), st));
             RTB_CUDA(cudaMemsetAsync(pb.cnt + (cur ^ 1), 0, 4, st));
             k_photon_shade<<<cap / kPB + 1, kPB, 0, st>>>(rv, pb, cur, max_depth, rr_depth, seed, flags);
             RTB_CUDA(cudaGetLastError());

@@ -228,7 +228,7 @@ __device__ __forceinline__ uint32_t shade_key(const RenderView &rv, const Buffer
     if (prim & RT_PRIM_SHAPE)
         mat = rv.sv.spheres[prim & ~RT_PRIM_SHAPE].material;
     else
-        mat = __ldg(rv.tri_mat + prim);
+        mat = __ldg(rv.rec_mat + prim);
     const uint32_t type = (uint32_t)rv.mats[min(mat, rv.nmats - 1)].type;
     return min(1u + type, (uint32_t)kSortKeys - 1u);
 }
@@ -579,53 +579,65 @@ __global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView r
     }
 }
 
-// Any-hit test of the wave's shadow rays (persistent warps, counter cnt[5]); an unoccluded
-// ray adds its contribution to the path it belongs to.
-__global__ void __launch_bounds__(kB, RTB_TRAV_MIN_BLOCKS) k_shadow(RenderView rv, Buffers bf, int nxt, GuideView gv)
+// Any-hit test of the wave's shadow rays (persistent warps, counter cnt[5]): an occluded ray's
+// contribution loses its target.
+constexpr uint32_t kNoTarget = 0xFFFFFFFFu;
+__global__ void __launch_bounds__(kB, RTB_TRAV_MIN_BLOCKS) k_shadow(RenderView rv, Buffers bf)
 {
+    __shared__ TravWarp scratch[kB / 32];
     const uint32_t n = min(bf.cnt[2], bf.scap);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, 12), (unsigned long long)n);  // stats
-    persistent_traverse(
-        rv.sv, n, bf.cnt + 5, true,
-        [&](uint32_t i, Trav &T) {
+    walk_queue<true, false>(
+        rv.sv, scratch[threadIdx.x >> 5], n, bf.cnt + 5, false,
+        [&](uint32_t i, Walk &W) {
             const float4 r0 = reinterpret_cast<const float4 *>(bf.srays)[2 * i];
             const float4 r1 = reinterpret_cast<const float4 *>(bf.srays)[2 * i + 1];
-            const uint32_t sub = __float_as_uint(r1.w) >> kShadowSceneShift;
-            trav_init(T, r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, scene_root(rv.sv, sub));
-            T.shadow = (__float_as_uint(r1.w) & 1u) != 0;
+            const uint32_t last = __float_as_uint(r1.w);
+            walk_init(W, r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, scene_root(rv.sv, last >> kShadowSceneShift),
+                      (last & 1u) != 0);
         },
-        [&](uint32_t i, Trav &T) {
-            const float tmax = T.w.tmax;
-            bool occ = T.best.prim >= 0 && T.best.t < tmax;
-            if (!occ && rv.sv.nspheres) {
-                float t = tmax;
-                int32_t prim = -1;
-                float b1 = 0, b2 = 0;
-                const uint32_t sub =
-                    __float_as_uint(reinterpret_cast<const float4 *>(bf.srays)[2 * i + 1].w) >> kShadowSceneShift;
-                intersect_spheres(rv.sv, sub, T.w.ox, T.w.oy, T.w.oz, T.dx, T.dy, T.dz, tmax, T.shadow, t, prim, b1,
-                                  b2);
-                occ = prim >= 0 && t < tmax;
-            }
-            if (occ) return;
-            const float4 c = bf.scontrib[i];
-            const uint32_t target = __float_as_uint(c.w);
-            float *dst = (target & kRetireTarget) ? reinterpret_cast<float *>(bf.retire + (target & ~kRetireTarget))
-                                                   : reinterpret_cast<float *>(bf.st1[nxt] + target);
-            atomicAdd(dst + 0, c.x);
-            atomicAdd(dst + 1, c.y);
-            atomicAdd(dst + 2, c.z);
-            if (gv.train) {
-                const uint32_t rec = (__float_as_uint(reinterpret_cast<const float4 *>(bf.srays)[2 * i + 1].w) >> 1) &
-                                     kRecNone;
-                if (rec != kRecNone) {
-                    float4 *e = &gv.recs[rec].e;
-                    atomicAdd(&e->x, c.x);
-                    atomicAdd(&e->y, c.y);
-                    atomicAdd(&e->z, c.z);
-                }
-            }
+        [&](uint32_t i, Walk &W, float2) {
+            if (W.brec != kNoRec && W.bt < W.lim) bf.scontrib[i].w = __uint_as_float(kNoTarget);
         });
+}
+
+// The wave's shadow rays that no triangle occludes: those that no analytic shape occludes either
+// add their contribution to the path they belong to (and, while the guide trains, to its record).
+// One thread per ray, so that the shape tests run with whole warps; at the end of each walk
+// in k_shadow they ran with the few lanes whose rays had just ended.
+__global__ void __launch_bounds__(kB) k_shadow_add(RenderView rv, Buffers bf, int nxt, GuideView gv)
+{
+    const uint32_t n = min(bf.cnt[2], bf.scap);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 c = bf.scontrib[i];
+        const uint32_t target = __float_as_uint(c.w);
+        if (target == kNoTarget) continue;
+        if (rv.sv.nspheres) {
+            const float4 r0 = reinterpret_cast<const float4 *>(bf.srays)[2 * i];
+            const float4 r1 = reinterpret_cast<const float4 *>(bf.srays)[2 * i + 1];
+            const uint32_t last = __float_as_uint(r1.w);
+            float t = r0.w, b1 = 0, b2 = 0;
+            int32_t prim = -1;
+            intersect_spheres(rv.sv, last >> kShadowSceneShift, r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w,
+                              (last & 1u) != 0, t, prim, b1, b2);
+            if (prim >= 0 && t < r0.w) continue;
+        }
+        float *dst = (target & kRetireTarget) ? reinterpret_cast<float *>(bf.retire + (target & ~kRetireTarget))
+                                               : reinterpret_cast<float *>(bf.st1[nxt] + target);
+        atomicAdd(dst + 0, c.x);
+        atomicAdd(dst + 1, c.y);
+        atomicAdd(dst + 2, c.z);
+        if (gv.train) {
+            const uint32_t rec =
+                (__float_as_uint(reinterpret_cast<const float4 *>(bf.srays)[2 * i + 1].w) >> 1) & kRecNone;
+            if (rec != kRecNone) {
+                float4 *e = &gv.recs[rec].e;
+                atomicAdd(&e->x, c.x);
+                atomicAdd(&e->y, c.y);
+                atomicAdd(&e->z, c.z);
+            }
+        }
+    }
 }
 
 // Photon-map gathers queued by k_shade: the density estimate (Scene::combinePhotonContributions,
@@ -1042,6 +1054,7 @@ int make_render_view(rt_scene *s, RenderView &rv)
     rv.mats = s->d_mats.as<rt_material>();
     rv.nmats = (uint32_t)s->materials.size();
     rv.tri_mat = s->d_tri_mat.as<uint32_t>();
+    rv.rec_mat = s->d_rec_mat.as<uint32_t>();
     rv.tri_shape = s->d_tri_shape.as<int32_t>();
     rv.tri_nidx = s->has_normals ? s->d_tri_nidx.as<int32_t>() : nullptr;
     rv.normals = s->has_normals ? s->d_normals.as<float>() : nullptr;
@@ -1200,7 +1213,6 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         }
     }
     RTB_CHECK(rs.cnt.reserve(256));
-    RTB_CHECK(s->scratch.queue.reserve(4ull * cap));
     RTB_CHECK(s->scratch.counters.reserve(64));
     if (!rs.host_cnt) RTB_CUDA(cudaMallocHost(&rs.host_cnt, 256));
 
@@ -1253,6 +1265,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     const unsigned retire_blocks = std::min(blocks, resident_grid(SLOT_RETIRE_RESIDENT, k_retire, kB));
     const unsigned shadow_blocks =
         std::min<unsigned>(resident_grid(SLOT_SHADOW_RESIDENT, k_shadow, kB), (scap + kB - 1) / kB);
+    const unsigned add_blocks = std::min<unsigned>((scap + kB - 1) / kB, 16u * device_sm_count());
     unsigned gather_resident = device_slot(SLOT_GATHER_RESIDENT);  // persistent gather warps: every resident block
     if (gathers && !gather_resident) {
         int per_sm = 0;
@@ -1301,8 +1314,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         for (int k = 0; k < 4; k++) {
             RTB_CHECK(mark(k, 0));
             RTB_CHECK(launch_trace_closest_dev(rv.sv, bf.rays[cur], bf.cnt + cur, cap, bf.hits, trace_flags,
-                                               s->scratch.queue.as<uint32_t>(), s->scratch.counters.as<uint32_t>(),
-                                               st));
+                                               s->scratch.counters.as<uint32_t>(), st));
             RTB_CHECK(mark(k, 1));
             if (gv.params) {
                 k_guide_infer<<<infer_blocks, kInferWarps * 32, kInferSmem, st>>>(
@@ -1320,7 +1332,9 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
             k_shade<<<blocks, kB, 0, st>>>(rv, bf, cur, gv);
             RTB_CUDA(cudaGetLastError());
             RTB_CHECK(mark(k, 4));
-            k_shadow<<<shadow_blocks, kB, 0, st>>>(rv, bf, cur ^ 1, gv);
+            k_shadow<<<shadow_blocks, kB, 0, st>>>(rv, bf);
+            RTB_CUDA(cudaGetLastError());
+            k_shadow_add<<<add_blocks, kB, 0, st>>>(rv, bf, cur ^ 1, gv);
             RTB_CUDA(cudaGetLastError());
             RTB_CHECK(mark(k, 5));
             if (gathers) {

@@ -190,27 +190,34 @@ void build_ref_tree(const float *tri9, uint32_t n, RefTreeHost &out);
 // ---------------------------------------------------------------- kernels
 
 struct TraceScratch {
-    DevBuf queue;   // ray indices needing the exact path
-    DevBuf counters;  // [0] queue length, [1] status word, [2..] stats
+    DevBuf counters;  // [0] rays that needed the reference tree, [1] status word, [2] replays, [3] work counter
 };
 
+// Internal trace flags (above the public RT_TRACE_* bits).
+// kTraceVisible: the hits are only for Scene::isVisible's decision (see k_trace_closest).
+constexpr uint32_t kTraceVisible = 0x80000000u;
+// kTraceRecords: rt_hit::prim holds the triangle's record index (the renderer's form, which reads
+// the record next) instead of its id; analytic shapes as in the public form.
+constexpr uint32_t kTraceRecords = 0x40000000u;
+// kTraceIds: the walk itself writes triangle ids (set by the launcher when nothing else is left to do).
+constexpr uint32_t kTraceIds = 0x20000000u;
 int launch_trace_closest(const SceneView &v, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags,
-                         uint32_t *queue, uint32_t queue_cap, uint32_t *counters, cudaStream_t s);
-// Same with the ray count read on the device (queues built by other kernels); cap bounds it.
+                         uint32_t *counters, cudaStream_t s);
+// Same with the ray count read on the device (queues built by other kernels); cap bounds it. The
+// hits are the renderer's form (kTraceRecords).
 int launch_trace_closest_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_dev, uint32_t cap, rt_hit *hits,
-                             uint32_t flags, uint32_t *queue, uint32_t *counters, cudaStream_t s);
-// Internal trace flag (above the public RT_TRACE_* bits): trace every ray with tmax = inf,
-// as the reference's shadow rays are, whatever tmax the ray carries.
-constexpr uint32_t kTraceUnbounded = 0x80000000u;
-// Occlusion decided from closest hits: hit and t <= the ray's tmax (Scene::isVisible).
-int launch_occlusion_from_hits(const rt_ray *rays, uint64_t n, const rt_hit *hits, void *out, bool bits,
-                               cudaStream_t s);
-// Any-hit occlusion of n rays: one byte per ray, or (bits) bit i % 32 of word i / 32 (the last
-// word's bits past n are 0).
+                             uint32_t flags, uint32_t *counters, cudaStream_t s);
+// Scene::isVisible: occluded when the reference's closest hit along the unbounded ray is no farther
+// than the ray's tmax. One byte per ray, or (bits) bit i % 32 of word i / 32 (the last word's bits
+// past n are 0). hits: n entries of scratch.
+int launch_trace_visible(const SceneView &v, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags, void *out,
+                         bool bits, uint32_t *counters, cudaStream_t s);
 int launch_trace_counts(const SceneView &v, const rt_ray *rays, uint64_t n, uint32_t flags, bool anyhit,
                         uint32_t *counts, uint32_t *counters, cudaStream_t s);
-int launch_trace_any(const SceneView &v, const rt_ray *rays, uint64_t n, void *out, bool bits, uint32_t flags,
-                     uint32_t *counters, cudaStream_t s);
+// Any-hit occlusion of n rays, in the same two forms. walk_out: n bytes of scratch (`out` itself
+// may serve for the byte form).
+int launch_trace_any(const SceneView &v, const rt_ray *rays, uint64_t n, uint8_t *walk_out, void *out, bool bits,
+                     uint32_t flags, uint32_t *counters, cudaStream_t s);
 
 // Wavefront buffers of rt_render (grown on demand, kept between calls).
 struct RenderScratch {
@@ -303,7 +310,7 @@ struct rt_scene {
     rtb::TraceScratch scratch;
     uint64_t last_rays = 0, last_fallback = 0;
     rtb::DevBuf h2d_rays, d2h_hits;  // device staging for the host-buffer entry points
-    rtb::DevBuf any_hits;            // closest hits behind rt_trace_any's reference-exact decision
+    rtb::DevBuf any_hits;            // rt_trace_any: closest hits, or the walk's bytes behind the bit mask
     // merged scene (rt_scene_merge): its scenes' roots and ranges and where each one's
     // triangles start (emitters are gathered per scene at upload)
     bool merged = false;
@@ -339,6 +346,7 @@ struct rt_scene {
     rtb::DevBuf d_texels, d_tex_info, d_tri_uv;
     bool tex_dirty = false;
     rtb::DevBuf d_mats, d_tri_mat, d_tri_shape, d_tri_nidx, d_normals, d_emit_tri, d_emit_cdf, d_plights;
+    rtb::DevBuf d_rec_mat;  // material id per triangle record (leaf order)
     rtb::RenderScratch rscratch;
     rtb::SceneView view() const;
     uint64_t device_bytes() const;

@@ -16,6 +16,7 @@ struct RenderView {
     SceneView sv;
     const rt_material *mats;
     const uint32_t *tri_mat;
+    const uint32_t *rec_mat;  // material id per triangle record
     const int32_t *tri_shape;  // shape id per triangle (the reference's meshId)
     const int32_t *tri_nidx;  // 3 per triangle, -1 when the mesh has no normals
     const float *normals;
@@ -100,7 +101,7 @@ struct Surface {
     float area_cos;  // for MIS: |cos| at the emitter
 };
 
-// Triangle / sphere hit -> surface (Triangle::intersect, Triangle.cu:319-428;
+// Triangle / sphere hit in the renderer's form (kTraceRecords) -> surface (Triangle::intersect, Triangle.cu:319-428;
 // Sphere::intersect, Sphere.cu:277-355).
 __device__ __forceinline__ Surface surface_at(const RenderView &rv, const rt_hit &h, V3 o, V3 d, bool compat)
 {
@@ -143,7 +144,8 @@ __device__ __forceinline__ Surface surface_at(const RenderView &rv, const rt_hit
         s.area_cos = 0.f;
         return s;
     }
-    const TriRecord tr = rv.sv.tris[rv.sv.leafpos[h.prim]];
+    const TriRecord tr = rv.sv.tris[h.prim];
+    const uint32_t tri = __float_as_uint(tr.v1.w);
     V3 p0 = v3(tr.v0.x, tr.v0.y, tr.v0.z), p1 = v3(tr.v1.x, tr.v1.y, tr.v1.z), p2 = v3(tr.v2.x, tr.v2.y, tr.v2.z);
     float b1 = h.b1, b2 = h.b2, b0 = 1.f - b1 - b2;
     s.p = p0 * b0 + p1 * b1 + p2 * b2;
@@ -152,8 +154,8 @@ __device__ __forceinline__ Surface surface_at(const RenderView &rv, const rt_hit
     s.n = ng;
     const float eb7 = error_bound(7);
     s.perr = (vabs(p0 * b0) + vabs(p1 * b1) + vabs(p2 * b2)) * eb7;
-    if (rv.tri_nidx && rv.tri_nidx[3 * h.prim] >= 0) {
-        const int32_t *ni = rv.tri_nidx + 3 * h.prim;
+    if (rv.tri_nidx && rv.tri_nidx[3 * tri] >= 0) {
+        const int32_t *ni = rv.tri_nidx + 3 * tri;
         V3 n0 = v3(rv.normals[3 * ni[0]], rv.normals[3 * ni[0] + 1], rv.normals[3 * ni[0] + 2]);
         V3 n1 = v3(rv.normals[3 * ni[1]], rv.normals[3 * ni[1] + 1], rv.normals[3 * ni[1] + 2]);
         V3 n2 = v3(rv.normals[3 * ni[2]], rv.normals[3 * ni[2] + 1], rv.normals[3 * ni[2] + 2]);
@@ -161,8 +163,8 @@ __device__ __forceinline__ Surface surface_at(const RenderView &rv, const rt_hit
         s.n = ns;
         if (compat) s.p = s.p + ns * 0.15f;  // Triangle.cu:418
     }
-    s.mat = rv.tri_mat[h.prim];
-    s.shape = rv.tri_shape ? rv.tri_shape[h.prim] : 0;
+    s.mat = rv.rec_mat[h.prim];
+    s.shape = rv.tri_shape ? rv.tri_shape[tri] : 0;
     s.emissive_tri = true;
     s.area_cos = fabsf(dot(ng, d));
     return s;
@@ -209,7 +211,7 @@ __device__ __forceinline__ float2 surface_uv(const RenderView &rv, const rt_hit 
     }
     const float b1 = h.b1, b2 = h.b2, b0 = 1.f - b1 - b2;
     if (!rv.tri_uv) return make_float2(b1 + b2, b2);  // (0,0) b0 + (1,0) b1 + (1,1) b2
-    const float *t = rv.tri_uv + 6ull * (uint32_t)h.prim;
+    const float *t = rv.tri_uv + 6ull * __float_as_uint(rv.sv.tris[h.prim].v1.w);
     return make_float2(b0 * t[0] + b1 * t[2] + b2 * t[4], b0 * t[1] + b1 * t[3] + b2 * t[5]);
 }
 

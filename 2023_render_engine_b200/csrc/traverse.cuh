@@ -9,30 +9,24 @@
 
 namespace rtb {
 
-// Entries of a walk's stack (8 bytes each, in local memory). A walk that would need more ends,
-// and its ray is replayed on the reference tree (exact); 32 entries overflowed on dense
-// triangle soups without changing the render's speed.
+// Entries of a walk's stack (8 bytes each, in local memory). A walk that would need more drops
+// the entries its best hit has already passed, and if that makes no room it ends, and its ray is
+// replayed on the reference tree (exact); 32 entries overflowed on dense triangle soups without
+// changing the render's speed.
 #ifndef RTB_KSTACK
-#define RTB_KSTACK 48
+#define RTB_KSTACK 56
 #endif
 constexpr int kStack = RTB_KSTACK;
 
 // Resident blocks of 128 threads per SM the traversal kernels are compiled for (register cap
-// 65536 / (128 * N)): 9 gives 56 registers and 36 warps per SM (measured on the BVH-stress
-// ray set: 2294 / 2410 / 2490 Mrays/s for 7 / 8 / 9 with the binned-SAH tree; 3134 / 2870 /
-// 2530 for 9 / 10 (48 registers) / 11 (40) with the PLOC tree).
+// 65536 / (128 * N)): 9 gives 56 registers and 36 warps per SM.
 #ifndef RTB_TRAV_MIN_BLOCKS
 #define RTB_TRAV_MIN_BLOCKS 9
 #endif
-constexpr uint32_t kQueueBlocker = 0x80000000u;  // queue entry flag: replay needed (not just ancestor walk)
-
-struct Best {
-    float t;
-    int32_t prim;
-    uint32_t rank;
-    float b1, b2;
-    float minblock;
-};
+// Idle lanes a warp collects before it fetches new rays for them.
+#ifndef RTB_REFILL
+#define RTB_REFILL 8
+#endif
 
 __device__ __forceinline__ uint32_t byte_of(uint32_t w, int k) { return (w >> (8 * k)) & 0xFFu; }
 
@@ -48,30 +42,6 @@ __device__ __forceinline__ void load_ray(const rt_ray *rays, uint64_t i, float4 
     const float4 *r4 = reinterpret_cast<const float4 *>(rays);
     a = ld_stream(r4 + 2 * i);
     b = ld_stream(r4 + 2 * i + 1);
-}
-
-// Tests one triangle record against the running best; see the file comment for the rule.
-__device__ __forceinline__ void test_triangle(const WatertightRay &w, const TriRecord *tris, uint32_t rec,
-                                              bool shadow, Best &best)
-{
-    const float4 *p = reinterpret_cast<const float4 *>(tris + rec);
-    float4 a = ld_scene(p), b = ld_scene(p + 1), c = ld_scene(p + 2);
-    if (shadow && (__float_as_uint(c.w) & 1u)) return;
-    TriHit h;
-    if (!watertight_test(w, a, b, c, h)) return;
-    uint32_t rank = __float_as_uint(a.w);
-    if (h.t > best.t) return;
-    if (h.t == best.t && best.prim >= 0 && rank < best.rank) return;
-    float dt = watertight_delta_t(h);
-    if (h.t <= dt) {
-        best.minblock = fminf(best.minblock, h.t);
-        return;
-    }
-    best.t = h.t;
-    best.prim = (int32_t)__float_as_uint(b.w);
-    best.rank = rank;
-    best.b1 = fmul(h.e1, h.invDet);
-    best.b2 = fmul(h.e2, h.invDet);
 }
 
 // Sorting network for 8 keys (ascending).
@@ -92,26 +62,39 @@ __device__ __forceinline__ void sort8(uint32_t k[8])
     cas(k[3], k[4]);
 }
 
-// Per-ray traversal state of the BVH8 walk. The walk advances one node per trav_step so a
-// persistent warp can retire finished rays and start new ones lane by lane.
-struct Trav {
-    WatertightRay w;
-    float dx, dy, dz;
-    float ix, iy, iz, oix, oiy, oiz;
-    uint32_t cur;
+constexpr unsigned kAllLanes = 0xFFFFFFFFu;
+constexpr uint32_t kNoRec = 0xFFFFFFFFu;  // no triangle record (record indices are below 2^30)
+
+// One ray's walk, held by one lane of a warp.
+struct Walk {
+    float ox, oy, oz;
+    float ix, iy, iz;  // 1 / direction
+    float Sx, Sy, Sz;  // shear of the watertight test (make_watertight)
+    uint32_t kz;       // its axis
+    float lim;         // nodes that the ray enters beyond this are skipped
+    uint32_t cur;      // node to visit next
     int sp;
     uint32_t steps;
-    bool ok;
+    bool ok;      // false: ran out of stack or steps
     bool shadow;  // checkShadow semantics: transparent primitives are skipped
-    Best best;
-    uint32_t tested;  // triangle records tested (counted by the COUNT walk only; steps counts nodes)
+    float bt;     // the best hit so far: offset, triangle record (its barycentrics: TravWarp::bary)
+    uint32_t brec;
+    float minblock;   // smallest offset that failed the error-bound test
+    uint32_t tested;  // triangle records tested (rt_trace_counts only; steps counts nodes)
     // node index, entry distance bits: one 8-byte local access per push / pop. Keeping the bottom
-    // 4 or 8 entries in shared memory instead (the rest in local memory) measured slower, render
-    // 2091 / 2100 against 2210 Mrays/s and 2^24-ray trace ~2800 against ~3100: the choice
-    // between the two memories at every push and pop costs registers (spills from 32 to 344
-    // bytes) and instructions that the saved local traffic does not repay
+    // 4 or 8 entries in shared memory instead (the rest in local memory) measured slower
     uint2 st[kStack];
 };
+
+// What the lanes of a warp exchange in shared memory while they test triangles.
+struct alignas(16) TravWarp {
+    float4 res[32];     // offset, record and flags, b1, b2 of the pair lane j tested
+    float2 bary[32];    // b1, b2 of each lane's best hit
+    uint16_t pair[32];  // lane that owns pair j, its triangle's offset in the node's block << 5
+};
+constexpr uint32_t kPairBlocked = 0x80000000u;      // TravWarp::res.y: fails the error-bound test
+constexpr uint32_t kPairTransparent = 0x40000000u;  // transparent to shadow rays
+constexpr uint32_t kPairRecord = 0x3FFFFFFFu;
 
 // BVH8 root of scene `sub` (0 for a plain scene) and its spheres [s0, s0 + ns).
 __device__ __forceinline__ uint32_t scene_root(const SceneView &v, uint32_t sub)
@@ -132,187 +115,277 @@ __device__ __forceinline__ void scene_spheres(const SceneView &v, uint32_t sub, 
 }
 
 // root: the BVH8 node the walk starts at (kNoRoot: the scene has no triangles; the walk is
-// skipped).
-__device__ __forceinline__ void trav_init(Trav &T, float ox, float oy, float oz, float dx, float dy, float dz,
-                                          float tmax, uint32_t root)
+// skipped). lim: the ray's limit (the walk's; the triangle test's too unless it is unbounded).
+__device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz, float dx, float dy, float dz,
+                                          float lim, uint32_t root, bool shadow)
 {
-    T.w = make_watertight(ox, oy, oz, dx, dy, dz, tmax);
-    T.dx = dx;
-    T.dy = dy;
-    T.dz = dz;
-    T.ix = 1.0f / dx;
-    T.iy = 1.0f / dy;
-    T.iz = 1.0f / dz;
-    T.oix = -ox * T.ix;
-    T.oiy = -oy * T.iy;
-    T.oiz = -oz * T.iz;
-    T.cur = root;
-    T.sp = 0;
-    T.steps = 0;
-    T.ok = true;
-    T.shadow = false;
-    T.best = Best{INFINITY, -1, 0u, 0.f, 0.f, INFINITY};
-    T.tested = 0;
+    W.ox = ox;
+    W.oy = oy;
+    W.oz = oz;
+    W.ix = 1.0f / dx;
+    W.iy = 1.0f / dy;
+    W.iz = 1.0f / dz;
+    const WatertightRay w = make_watertight(ox, oy, oz, dx, dy, dz, lim);
+    W.Sx = w.Sx;
+    W.Sy = w.Sy;
+    W.Sz = w.Sz;
+    W.kz = (uint32_t)w.kz;
+    W.lim = lim;
+    W.cur = root;
+    W.sp = 0;
+    W.steps = 0;
+    W.ok = true;
+    W.shadow = shadow;
+    W.bt = INFINITY;
+    W.brec = kNoRec;
+    W.minblock = INFINITY;
+    W.tested = 0;
 }
 
-// Visits node T.cur: tests its eight quantized child boxes (unrolled), the triangles of the
-// hit leaves (rolled, so the long exact triangle test exists once in the instruction
-// stream), pushes the hit interior children far-to-near and selects the next node.
-// Postponing the leaf tests to separate warp-wide triangle steps (one triangle per lane per
-// step, taken when enough lanes have triangles waiting) visits the same nodes in the same
-// order but was slower on the BVH-stress scene: render 1683 / 1714 / 1654 against 1832
-// Mrays/s, 2^24-ray trace ~2900 against 3123, for triangle-step ratios 3 / 2 / 5 (leaves
-// hold at most 3 triangles, so the per-step phase vote costs more than the packing saves).
-// Two smaller rewrites of the box test were slower too (render / trace Mrays/s, against
-// 1837 / 3130): bytes turned into floats through the mantissa of 2^23 (1815 / 3067), and a
-// minimum instead of the sorting network when one interior child is hit (1824 / 3086). Shadow
-// rays (any hit) gain from the near-to-far order too: pushing their children unsorted, or only
-// the nearest first, rendered at 2140 and 2112 against 2228 Mrays/s (2^26 paths).
-// Returns true when the ray is done (T.ok = false if the stack or step cap was exceeded).
-template <bool COUNT = false>
-__device__ __forceinline__ bool trav_step(const SceneView &v, Trav &T, bool anyhit)
-{
-    const bool shadow = T.shadow;
-    if (++T.steps > v.nnodes + 1) {
-        T.ok = false;
-        return true;
-    }
-    const uint4 *np = reinterpret_cast<const uint4 *>(v.nodes + T.cur);
-    const uint4 n0 = ld_scene(np), n1 = ld_scene(np + 1), n2 = ld_scene(np + 2), n3 = ld_scene(np + 3),
-                n4 = ld_scene(np + 4);
-    const float sx = __uint_as_float((n0.w & 0xFFu) << 23);
-    const float sy = __uint_as_float(((n0.w >> 8) & 0xFFu) << 23);
-    const float sz = __uint_as_float(((n0.w >> 16) & 0xFFu) << 23);
-    const uint32_t imask = n0.w >> 24;
-    const uint32_t child_base = n1.x, tri_base = n1.y;
-    const uint32_t meta_lo = n1.z, meta_hi = n1.w;
-    // per-axis affine map t = q * (s * inv) + (p * inv - o * inv)
-    const float ax = sx * T.ix, bx = fmaf(__uint_as_float(n0.x), T.ix, T.oix);
-    const float ay = sy * T.iy, by = fmaf(__uint_as_float(n0.y), T.iy, T.oiy);
-    const float az = sz * T.iz, bz = fmaf(__uint_as_float(n0.z), T.iz, T.oiz);
-    const float tlimit = fminf(T.best.t, T.w.tmax);
-    uint32_t keys[8];
-    uint32_t nint = 0, leafmask = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int b = k & 3;
-        const uint32_t meta = byte_of(k < 4 ? meta_lo : meta_hi, b);
-        const float qlx = (float)byte_of(k < 4 ? n2.x : n2.y, b);
-        const float qly = (float)byte_of(k < 4 ? n2.z : n2.w, b);
-        const float qlz = (float)byte_of(k < 4 ? n3.x : n3.y, b);
-        const float qhx = (float)byte_of(k < 4 ? n3.z : n3.w, b);
-        const float qhy = (float)byte_of(k < 4 ? n4.x : n4.y, b);
-        const float qhz = (float)byte_of(k < 4 ? n4.z : n4.w, b);
-        const float t1x = fmaf(qlx, ax, bx), t2x = fmaf(qhx, ax, bx);
-        const float t1y = fmaf(qly, ay, by), t2y = fmaf(qhy, ay, by);
-        const float t1z = fmaf(qlz, az, bz), t2z = fmaf(qhz, az, bz);
-        const float tn = fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fmaxf(fminf(t1z, t2z), 0.0f));
-        const float tf = fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fminf(fmaxf(t1z, t2z), tlimit));
-        const bool hit = (meta != 0xFFu) && (tn <= tf);
-        const bool interior = (imask >> k) & 1u;
-        keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
-        nint += (hit && interior) ? 1u : 0u;
-        leafmask |= (hit && !interior) ? (1u << k) : 0u;
-    }
-#pragma unroll 1
-    while (leafmask) {
-        const int k = __ffs(leafmask) - 1;
-        leafmask &= leafmask - 1;
-        const uint32_t meta = byte_of(k < 4 ? meta_lo : meta_hi, k & 3);
-        const uint32_t first = tri_base + (meta & 31u), cnt = (meta >> 5) + 1;
-        if (COUNT) T.tested += cnt;
-#pragma unroll 1
-        for (uint32_t j = 0; j < cnt; j++) test_triangle(T.w, v.tris, first + j, shadow, T.best);
-        if (anyhit && T.best.prim >= 0) return true;
-    }
-    uint32_t next = 0xFFFFFFFFu;
-    const float tl = fminf(T.best.t, T.w.tmax);
-    if (nint) {
-        sort8(keys);
-#pragma unroll
-        for (int j = 7; j >= 1; j--) {
-            if (j < (int)nint) {
-                const uint32_t slot = keys[j] & 7u;
-                const float tn = __uint_as_float(keys[j] & ~7u);
-                if (tn <= tl) {
-                    if (T.sp >= kStack) {
-                        T.ok = false;
-                        return true;
-                    }
-                    T.st[T.sp] = make_uint2(child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3),
-                                            __float_as_uint(tn));
-                    T.sp++;
-                }
-            }
-        }
-        const uint32_t slot = keys[0] & 7u;
-        if (__uint_as_float(keys[0] & ~7u) <= tl) next = child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3);
-    }
-    if (next == 0xFFFFFFFFu) {
-#pragma unroll 1
-        while (T.sp > 0) {
-            T.sp--;
-            const uint2 e = T.st[T.sp];
-            if (__uint_as_float(e.y) <= tl) {
-                next = e.x;
-                break;
-            }
-        }
-    }
-    if (next == 0xFFFFFFFFu) return true;
-    T.cur = next;
-    return false;
-}
-
-// Whole traversal of one ray; returns false if the stack would overflow (result then
-// unreliable).
-__device__ __forceinline__ bool traverse_bvh8(const SceneView &v, const WatertightRay &w, float dx, float dy, float dz,
-                                              bool shadow, bool anyhit, Best &best)
-{
-    Trav T;
-    trav_init(T, w.ox, w.oy, w.oz, dx, dy, dz, w.tmax, scene_root(v, 0));
-    T.shadow = shadow;
-    T.best = best;
-    if (T.cur != kNoRoot)
-        while (!trav_step(v, T, anyhit)) {
-        }
-    best = T.best;
-    return T.ok;
-}
-
-// Persistent-warp driver: every lane runs its own ray; a lane whose ray is done fetches the
-// next ray index from *work (one atomic per fetching warp) until n is exhausted.
-// init(i, T) prepares ray i (trav_init + T.shadow), finish(i, T) consumes the result.
-// COUNT: the walk also counts the triangle records it tests (T.tested), for rt_trace_counts.
-template <bool COUNT = false, typename Init, typename Finish>
-__device__ __forceinline__ void persistent_traverse(const SceneView &v, uint32_t n, uint32_t *work, bool anyhit,
-                                                    Init init, Finish finish)
+// Walks the rays [0, n) of a queue: every lane of a persistent warp runs its own ray, and lanes
+// whose rays are done fetch the next ones together. A step visits one node per lane and then
+// tests the triangles of the leaves the whole warp hit, one (ray, triangle) pair per lane:
+// the pairs are numbered by a prefix sum over the lanes, each lane reads its pair's ray from the
+// owner by shuffles, and the owner takes the results in its own triangle order, so a walk gives
+// what it gives when every lane tests its own triangles one after the other. A step hits about
+// as many triangles as a warp has lanes, so they mostly take one round, where the serial loop
+// took as many as the lane with the most of them, with a few lanes active in each and a triangle
+// fetch of latency per round.
+//
+// init(i, W) prepares ray i (walk_init); finish(i, W, bary) consumes its result. ANY: the walk
+// ends at the first accepted hit in triangle order (in the node that has one). unbounded: the
+// triangle test has no limit (lim only bounds the nodes). COUNT: also counts the triangles a
+// serial walk would test (whole leaves, up to the leaf of the accepted hit under ANY).
+template <bool ANY, bool COUNT, typename Init, typename Finish>
+__device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uint32_t n, uint32_t *work,
+                                           bool unbounded, Init init, Finish finish)
 {
     const unsigned lane = threadIdx.x & 31u;
     uint32_t ray = 0xFFFFFFFFu;
     bool exhausted = false;
-    Trav T;
+    Walk W;
     for (;;) {
-        const bool idle = ray == 0xFFFFFFFFu;
-        const unsigned idle_mask = __ballot_sync(0xFFFFFFFFu, idle);
-        if (idle_mask && !exhausted) {
-            const unsigned leader = __ffs(idle_mask) - 1;
+        const unsigned idle = __ballot_sync(kAllLanes, ray == 0xFFFFFFFFu);
+        if (!exhausted && __popc(idle) >= RTB_REFILL) {
             uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(work, (uint32_t)__popc(idle_mask));
-            base = __shfl_sync(0xFFFFFFFFu, base, leader);
-            if (base >= n) exhausted = true;
-            if (idle) {
-                const uint32_t mine = base + __popc(idle_mask & ((1u << lane) - 1u));
+            if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
+            base = __shfl_sync(kAllLanes, base, 0);
+            if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
+            if (ray == 0xFFFFFFFFu) {
+                const uint32_t mine = base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < n) {
                     ray = mine;
-                    init(ray, T);
+                    init(ray, W);
+                    if (W.cur == kNoRoot) {
+                        finish(ray, W, make_float2(0.f, 0.f));
+                        ray = 0xFFFFFFFFu;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        const bool active = ray != 0xFFFFFFFFu;
+        if (!__any_sync(kAllLanes, active)) {
+            if (exhausted) break;
+            continue;
+        }
+        // visit a node: its eight quantized child boxes; the triangles of the hit leaves as a
+        // mask over the node's block of records, the hit interior children pushed far to near
+        uint32_t trimask = 0, leafend = 0, tri_base = 0, next = kNoRoot;
+        float next_t = 0.f;
+        bool done = false;
+        if (active) {
+            if (++W.steps > v.nnodes + 1) {
+                W.ok = false;
+                done = true;
+            } else {
+                const uint4 *np = reinterpret_cast<const uint4 *>(v.nodes + W.cur);
+                const uint4 n0 = ld_scene(np), n1 = ld_scene(np + 1), n2 = ld_scene(np + 2), n3 = ld_scene(np + 3),
+                            n4 = ld_scene(np + 4);
+                const float sx = __uint_as_float((n0.w & 0xFFu) << 23);
+                const float sy = __uint_as_float(((n0.w >> 8) & 0xFFu) << 23);
+                const float sz = __uint_as_float(((n0.w >> 16) & 0xFFu) << 23);
+                const uint32_t imask = n0.w >> 24;
+                const uint32_t child_base = n1.x;
+                tri_base = n1.y;
+                const uint32_t meta_lo = n1.z, meta_hi = n1.w;
+                // per-axis affine map t = q * (s * inv) + (p * inv - o * inv)
+                const float ax = sx * W.ix, bx = fmaf(__uint_as_float(n0.x), W.ix, -W.ox * W.ix);
+                const float ay = sy * W.iy, by = fmaf(__uint_as_float(n0.y), W.iy, -W.oy * W.iy);
+                const float az = sz * W.iz, bz = fmaf(__uint_as_float(n0.z), W.iz, -W.oz * W.iz);
+                const float tlimit = fminf(W.bt, W.lim);
+                uint32_t keys[8];
+                uint32_t nint = 0;
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const int b = k & 3;
+                    const uint32_t meta = byte_of(k < 4 ? meta_lo : meta_hi, b);
+                    const float qlx = (float)byte_of(k < 4 ? n2.x : n2.y, b);
+                    const float qly = (float)byte_of(k < 4 ? n2.z : n2.w, b);
+                    const float qlz = (float)byte_of(k < 4 ? n3.x : n3.y, b);
+                    const float qhx = (float)byte_of(k < 4 ? n3.z : n3.w, b);
+                    const float qhy = (float)byte_of(k < 4 ? n4.x : n4.y, b);
+                    const float qhz = (float)byte_of(k < 4 ? n4.z : n4.w, b);
+                    const float t1x = fmaf(qlx, ax, bx), t2x = fmaf(qhx, ax, bx);
+                    const float t1y = fmaf(qly, ay, by), t2y = fmaf(qhy, ay, by);
+                    const float t1z = fmaf(qlz, az, bz), t2z = fmaf(qhz, az, bz);
+                    const float tn =
+                        fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fmaxf(fminf(t1z, t2z), 0.0f));
+                    const float tf =
+                        fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fminf(fmaxf(t1z, t2z), tlimit));
+                    const bool hit = (meta != 0xFFu) && (tn <= tf);
+                    const bool interior = (imask >> k) & 1u;
+                    keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
+                    nint += (hit && interior) ? 1u : 0u;
+                    if (hit && !interior) {
+                        trimask |= ((2u << (meta >> 5)) - 1u) << (meta & 31u);
+                        if (COUNT) leafend |= (1u << (meta >> 5)) << (meta & 31u);
+                    }
+                }
+                if (nint) {
+                    sort8(keys);
+                    if (W.sp + (int)nint - 1 > kStack) {  // drop the entries beyond the best hit
+                        int kept = 0;
+#pragma unroll 1
+                        for (int e = 0; e < W.sp; e++) {
+                            const uint2 x = W.st[e];
+                            if (__uint_as_float(x.y) <= tlimit) W.st[kept++] = x;
+                        }
+                        W.sp = kept;
+                        if (W.sp + (int)nint - 1 > kStack) {
+                            W.ok = false;
+                            done = true;
+                        }
+                    }
+                    if (!done) {
+#pragma unroll
+                        for (int j = 7; j >= 1; j--)
+                            if (j < (int)nint) {
+                                const uint32_t slot = keys[j] & 7u;
+                                W.st[W.sp] = make_uint2(child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3),
+                                                        keys[j] & ~7u);
+                                W.sp++;
+                            }
+                    }
+                    const uint32_t slot = keys[0] & 7u;
+                    next = child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3);
+                    next_t = __uint_as_float(keys[0] & ~7u);
                 }
             }
         }
-        if (__all_sync(0xFFFFFFFFu, ray == 0xFFFFFFFFu)) break;
-        if (ray != 0xFFFFFFFFu) {
-            if (T.cur == kNoRoot || trav_step<COUNT>(v, T, anyhit)) {
-                finish(ray, T);
+        // the triangles of the whole warp, 32 pairs a round
+        const uint32_t mytris = (uint32_t)__popc(trimask);
+        if (__any_sync(kAllLanes, trimask != 0)) {
+            uint32_t incl = mytris;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kAllLanes, incl, o);
+                if (lane >= (unsigned)o) incl += y;
+            }
+            const uint32_t total = __shfl_sync(kAllLanes, incl, 31);
+            uint32_t at = incl - mytris, left = trimask;
+            if (COUNT && !ANY) W.tested += mytris;
+            uint32_t before = 0;  // triangles of this lane offered in earlier rounds (COUNT)
+            for (uint32_t r0 = 0; r0 < total; r0 += 32) {
+                const uint32_t first = at;
+#pragma unroll 1
+                while (left && at < r0 + 32) {
+                    const uint32_t off = (uint32_t)__ffs(left) - 1u;
+                    left &= left - 1u;
+                    sm.pair[at - r0] = (uint16_t)(lane | (off << 5));
+                    at++;
+                }
+                __syncwarp();
+                const bool on = r0 + lane < total;
+                const uint32_t e = on ? sm.pair[lane] : lane;
+                const int src = (int)(e & 31u);
+                WatertightRay w;
+                w.ox = __shfl_sync(kAllLanes, W.ox, src);
+                w.oy = __shfl_sync(kAllLanes, W.oy, src);
+                w.oz = __shfl_sync(kAllLanes, W.oz, src);
+                w.Sx = __shfl_sync(kAllLanes, W.Sx, src);
+                w.Sy = __shfl_sync(kAllLanes, W.Sy, src);
+                w.Sz = __shfl_sync(kAllLanes, W.Sz, src);
+                const float lim = __shfl_sync(kAllLanes, W.lim, src);
+                const uint32_t axis_base = __shfl_sync(kAllLanes, (tri_base << 2) | (W.kz & 3u), src);
+                w.tmax = unbounded ? INFINITY : lim;
+                w.kz = (int)(axis_base & 3u);
+                w.kx = w.kz == 2 ? 0 : w.kz + 1;
+                w.ky = w.kx == 2 ? 0 : w.kx + 1;
+                bool hit = false;
+                if (on) {
+                    const uint32_t rec = (axis_base >> 2) + (e >> 5);
+                    const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
+                    const float4 a = ld_scene(p), b = ld_scene(p + 1), c = ld_scene(p + 2);
+                    TriHit h;
+                    hit = watertight_test(w, a, b, c, h);
+                    if (hit) {
+                        const float dt = watertight_delta_t(h);
+                        const uint32_t fl = rec | (h.t <= dt ? kPairBlocked : 0u) |
+                                            ((__float_as_uint(c.w) & 1u) ? kPairTransparent : 0u);
+                        sm.res[lane] =
+                            make_float4(h.t, __uint_as_float(fl), fmul(h.e1, h.invDet), fmul(h.e2, h.invDet));
+                    }
+                }
+                uint32_t mine = __ballot_sync(kAllLanes, hit);
+                __syncwarp();
+                // the owner takes the results of its own pairs, in order
+                mine = at > first ? (mine >> (first - r0)) & ((1u << (at - first)) - 1u) : 0u;
+                if (ANY && W.brec != kNoRec) mine = 0;
+#pragma unroll 1
+                while (mine) {
+                    const uint32_t j = first - r0 + (uint32_t)__ffs(mine) - 1u;
+                    mine &= mine - 1u;
+                    const float2 tf = *reinterpret_cast<const float2 *>(&sm.res[j]);
+                    const uint32_t fl = __float_as_uint(tf.y), rec = fl & kPairRecord;
+                    if (W.shadow && (fl & kPairTransparent)) continue;
+                    if (tf.x > W.bt) continue;
+                    if (tf.x == W.bt && W.brec != kNoRec &&
+                        __float_as_uint(__ldg(&v.tris[rec].v0.w)) < __float_as_uint(__ldg(&v.tris[W.brec].v0.w)))
+                        continue;
+                    if (fl & kPairBlocked) {
+                        W.minblock = fminf(W.minblock, tf.x);
+                        continue;
+                    }
+                    W.bt = tf.x;
+                    W.brec = rec;
+                    sm.bary[lane] = *(reinterpret_cast<const float2 *>(&sm.res[j]) + 1);
+                    if (ANY) {
+                        if (COUNT) {  // the triangles up to the end of this one's leaf
+                            const uint32_t off = sm.pair[j] >> 5;
+                            const uint32_t end = (uint32_t)__ffs(leafend >> off) - 1u + off;
+                            before = (uint32_t)__popc(trimask & ((2u << end) - 1u));
+                        }
+                        break;
+                    }
+                }
+            }
+            if (COUNT && ANY) W.tested += W.brec != kNoRec ? before : mytris;
+            __syncwarp();
+        }
+        if (active) {
+            // the nearest hit child, or the top stack entry the best hit has not passed
+            const float tl = fminf(W.bt, W.lim);
+            if (ANY && W.brec != kNoRec) done = true;
+            if (!done) {
+                if (next != kNoRoot && next_t <= tl) {
+                    W.cur = next;
+                } else {
+                    done = true;
+#pragma unroll 1
+                    while (W.sp > 0) {
+                        W.sp--;
+                        const uint2 e = W.st[W.sp];
+                        if (__uint_as_float(e.y) <= tl) {
+                            W.cur = e.x;
+                            done = false;
+                            break;
+                        }
+                    }
+                }
+            }
+            if (done) {
+                finish(ray, W, W.brec != kNoRec ? sm.bary[lane] : make_float2(0.f, 0.f));
                 ray = 0xFFFFFFFFu;
             }
         }

@@ -163,9 +163,9 @@ RT_API int rt_trace_closest_host(rt_scene *scene, const rt_ray *rays, uint64_t n
 /* Closest hit exactly like rt_trace_closest, for callers that must not allocate device
  * memory while they trace (a render thread that cannot afford the device synchronisation an
  * allocation may cause, or a host whose own pool allocator owns all device memory). It has
- * no counterpart in the reference. Its scratch (the reference-order replay queue and the
- * counters) is a fixed device array inside this library, about 4 MiB, held on every GPU
- * that loads the library until the process exits. At most 1048576 rays per call
+ * no counterpart in the reference. Its scratch (status and work counters) is a fixed device
+ * array inside this library, held on every GPU that loads the library until the process
+ * exits. At most 1048576 rays per call
  * (RT_ERR_CAPACITY above that). The first call on a device looks up the array's device
  * address (make that first call before any stream capture) and keeps it for the process's
  * life, so do not call it after a cudaDeviceReset of that device. All calls share the array:
