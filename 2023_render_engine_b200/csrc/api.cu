@@ -281,6 +281,7 @@ int rt_scene_add_sphere(rt_scene *s, const float o2w[16], const float w2o[16], f
     r.material = material;
     r.shape_id = shape_id;
     r.flags = transparent ? 3u : 0u;  // bit 1: requested at add time, bit 0: effective
+    if (w2o[12] == 0.f && w2o[13] == 0.f && w2o[14] == 0.f && w2o[15] == 1.f) r.flags |= kShapeAffine;
     if (index) *index = (uint32_t)s->spheres.size();
     s->spheres.push_back(r);
     s->committed = false;

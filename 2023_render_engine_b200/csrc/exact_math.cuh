@@ -170,6 +170,35 @@ __device__ __forceinline__ EF ef_sqrt(EF f)
     return {v, __double2float_rn(__ddiv_rn(__dmul_rn(0.5, (double)f.e), (double)v))};
 }
 
+// Whether sphere_test certainly rejects the ray, for an affine world->object matrix (its last row
+// (0, 0, 0, 1)): most of a scene's rays pass most of its spheres by a margin far above the
+// rounding of the exact test, whose error-bounded quadratic takes some 250 operations with
+// six divisions and a double-precision root. With p, d the object-space origin and direction
+// exactly as sphere_test computes them first (it then moves p along d, which leaves the line
+// where it is, and scales d to unit length): the line misses the sphere when
+// (d.p)^2 < |d|^2 (|p|^2 - r^2), and a ray that starts outside and moves away has both roots
+// negative. Each comparison keeps 1e-4 of the terms' size, against about 2e-6 of rounding in
+// either evaluation; a NaN never rejects.
+// (rows 0..2 of the matrix as float4)
+__device__ __forceinline__ bool sphere_missed(const float4 *m, float radius, float ox, float oy, float oz, float dx,
+                                              float dy, float dz)
+{
+    float po[3], pd[3];
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        const float4 row = __ldg(m + r);
+        po[r] = fadd(fadd(fadd(fmul(row.x, ox), fmul(row.y, oy)), fmul(row.z, oz)), row.w);
+        pd[r] = fadd(fadd(fmul(row.x, dx), fmul(row.y, dy)), fmul(row.z, dz));
+    }
+    const float dd = pd[0] * pd[0] + pd[1] * pd[1] + pd[2] * pd[2];
+    const float b = pd[0] * po[0] + pd[1] * po[1] + pd[2] * po[2];
+    const float pp = po[0] * po[0] + po[1] * po[1] + po[2] * po[2], rr = radius * radius;
+    const float tol = 1e-4f * (pp + rr), c = pp - rr;
+    // squares that leave the normal range (scales near 1e-19 or 1e19) decide nothing
+    if (!(dd > 1e-30f && dd < 1e30f && rr > 1e-30f && pp + rr < 1e30f)) return false;
+    return b * b < dd * (c - tol) || (b > 0.f && c > tol);
+}
+
 // Sphere::intersects (shapes/Sphere.cu:357-398) for a full sphere: ray to object space
 // with error bounds (Transform.cu:328-404), normalized direction, ErrorFloat quadratic
 // (math.cu:91-115), bound checks (Sphere.cu:41-81). Returns the object-space offset.

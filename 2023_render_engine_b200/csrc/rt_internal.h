@@ -124,13 +124,14 @@ struct alignas(16) TriRecord {
 // Analytic shape as the reference stores it: world->object matrix (rows 0..3), radius
 // (spheres) and object->world matrix. A plane (kShapePlane) is the unit square [0,1]^2 of its
 // object space (shapes/Plane.cu).
-constexpr uint32_t kShapePlane = 4u;  // SphereRecord.flags: the record is a Plane
+constexpr uint32_t kShapePlane = 4u;   // SphereRecord.flags: the record is a Plane
+constexpr uint32_t kShapeAffine = 8u;  // a sphere whose world->object matrix ends in (0, 0, 0, 1)
 struct alignas(16) SphereRecord {
     float w2o[16];
     float radius;
     uint32_t material;
     int32_t shape_id;
-    uint32_t flags;  // bit 0: transparent to shadow rays; bit 1: transparent as added; kShapePlane
+    uint32_t flags;  // bit 0: transparent to shadow rays; bit 1: transparent as added; kShape*
     float o2w[16];
 };
 

@@ -113,14 +113,16 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_counts(Sc
 // the replay of the reference's answer (see the file comment); the analytic shapes; triangle
 // ids (kTraceRecords: the renderer's form, triangle records) or, for kTraceVisible, the occlusion
 // decision in `out` (one byte per ray, or with bits one word per 32 rays). With nothing of that
-// to do it only looks at the rays whose walk could not finish (counters[0] of them).
-__global__ void __launch_bounds__(kBlock) k_trace_finish(SceneView v, const rt_ray *__restrict__ rays, uint64_t n,
+// to do it only looks at the rays whose walk could not finish (counters[0] of them). EXACT: without
+// RT_TRACE_FAST.
+template <bool EXACT>
+__global__ void __launch_bounds__(kBlock, EXACT ? 8 : 12) k_trace_finish(SceneView v, const rt_ray *__restrict__ rays, uint64_t n,
                                                          const uint32_t *__restrict__ n_dev, rt_hit *__restrict__ hits,
                                                          uint32_t flags, void *__restrict__ out, bool bits,
                                                          uint32_t *__restrict__ counters)
 {
     if (n_dev) n = min((uint64_t)*n_dev, n);
-    const bool exact = !(flags & RT_TRACE_FAST), visible = (flags & kTraceVisible) != 0;
+    const bool exact = EXACT, visible = EXACT && (flags & kTraceVisible) != 0;
     if (!exact && !v.nspheres && *(volatile uint32_t *)counters == 0u) return;
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
     // whole warps stay in the loop (the bit mask is gathered with a ballot)
@@ -129,12 +131,12 @@ __global__ void __launch_bounds__(kBlock) k_trace_finish(SceneView v, const rt_r
         bool occ = false;
         if (i < n) {
             const float4 hv = reinterpret_cast<const float4 *>(hits)[i];
+            float4 ra, rb;
+            load_ray(rays, i, ra, rb);
             float t = hv.x, b1 = hv.z, b2 = hv.w;
             int32_t rec = __float_as_int(hv.y), prim = rec;
             bool replay = rec == kHitReplay;
             if (exact || v.nspheres || replay) {
-                float4 ra, rb;
-                load_ray(rays, i, ra, rb);
                 const float tri_max = visible ? INFINITY : ra.w;
                 if (exact && rec >= 0 && !replay) {
                     const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
@@ -261,6 +263,10 @@ static unsigned persistent_blocks()
     return cached;
 }
 
+// Blocks of a walk over n rays: all that are resident, or one per 16 rays (4 per warp) where that is
+// fewer.
+static uint64_t walk_blocks(uint64_t n) { return std::min<uint64_t>((n + 15) / 16, persistent_blocks()); }
+
 // The walk, then k_trace_finish. n_dev: the count, when it is on the device (n bounds it).
 static int launch_trace(const SceneView &v, const rt_ray *rays, uint64_t n, const uint32_t *n_dev, rt_hit *hits,
                         uint32_t flags, void *out, bool bits, uint32_t *counters, cudaStream_t s)
@@ -269,11 +275,12 @@ static int launch_trace(const SceneView &v, const rt_ray *rays, uint64_t n, cons
     // fast, triangles only, ids wanted: the walk writes the ids itself and nothing is left to finish
     if ((flags & RT_TRACE_FAST) && !v.nspheres && !(flags & kTraceRecords)) flags |= kTraceIds;
     RTB_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(uint32_t), s));
-    const uint64_t blocks = std::min<uint64_t>((n + kBlock - 1) / kBlock, persistent_blocks());
+    const uint64_t blocks = walk_blocks(n);
     k_trace_closest<<<(unsigned)blocks, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, counters);
     RTB_CUDA(cudaGetLastError());
     const uint64_t finish = std::min<uint64_t>((n + kBlock - 1) / kBlock, 16ull * device_sm_count());
-    k_trace_finish<<<(unsigned)finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, out, bits, counters);
+    auto kernel = (flags & RT_TRACE_FAST) ? k_trace_finish<false> : k_trace_finish<true>;
+    kernel<<<(unsigned)finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, out, bits, counters);
     RTB_CUDA(cudaGetLastError());
     return RT_OK;
 }
@@ -315,7 +322,7 @@ int launch_trace_any(const SceneView &v, const rt_ray *rays, uint64_t n, uint8_t
 {
     if (n == 0) return RT_OK;
     RTB_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(uint32_t), s));
-    const uint64_t blocks = std::min<uint64_t>((n + kBlock - 1) / kBlock, persistent_blocks());
+    const uint64_t blocks = walk_blocks(n);
     k_trace_any<<<(unsigned)blocks, kBlock, 0, s>>>(v, rays, n, walk_out, flags, counters);
     RTB_CUDA(cudaGetLastError());
     if (bits || v.nspheres) {

@@ -70,7 +70,7 @@ struct Walk {
     float ox, oy, oz;
     float ix, iy, iz;  // 1 / direction
     float Sx, Sy, Sz;  // shear of the watertight test (make_watertight)
-    uint32_t kz;       // its axis
+    uint32_t kz;       // its axis; bits 2..6: the lane that fetched the ray (walk_queue's groups)
     float lim;         // nodes that the ray enters beyond this are skipped
     uint32_t cur;      // node to visit next
     int sp;
@@ -91,6 +91,11 @@ struct alignas(16) TravWarp {
     float4 res[32];     // offset, record and flags, b1, b2 of the pair lane j tested
     float2 bary[32];    // b1, b2 of each lane's best hit
     uint16_t pair[32];  // lane that owns pair j, its triangle's offset in the node's block << 5
+    // per ray in flight, at the lane that fetched it: how many lanes walk it, and what the lanes
+    // that ended have found between them
+    uint32_t lanes[32];
+    float4 found[32];   // offset, triangle record, b1, b2
+    float blocked[32];  // minblock; -1: a lane ran out of stack or steps
 };
 constexpr uint32_t kPairBlocked = 0x80000000u;      // TravWarp::res.y: fails the error-bound test
 constexpr uint32_t kPairTransparent = 0x40000000u;  // transparent to shadow rays
@@ -129,7 +134,7 @@ __device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz,
     W.Sx = w.Sx;
     W.Sy = w.Sy;
     W.Sz = w.Sz;
-    W.kz = (uint32_t)w.kz;
+    W.kz = (uint32_t)w.kz | ((threadIdx.x & 31u) << 2);
     W.lim = lim;
     W.cur = root;
     W.sp = 0;
@@ -142,254 +147,378 @@ __device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz,
     W.tested = 0;
 }
 
+// One step of a warp's walks: each active lane visits its next node, then the warp tests the
+// triangles of the leaves its lanes hit, one (ray, triangle) pair per lane: the pairs are numbered
+// by a prefix sum over the lanes, each lane reads its pair's ray from the owner by shuffles, and the
+// owner takes the results in its own triangle order, so a walk gives what it gives when every
+// lane tests its own triangles one after the other. A step hits about as many triangles as a
+// warp has lanes, so they mostly take one round, where the serial loop took as many as the lane
+// with the most of them, with a few lanes active in each and a triangle fetch of latency per round.
+// shared_t: the ray's best offset among other lanes (INFINITY: none). Returns whether the walk ended.
+template <bool ANY, bool COUNT>
+__device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk &W, bool active, bool unbounded,
+                                          float shared_t)
+{
+    const unsigned lane = threadIdx.x & 31u;
+    // visit a node: its eight quantized child boxes; the triangles of the hit leaves as a
+    // mask over the node's block of records, the hit interior children pushed far to near
+    uint32_t trimask = 0, leafend = 0, tri_base = 0, next = kNoRoot;
+    float next_t = 0.f;
+    bool done = false;
+    if (active) {
+        if (++W.steps > v.nnodes + 1) {
+            W.ok = false;
+            done = true;
+        } else {
+            const uint4 *np = reinterpret_cast<const uint4 *>(v.nodes + W.cur);
+            const uint4 n0 = ld_scene(np), n1 = ld_scene(np + 1), n2 = ld_scene(np + 2), n3 = ld_scene(np + 3),
+                        n4 = ld_scene(np + 4);
+            const float sx = __uint_as_float((n0.w & 0xFFu) << 23);
+            const float sy = __uint_as_float(((n0.w >> 8) & 0xFFu) << 23);
+            const float sz = __uint_as_float(((n0.w >> 16) & 0xFFu) << 23);
+            const uint32_t imask = n0.w >> 24;
+            const uint32_t child_base = n1.x;
+            tri_base = n1.y;
+            const uint32_t meta_lo = n1.z, meta_hi = n1.w;
+            // per-axis affine map t = q * (s * inv) + (p * inv - o * inv)
+            const float ax = sx * W.ix, bx = fmaf(__uint_as_float(n0.x), W.ix, -W.ox * W.ix);
+            const float ay = sy * W.iy, by = fmaf(__uint_as_float(n0.y), W.iy, -W.oy * W.iy);
+            const float az = sz * W.iz, bz = fmaf(__uint_as_float(n0.z), W.iz, -W.oz * W.iz);
+            const float tlimit = fminf(fminf(W.bt, W.lim), shared_t);
+            uint32_t keys[8];
+            uint32_t nint = 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int b = k & 3;
+                const uint32_t meta = byte_of(k < 4 ? meta_lo : meta_hi, b);
+                const float qlx = (float)byte_of(k < 4 ? n2.x : n2.y, b);
+                const float qly = (float)byte_of(k < 4 ? n2.z : n2.w, b);
+                const float qlz = (float)byte_of(k < 4 ? n3.x : n3.y, b);
+                const float qhx = (float)byte_of(k < 4 ? n3.z : n3.w, b);
+                const float qhy = (float)byte_of(k < 4 ? n4.x : n4.y, b);
+                const float qhz = (float)byte_of(k < 4 ? n4.z : n4.w, b);
+                const float t1x = fmaf(qlx, ax, bx), t2x = fmaf(qhx, ax, bx);
+                const float t1y = fmaf(qly, ay, by), t2y = fmaf(qhy, ay, by);
+                const float t1z = fmaf(qlz, az, bz), t2z = fmaf(qhz, az, bz);
+                const float tn =
+                    fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fmaxf(fminf(t1z, t2z), 0.0f));
+                const float tf =
+                    fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fminf(fmaxf(t1z, t2z), tlimit));
+                const bool hit = (meta != 0xFFu) && (tn <= tf);
+                const bool interior = (imask >> k) & 1u;
+                keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
+                nint += (hit && interior) ? 1u : 0u;
+                if (hit && !interior) {
+                    trimask |= ((2u << (meta >> 5)) - 1u) << (meta & 31u);
+                    if (COUNT) leafend |= (1u << (meta >> 5)) << (meta & 31u);
+                }
+            }
+            if (nint) {
+                sort8(keys);
+                if (W.sp + (int)nint - 1 > kStack) {  // drop the entries beyond the best hit
+                    int kept = 0;
+#pragma unroll 1
+                    for (int e = 0; e < W.sp; e++) {
+                        const uint2 x = W.st[e];
+                        if (__uint_as_float(x.y) <= tlimit) W.st[kept++] = x;
+                    }
+                    W.sp = kept;
+                    if (W.sp + (int)nint - 1 > kStack) {
+                        W.ok = false;
+                        done = true;
+                    }
+                }
+                if (!done) {
+#pragma unroll
+                    for (int j = 7; j >= 1; j--)
+                        if (j < (int)nint) {
+                            const uint32_t slot = keys[j] & 7u;
+                            W.st[W.sp] = make_uint2(child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3),
+                                                    keys[j] & ~7u);
+                            W.sp++;
+                        }
+                }
+                const uint32_t slot = keys[0] & 7u;
+                next = child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3);
+                next_t = __uint_as_float(keys[0] & ~7u);
+            }
+        }
+    }
+    // the triangles of the whole warp, 32 pairs a round
+    const uint32_t mytris = (uint32_t)__popc(trimask);
+    if (__any_sync(kAllLanes, trimask != 0)) {
+        uint32_t incl = mytris;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kAllLanes, incl, o);
+            if (lane >= (unsigned)o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(kAllLanes, incl, 31);
+        uint32_t at = incl - mytris, left = trimask;
+        if (COUNT && !ANY) W.tested += mytris;
+        uint32_t before = 0;  // triangles of this lane offered in earlier rounds (COUNT)
+        for (uint32_t r0 = 0; r0 < total; r0 += 32) {
+            const uint32_t first = at;
+#pragma unroll 1
+            while (left && at < r0 + 32) {
+                const uint32_t off = (uint32_t)__ffs(left) - 1u;
+                left &= left - 1u;
+                sm.pair[at - r0] = (uint16_t)(lane | (off << 5));
+                at++;
+            }
+            __syncwarp();
+            const bool on = r0 + lane < total;
+            const uint32_t e = on ? sm.pair[lane] : lane;
+            const int src = (int)(e & 31u);
+            WatertightRay w;
+            w.ox = __shfl_sync(kAllLanes, W.ox, src);
+            w.oy = __shfl_sync(kAllLanes, W.oy, src);
+            w.oz = __shfl_sync(kAllLanes, W.oz, src);
+            w.Sx = __shfl_sync(kAllLanes, W.Sx, src);
+            w.Sy = __shfl_sync(kAllLanes, W.Sy, src);
+            w.Sz = __shfl_sync(kAllLanes, W.Sz, src);
+            const float lim = __shfl_sync(kAllLanes, W.lim, src);
+            const uint32_t axis_base = __shfl_sync(kAllLanes, (tri_base << 2) | (W.kz & 3u), src);
+            w.tmax = unbounded ? INFINITY : lim;
+            w.kz = (int)(axis_base & 3u);
+            w.kx = w.kz == 2 ? 0 : w.kz + 1;
+            w.ky = w.kx == 2 ? 0 : w.kx + 1;
+            bool hit = false;
+            if (on) {
+                const uint32_t rec = (axis_base >> 2) + (e >> 5);
+                const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
+                const float4 a = ld_scene(p), b = ld_scene(p + 1), c = ld_scene(p + 2);
+                TriHit h;
+                hit = watertight_test(w, a, b, c, h);
+                if (hit) {
+                    const float dt = watertight_delta_t(h);
+                    const uint32_t fl = rec | (h.t <= dt ? kPairBlocked : 0u) |
+                                        ((__float_as_uint(c.w) & 1u) ? kPairTransparent : 0u);
+                    sm.res[lane] =
+                        make_float4(h.t, __uint_as_float(fl), fmul(h.e1, h.invDet), fmul(h.e2, h.invDet));
+                }
+            }
+            uint32_t mine = __ballot_sync(kAllLanes, hit);
+            __syncwarp();
+            // the owner takes the results of its own pairs, in order
+            mine = at > first ? (mine >> (first - r0)) & ((1u << (at - first)) - 1u) : 0u;
+            if (ANY && W.brec != kNoRec) mine = 0;
+#pragma unroll 1
+            while (mine) {
+                const uint32_t j = first - r0 + (uint32_t)__ffs(mine) - 1u;
+                mine &= mine - 1u;
+                const float2 tf = *reinterpret_cast<const float2 *>(&sm.res[j]);
+                const uint32_t fl = __float_as_uint(tf.y), rec = fl & kPairRecord;
+                if (W.shadow && (fl & kPairTransparent)) continue;
+                if (tf.x > W.bt) continue;
+                if (tf.x == W.bt && W.brec != kNoRec &&
+                    __float_as_uint(__ldg(&v.tris[rec].v0.w)) < __float_as_uint(__ldg(&v.tris[W.brec].v0.w)))
+                    continue;
+                if (fl & kPairBlocked) {
+                    W.minblock = fminf(W.minblock, tf.x);
+                    continue;
+                }
+                W.bt = tf.x;
+                W.brec = rec;
+                sm.bary[lane] = *(reinterpret_cast<const float2 *>(&sm.res[j]) + 1);
+                if (ANY) {
+                    if (COUNT) {  // the triangles up to the end of this one's leaf
+                        const uint32_t off = sm.pair[j] >> 5;
+                        const uint32_t end = (uint32_t)__ffs(leafend >> off) - 1u + off;
+                        before = (uint32_t)__popc(trimask & ((2u << end) - 1u));
+                    }
+                    break;
+                }
+            }
+        }
+        if (COUNT && ANY) W.tested += W.brec != kNoRec ? before : mytris;
+        __syncwarp();
+    }
+    if (active) {
+        // the nearest hit child, or the top stack entry the best hit has not passed
+        const float tl = fminf(fminf(W.bt, W.lim), shared_t);
+        if (ANY && (W.brec != kNoRec || shared_t < INFINITY)) done = true;
+        if (!done) {
+            if (next != kNoRoot && next_t <= tl) {
+                W.cur = next;
+            } else {
+                done = true;
+#pragma unroll 1
+                while (W.sp > 0) {
+                    W.sp--;
+                    const uint2 e = W.st[W.sp];
+                    if (__uint_as_float(e.y) <= tl) {
+                        W.cur = e.x;
+                        done = false;
+                        break;
+                    }
+                }
+            }
+        }
+    }
+    return active && done;
+}
+
 // Walks the rays [0, n) of a queue: every lane of a persistent warp runs its own ray, and lanes
-// whose rays are done fetch the next ones together. A step visits one node per lane and then
-// tests the triangles of the leaves the whole warp hit, one (ray, triangle) pair per lane:
-// the pairs are numbered by a prefix sum over the lanes, each lane reads its pair's ray from the
-// owner by shuffles, and the owner takes the results in its own triangle order, so a walk gives
-// what it gives when every lane tests its own triangles one after the other. A step hits about
-// as many triangles as a warp has lanes, so they mostly take one round, where the serial loop
-// took as many as the lane with the most of them, with a few lanes active in each and a triangle
-// fetch of latency per round.
+// whose rays are done fetch the next ones together (measured for 1 / 4 / 8 / 16 idle lanes:
+// 2^24 rays of the BVH-stress scene 4.60 / 4.60 / 4.58 / 4.98 ms, its 1080p x 64 spp frame 212 / 209
+// / 209 / 217 ms).
+//
+// Once the queue is empty, idle lanes help: each takes the top stack entry of a lane that has one
+// and walks that subtree for the same ray, so the few longest rays, which pass hundreds of nodes,
+// no longer hold the kernel up one node at a time (2^22 rays: the last SM ran 0.4 of 1.3 ms by
+// itself). The lanes of a ray share its best offset for skipping nodes, and the last of them to
+// end reports what they found together: the nearest hit, ties to the higher rank, which does not
+// depend on who found it. A short queue is dealt out over all warps (quota rays each), so that
+// there are idle lanes to help from the start.
 //
 // init(i, W) prepares ray i (walk_init); finish(i, W, bary) consumes its result. ANY: the walk
 // ends at the first accepted hit in triangle order (in the node that has one). unbounded: the
 // triangle test has no limit (lim only bounds the nodes). COUNT: also counts the triangles a
-// serial walk would test (whole leaves, up to the leaf of the accepted hit under ANY).
+// serial walk would test (whole leaves, up to the leaf of the accepted hit under ANY), and every
+// ray keeps its own lane.
 template <bool ANY, bool COUNT, typename Init, typename Finish>
 __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uint32_t n, uint32_t *work,
                                            bool unbounded, Init init, Finish finish)
 {
     const unsigned lane = threadIdx.x & 31u;
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    const uint32_t quota = COUNT ? 32u : min(max((n + warps - 1u) / warps, 1u), 32u);
+    // with quota * warps >= n the first fetch of each warp takes all there is for it
+    const bool single = !COUNT && (uint64_t)quota * warps >= n;
     uint32_t ray = 0xFFFFFFFFu;
     bool exhausted = false;
     Walk W;
     for (;;) {
         const unsigned idle = __ballot_sync(kAllLanes, ray == 0xFFFFFFFFu);
-        if (!exhausted && __popc(idle) >= RTB_REFILL) {
+        const uint32_t busy = 32u - (uint32_t)__popc(idle);
+        if (!exhausted && busy + min(quota, (uint32_t)RTB_REFILL) <= quota) {
+            const uint32_t want = quota - busy;
             uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
+            if (lane == 0) base = atomicAdd(work, want);
             base = __shfl_sync(kAllLanes, base, 0);
-            if (base + (uint32_t)__popc(idle) >= n) exhausted = true;
-            if (ray == 0xFFFFFFFFu) {
-                const uint32_t mine = base + __popc(idle & ((1u << lane) - 1u));
-                if (mine < n) {
-                    ray = mine;
-                    init(ray, W);
-                    if (W.cur == kNoRoot) {
-                        finish(ray, W, make_float2(0.f, 0.f));
-                        ray = 0xFFFFFFFFu;
-                    }
+            exhausted = single || base + want >= n;
+            const uint32_t rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+            if (ray == 0xFFFFFFFFu && rank < want && base + rank < n) {
+                ray = base + rank;
+                init(ray, W);
+                if (W.cur == kNoRoot) {
+                    finish(ray, W, make_float2(0.f, 0.f));
+                    ray = 0xFFFFFFFFu;
                 }
+            }
+            __syncwarp();
+            if (!COUNT && exhausted) break;
+        }
+        const bool active = ray != 0xFFFFFFFFu;
+        if (!__any_sync(kAllLanes, active)) {
+            if (exhausted) return;
+            continue;
+        }
+        if (walk_step<ANY, COUNT>(v, sm, W, active, unbounded, INFINITY)) {
+            finish(ray, W, W.brec != kNoRec ? sm.bary[lane] : make_float2(0.f, 0.f));
+            ray = 0xFFFFFFFFu;
+        }
+    }
+    if (COUNT) return;
+    // the queue is empty: the warp's last rays, with all its lanes
+    sm.lanes[lane] = 1;
+    sm.found[lane] = make_float4(INFINITY, __uint_as_float(kNoRec), 0.f, 0.f);
+    sm.blocked[lane] = INFINITY;
+    __syncwarp();
+    for (;;) {
+        const unsigned idle = __ballot_sync(kAllLanes, ray == 0xFFFFFFFFu);
+        if (idle == kAllLanes) return;
+        // idle lane k takes the top entry of the k-th lane that has one
+        const bool give = ray != 0xFFFFFFFFu && W.sp > 0;
+        const unsigned givers = __ballot_sync(kAllLanes, give);
+        if (idle && givers) {
+            const uint32_t below = (1u << lane) - 1u;
+            const uint32_t moves = min((uint32_t)__popc(idle), (uint32_t)__popc(givers));
+            const uint32_t k = (uint32_t)__popc((give ? givers : idle) & below);
+            uint2 e = make_uint2(0u, 0u);
+            if (give && k < moves) {
+                e = W.st[--W.sp];
+                sm.pair[k] = (uint16_t)lane;
+            }
+            __syncwarp();
+            const bool take = ray == 0xFFFFFFFFu && k < moves;
+            const int src = take ? (int)sm.pair[k] : (int)lane;
+            const uint32_t ex = __shfl_sync(kAllLanes, e.x, src), ey = __shfl_sync(kAllLanes, e.y, src);
+            const uint32_t r = __shfl_sync(kAllLanes, ray, src), kz = __shfl_sync(kAllLanes, W.kz, src);
+            const float ox = __shfl_sync(kAllLanes, W.ox, src), oy = __shfl_sync(kAllLanes, W.oy, src),
+                        oz = __shfl_sync(kAllLanes, W.oz, src);
+            const float ix = __shfl_sync(kAllLanes, W.ix, src), iy = __shfl_sync(kAllLanes, W.iy, src),
+                        iz = __shfl_sync(kAllLanes, W.iz, src);
+            const float Sx = __shfl_sync(kAllLanes, W.Sx, src), Sy = __shfl_sync(kAllLanes, W.Sy, src),
+                        Sz = __shfl_sync(kAllLanes, W.Sz, src);
+            const float lim = __shfl_sync(kAllLanes, W.lim, src), bt = __shfl_sync(kAllLanes, W.bt, src);
+            const bool shadow = __shfl_sync(kAllLanes, (int)W.shadow, src) != 0;
+            // an entry the giver's best hit has passed is dropped
+            if (take && __uint_as_float(ey) <= fminf(bt, lim)) {
+                ray = r;
+                W.ox = ox, W.oy = oy, W.oz = oz;
+                W.ix = ix, W.iy = iy, W.iz = iz;
+                W.Sx = Sx, W.Sy = Sy, W.Sz = Sz;
+                W.kz = kz;
+                W.lim = lim;
+                W.cur = ex;
+                W.sp = 0;
+                W.steps = 0;
+                W.ok = true;
+                W.shadow = shadow;
+                W.bt = INFINITY;
+                W.brec = kNoRec;
+                W.minblock = INFINITY;
+                atomicAdd(&sm.lanes[kz >> 2], 1u);
             }
             __syncwarp();
         }
         const bool active = ray != 0xFFFFFFFFu;
-        if (!__any_sync(kAllLanes, active)) {
-            if (exhausted) break;
-            continue;
-        }
-        // visit a node: its eight quantized child boxes; the triangles of the hit leaves as a
-        // mask over the node's block of records, the hit interior children pushed far to near
-        uint32_t trimask = 0, leafend = 0, tri_base = 0, next = kNoRoot;
-        float next_t = 0.f;
-        bool done = false;
-        if (active) {
-            if (++W.steps > v.nnodes + 1) {
-                W.ok = false;
-                done = true;
-            } else {
-                const uint4 *np = reinterpret_cast<const uint4 *>(v.nodes + W.cur);
-                const uint4 n0 = ld_scene(np), n1 = ld_scene(np + 1), n2 = ld_scene(np + 2), n3 = ld_scene(np + 3),
-                            n4 = ld_scene(np + 4);
-                const float sx = __uint_as_float((n0.w & 0xFFu) << 23);
-                const float sy = __uint_as_float(((n0.w >> 8) & 0xFFu) << 23);
-                const float sz = __uint_as_float(((n0.w >> 16) & 0xFFu) << 23);
-                const uint32_t imask = n0.w >> 24;
-                const uint32_t child_base = n1.x;
-                tri_base = n1.y;
-                const uint32_t meta_lo = n1.z, meta_hi = n1.w;
-                // per-axis affine map t = q * (s * inv) + (p * inv - o * inv)
-                const float ax = sx * W.ix, bx = fmaf(__uint_as_float(n0.x), W.ix, -W.ox * W.ix);
-                const float ay = sy * W.iy, by = fmaf(__uint_as_float(n0.y), W.iy, -W.oy * W.iy);
-                const float az = sz * W.iz, bz = fmaf(__uint_as_float(n0.z), W.iz, -W.oz * W.iz);
-                const float tlimit = fminf(W.bt, W.lim);
-                uint32_t keys[8];
-                uint32_t nint = 0;
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const int b = k & 3;
-                    const uint32_t meta = byte_of(k < 4 ? meta_lo : meta_hi, b);
-                    const float qlx = (float)byte_of(k < 4 ? n2.x : n2.y, b);
-                    const float qly = (float)byte_of(k < 4 ? n2.z : n2.w, b);
-                    const float qlz = (float)byte_of(k < 4 ? n3.x : n3.y, b);
-                    const float qhx = (float)byte_of(k < 4 ? n3.z : n3.w, b);
-                    const float qhy = (float)byte_of(k < 4 ? n4.x : n4.y, b);
-                    const float qhz = (float)byte_of(k < 4 ? n4.z : n4.w, b);
-                    const float t1x = fmaf(qlx, ax, bx), t2x = fmaf(qhx, ax, bx);
-                    const float t1y = fmaf(qly, ay, by), t2y = fmaf(qhy, ay, by);
-                    const float t1z = fmaf(qlz, az, bz), t2z = fmaf(qhz, az, bz);
-                    const float tn =
-                        fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fmaxf(fminf(t1z, t2z), 0.0f));
-                    const float tf =
-                        fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fminf(fmaxf(t1z, t2z), tlimit));
-                    const bool hit = (meta != 0xFFu) && (tn <= tf);
-                    const bool interior = (imask >> k) & 1u;
-                    keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
-                    nint += (hit && interior) ? 1u : 0u;
-                    if (hit && !interior) {
-                        trimask |= ((2u << (meta >> 5)) - 1u) << (meta & 31u);
-                        if (COUNT) leafend |= (1u << (meta >> 5)) << (meta & 31u);
-                    }
-                }
-                if (nint) {
-                    sort8(keys);
-                    if (W.sp + (int)nint - 1 > kStack) {  // drop the entries beyond the best hit
-                        int kept = 0;
-#pragma unroll 1
-                        for (int e = 0; e < W.sp; e++) {
-                            const uint2 x = W.st[e];
-                            if (__uint_as_float(x.y) <= tlimit) W.st[kept++] = x;
-                        }
-                        W.sp = kept;
-                        if (W.sp + (int)nint - 1 > kStack) {
-                            W.ok = false;
-                            done = true;
-                        }
-                    }
-                    if (!done) {
-#pragma unroll
-                        for (int j = 7; j >= 1; j--)
-                            if (j < (int)nint) {
-                                const uint32_t slot = keys[j] & 7u;
-                                W.st[W.sp] = make_uint2(child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3),
-                                                        keys[j] & ~7u);
-                                W.sp++;
-                            }
-                    }
-                    const uint32_t slot = keys[0] & 7u;
-                    next = child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3);
-                    next_t = __uint_as_float(keys[0] & ~7u);
-                }
-            }
-        }
-        // the triangles of the whole warp, 32 pairs a round
-        const uint32_t mytris = (uint32_t)__popc(trimask);
-        if (__any_sync(kAllLanes, trimask != 0)) {
-            uint32_t incl = mytris;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(kAllLanes, incl, o);
-                if (lane >= (unsigned)o) incl += y;
-            }
-            const uint32_t total = __shfl_sync(kAllLanes, incl, 31);
-            uint32_t at = incl - mytris, left = trimask;
-            if (COUNT && !ANY) W.tested += mytris;
-            uint32_t before = 0;  // triangles of this lane offered in earlier rounds (COUNT)
-            for (uint32_t r0 = 0; r0 < total; r0 += 32) {
-                const uint32_t first = at;
-#pragma unroll 1
-                while (left && at < r0 + 32) {
-                    const uint32_t off = (uint32_t)__ffs(left) - 1u;
-                    left &= left - 1u;
-                    sm.pair[at - r0] = (uint16_t)(lane | (off << 5));
-                    at++;
-                }
-                __syncwarp();
-                const bool on = r0 + lane < total;
-                const uint32_t e = on ? sm.pair[lane] : lane;
-                const int src = (int)(e & 31u);
-                WatertightRay w;
-                w.ox = __shfl_sync(kAllLanes, W.ox, src);
-                w.oy = __shfl_sync(kAllLanes, W.oy, src);
-                w.oz = __shfl_sync(kAllLanes, W.oz, src);
-                w.Sx = __shfl_sync(kAllLanes, W.Sx, src);
-                w.Sy = __shfl_sync(kAllLanes, W.Sy, src);
-                w.Sz = __shfl_sync(kAllLanes, W.Sz, src);
-                const float lim = __shfl_sync(kAllLanes, W.lim, src);
-                const uint32_t axis_base = __shfl_sync(kAllLanes, (tri_base << 2) | (W.kz & 3u), src);
-                w.tmax = unbounded ? INFINITY : lim;
-                w.kz = (int)(axis_base & 3u);
-                w.kx = w.kz == 2 ? 0 : w.kz + 1;
-                w.ky = w.kx == 2 ? 0 : w.kx + 1;
-                bool hit = false;
-                if (on) {
-                    const uint32_t rec = (axis_base >> 2) + (e >> 5);
-                    const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
-                    const float4 a = ld_scene(p), b = ld_scene(p + 1), c = ld_scene(p + 2);
-                    TriHit h;
-                    hit = watertight_test(w, a, b, c, h);
-                    if (hit) {
-                        const float dt = watertight_delta_t(h);
-                        const uint32_t fl = rec | (h.t <= dt ? kPairBlocked : 0u) |
-                                            ((__float_as_uint(c.w) & 1u) ? kPairTransparent : 0u);
-                        sm.res[lane] =
-                            make_float4(h.t, __uint_as_float(fl), fmul(h.e1, h.invDet), fmul(h.e2, h.invDet));
-                    }
-                }
-                uint32_t mine = __ballot_sync(kAllLanes, hit);
-                __syncwarp();
-                // the owner takes the results of its own pairs, in order
-                mine = at > first ? (mine >> (first - r0)) & ((1u << (at - first)) - 1u) : 0u;
-                if (ANY && W.brec != kNoRec) mine = 0;
-#pragma unroll 1
-                while (mine) {
-                    const uint32_t j = first - r0 + (uint32_t)__ffs(mine) - 1u;
-                    mine &= mine - 1u;
-                    const float2 tf = *reinterpret_cast<const float2 *>(&sm.res[j]);
-                    const uint32_t fl = __float_as_uint(tf.y), rec = fl & kPairRecord;
-                    if (W.shadow && (fl & kPairTransparent)) continue;
-                    if (tf.x > W.bt) continue;
-                    if (tf.x == W.bt && W.brec != kNoRec &&
-                        __float_as_uint(__ldg(&v.tris[rec].v0.w)) < __float_as_uint(__ldg(&v.tris[W.brec].v0.w)))
-                        continue;
-                    if (fl & kPairBlocked) {
-                        W.minblock = fminf(W.minblock, tf.x);
-                        continue;
-                    }
-                    W.bt = tf.x;
-                    W.brec = rec;
-                    sm.bary[lane] = *(reinterpret_cast<const float2 *>(&sm.res[j]) + 1);
-                    if (ANY) {
-                        if (COUNT) {  // the triangles up to the end of this one's leaf
-                            const uint32_t off = sm.pair[j] >> 5;
-                            const uint32_t end = (uint32_t)__ffs(leafend >> off) - 1u + off;
-                            before = (uint32_t)__popc(trimask & ((2u << end) - 1u));
-                        }
-                        break;
-                    }
-                }
-            }
-            if (COUNT && ANY) W.tested += W.brec != kNoRec ? before : mytris;
-            __syncwarp();
-        }
-        if (active) {
-            // the nearest hit child, or the top stack entry the best hit has not passed
-            const float tl = fminf(W.bt, W.lim);
-            if (ANY && W.brec != kNoRec) done = true;
-            if (!done) {
-                if (next != kNoRoot && next_t <= tl) {
-                    W.cur = next;
+        const float shared_t = active ? sm.found[W.kz >> 2].x : INFINITY;
+        const bool done = walk_step<ANY, COUNT>(v, sm, W, active, unbounded, shared_t);
+        // one ended lane after the other adds what it found to its ray's; the last reports it
+        unsigned ended = __ballot_sync(kAllLanes, done);
+        while (ended) {
+            const unsigned who = __ffs(ended) - 1;
+            ended &= ended - 1u;
+            if (lane == who) {
+                const uint32_t home = W.kz >> 2;
+                const float4 f = sm.found[home];
+                const uint32_t frec = __float_as_uint(f.y);
+                const bool take = W.brec != kNoRec && !(W.bt > f.x) &&
+                                  !(W.bt == f.x && frec != kNoRec &&
+                                    __float_as_uint(__ldg(&v.tris[W.brec].v0.w)) <
+                                        __float_as_uint(__ldg(&v.tris[frec].v0.w)));
+                const float4 g = take ? make_float4(W.bt, __uint_as_float(W.brec), sm.bary[lane].x, sm.bary[lane].y)
+                                      : f;
+                const float mb = W.ok ? fminf(sm.blocked[home], W.minblock) : -1.f;
+                if (--sm.lanes[home] == 0) {
+                    W.ok = mb >= 0.f;
+                    W.bt = g.x;
+                    W.brec = __float_as_uint(g.y);
+                    W.minblock = mb;
+                    finish(ray, W, make_float2(g.z, g.w));
                 } else {
-                    done = true;
-#pragma unroll 1
-                    while (W.sp > 0) {
-                        W.sp--;
-                        const uint2 e = W.st[W.sp];
-                        if (__uint_as_float(e.y) <= tl) {
-                            W.cur = e.x;
-                            done = false;
-                            break;
-                        }
-                    }
+                    sm.found[home] = g;
+                    sm.blocked[home] = mb;
                 }
-            }
-            if (done) {
-                finish(ray, W, W.brec != kNoRec ? sm.bary[lane] : make_float2(0.f, 0.f));
                 ray = 0xFFFFFFFFu;
             }
+            __syncwarp();
         }
     }
+}
+
+// The exact test of one analytic shape, out of line: a ray comes here for the few shapes it may hit.
+__device__ __noinline__ static bool shape_test(const SphereRecord *sr, float ox, float oy, float oz, float dx, float dy,
+                                               float dz, float tmax, float3 *hit)
+{
+    float t, u = 0.f, v = 0.f;
+    const bool ok = (sr->flags & kShapePlane) ? plane_test(sr->w2o, ox, oy, oz, dx, dy, dz, tmax, t, u, v)
+                                              : sphere_test(sr->w2o, sr->radius, ox, oy, oz, dx, dy, dz, tmax, t);
+    if (ok) *hit = make_float3(t, u, v);
+    return ok;
 }
 
 // Scene::intersects' loop over the analytic shapes (Scene.cu:141-146) of scene `sub`.
@@ -400,16 +529,18 @@ __device__ __forceinline__ void intersect_spheres(const SceneView &v, uint32_t s
     uint32_t s0, ns;
     scene_spheres(v, sub, s0, ns);
     for (uint32_t s = s0; s < s0 + ns; s++) {
-        const SphereRecord &sr = v.spheres[s];
-        if (shadow && (sr.flags & 1u)) continue;
-        float ts, pu = 0.f, pv = 0.f;
-        const bool hit = (sr.flags & kShapePlane) ? plane_test(sr.w2o, ox, oy, oz, dx, dy, dz, tmax, ts, pu, pv)
-                                                  : sphere_test(sr.w2o, sr.radius, ox, oy, oz, dx, dy, dz, tmax, ts);
-        if (hit && ts < t) {
-            t = ts;
+        const SphereRecord *sr = v.spheres + s;
+        const float4 *m = reinterpret_cast<const float4 *>(sr->w2o);
+        const float4 tail = __ldg(reinterpret_cast<const float4 *>(&sr->radius));  // radius, material, shape id, flags
+        const uint32_t flags = __float_as_uint(tail.w);
+        if (shadow && (flags & 1u)) continue;
+        if ((flags & kShapeAffine) && sphere_missed(m, tail.x, ox, oy, oz, dx, dy, dz)) continue;
+        float3 hit;  // offset; a plane hit reports its object-space (x, y); 0 for spheres
+        if (shape_test(sr, ox, oy, oz, dx, dy, dz, tmax, &hit) && hit.x < t) {
+            t = hit.x;
             prim = RT_PRIM_SHAPE | (int32_t)s;
-            b1 = pu;  // a plane hit reports its object-space (x, y); 0 for spheres
-            b2 = pv;
+            b1 = hit.y;
+            b2 = hit.z;
         }
     }
 }
