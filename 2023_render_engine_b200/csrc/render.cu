@@ -58,13 +58,26 @@ struct Buffers {
     float4 *gather;    // photon-map gather requests, 4 float4 each: p+shape, n+material, wo+target, beta
     const uint32_t *perm;  // shading order of the wave's queue slots (material sort), or null
     uint32_t cap, scap, gcap;
-    // counters (uint32): [0],[1] queue sizes of buffers 0/1, [2] shadow count, [3] retire count,
-    // [4] status, [5] shadow-kernel work counter, [6] gather requests, [7] gather-kernel work
-    // counter; u64 at [8]: next sample,
-    // [10] extension rays, [12] shadow rays, [14] gathers; [16] guide wait timed out, [18] waves
-    // of the device-side loop, [19] wave cap reached
-    uint32_t *cnt;
+    uint32_t *cnt;  // counters, at the word offsets below
+    uint32_t *trace_cnt;  // the closest-hit trace's counters (4 words)
 };
+
+// Word offsets of the counters. Those that every block of a kernel adds to lie 128 bytes apart:
+// side by side they share an L2 slice, which takes one atomic at a time.
+constexpr int kCntQueue = 0;          // + 32 b: paths in buffer b
+constexpr int kCntShadow = 64;        // shadow rays of the wave
+constexpr int kCntRetire = 96;        // retired paths of the wave
+constexpr int kCntShadowWork = 128;   // k_shadow's work counter
+constexpr int kCntGather = 160;       // gather requests of the wave
+constexpr int kCntGatherWork = 192;   // k_gather's work counter
+constexpr int kCntSample = 224;       // u64: next camera sample
+constexpr int kCntRays = 256;         // u64: extension rays
+constexpr int kCntShadowRays = 258;   // u64
+constexpr int kCntGathers = 260;      // u64
+constexpr int kCntGuideTimeout = 264; // the guide's tensor-core wait timed out
+constexpr int kCntWaves = 266;        // waves of the device-side loop
+constexpr int kCntCapped = 267;       // its wave cap was reached
+constexpr int kCntWords = 288;
 
 struct GuideView {
     const GuideParams *params;  // per queue slot; null while the guide is untrained (BSDF sampling)
@@ -152,10 +165,10 @@ __device__ __forceinline__ void regenerate(const RenderView &rv, const Buffers &
 {
     cg::coalesced_group grp = cg::coalesced_threads();
     unsigned long long base = 0;
-    if (grp.thread_rank() == 0) base = atomicAdd(cnt64(bf.cnt, 8), (unsigned long long)grp.size());
+    if (grp.thread_rank() == 0) base = atomicAdd(cnt64(bf.cnt, kCntSample), (unsigned long long)grp.size());
     const unsigned long long g = grp.shfl(base, 0) + grp.thread_rank();
     if (g >= rv.total) return;
-    uint32_t q = append(bf.cnt + b);
+    uint32_t q = append(bf.cnt + kCntQueue + 32 * b);
     start_path(rv, bf, b, q, g);
 }
 
@@ -177,7 +190,7 @@ constexpr uint32_t kShadowSceneShift = 24;
 __device__ __forceinline__ void push_shadow(const Buffers &bf, V3 o, V3 d, float tmax, V3 contrib, uint32_t target,
                                             bool skip_transparent, uint32_t sub, uint32_t rec = kRecNone)
 {
-    uint32_t i = append(bf.cnt + 2);
+    uint32_t i = append(bf.cnt + kCntShadow);
     if (i >= bf.scap) return;
     reinterpret_cast<float4 *>(bf.srays)[2 * i] = make_float4(o.x, o.y, o.z, tmax);
     reinterpret_cast<float4 *>(bf.srays)[2 * i + 1] = make_float4(
@@ -196,7 +209,7 @@ constexpr int kGatherWords = 5;
 __device__ __forceinline__ void push_gather(const Buffers &bf, const Surface &sf, V3 wo_w, V3 weight, uint32_t target,
                                             uint32_t kind, uint32_t rec, V3 kd)
 {
-    const uint32_t gi = append(bf.cnt + 6);
+    const uint32_t gi = append(bf.cnt + kCntGather);
     if (gi >= bf.gcap) return;
     float4 *g = bf.gather + (uint64_t)kGatherWords * gi;
     g[0] = make_float4(sf.p.x, sf.p.y, sf.p.z, __int_as_float(sf.shape));
@@ -239,7 +252,7 @@ __global__ void __launch_bounds__(kSortBlock) k_material_sort(RenderView rv, Buf
     __shared__ uint32_t count[kSortKeys], start[kSortKeys];
     __shared__ uint8_t key[1u << kSortMaxLog2];
     __shared__ uint32_t wcount[kSortBlock / 32][kSortKeys];
-    const uint32_t n = min(bf.cnt[cur], bf.cap);
+    const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
     // chunks in a grid-stride loop over the resident blocks (c0 is the same for the whole block)
     for (uint32_t c0 = blockIdx.x << log2; c0 < n; c0 += gridDim.x << log2) {
         const uint32_t len = min(1u << log2, n - c0);
@@ -293,17 +306,17 @@ __global__ void __launch_bounds__(kSortBlock) k_material_sort(RenderView rv, Buf
 // End of one 4-wave group of the device-side wave loop: counts the waves and sets the loop's
 // condition to 0 once every queue has drained and every camera sample has started (what the
 // host loop checks after each group), when the guide's tensor-core wait timed out, or at the
-// wave cap (cnt[19] = 1 then). cnt[18] counts the waves.
+// wave cap (kCntCapped = 1 then). kCntWaves counts the waves.
 __global__ void k_wave_check(uint32_t *cnt, uint64_t total, uint32_t max_waves, cudaGraphConditionalHandle loop)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const uint32_t waves = cnt[18] + 4;
-    cnt[18] = waves;
-    const unsigned long long next = *reinterpret_cast<const unsigned long long *>(cnt + 8);
-    const bool done = cnt[0] == 0 && next >= total;
+    const uint32_t waves = cnt[kCntWaves] + 4;
+    cnt[kCntWaves] = waves;
+    const unsigned long long next = *reinterpret_cast<const unsigned long long *>(cnt + kCntSample);
+    const bool done = cnt[kCntQueue] == 0 && next >= total;
     const bool capped = !done && waves >= max_waves;
-    if (capped) cnt[19] = 1;
-    cudaGraphSetConditional(loop, (done || capped || cnt[16] != 0) ? 0u : 1u);
+    if (capped) cnt[kCntCapped] = 1;
+    cudaGraphSetConditional(loop, (done || capped || cnt[kCntGuideTimeout] != 0) ? 0u : 1u);
 }
 
 // Resident blocks per SM k_shade is compiled for: more resident warps hide its scattered
@@ -320,8 +333,8 @@ __global__ void k_wave_check(uint32_t *cnt, uint64_t total, uint32_t max_waves, 
 __global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView rv, Buffers bf, int cur, GuideView gv)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = min(bf.cnt[cur], bf.cap);
-    if (i == 0) atomicAdd(cnt64(bf.cnt, 10), (unsigned long long)n);  // extension rays of this wave
+    const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
+    if (i == 0) atomicAdd(cnt64(bf.cnt, kCntRays), (unsigned long long)n);  // extension rays of this wave
     if (i >= n) return;
     // the queue slot this thread shades. Forwarding the slot's hit, triangle record position and
     // material through the sort (32 B per path, read here in one coalesced load, so that the
@@ -458,7 +471,7 @@ __global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView r
             // RENDER_MODE PHOTON_MAPPING: the density estimate at this hit ends the path
             // (Scene::getPhotonContributions, Scene.cu:822-840; finishStep, pathTracing.cu:85-89)
             finished = true;
-            const uint32_t rt = kRetireTarget | append(bf.cnt + 3);
+            const uint32_t rt = kRetireTarget | append(bf.cnt + kCntRetire);
             push_gather(bf, sf, wo_w, beta_in, rt, kGatherDensity, rec_in, bs.color);
             if (subsurface && bs.type == RT_MAT_SUBSURFACE && (flags & kCameraRay))
                 push_gather(bf, sf, wo_w, beta_in, rt, kGatherSubsurface, rec_in, bs.color);
@@ -479,7 +492,7 @@ __global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView r
         if (!finished && depth + 1 >= vw.max_depth) finished = true;  // loop bound (pathTracing.cu:296)
         // reserve the path's slot for the shadow contributions
         if (!finished) {
-            uint32_t qn = append(bf.cnt + nxt);
+            uint32_t qn = append(bf.cnt + kCntQueue + 32 * nxt);
             target = qn;
             cont = true;
             next_o = spawn_origin(sf.p, sf.n, sf.perr, wi_w);
@@ -488,7 +501,7 @@ __global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView r
             next_flags = (depth + 1) | (delta ? kLastSpecular : 0u) |
                          (((flags & kCameraRay) && specular) ? kCameraRay : 0u) | (rec << kRecShift);
         } else {
-            target = kRetireTarget | append(bf.cnt + 3);
+            target = kRetireTarget | append(bf.cnt + kCntRetire);
         }
         // next-event estimation with beta before this bounce (pathTracing.cu:173-205). The
         // direct-light term of a vertex (Scene::sampleDirectLight, Scene.cu:914-969) also holds
@@ -562,7 +575,7 @@ __global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView r
             }
         }
     } else {
-        target = kRetireTarget | append(bf.cnt + 3);
+        target = kRetireTarget | append(bf.cnt + kCntRetire);
     }
     if (cont) {
         const uint32_t qn = target;
@@ -579,16 +592,16 @@ __global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView r
     }
 }
 
-// Any-hit test of the wave's shadow rays (persistent warps, counter cnt[5]): an occluded ray's
+// Any-hit test of the wave's shadow rays (persistent warps, counter kCntShadowWork): an occluded ray's
 // contribution loses its target.
 constexpr uint32_t kNoTarget = 0xFFFFFFFFu;
 __global__ void __launch_bounds__(kB, RTB_TRAV_MIN_BLOCKS) k_shadow(RenderView rv, Buffers bf)
 {
     __shared__ TravWarp scratch[kB / 32];
-    const uint32_t n = min(bf.cnt[2], bf.scap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, 12), (unsigned long long)n);  // stats
+    const uint32_t n = min(bf.cnt[kCntShadow], bf.scap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, kCntShadowRays), (unsigned long long)n);  // stats
     walk_queue<true, false>(
-        rv.sv, scratch[threadIdx.x >> 5], n, bf.cnt + 5, false,
+        rv.sv, scratch[threadIdx.x >> 5], n, bf.cnt + kCntShadowWork, false,
         [&](uint32_t i, Walk &W) {
             const float4 r0 = reinterpret_cast<const float4 *>(bf.srays)[2 * i];
             const float4 r1 = reinterpret_cast<const float4 *>(bf.srays)[2 * i + 1];
@@ -605,9 +618,9 @@ __global__ void __launch_bounds__(kB, RTB_TRAV_MIN_BLOCKS) k_shadow(RenderView r
 // add their contribution to the path they belong to (and, while the guide trains, to its record).
 // One thread per ray, so that the shape tests run with whole warps; at the end of each walk
 // in k_shadow they ran with the few lanes whose rays had just ended.
-__global__ void __launch_bounds__(kB) k_shadow_add(RenderView rv, Buffers bf, int nxt, GuideView gv)
+__global__ void __launch_bounds__(kB, 12) k_shadow_add(RenderView rv, Buffers bf, int nxt, GuideView gv)
 {
-    const uint32_t n = min(bf.cnt[2], bf.scap);
+    const uint32_t n = min(bf.cnt[kCntShadow], bf.scap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 c = bf.scontrib[i];
         const uint32_t target = __float_as_uint(c.w);
@@ -644,7 +657,7 @@ __global__ void __launch_bounds__(kB) k_shadow_add(RenderView rv, Buffers bf, in
 // zero on subsurface materials, Scene.cu:611-612) or the subsurface dipole estimate
 // (Scene::combinePhotonsSubsurface), times the request's weight, added to the path's radiance
 // and, while the guide trains, to the guide record of the vertex before it (as k_shadow does).
-// One warp per request; warps take requests from counter cnt[7] until the wave's are done.
+// One warp per request; warps take requests from counter kCntGatherWork until the wave's are done.
 constexpr int kGatherBlock = 128;
 // Resident blocks per SM k_gather is compiled for (64 registers). Config-4 render at 3840x2160,
 // 4 spp: 538 / 513 / 464 / 467 ms for no bound (118 registers) / 5 / 6 / 8.
@@ -657,12 +670,12 @@ __global__ void __launch_bounds__(kGatherBlock, RTB_GATHER_MIN_BLOCKS) k_gather(
     __shared__ PhotonWarpScratch scratch[kGatherBlock / 32];
     PhotonWarpScratch &sm = scratch[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = min(bf.cnt[6], bf.gcap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, 14), (unsigned long long)n);  // stats
+    const uint32_t n = min(bf.cnt[kCntGather], bf.gcap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, kCntGathers), (unsigned long long)n);  // stats
     const bool compat = (rv.flags & RT_RENDER_COMPAT) != 0;
     for (;;) {
         uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(bf.cnt + 7, 1u);
+        if (lane == 0) i = atomicAdd(bf.cnt + kCntGatherWork, 1u);
         i = __shfl_sync(kFullMask, i, 0);
         if (i >= n) return;  // warp-uniform
         const float4 *g = bf.gather + (uint64_t)kGatherWords * i;
@@ -748,7 +761,7 @@ __device__ __forceinline__ void retire_path(const Buffers &bf, float *sum, uint3
 // the resident blocks: a grid of the capacity would spend most of its blocks exiting.
 __global__ void __launch_bounds__(kB) k_retire(Buffers bf, float *sum, uint32_t *count, double *sum64, GuideView gv)
 {
-    const uint32_t n = min(bf.cnt[3], bf.cap);
+    const uint32_t n = min(bf.cnt[kCntRetire], bf.cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         retire_path(bf, sum, count, sum64, gv, i);
 }
@@ -758,8 +771,8 @@ __global__ void __launch_bounds__(kB) k_retire(Buffers bf, float *sum, uint32_t 
 __global__ void __launch_bounds__(kInferWarps * 32, 1) k_guide_infer(RenderView rv, Buffers bf, int cur, const uint4 *img,
                                                                    GuideBox box, GuideParams *params, uint32_t max_depth)
 {
-    // cnt[16]: set when a tensor-core completion wait ran out (checked after every wave group)
-    const uint32_t n = min(bf.cnt[cur], bf.cap);
+    // kCntGuideTimeout: set when a tensor-core completion wait ran out (checked after every wave group)
+    const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
     const bool compat = (rv.flags & RT_RENDER_COMPAT) != 0;
     auto src = [&](uint32_t q, float *out) -> bool {
         const float4 hv = reinterpret_cast<const float4 *>(bf.hits)[q];
@@ -791,7 +804,7 @@ __global__ void __launch_bounds__(kInferWarps * 32, 1) k_guide_infer(RenderView 
         guide_decode(o, P);
         params[q] = P;
     };
-    guide_infer_rows(img, box, n, src, sink, bf.cnt + 16);
+    guide_infer_rows(img, box, n, src, sink, bf.cnt + kCntGuideTimeout);
 }
 
 __global__ void k_texture_lookup(RenderView rv, uint32_t id, const float *uv, uint64_t n, float *rgb)
@@ -1212,9 +1225,9 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
             gv.rec_cap = guide->rec_cap;
         }
     }
-    RTB_CHECK(rs.cnt.reserve(256));
+    RTB_CHECK(rs.cnt.reserve(4 * kCntWords));
     RTB_CHECK(s->scratch.counters.reserve(64));
-    if (!rs.host_cnt) RTB_CUDA(cudaMallocHost(&rs.host_cnt, 256));
+    if (!rs.host_cnt) RTB_CUDA(cudaMallocHost(&rs.host_cnt, 4 * kCntWords));
 
     Buffers bf;
     for (int b = 0; b < 2; b++) {
@@ -1246,6 +1259,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     if (sort_log2) RTB_CHECK(rs.perm.reserve(4ull * cap));
     bf.perm = sort_log2 ? rs.perm.as<uint32_t>() : nullptr;
     bf.cnt = rs.cnt.as<uint32_t>();
+    bf.trace_cnt = s->scratch.counters.as<uint32_t>();
 
     RenderView rv{};
     RTB_CHECK(make_render_view(s, rv));
@@ -1260,7 +1274,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     RTB_CUDA(cudaEventCreate(&e0));
     RTB_CUDA(cudaEventCreate(&e1));
     RTB_CUDA(cudaEventRecord(e0, st));
-    RTB_CUDA(cudaMemsetAsync(bf.cnt, 0, 256, st));
+    RTB_CUDA(cudaMemsetAsync(bf.cnt, 0, 4 * kCntWords, st));
     const unsigned blocks = cap / kB;
     const unsigned retire_blocks = std::min(blocks, resident_grid(SLOT_RETIRE_RESIDENT, k_retire, kB));
     const unsigned shadow_blocks =
@@ -1313,7 +1327,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         int cur = 0;
         for (int k = 0; k < 4; k++) {
             RTB_CHECK(mark(k, 0));
-            RTB_CHECK(launch_trace_closest_dev(rv.sv, bf.rays[cur], bf.cnt + cur, cap, bf.hits, trace_flags,
+            RTB_CHECK(launch_trace_closest_dev(rv.sv, bf.rays[cur], bf.cnt + kCntQueue + 32 * cur, cap, bf.hits, trace_flags,
                                                s->scratch.counters.as<uint32_t>(), st));
             RTB_CHECK(mark(k, 1));
             if (gv.params) {
@@ -1322,8 +1336,8 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
                 RTB_CUDA(cudaGetLastError());
             }
             RTB_CHECK(mark(k, 2));
-            RTB_CUDA(cudaMemsetAsync(bf.cnt + ((cur ^ 1)), 0, 4, st));
-            RTB_CUDA(cudaMemsetAsync(bf.cnt + 2, 0, 24, st));
+            RTB_CUDA(cudaMemsetAsync(bf.cnt + kCntQueue + 32 * (cur ^ 1), 0, 4, st));
+            RTB_CUDA(cudaMemsetAsync(bf.cnt + kCntShadow, 0, 4 * (kCntSample - kCntShadow), st));
             if (sort_log2) {
                 k_material_sort<<<sort_blocks, kSortBlock, 0, st>>>(rv, bf, cur, rs.perm.as<uint32_t>(), sort_log2);
                 RTB_CUDA(cudaGetLastError());
@@ -1403,14 +1417,14 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     }
     if (device_loop) {
         cudaError_t ce = cudaGraphLaunch(graph, st);
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(rs.host_cnt, bf.cnt, 128, cudaMemcpyDeviceToHost, st);
+        if (ce == cudaSuccess) ce = cudaMemcpyAsync(rs.host_cnt, bf.cnt, 4 * kCntWords, cudaMemcpyDeviceToHost, st);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
         release_graph();
         if (ce != cudaSuccess) return cuda_status(ce, "device wave loop");
         const uint32_t *hc = static_cast<const uint32_t *>(rs.host_cnt);
-        waves = hc[18];
-        if (hc[16]) return fail(RT_ERR_TIMEOUT, name + ": guide tensor-core completion wait timed out");
-        if (hc[19]) return fail(RT_ERR_TIMEOUT, name + ": wave cap exceeded");
+        waves = hc[kCntWaves];
+        if (hc[kCntGuideTimeout]) return fail(RT_ERR_TIMEOUT, name + ": guide tensor-core completion wait timed out");
+        if (hc[kCntCapped]) return fail(RT_ERR_TIMEOUT, name + ": wave cap exceeded");
     }
     for (uint64_t group = 0; !device_loop; group++) {
         int rc = RT_OK;
@@ -1441,7 +1455,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
             if (rc != RT_OK) return rc;
         }
         waves += 4;
-        cudaError_t ce = cudaMemcpyAsync(rs.host_cnt, bf.cnt, 128, cudaMemcpyDeviceToHost, st);
+        cudaError_t ce = cudaMemcpyAsync(rs.host_cnt, bf.cnt, 4 * kCntWords, cudaMemcpyDeviceToHost, st);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
         if (ce != cudaSuccess) {
             release_graph();
@@ -1458,12 +1472,12 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         }
         const uint32_t *hc = static_cast<const uint32_t *>(rs.host_cnt);
         uint64_t next_sample;
-        std::memcpy(&next_sample, hc + 8, 8);
-        if (hc[16]) {
+        std::memcpy(&next_sample, hc + kCntSample, 8);
+        if (hc[kCntGuideTimeout]) {
             release_graph();
             return fail(RT_ERR_TIMEOUT, name + ": guide tensor-core completion wait timed out");
         }
-        if (hc[0] == 0 && next_sample >= total) break;
+        if (hc[kCntQueue] == 0 && next_sample >= total) break;
         if (waves > max_waves) {
             release_graph();
             return fail(RT_ERR_TIMEOUT, name + ": wave cap exceeded");
@@ -1479,13 +1493,13 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     if (stats) {
         const uint32_t *hc = static_cast<const uint32_t *>(rs.host_cnt);
         uint64_t v;
-        std::memcpy(&v, hc + 10, 8);
+        std::memcpy(&v, hc + kCntRays, 8);
         stats->extension_rays = v;
-        std::memcpy(&v, hc + 12, 8);
+        std::memcpy(&v, hc + kCntShadowRays, 8);
         stats->shadow_rays = v;
-        std::memcpy(&v, hc + 8, 8);
+        std::memcpy(&v, hc + kCntSample, 8);
         stats->camera_rays = std::min<uint64_t>(v, total);
-        std::memcpy(&v, hc + 14, 8);
+        std::memcpy(&v, hc + kCntGathers, 8);
         stats->gathers = v;
         stats->waves = waves;
         stats->ms = ms;
