@@ -58,6 +58,7 @@ struct Buffers {
     float4 *gather;    // photon-map gather requests, 4 float4 each: p+shape, n+material, wo+target, beta
     const uint32_t *perm;  // shading order of the wave's queue slots (material sort), or null
     uint32_t cap, scap, gcap;
+    bool regen;  // there are more camera samples than queue slots: finished paths make room for them
     uint32_t *cnt;  // counters, at the word offsets below
     uint32_t *trace_cnt;  // the closest-hit trace's counters (4 words)
 };
@@ -121,8 +122,14 @@ __device__ void start_path(const RenderView &rv, const Buffers &bf, int b, uint3
     const rt_camera &cam = vw.camera;
     g -= rv.view_sample0[vi];
     const uint32_t W = cam.width, H = cam.height;
-    const uint32_t pix = (uint32_t)(g / vw.spp);
-    const uint32_t j = vw.sample_offset + (uint32_t)(g % vw.spp);
+    uint32_t pix, j;
+    if (g >> 32) {
+        pix = (uint32_t)(g / vw.spp);
+        j = vw.sample_offset + (uint32_t)(g % vw.spp);
+    } else {  // a 64-bit division costs more than the rest of this function
+        pix = (uint32_t)g / vw.spp;
+        j = vw.sample_offset + (uint32_t)g % vw.spp;
+    }
     const uint32_t px = pix % W, py = pix / W;
     Pcg r = pcg_init(pix, j, vw.seed);
     float fx = fminf(fmaxf((float)px + pcg_float(r), 0.f), (float)W);
@@ -159,24 +166,16 @@ __device__ void start_path(const RenderView &rv, const Buffers &bf, int b, uint3
     bf.st2[b][q] = make_uint4((uint32_t)r.state, (uint32_t)(r.state >> 32), j, kCameraRay | kRecBits);
 }
 
-// Takes the next camera sample (if any) and appends it to buffer b.
-// Sample indices are handed out with one atomic per group of converged lanes.
-__device__ __forceinline__ void regenerate(const RenderView &rv, const Buffers &bf, int b)
-{
-    cg::coalesced_group grp = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (grp.thread_rank() == 0) base = atomicAdd(cnt64(bf.cnt, kCntSample), (unsigned long long)grp.size());
-    const unsigned long long g = grp.shfl(base, 0) + grp.thread_rank();
-    if (g >= rv.total) return;
-    uint32_t q = append(bf.cnt + kCntQueue + 32 * b);
-    start_path(rv, bf, b, q, g);
-}
-
+// The first camera samples, one per queue slot.
 __global__ void __launch_bounds__(kB) k_start(RenderView rv, Buffers bf)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= bf.cap) return;
-    regenerate(rv, bf, 0);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t n = (uint32_t)min((unsigned long long)bf.cap, (unsigned long long)rv.total);
+    if (i == 0) {
+        bf.cnt[kCntQueue] = n;
+        *cnt64(bf.cnt, kCntSample) = n;
+    }
+    if (i < n) start_path(rv, bf, 0, i, i);
 }
 
 // skip_transparent: the reference's checkShadow semantics (Scene::isVisible ->
@@ -319,276 +318,313 @@ __global__ void k_wave_check(uint32_t *cnt, uint64_t total, uint32_t max_waves, 
     cudaGraphSetConditional(loop, (done || capped || cnt[kCntGuideTimeout] != 0) ? 0u : 1u);
 }
 
-// Resident blocks per SM k_shade is compiled for: more resident warps hide its scattered
-// loads better than the spills they cost. BVH-stress render, Mrays/s: 1465 / 1494 / 1507 for
-// 4 (127 registers, no bound) / 5 (96) / 6 (80) with the binned-SAH tree; 1559 / 1583 / 1588
-// for 6 / 7 (72) / 8 (64) with the PLOC tree.
-#ifndef RTB_SHADE_MIN_BLOCKS
-#define RTB_SHADE_MIN_BLOCKS 8
-#endif
+// Resident blocks per SM k_shade is compiled for: its scattered loads want many resident warps,
+// its state registers. 1080p x 64 spp BVH-stress frame and 256x256 x 16 spp Cornell frame (without
+// REST), hybrid 960x540 terrain frame (REST), ms: 194.3 / 1.83 / 11.4 for 5 (96 registers), 193.4 /
+// 1.85 / 11.7 for 6 (80), 193.0 / 1.88 / 11.6 for 7 (72), 193.1 / 1.88 / 11.6 for 8 (64).
+constexpr int kShadeBlocks = 7, kShadeBlocksRest = 5;
+
+// The queue slots of a block's paths, taken with one atomic per counter and block: k_shade is
+// bound by latency, and the wave's tens of millions of appends to the same few counters cost
+// more than its arithmetic when every warp makes its own.
+struct ShadeShared {
+    uint32_t cont[kB / 32], fin[kB / 32];  // per warp: continuing and finished paths
+    uint32_t qbase, rbase;                 // their first slots in the next queue and the retire list
+    unsigned long long sample;             // first of the camera samples taken for the finished ones
+    uint32_t fresh, fbase;                 // how many of them exist, their first slot in the next queue
+};
+
 // One thread per queue position i of the wave (the slot perm[i] when the queue is sorted), on a
-// grid of the queue's capacity. A grid-stride loop over the resident blocks instead nearly
-// doubles the spills at the 64-register bound (708 -> 1300 bytes of spill stores) and was 13%
-// slower on the BVH-stress render (1806 -> 1578 Mrays/s at 2^22 paths).
-__global__ void __launch_bounds__(kB, RTB_SHADE_MIN_BLOCKS) k_shade(RenderView rv, Buffers bf, int cur, GuideView gv)
+// grid of the queue's capacity. GUIDE: the render samples with a guide. REST: it has any of
+// the reference's estimator quirks, photon-map gathers, point lights, textures, several scenes or
+// materials beyond Lambertian, Trowbridge, dielectric, light and mirror; without them it
+// holds much less state.
+template <bool GUIDE, bool REST>
+__global__ void __launch_bounds__(kB, REST ? kShadeBlocksRest : kShadeBlocks) k_shade(RenderView rv, Buffers bf, int cur, GuideView gv)
 {
+    __shared__ ShadeShared sm;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
     if (i == 0) atomicAdd(cnt64(bf.cnt, kCntRays), (unsigned long long)n);  // extension rays of this wave
-    if (i >= n) return;
-    // the queue slot this thread shades. Forwarding the slot's hit, triangle record position and
-    // material through the sort (32 B per path, read here in one coalesced load, so that the
-    // record and material loads start one hop earlier) measured slower: 2189 against 2209 Mrays/s
-    // on the BVH-stress render (more spills here, more traffic in the sort)
-    const uint32_t q = bf.perm ? __ldg(bf.perm + i) : i;
+    if (blockIdx.x * kB >= n) return;
+    const bool live = i < n;
     const int nxt = cur ^ 1;
-    const bool compat = (rv.flags & RT_RENDER_COMPAT) != 0;
-    const uint32_t sub = rv.sv.subs ? __float_as_uint(__ldg(reinterpret_cast<const float *>(bf.rays[cur]) + 8 * q + 7)) : 0u;
-    const SceneLights lights = scene_lights(rv, sub);
-    const bool nee_area = (rv.flags & RT_RENDER_NEE_AREA) != 0 && lights.ne > 0;
-    const bool photon_mode = (rv.flags & RT_RENDER_PHOTON_MAP) != 0;
-    const bool hybrid = (rv.flags & RT_RENDER_HYBRID) != 0;
-    const bool subsurface = (rv.flags & RT_RENDER_SUBSURFACE) != 0;
-    float4 r0 = reinterpret_cast<const float4 *>(bf.rays[cur])[2 * q];
-    float4 r1 = reinterpret_cast<const float4 *>(bf.rays[cur])[2 * q + 1];
-    float4 s0 = bf.st0[cur][q], s1 = bf.st1[cur][q];
-    uint4 s2 = bf.st2[cur][q];
-    float4 hv = reinterpret_cast<const float4 *>(bf.hits)[q];
-    rt_hit h{hv.x, __float_as_int(hv.y), hv.z, hv.w};
-    V3 o = v3(r0.x, r0.y, r0.z), d = v3(r1.x, r1.y, r1.z);
-    V3 beta = v3(s0.x, s0.y, s0.z), L = v3(s1.x, s1.y, s1.z);
-    const float last_pdf = s0.w;
-    const uint32_t pix = __float_as_uint(s1.w);
-    uint32_t flags = s2.w;
-    const uint32_t depth = flags & kDepthMask;
-    uint32_t rec = (flags >> kRecShift) & kRecNone;  // newest guide record of this path
+    const bool compat = REST && (rv.flags & RT_RENDER_COMPAT) != 0;
+    const bool photon_mode = REST && (rv.flags & RT_RENDER_PHOTON_MAP) != 0;
+    const bool hybrid = REST && (rv.flags & RT_RENDER_HYBRID) != 0 && !photon_mode;
+    const bool subsurface = REST && (rv.flags & RT_RENDER_SUBSURFACE) != 0;
+    // path state, between the bounce and the next-event estimation
+    uint32_t sub = 0, pix = 0, flags = 0, rec = kRecNone, rec_in = kRecNone, sample_hi = 0;
+    SceneLights lights;
+    bool nee_area = false, finished = true, scattering = false, guided = false;
+    V3 L, beta, beta_in, wo, wo_w, t, bvec, next_d;
+    Surface sf;
+    Bsdf bs;
     Pcg rng;
-    rng.state = ((uint64_t)s2.y << 32) | s2.x;
-    const rt_view &vw = rv.views[view_of_pixel(rv, pix)];
-    rng.inc = ((((uint64_t)s2.z << 32) | vw.seed) << 1u) | 1u;
-
-    bool finished = h.prim < 0;  // missed: no environment light (Scene::getEnvironmentLight = 0)
-    uint32_t target = 0;
-    bool cont = false;
-    V3 next_o, next_d;
-    float next_pdf = 0.f;
+    float alpha = 0.f, next_pdf = 0.f;
     uint32_t next_flags = 0;
-    if (!finished) {
-        Surface sf = surface_at(rv, h, o, d, compat);
-        const rt_material &m = rv.mats[min(sf.mat, rv.nmats - 1)];
-        Bsdf bs = load_bsdf(m);
-        V3 t, bvec;
-        onb(sf.n, t, bvec);
-        V3 wo_w = -d;
-        V3 wo = v3(dot(wo_w, t), dot(wo_w, bvec), dot(wo_w, sf.n));
-        // the reference decides these from the material's own kd, before any texture
-        const bool scattering = is_scattering(bs);
-        const bool specular = is_specular(bs);
-        const bool guide_ok = guide_vertex(bs, wo.z);
-        if (m.texture) {
-            const float2 uv = surface_uv(rv, h, sf);
-            texture_bsdf(bs, tex_color(rv, m.texture - 1u, uv.x, uv.y));
-        }
-        // where this path's radiance will live after this bounce: decided below, but shadow
-        // rays need the target now, so reserve it first.
-        // BSDF sample first (its outcome decides continue/retire), NEE uses beta before update.
-        V3 wi_l;
-        float pdf_b;
-        bool delta;
-        V3 beta_in = beta;
-        // emission of the hit surface (pathTracing.cu:49-50)
-        V3 Le = v3(0, 0, 0);
-        if (bs.type == RT_MAT_LIGHT) {
-            Le = bs.color * m.intensity;
-        } else if (bs.type == RT_MAT_PLAIN && (flags & kCameraRay)) {
-            Le = bs.color;  // PlainMaterial::getEmittedRadiance on camera rays
-        } else if (bs.type == RT_MAT_FRESNEL_BLEND) {
-            Le = v3(m.extra[0], m.extra[1], m.extra[2]);  // FresnelBlendMaterial::getEmittedRadiance: ke
-        }
-        if (!is_black(Le)) {
-            float w = 1.f;
-            if (nee_area && bs.type == RT_MAT_LIGHT && depth > 0 && !(flags & kLastSpecular) && sf.emissive_tri) {
-                float pl = emitter_pdf(lights.etotal, Le, h.t * h.t, sf.area_cos);
-                w = (last_pdf * last_pdf) / (last_pdf * last_pdf + pl * pl);
+    const GuideParams *gp = nullptr;
+    if (live) {
+        // the queue slot this thread shades. Forwarding the slot's hit, triangle record position and
+        // material through the sort (32 B per path, read here in one coalesced load, so that the
+        // record and material loads start one hop earlier) measured slower: 2189 against 2209
+        // Mrays/s on the BVH-stress render (more spills here, more traffic in the sort)
+        const uint32_t q = bf.perm ? __ldg(bf.perm + i) : i;
+        if (REST && rv.sv.subs) sub = __float_as_uint(__ldg(reinterpret_cast<const float *>(bf.rays[cur]) + 8 * q + 7));
+        lights = scene_lights(rv, sub);
+        nee_area = (rv.flags & RT_RENDER_NEE_AREA) != 0 && lights.ne > 0;
+        float4 r0 = reinterpret_cast<const float4 *>(bf.rays[cur])[2 * q];
+        float4 r1 = reinterpret_cast<const float4 *>(bf.rays[cur])[2 * q + 1];
+        float4 s0 = bf.st0[cur][q], s1 = bf.st1[cur][q];
+        uint4 s2 = bf.st2[cur][q];
+        float4 hv = reinterpret_cast<const float4 *>(bf.hits)[q];
+        rt_hit h{hv.x, __float_as_int(hv.y), hv.z, hv.w};
+        V3 o = v3(r0.x, r0.y, r0.z), d = v3(r1.x, r1.y, r1.z);
+        beta = v3(s0.x, s0.y, s0.z);
+        L = v3(s1.x, s1.y, s1.z);
+        const float last_pdf = s0.w;
+        pix = __float_as_uint(s1.w);
+        flags = s2.w;
+        const uint32_t depth = flags & kDepthMask;
+        if (GUIDE) rec = (flags >> kRecShift) & kRecNone;  // newest guide record of this path
+        rng.state = ((uint64_t)s2.y << 32) | s2.x;
+        sample_hi = s2.z;
+        const rt_view &vw = rv.views[view_of_pixel(rv, pix)];
+        rng.inc = ((((uint64_t)s2.z << 32) | vw.seed) << 1u) | 1u;
+        finished = h.prim < 0;  // missed: no environment light (Scene::getEnvironmentLight = 0)
+        if (!finished) {
+            sf = surface_at(rv, h, o, d, compat);
+            const rt_material &m = rv.mats[min(sf.mat, rv.nmats - 1)];
+            bs = load_bsdf(m);
+            if (!REST) __builtin_assume(bs.type <= RT_MAT_MIRROR);
+            onb(sf.n, t, bvec);
+            wo_w = -d;
+            wo = v3(dot(wo_w, t), dot(wo_w, bvec), dot(wo_w, sf.n));
+            // the reference decides these from the material's own kd, before any texture
+            scattering = is_scattering(bs);
+            const bool specular = is_specular(bs);
+            const bool guide_ok = guide_vertex(bs, wo.z);
+            if (REST && m.texture) {
+                const float2 uv = surface_uv(rv, h, sf);
+                texture_bsdf(bs, tex_color(rv, m.texture - 1u, uv.x, uv.y));
             }
-            L = L + beta_in * Le * w;
-            // the guide is not trained on emitters that next-event estimation samples: with
-            // area NEE on, the direct light is NEE's job and the guide learns the rest
-            if (gv.train && rec != kRecNone && !(nee_area && bs.type == RT_MAT_LIGHT && sf.emissive_tri)) {
-                float4 &e = gv.recs[rec].e;
-                e.x += beta_in.x * Le.x * w;
-                e.y += beta_in.y * Le.y * w;
-                e.z += beta_in.z * Le.z * w;
+            V3 wi_l;
+            float pdf_b;
+            bool delta;
+            beta_in = beta;
+            // emission of the hit surface (pathTracing.cu:49-50)
+            V3 Le = v3(0, 0, 0);
+            if (bs.type == RT_MAT_LIGHT) {
+                Le = bs.color * m.intensity;
+            } else if (bs.type == RT_MAT_PLAIN && (flags & kCameraRay)) {
+                Le = bs.color;  // PlainMaterial::getEmittedRadiance on camera rays
+            } else if (bs.type == RT_MAT_FRESNEL_BLEND) {
+                Le = v3(m.extra[0], m.extra[1], m.extra[2]);  // FresnelBlendMaterial::getEmittedRadiance: ke
             }
-        }
-        const bool guided = gv.enabled && depth < gv.max_depth && guide_ok;
-        const uint32_t rec_in = rec;  // this vertex's NEE belongs to the previous record
-        float alpha = 0.f;
-        const GuideParams *gp = nullptr;
-        if (guided && gv.params) {
-            gp = gv.params + q;
-            alpha = gp->alpha;
-        }
-        V3 f, wi_w;
-        if (guided) {
-            // one-sample MIS between the guide's vMF mixture and the BSDF
-            const float usel = pcg_float(rng);
-            if (usel < alpha) {
-                const float u1 = pcg_float(rng), u2 = pcg_float(rng);
-                wi_w = guide_sample(*gp, usel / alpha, u1, u2);
-                wi_l = v3(dot(wi_w, t), dot(wi_w, bvec), dot(wi_w, sf.n));
-            } else {
-                (void)bsdf_sample(bs, wo, rng, compat, wi_l, pdf_b, delta);
-                wi_w = t * wi_l.x + bvec * wi_l.y + sf.n * wi_l.z;
-            }
-            float pe;
-            V3 fc = bsdf_eval(bs, wo, wi_l, pe);
-            pdf_b = bsdf_sampling_pdf(bs, wo, wi_l);
-            const float pmix = (alpha > 0.f ? alpha * guide_pdf(*gp, wi_w) : 0.f) + (1.f - alpha) * pdf_b;
-            f = (pdf_b > 0.f && pmix > 0.f) ? fc * (1.f / pmix) : v3(0, 0, 0);
-            delta = false;
-            if (gv.train && !is_black(f)) {
-                const uint32_t ri = append(gv.rcnt);
-                if (ri < gv.rec_cap) {
-                    GuideRecord r;
-                    r.a = make_float4(sf.p.x, sf.p.y, sf.p.z, sf.n.x);
-                    r.b = make_float4(sf.n.y, sf.n.z, wo_w.x, wo_w.y);
-                    r.c = make_float4(wo_w.z, wi_w.x, wi_w.y, wi_w.z);
-                    r.d = make_float4(pdf_b, beta_in.x, beta_in.y, beta_in.z);
-                    r.e = make_float4(0.f, 0.f, 0.f, __uint_as_float(rec));
-                    gv.recs[ri] = r;
-                    rec = ri;
+            if (!is_black(Le)) {
+                float w = 1.f;
+                if (nee_area && bs.type == RT_MAT_LIGHT && depth > 0 && !(flags & kLastSpecular) && sf.emissive_tri) {
+                    float pl = emitter_pdf(lights.etotal, Le, h.t * h.t, sf.area_cos);
+                    w = (last_pdf * last_pdf) / (last_pdf * last_pdf + pl * pl);
+                }
+                L = L + beta_in * Le * w;
+                // the guide is not trained on emitters that next-event estimation samples: with
+                // area NEE on, the direct light is NEE's job and the guide learns the rest
+                if (GUIDE && gv.train && rec != kRecNone && !(nee_area && bs.type == RT_MAT_LIGHT && sf.emissive_tri)) {
+                    float4 &e = gv.recs[rec].e;
+                    e.x += beta_in.x * Le.x * w;
+                    e.y += beta_in.y * Le.y * w;
+                    e.z += beta_in.z * Le.z * w;
                 }
             }
-            pdf_b = pmix;  // the density MIS pairs with area-light sampling
-        } else {
-            f = bsdf_sample(bs, wo, rng, compat, wi_l, pdf_b, delta);
-            wi_w = t * wi_l.x + bvec * wi_l.y + sf.n * wi_l.z;
-        }
-        beta = beta * f;
-        finished = is_black(f);
-        if (photon_mode && scattering) {
+            guided = GUIDE && gv.enabled && depth < gv.max_depth && guide_ok;
+            rec_in = rec;  // this vertex's NEE belongs to the previous record
+            if (guided && gv.params) {
+                gp = gv.params + q;
+                alpha = gp->alpha;
+            }
+            V3 f, wi_w;
+            if (guided) {
+                // one-sample MIS between the guide's vMF mixture and the BSDF
+                const float usel = pcg_float(rng);
+                if (usel < alpha) {
+                    const float u1 = pcg_float(rng), u2 = pcg_float(rng);
+                    wi_w = guide_sample(*gp, usel / alpha, u1, u2);
+                    wi_l = v3(dot(wi_w, t), dot(wi_w, bvec), dot(wi_w, sf.n));
+                } else {
+                    (void)bsdf_sample(bs, wo, rng, compat, wi_l, pdf_b, delta);
+                    wi_w = t * wi_l.x + bvec * wi_l.y + sf.n * wi_l.z;
+                }
+                float pe;
+                V3 fc = bsdf_eval(bs, wo, wi_l, pe);
+                pdf_b = bsdf_sampling_pdf(bs, wo, wi_l);
+                const float pmix = (alpha > 0.f ? alpha * guide_pdf(*gp, wi_w) : 0.f) + (1.f - alpha) * pdf_b;
+                f = (pdf_b > 0.f && pmix > 0.f) ? fc * (1.f / pmix) : v3(0, 0, 0);
+                delta = false;
+                if (gv.train && !is_black(f)) {
+                    const uint32_t ri = append(gv.rcnt);
+                    if (ri < gv.rec_cap) {
+                        GuideRecord r;
+                        r.a = make_float4(sf.p.x, sf.p.y, sf.p.z, sf.n.x);
+                        r.b = make_float4(sf.n.y, sf.n.z, wo_w.x, wo_w.y);
+                        r.c = make_float4(wo_w.z, wi_w.x, wi_w.y, wi_w.z);
+                        r.d = make_float4(pdf_b, beta_in.x, beta_in.y, beta_in.z);
+                        r.e = make_float4(0.f, 0.f, 0.f, __uint_as_float(rec));
+                        gv.recs[ri] = r;
+                        rec = ri;
+                    }
+                }
+                pdf_b = pmix;  // the density MIS pairs with area-light sampling
+            } else {
+                f = bsdf_sample(bs, wo, rng, compat, wi_l, pdf_b, delta);
+                wi_w = t * wi_l.x + bvec * wi_l.y + sf.n * wi_l.z;
+            }
+            beta = beta * f;
+            finished = is_black(f);
             // RENDER_MODE PHOTON_MAPPING: the density estimate at this hit ends the path
             // (Scene::getPhotonContributions, Scene.cu:822-840; finishStep, pathTracing.cu:85-89)
-            finished = true;
-            const uint32_t rt = kRetireTarget | append(bf.cnt + kCntRetire);
-            push_gather(bf, sf, wo_w, beta_in, rt, kGatherDensity, rec_in, bs.color);
-            if (subsurface && bs.type == RT_MAT_SUBSURFACE && (flags & kCameraRay))
-                push_gather(bf, sf, wo_w, beta_in, rt, kGatherSubsurface, rec_in, bs.color);
-            bf.retire[rt & ~kRetireTarget] = make_float4(L.x, L.y, L.z, __uint_as_float(pix));
-            regenerate(rv, bf, nxt);
-            return;
-        }
-        // Russian roulette (pathTracing.cu:91-102) on the reference's brightness (luminance) in
-        // compat mode; on the largest component otherwise, so that no channel of a surviving
-        // path's throughput grows past 1 (luminance lets a saturated red path grow 4.7x)
-        if (!finished && scattering && depth > vw.rr_depth) {
-            float qrr = fmaxf(0.05f, 1.f - (compat ? luminance(beta) : fmaxf(beta.x, fmaxf(beta.y, beta.z))));
-            if (pcg_float(rng) < qrr)
-                finished = true;
-            else
-                beta = beta * (1.f / (1.f - qrr));
-        }
-        if (!finished && depth + 1 >= vw.max_depth) finished = true;  // loop bound (pathTracing.cu:296)
-        // reserve the path's slot for the shadow contributions
-        if (!finished) {
-            uint32_t qn = append(bf.cnt + kCntQueue + 32 * nxt);
-            target = qn;
-            cont = true;
-            next_o = spawn_origin(sf.p, sf.n, sf.perr, wi_w);
+            if (photon_mode && scattering) finished = true;
+            // Russian roulette (pathTracing.cu:91-102) on the reference's brightness (luminance) in
+            // compat mode; on the largest component otherwise, so that no channel of a surviving
+            // path's throughput grows past 1 (luminance lets a saturated red path grow 4.7x)
+            if (!finished && scattering && depth > vw.rr_depth) {
+                float qrr = fmaxf(0.05f, 1.f - (compat ? luminance(beta) : fmaxf(beta.x, fmaxf(beta.y, beta.z))));
+                if (pcg_float(rng) < qrr)
+                    finished = true;
+                else
+                    beta = beta * (1.f / (1.f - qrr));
+            }
+            if (!finished && depth + 1 >= vw.max_depth) finished = true;  // loop bound (pathTracing.cu:296)
             next_d = wi_w;
             next_pdf = delta ? 0.f : pdf_b;
             next_flags = (depth + 1) | (delta ? kLastSpecular : 0u) |
                          (((flags & kCameraRay) && specular) ? kCameraRay : 0u) | (rec << kRecShift);
-        } else {
-            target = kRetireTarget | append(bf.cnt + kCntRetire);
         }
+    }
+    // slots: in the next queue for the paths that go on, in the retire list for the others, whose
+    // places in the next queue the next camera samples take
+    const bool cont = live && !finished, fin = live && finished;
+    const unsigned mc = __ballot_sync(0xFFFFFFFFu, cont), mf = __ballot_sync(0xFFFFFFFFu, fin);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        sm.cont[warp] = (uint32_t)__popc(mc);
+        sm.fin[warp] = (uint32_t)__popc(mf);
+    }
+    __syncthreads();
+    if (lane == 0 && warp < 3) {  // one counter per warp, so that the round trips overlap
+        uint32_t c = 0, f = 0;
+        for (int w = 0; w < kB / 32; w++) {
+            c += sm.cont[w];
+            f += sm.fin[w];
+        }
+        if (warp == 0) sm.qbase = c ? atomicAdd(bf.cnt + kCntQueue + 32 * nxt, c) : 0u;
+        if (warp == 1) sm.rbase = f ? atomicAdd(bf.cnt + kCntRetire, f) : 0u;
+        if (warp == 2) sm.sample = bf.regen && f ? atomicAdd(cnt64(bf.cnt, kCntSample), (unsigned long long)f) : rv.total;
+    }
+    __syncthreads();
+    uint32_t slot = 0;  // place among the block's continuing or finished paths
+    for (uint32_t w = 0; w < warp; w++) slot += fin ? sm.fin[w] : sm.cont[w];
+    slot += (uint32_t)__popc((fin ? mf : mc) & ((1u << lane) - 1u));
+    if (bf.regen && threadIdx.x == 96) {
+        uint32_t f = 0;
+        for (int w = 0; w < kB / 32; w++) f += sm.fin[w];
+        sm.fresh = sm.sample < rv.total ? (uint32_t)min((unsigned long long)f, (unsigned long long)(rv.total - sm.sample)) : 0u;
+        sm.fbase = sm.fresh ? atomicAdd(bf.cnt + kCntQueue + 32 * nxt, sm.fresh) : 0u;
+    }
+    if (live) {
+        const uint32_t target = cont ? sm.qbase + slot : kRetireTarget | (sm.rbase + slot);
         // next-event estimation with beta before this bounce (pathTracing.cu:173-205). The
         // direct-light term of a vertex (Scene::sampleDirectLight, Scene.cu:914-969) also holds
         // the subsurface estimate at camera-ray hits and, in hybrid mode, the photon density,
         // with the sum halved.
         const float dscale = hybrid ? 0.5f : 1.0f;
         if (scattering) {
-            if (subsurface && bs.type == RT_MAT_SUBSURFACE && (flags & kCameraRay))
-                push_gather(bf, sf, wo_w, beta_in * dscale, target, kGatherSubsurface, rec_in, bs.color);
-            if (hybrid) push_gather(bf, sf, wo_w, beta_in * dscale, target, kGatherDensity, rec_in, bs.color);
-            for (uint32_t li = lights.pl0; li < lights.pl0 + lights.npl; li++) {  // Scene::estimateAllDirectLights
-                float4 lp = rv.plights[2 * li], li4 = rv.plights[2 * li + 1];
-                V3 tol = v3(lp.x, lp.y, lp.z) - sf.p;
-                float dist2 = dot(tol, tol), dist = sqrtf(dist2);
-                V3 wl = tol * (1.0f / dist);
-                float ul1 = pcg_float(rng), ul2 = pcg_float(rng);
-                (void)ul1;
-                (void)ul2;
-                if (!(dot(wl, sf.n) > 0)) continue;  // isOrientedTo
-                V3 wls = v3(dot(wl, t), dot(wl, bvec), dot(wl, sf.n));
-                float pb;
-                V3 fl = bsdf_eval(bs, wo, wls, pb);
-                V3 Li = v3(li4.x, li4.y, li4.z) * (1.0f / dist2);
-                if (is_black(fl) || is_black(Li)) continue;
-                float w = compat ? 1.0f / (1.0f + pb * pb) : 1.0f;  // powerHeuristic(1,1,1,pdf), Scene.cu:331
-                V3 c = beta_in * fl * Li * (w * dscale);
-                V3 so = spawn_origin(sf.p, sf.n, sf.perr, wl);
-                push_shadow(bf, so, wl, dist, c, target, compat, sub, rec_in);
+            if (REST && (photon_mode || hybrid || subsurface)) {
+                if (photon_mode) push_gather(bf, sf, wo_w, beta_in, target, kGatherDensity, rec_in, bs.color);
+                if (subsurface && bs.type == RT_MAT_SUBSURFACE && (flags & kCameraRay))
+                    push_gather(bf, sf, wo_w, beta_in * dscale, target, kGatherSubsurface, rec_in, bs.color);
+                if (hybrid) push_gather(bf, sf, wo_w, beta_in * dscale, target, kGatherDensity, rec_in, bs.color);
             }
-            if (nee_area) {
-                float u0 = pcg_float(rng), u1 = pcg_float(rng), u2 = pcg_float(rng);
-                // pick an emitter by area * luminance
-                float x = u0 * lights.etotal;
-                uint32_t lo = lights.e0, hi = lights.e0 + lights.ne - 1;
-                while (lo < hi) {
-                    uint32_t mid = (lo + hi) >> 1;
-                    if (rv.emit_cdf[mid] <= x)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                uint32_t etri = rv.emit_tri[lo];
-                const TriRecord er = rv.sv.tris[rv.sv.leafpos[etri]];
-                V3 e0 = v3(er.v0.x, er.v0.y, er.v0.z), e1 = v3(er.v1.x, er.v1.y, er.v1.z),
-                   e2 = v3(er.v2.x, er.v2.y, er.v2.z);
-                float su = sqrtf(u1);
-                float c0 = 1 - su, c1 = u2 * su;
-                V3 xl = e0 * c0 + e1 * c1 + e2 * (1 - c0 - c1);
-                V3 nl = normalize(cross(e1 - e0, e2 - e0));
-                V3 tol = xl - sf.p;
-                float dist2 = dot(tol, tol), dist = sqrtf(dist2);
-                V3 wl = tol * (1.0f / dist);
-                float cosl = fabsf(dot(nl, wl));
-                const rt_material &em = rv.mats[min(rv.tri_mat[etri], rv.nmats - 1)];
-                V3 Lel = v3(em.color[0], em.color[1], em.color[2]) * em.intensity;
-                float pl = emitter_pdf(lights.etotal, Lel, dist2, cosl);
-                if (pl > 0 && dot(wl, sf.n) > 0) {
+            if (!photon_mode) {
+                for (uint32_t li = lights.pl0; li < lights.pl0 + lights.npl; li++) {  // Scene::estimateAllDirectLights
+                    float4 lp = rv.plights[2 * li], li4 = rv.plights[2 * li + 1];
+                    V3 tol = v3(lp.x, lp.y, lp.z) - sf.p;
+                    float dist2 = dot(tol, tol), dist = sqrtf(dist2);
+                    V3 wl = tol * (1.0f / dist);
+                    float ul1 = pcg_float(rng), ul2 = pcg_float(rng);
+                    (void)ul1;
+                    (void)ul2;
+                    if (!(dot(wl, sf.n) > 0)) continue;  // isOrientedTo
                     V3 wls = v3(dot(wl, t), dot(wl, bvec), dot(wl, sf.n));
                     float pb;
                     V3 fl = bsdf_eval(bs, wo, wls, pb);
-                    if (guided)
-                        pb = (alpha > 0.f ? alpha * guide_pdf(*gp, wl) : 0.f) +
-                             (1.f - alpha) * bsdf_sampling_pdf(bs, wo, wls);
-                    if (!is_black(fl)) {
-                        float w = (pl * pl) / (pl * pl + pb * pb);
-                        V3 c = beta_in * fl * Lel * (w * dscale / pl);
-                        V3 so = spawn_origin(sf.p, sf.n, sf.perr, wl);
-                        push_shadow(bf, so, wl, dist * (1.0f - 1e-4f), c, target, false, sub, rec_in);
+                    V3 Li = v3(li4.x, li4.y, li4.z) * (1.0f / dist2);
+                    if (is_black(fl) || is_black(Li)) continue;
+                    float w = compat ? 1.0f / (1.0f + pb * pb) : 1.0f;  // powerHeuristic(1,1,1,pdf), Scene.cu:331
+                    V3 c = beta_in * fl * Li * (w * dscale);
+                    V3 so = spawn_origin(sf.p, sf.n, sf.perr, wl);
+                    push_shadow(bf, so, wl, dist, c, target, compat, sub, rec_in);
+                }
+                if (nee_area) {
+                    float u0 = pcg_float(rng), u1 = pcg_float(rng), u2 = pcg_float(rng);
+                    // pick an emitter by area * luminance
+                    float x = u0 * lights.etotal;
+                    uint32_t lo = lights.e0, hi = lights.e0 + lights.ne - 1;
+                    while (lo < hi) {
+                        uint32_t mid = (lo + hi) >> 1;
+                        if (rv.emit_cdf[mid] <= x)
+                            lo = mid + 1;
+                        else
+                            hi = mid;
+                    }
+                    uint32_t etri = rv.emit_tri[lo];
+                    const TriRecord er = rv.sv.tris[rv.sv.leafpos[etri]];
+                    V3 e0 = v3(er.v0.x, er.v0.y, er.v0.z), e1 = v3(er.v1.x, er.v1.y, er.v1.z),
+                       e2 = v3(er.v2.x, er.v2.y, er.v2.z);
+                    float su = sqrtf(u1);
+                    float c0 = 1 - su, c1 = u2 * su;
+                    V3 xl = e0 * c0 + e1 * c1 + e2 * (1 - c0 - c1);
+                    V3 nl = normalize(cross(e1 - e0, e2 - e0));
+                    V3 tol = xl - sf.p;
+                    float dist2 = dot(tol, tol), dist = sqrtf(dist2);
+                    V3 wl = tol * (1.0f / dist);
+                    float cosl = fabsf(dot(nl, wl));
+                    const rt_material &em = rv.mats[min(rv.tri_mat[etri], rv.nmats - 1)];
+                    V3 Lel = v3(em.color[0], em.color[1], em.color[2]) * em.intensity;
+                    float pl = emitter_pdf(lights.etotal, Lel, dist2, cosl);
+                    if (pl > 0 && dot(wl, sf.n) > 0) {
+                        V3 wls = v3(dot(wl, t), dot(wl, bvec), dot(wl, sf.n));
+                        float pb;
+                        V3 fl = bsdf_eval(bs, wo, wls, pb);
+                        if (guided)
+                            pb = (alpha > 0.f ? alpha * guide_pdf(*gp, wl) : 0.f) +
+                                 (1.f - alpha) * bsdf_sampling_pdf(bs, wo, wls);
+                        if (!is_black(fl)) {
+                            float w = (pl * pl) / (pl * pl + pb * pb);
+                            V3 c = beta_in * fl * Lel * (w * dscale / pl);
+                            V3 so = spawn_origin(sf.p, sf.n, sf.perr, wl);
+                            push_shadow(bf, so, wl, dist * (1.0f - 1e-4f), c, target, false, sub, rec_in);
+                        }
                     }
                 }
             }
         }
-    } else {
-        target = kRetireTarget | append(bf.cnt + kCntRetire);
+        if (cont) {
+            const V3 next_o = spawn_origin(sf.p, sf.n, sf.perr, next_d);
+            reinterpret_cast<float4 *>(bf.rays[nxt])[2 * target] = make_float4(next_o.x, next_o.y, next_o.z, INFINITY);
+            reinterpret_cast<float4 *>(bf.rays[nxt])[2 * target + 1] =
+                make_float4(next_d.x, next_d.y, next_d.z, __uint_as_float(sub));
+            bf.st0[nxt][target] = make_float4(beta.x, beta.y, beta.z, next_pdf);
+            bf.st1[nxt][target] = make_float4(L.x, L.y, L.z, __uint_as_float(pix));
+            bf.st2[nxt][target] = make_uint4((uint32_t)rng.state, (uint32_t)(rng.state >> 32), sample_hi, next_flags);
+        } else {
+            bf.retire[target & ~kRetireTarget] = make_float4(L.x, L.y, L.z, __uint_as_float(pix));
+            if (GUIDE && gv.train) gv.retire_rec[target & ~kRetireTarget] = rec;
+        }
     }
-    if (cont) {
-        const uint32_t qn = target;
-        reinterpret_cast<float4 *>(bf.rays[nxt])[2 * qn] = make_float4(next_o.x, next_o.y, next_o.z, INFINITY);
-        reinterpret_cast<float4 *>(bf.rays[nxt])[2 * qn + 1] =
-            make_float4(next_d.x, next_d.y, next_d.z, __uint_as_float(sub));
-        bf.st0[nxt][qn] = make_float4(beta.x, beta.y, beta.z, next_pdf);
-        bf.st1[nxt][qn] = make_float4(L.x, L.y, L.z, __uint_as_float(pix));
-        bf.st2[nxt][qn] = make_uint4((uint32_t)rng.state, (uint32_t)(rng.state >> 32), s2.z, next_flags);
-    } else {
-        bf.retire[target & ~kRetireTarget] = make_float4(L.x, L.y, L.z, __uint_as_float(pix));
-        if (gv.train) gv.retire_rec[target & ~kRetireTarget] = rec;
-        regenerate(rv, bf, nxt);
+    if (bf.regen) {
+        __syncthreads();
+        if (fin && slot < sm.fresh) start_path(rv, bf, nxt, sm.fbase + slot, sm.sample + slot);
     }
 }
 
@@ -1250,6 +1286,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     bf.cap = cap;
     bf.scap = scap;
     bf.gcap = gcap;
+    bf.regen = total > cap;
     // material sort of the shading order, chunks of 2^sort_log2 queue slots (0: off)
     const uint32_t sort_log2 = s->sort_log2 ? std::min<uint32_t>(std::max<uint32_t>(s->sort_log2, 5u), kSortMaxLog2) : 0u;
     const unsigned sort_blocks =
@@ -1321,6 +1358,12 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         if (stage_times) RTB_CUDA(cudaEventRecord(sev.e[k][b], st));
         return RT_OK;
     };
+    // k_shade's form (see there)
+    bool rest = (flags & (RT_RENDER_COMPAT | RT_RENDER_PHOTON_MAP | RT_RENDER_HYBRID | RT_RENDER_SUBSURFACE)) != 0 ||
+                s->merged || !s->plights.empty();
+    for (const rt_material &m : s->materials) rest |= m.type > RT_MAT_MIRROR || m.texture != 0;
+    auto shade = guided ? (rest ? k_shade<true, true> : k_shade<true, false>)
+                        : (rest ? k_shade<false, true> : k_shade<false, false>);
     // One group = 4 waves (cur 0, 1, 0, 1). The first group is launched directly; the rest
     // replay it as a CUDA graph captured from the second group's launches.
     auto wave_group = [&]() -> int {
@@ -1343,7 +1386,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
                 RTB_CUDA(cudaGetLastError());
             }
             RTB_CHECK(mark(k, 3));
-            k_shade<<<blocks, kB, 0, st>>>(rv, bf, cur, gv);
+            shade<<<blocks, kB, 0, st>>>(rv, bf, cur, gv);
             RTB_CUDA(cudaGetLastError());
             RTB_CHECK(mark(k, 4));
             k_shadow<<<shadow_blocks, kB, 0, st>>>(rv, bf);
