@@ -77,7 +77,7 @@ constexpr int kCntShadowRays = 258;   // u64
 constexpr int kCntGathers = 260;      // u64
 constexpr int kCntGuideTimeout = 264; // the guide's tensor-core wait timed out
 constexpr int kCntWaves = 266;        // waves of the device-side loop
-constexpr int kCntCapped = 267;       // its wave cap was reached
+constexpr int kCntCapped = 267;       // its wave cap was reached; k_wave_count: the queues have drained
 constexpr int kCntWords = 288;
 
 struct GuideView {
@@ -229,12 +229,14 @@ struct PhotonView {
 // a stable counting sort in shared memory; k_shade's thread i then shades slot perm[i]. Lanes of a warp
 // then mostly run the same BSDF code, while the chunk keeps the state reads of a warp within a
 // few kilobytes. The chunk size is the sort granularity (rt_render_set_sort).
+// finish: the hits are a walk's (launch_walk_dev), and this kernel, which reads them all anyway, does
+// what the walk left to do: a pass over hits and rays by itself cost up to 40 us a wave of 2^20 paths.
+// It also clears the wave's counters, which are not in use while it runs.
 constexpr int kSortBlock = 256;
 constexpr int kSortKeys = 16;  // 0: miss, 1 + rt_material_type
 constexpr uint32_t kSortMaxLog2 = 13;
-__device__ __forceinline__ uint32_t shade_key(const RenderView &rv, const Buffers &bf, uint32_t q)
+__device__ __forceinline__ uint32_t shade_key(const RenderView &rv, int32_t prim)
 {
-    const int32_t prim = __float_as_int(__ldg(reinterpret_cast<const float *>(bf.hits) + 4 * (uint64_t)q + 1));
     if (prim < 0) return 0;
     uint32_t mat;
     if (prim & RT_PRIM_SHAPE)
@@ -246,11 +248,15 @@ __device__ __forceinline__ uint32_t shade_key(const RenderView &rv, const Buffer
 }
 
 __global__ void __launch_bounds__(kSortBlock) k_material_sort(RenderView rv, Buffers bf, int cur, uint32_t *perm,
-                                                               uint32_t log2)
+                                                               uint32_t log2, bool finish)
 {
     __shared__ uint32_t count[kSortKeys], start[kSortKeys];
     __shared__ uint8_t key[1u << kSortMaxLog2];
     __shared__ uint32_t wcount[kSortBlock / 32][kSortKeys];
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) bf.cnt[kCntQueue + 32 * (cur ^ 1)] = 0;
+        if (threadIdx.x < 5) bf.cnt[kCntShadow + 32 * threadIdx.x] = 0;
+    }
     const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
     // chunks in a grid-stride loop over the resident blocks (c0 is the same for the whole block)
     for (uint32_t c0 = blockIdx.x << log2; c0 < n; c0 += gridDim.x << log2) {
@@ -258,7 +264,13 @@ __global__ void __launch_bounds__(kSortBlock) k_material_sort(RenderView rv, Buf
         if (threadIdx.x < kSortKeys) count[threadIdx.x] = 0;
         __syncthreads();
         for (uint32_t j = threadIdx.x; j < len; j += kSortBlock) {
-            const uint32_t k = shade_key(rv, bf, c0 + j);
+            float4 *h = reinterpret_cast<float4 *>(bf.hits) + c0 + j;
+            float4 hv = *h;
+            if (finish && (rv.sv.nspheres || __float_as_int(hv.y) == kHitReplay)) {
+                hv = finish_fast(rv.sv, bf.rays[cur], c0 + j, RT_TRACE_FAST | kTraceRecords, hv, bf.trace_cnt);
+                *h = hv;
+            }
+            const uint32_t k = shade_key(rv, __float_as_int(hv.y));
             key[j] = (uint8_t)k;
             atomicAdd(&count[k], 1u);
         }
@@ -318,6 +330,15 @@ __global__ void k_wave_check(uint32_t *cnt, uint64_t total, uint32_t max_waves, 
     cudaGraphSetConditional(loop, (done || capped || cnt[kCntGuideTimeout] != 0) ? 0u : 1u);
 }
 
+// Counts the waves of a 4-wave group launched without a loop, until the queues have drained.
+__global__ void k_wave_count(uint32_t *cnt)
+{
+    if (cnt[kCntCapped]) return;
+    cnt[kCntWaves] += 4;
+    if (cnt[kCntQueue] == 0) cnt[kCntCapped] = 1;
+}
+constexpr uint32_t kDirectDepth = 64;
+
 // Resident blocks per SM k_shade is compiled for: its scattered loads want many resident warps,
 // its state registers. 1080p x 64 spp BVH-stress frame and 256x256 x 16 spp Cornell frame (without
 // REST), hybrid 960x540 terrain frame (REST), ms: 194.3 / 1.83 / 11.4 for 5 (96 registers), 193.4 /
@@ -345,7 +366,10 @@ __global__ void __launch_bounds__(kB, REST ? kShadeBlocksRest : kShadeBlocks) k_
     __shared__ ShadeShared sm;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
-    if (i == 0) atomicAdd(cnt64(bf.cnt, kCntRays), (unsigned long long)n);  // extension rays of this wave
+    if (i == 0) {
+        atomicAdd(cnt64(bf.cnt, kCntRays), (unsigned long long)n);  // extension rays of this wave
+        *reinterpret_cast<uint4 *>(bf.trace_cnt) = make_uint4(0, 0, 0, 0);  // for the next wave's trace
+    }
     if (blockIdx.x * kB >= n) return;
     const bool live = i < n;
     const int nxt = cur ^ 1;
@@ -1312,6 +1336,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     RTB_CUDA(cudaEventCreate(&e1));
     RTB_CUDA(cudaEventRecord(e0, st));
     RTB_CUDA(cudaMemsetAsync(bf.cnt, 0, 4 * kCntWords, st));
+    RTB_CUDA(cudaMemsetAsync(bf.trace_cnt, 0, 16, st));
     const unsigned blocks = cap / kB;
     const unsigned retire_blocks = std::min(blocks, resident_grid(SLOT_RETIRE_RESIDENT, k_retire, kB));
     const unsigned shadow_blocks =
@@ -1366,25 +1391,34 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
                         : (rest ? k_shade<false, true> : k_shade<false, false>);
     // One group = 4 waves (cur 0, 1, 0, 1). The first group is launched directly; the rest
     // replay it as a CUDA graph captured from the second group's launches.
+    // fused: the material sort finishes the walk's hits (timed stages keep them apart)
+    const bool fused = sort_log2 != 0 && trace_flags == RT_TRACE_FAST && !stage_times;
     auto wave_group = [&]() -> int {
         int cur = 0;
+        auto infer = [&]() -> int {
+            k_guide_infer<<<infer_blocks, kInferWarps * 32, kInferSmem, st>>>(
+                rv, bf, cur, guide->img.as<uint4>(), gbox, guide->params.as<GuideParams>(), gv.max_depth);
+            RTB_CUDA(cudaGetLastError());
+            return RT_OK;
+        };
         for (int k = 0; k < 4; k++) {
             RTB_CHECK(mark(k, 0));
-            RTB_CHECK(launch_trace_closest_dev(rv.sv, bf.rays[cur], bf.cnt + kCntQueue + 32 * cur, cap, bf.hits, trace_flags,
-                                               s->scratch.counters.as<uint32_t>(), st));
+            const uint32_t *paths = bf.cnt + kCntQueue + 32 * cur;
+            if (fused)
+                RTB_CHECK(launch_walk_dev(rv.sv, bf.rays[cur], paths, cap, bf.hits, bf.trace_cnt, st));
+            else
+                RTB_CHECK(launch_trace_closest_dev(rv.sv, bf.rays[cur], paths, cap, bf.hits, trace_flags, bf.trace_cnt, st));
             RTB_CHECK(mark(k, 1));
-            if (gv.params) {
-                k_guide_infer<<<infer_blocks, kInferWarps * 32, kInferSmem, st>>>(
-                    rv, bf, cur, guide->img.as<uint4>(), gbox, guide->params.as<GuideParams>(), gv.max_depth);
-                RTB_CUDA(cudaGetLastError());
-            }
+            if (gv.params && !fused) RTB_CHECK(infer());
             RTB_CHECK(mark(k, 2));
-            RTB_CUDA(cudaMemsetAsync(bf.cnt + kCntQueue + 32 * (cur ^ 1), 0, 4, st));
-            RTB_CUDA(cudaMemsetAsync(bf.cnt + kCntShadow, 0, 4 * (kCntSample - kCntShadow), st));
             if (sort_log2) {
-                k_material_sort<<<sort_blocks, kSortBlock, 0, st>>>(rv, bf, cur, rs.perm.as<uint32_t>(), sort_log2);
+                k_material_sort<<<sort_blocks, kSortBlock, 0, st>>>(rv, bf, cur, rs.perm.as<uint32_t>(), sort_log2, fused);
                 RTB_CUDA(cudaGetLastError());
+            } else {
+                RTB_CUDA(cudaMemsetAsync(bf.cnt + kCntQueue + 32 * (cur ^ 1), 0, 4, st));
+                RTB_CUDA(cudaMemsetAsync(bf.cnt + kCntShadow, 0, 4 * (kCntSample - kCntShadow), st));
             }
+            if (gv.params && fused) RTB_CHECK(infer());
             RTB_CHECK(mark(k, 3));
             shade<<<blocks, kB, 0, st>>>(rv, bf, cur, gv);
             RTB_CUDA(cudaGetLastError());
@@ -1415,9 +1449,28 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     // group, ended by k_wave_check on the device, so the host waits once per frame instead of
     // after every group. Where conditional graphs cannot be built (the legacy default stream
     // cannot be captured) the host loop below runs instead.
-    bool device_loop = false;
+    bool device_loop = false, done = false;
+    // Where every sample has a queue slot from the start, max_depth waves are all there can be: their
+    // launches go straight into the stream, which costs less than building and instantiating a
+    // graph (about 0.4 ms a call), and the waves that find no path left take a few microseconds
+    // each.
+    if (!bf.regen && depth_max <= kDirectDepth && !(flags & (RT_RENDER_HOST_LOOP | RT_RENDER_STAGE_TIMES))) {
+        for (uint32_t w = 0; w < depth_max; w += 4) {
+            RTB_CHECK(wave_group());
+            k_wave_count<<<1, 1, 0, st>>>(bf.cnt);
+            RTB_CUDA(cudaGetLastError());
+        }
+        RTB_CUDA(cudaMemcpyAsync(rs.host_cnt, bf.cnt, 4 * kCntWords, cudaMemcpyDeviceToHost, st));
+        RTB_CUDA(cudaStreamSynchronize(st));
+        const uint32_t *hc = static_cast<const uint32_t *>(rs.host_cnt);
+        waves = hc[kCntWaves];
+        if (hc[kCntGuideTimeout])
+            return fail(RT_ERR_TIMEOUT, name + ": guide tensor-core completion wait timed out");
+        if (hc[kCntQueue] != 0) return fail(RT_ERR_TIMEOUT, name + ": wave cap exceeded");
+        done = true;
+    }
     const uint32_t wave_cap = (uint32_t)std::min<uint64_t>(max_waves, 0x7FFFFFF0u);
-    if (st != nullptr && st != cudaStreamLegacy && !(flags & (RT_RENDER_HOST_LOOP | RT_RENDER_STAGE_TIMES))) {
+    if (!done && st != nullptr && st != cudaStreamLegacy && !(flags & (RT_RENDER_HOST_LOOP | RT_RENDER_STAGE_TIMES))) {
         cudaGraph_t g = nullptr;
         cudaGraphConditionalHandle loop_handle;
         bool ok = cudaGraphCreate(&g, 0) == cudaSuccess &&
@@ -1469,7 +1522,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         if (hc[kCntGuideTimeout]) return fail(RT_ERR_TIMEOUT, name + ": guide tensor-core completion wait timed out");
         if (hc[kCntCapped]) return fail(RT_ERR_TIMEOUT, name + ": wave cap exceeded");
     }
-    for (uint64_t group = 0; !device_loop; group++) {
+    for (uint64_t group = 0; !device_loop && !done; group++) {
         int rc = RT_OK;
         // the legacy default stream cannot be captured: there every group is launched directly
         if (group == 1 && !stage_times && st != nullptr && st != cudaStreamLegacy &&

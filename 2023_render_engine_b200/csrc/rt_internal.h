@@ -208,6 +208,10 @@ int launch_trace_closest(const SceneView &v, const rt_ray *rays, uint64_t n, rt_
 // hits are the renderer's form (kTraceRecords).
 int launch_trace_closest_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_dev, uint32_t cap, rt_hit *hits,
                              uint32_t flags, uint32_t *counters, cudaStream_t s);
+// Only the fast-mode walk of it: the caller's next kernel applies finish_fast (traverse.cuh) to each
+// hit, and the caller's kernels clear the counters between walks.
+int launch_walk_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_dev, uint32_t cap, rt_hit *hits,
+                    uint32_t *counters, cudaStream_t s);
 // Scene::isVisible: occluded when the reference's closest hit along the unbounded ray is no farther
 // than the ray's tmax. One byte per ray, or (bits) bit i % 32 of word i / 32 (the last word's bits
 // past n are 0). hits: n entries of scratch.

@@ -27,9 +27,6 @@ namespace {
 
 constexpr int kBlock = 128;
 
-// rt_hit::prim between the walk and k_trace_finish: a triangle record, -1, or
-constexpr int32_t kHitReplay = 0x7FFFFFFE;  // the reference traversal decides
-
 // Scene index a ray carries in its last word (merged scenes only; 0 otherwise).
 __device__ __forceinline__ uint32_t ray_scene(const SceneView &v, const rt_ray *rays, uint64_t i)
 {
@@ -109,22 +106,18 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_counts(Sc
         });
 }
 
-// The walk's hits -> the call's results, one thread per ray: with exactness wanted, the proof or
-// the replay of the reference's answer (see the file comment); the analytic shapes; triangle
-// ids (kTraceRecords: the renderer's form, triangle records) or, for kTraceVisible, the occlusion
-// decision in `out` (one byte per ray, or with bits one word per 32 rays). With nothing of that
-// to do it only looks at the rays whose walk could not finish (counters[0] of them). EXACT: without
-// RT_TRACE_FAST.
-template <bool EXACT>
-__global__ void __launch_bounds__(kBlock, EXACT ? 8 : 12) k_trace_finish(SceneView v, const rt_ray *__restrict__ rays, uint64_t n,
-                                                         const uint32_t *__restrict__ n_dev, rt_hit *__restrict__ hits,
-                                                         uint32_t flags, void *__restrict__ out, bool bits,
-                                                         uint32_t *__restrict__ counters)
+// The walk's hits -> the call's results, one thread per ray, without RT_TRACE_FAST: the proof or the
+// replay of the reference's answer (see the file comment); the analytic shapes; triangle ids
+// (kTraceRecords: the renderer's form, triangle records) or, for kTraceVisible, the occlusion
+// decision in `out` (one byte per ray, or with bits one word per 32 rays).
+__global__ void __launch_bounds__(kBlock, 8) k_trace_finish(SceneView v, const rt_ray *__restrict__ rays, uint64_t n,
+                                                            const uint32_t *__restrict__ n_dev,
+                                                            rt_hit *__restrict__ hits, uint32_t flags,
+                                                            void *__restrict__ out, bool bits,
+                                                            uint32_t *__restrict__ counters)
 {
     if (n_dev) n = min((uint64_t)*n_dev, n);
-    const bool exact = EXACT, visible = EXACT && (flags & kTraceVisible) != 0;
-    if (!exact && !v.nspheres && *(volatile uint32_t *)counters == 0u) return;
-    const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
+    const bool visible = (flags & kTraceVisible) != 0, shadow = (flags & RT_TRACE_SHADOW) != 0;
     // whole warps stay in the loop (the bit mask is gathered with a ballot)
     for (uint64_t i0 = (uint64_t)blockIdx.x * kBlock; i0 < n; i0 += (uint64_t)gridDim.x * kBlock) {
         const uint64_t i = i0 + threadIdx.x;
@@ -136,58 +129,54 @@ __global__ void __launch_bounds__(kBlock, EXACT ? 8 : 12) k_trace_finish(SceneVi
             float t = hv.x, b1 = hv.z, b2 = hv.w;
             int32_t rec = __float_as_int(hv.y), prim = rec;
             bool replay = rec == kHitReplay;
-            if (exact || v.nspheres || replay) {
-                const float tri_max = visible ? INFINITY : ra.w;
-                if (exact && rec >= 0 && !replay) {
-                    const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
-                    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-                    prim = (int32_t)__float_as_uint(b.w);
-                    const float ix = fdiv(1.0f, rb.x), iy = fdiv(1.0f, rb.y), iz = fdiv(1.0f, rb.z);
-                    const float lx = fminf(fminf(a.x, b.x), c.x), ly = fminf(fminf(a.y, b.y), c.y),
-                                lz = fminf(fminf(a.z, b.z), c.z);
-                    const float hx = fmaxf(fmaxf(a.x, b.x), c.x), hy = fmaxf(fmaxf(a.y, b.y), c.y),
-                                hz = fmaxf(fmaxf(a.z, b.z), c.z);
-                    if (!(tri_max == INFINITY) || rb.x == 0.f || rb.y == 0.f || rb.z == 0.f ||
-                        !ref_box_test(lx, ly, lz, hx, hy, hz, ra.x, ra.y, ra.z, ix, iy, iz, tri_max)) {
-                        // walk the winner's ancestors in the reference tree (the root is never
-                        // box-tested)
-                        atomicAdd(counters, 1u);
-                        uint32_t j = v.ref_pos[prim];
-                        const uint32_t m = v.ntri, root = 2 * m - 2;
-                        while (m > 1) {
-                            const uint32_t q = m + j / 2;
-                            if (q >= root) break;
-                            const float2 *bx = v.ref_boxes + 3 * (size_t)q;
-                            const float2 b0 = __ldg(bx), b1v = __ldg(bx + 1), b2v = __ldg(bx + 2);
-                            if (!ref_box_test(b0.x, b0.y, b1v.x, b1v.y, b2v.x, b2v.y, ra.x, ra.y, ra.z, ix, iy, iz,
-                                              tri_max)) {
-                                replay = true;
-                                break;
-                            }
-                            j = q;
+            const float tri_max = visible ? INFINITY : ra.w;
+            if (rec >= 0 && !replay) {
+                const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
+                const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+                prim = (int32_t)__float_as_uint(b.w);
+                const float ix = fdiv(1.0f, rb.x), iy = fdiv(1.0f, rb.y), iz = fdiv(1.0f, rb.z);
+                const float lx = fminf(fminf(a.x, b.x), c.x), ly = fminf(fminf(a.y, b.y), c.y),
+                            lz = fminf(fminf(a.z, b.z), c.z);
+                const float hx = fmaxf(fmaxf(a.x, b.x), c.x), hy = fmaxf(fmaxf(a.y, b.y), c.y),
+                            hz = fmaxf(fmaxf(a.z, b.z), c.z);
+                if (!(tri_max == INFINITY) || rb.x == 0.f || rb.y == 0.f || rb.z == 0.f ||
+                    !ref_box_test(lx, ly, lz, hx, hy, hz, ra.x, ra.y, ra.z, ix, iy, iz, tri_max)) {
+                    // walk the winner's ancestors in the reference tree (the root is never
+                    // box-tested)
+                    atomicAdd(counters, 1u);
+                    uint32_t j = v.ref_pos[prim];
+                    const uint32_t m = v.ntri, root = 2 * m - 2;
+                    while (m > 1) {
+                        const uint32_t q = m + j / 2;
+                        if (q >= root) break;
+                        const float2 *bx = v.ref_boxes + 3 * (size_t)q;
+                        const float2 b0 = __ldg(bx), b1v = __ldg(bx + 1), b2v = __ldg(bx + 2);
+                        if (!ref_box_test(b0.x, b0.y, b1v.x, b1v.y, b2v.x, b2v.y, ra.x, ra.y, ra.z, ix, iy, iz,
+                                          tri_max)) {
+                            replay = true;
+                            break;
                         }
+                        j = q;
                     }
-                } else if (rec >= 0 && !replay && !(flags & (kTraceRecords | kTraceIds))) {
-                    prim = (int32_t)__float_as_uint(__ldg(&v.tris[rec].v1.w));
                 }
-                if (replay) {
-                    const WatertightRay w = make_watertight(ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max);
-                    bool overflow = false;
-                    prim = replay_reference(v, w, fdiv(1.0f, rb.x), fdiv(1.0f, rb.y), fdiv(1.0f, rb.z), shadow, t, b1,
-                                            b2, overflow);
-                    if (overflow) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
-                    atomicAdd(counters + 2, 1u);
-                }
-                if (prim < 0) t = INFINITY;
-                if ((flags & kTraceRecords) && prim >= 0 && (exact || replay)) prim = (int32_t)v.leafpos[prim];
-                if (v.nspheres)
-                    intersect_spheres(v, ray_scene(v, rays, i), ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max, shadow, t,
-                                      prim, b1, b2);
-                if (visible)
-                    occ = prim != RT_PRIM_NONE && t <= ra.w;
-                else
-                    reinterpret_cast<float4 *>(hits)[i] = make_float4(t, __int_as_float(prim), b1, b2);
             }
+            if (replay) {
+                const WatertightRay w = make_watertight(ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max);
+                bool overflow = false;
+                prim = replay_reference(v, w, fdiv(1.0f, rb.x), fdiv(1.0f, rb.y), fdiv(1.0f, rb.z), shadow, t, b1,
+                                        b2, overflow);
+                if (overflow) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
+                atomicAdd(counters + 2, 1u);
+            }
+            if (prim < 0) t = INFINITY;
+            if ((flags & kTraceRecords) && prim >= 0) prim = (int32_t)v.leafpos[prim];
+            if (v.nspheres)
+                intersect_spheres(v, ray_scene(v, rays, i), ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max, shadow, t,
+                                  prim, b1, b2);
+            if (visible)
+                occ = prim != RT_PRIM_NONE && t <= ra.w;
+            else
+                reinterpret_cast<float4 *>(hits)[i] = make_float4(t, __int_as_float(prim), b1, b2);
         }
         if (visible) {
             if (bits) {
@@ -197,6 +186,21 @@ __global__ void __launch_bounds__(kBlock, EXACT ? 8 : 12) k_trace_finish(SceneVi
                 static_cast<uint8_t *>(out)[i] = occ ? 1 : 0;
             }
         }
+    }
+}
+
+// The same in fast mode (finish_fast). With nothing to do for most rays it only looks at those whose
+// walk could not finish (counters[0] of them).
+__global__ void __launch_bounds__(kBlock, 12) k_trace_finish_fast(SceneView v, const rt_ray *__restrict__ rays, uint64_t n,
+                                                                  const uint32_t *__restrict__ n_dev,
+                                                                  rt_hit *__restrict__ hits, uint32_t flags,
+                                                                  uint32_t *__restrict__ counters)
+{
+    if (n_dev) n = min((uint64_t)*n_dev, n);
+    if (!v.nspheres && *(volatile uint32_t *)counters == 0u) return;
+    for (uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kBlock) {
+        float4 *h = reinterpret_cast<float4 *>(hits) + i;
+        *h = finish_fast(v, rays, i, flags, *h, counters);
     }
 }
 
@@ -267,7 +271,16 @@ static unsigned persistent_blocks()
 // fewer.
 static uint64_t walk_blocks(uint64_t n) { return std::min<uint64_t>((n + 15) / 16, persistent_blocks()); }
 
-// The walk, then k_trace_finish. n_dev: the count, when it is on the device (n bounds it).
+// The walk. n_dev: the count, when it is on the device (n bounds it).
+static int launch_walk(const SceneView &v, const rt_ray *rays, uint64_t n, const uint32_t *n_dev, rt_hit *hits,
+                       uint32_t flags, uint32_t *counters, cudaStream_t s)
+{
+    k_trace_closest<<<(unsigned)walk_blocks(n), kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, counters);
+    RTB_CUDA(cudaGetLastError());
+    return RT_OK;
+}
+
+// The walk and what it leaves to do.
 static int launch_trace(const SceneView &v, const rt_ray *rays, uint64_t n, const uint32_t *n_dev, rt_hit *hits,
                         uint32_t flags, void *out, bool bits, uint32_t *counters, cudaStream_t s)
 {
@@ -275,12 +288,12 @@ static int launch_trace(const SceneView &v, const rt_ray *rays, uint64_t n, cons
     // fast, triangles only, ids wanted: the walk writes the ids itself and nothing is left to finish
     if ((flags & RT_TRACE_FAST) && !v.nspheres && !(flags & kTraceRecords)) flags |= kTraceIds;
     RTB_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(uint32_t), s));
-    const uint64_t blocks = walk_blocks(n);
-    k_trace_closest<<<(unsigned)blocks, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, counters);
-    RTB_CUDA(cudaGetLastError());
-    const uint64_t finish = std::min<uint64_t>((n + kBlock - 1) / kBlock, 16ull * device_sm_count());
-    auto kernel = (flags & RT_TRACE_FAST) ? k_trace_finish<false> : k_trace_finish<true>;
-    kernel<<<(unsigned)finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, out, bits, counters);
+    RTB_CHECK(launch_walk(v, rays, n, n_dev, hits, flags, counters, s));
+    const unsigned finish = (unsigned)std::min<uint64_t>((n + kBlock - 1) / kBlock, 16ull * device_sm_count());
+    if (flags & RT_TRACE_FAST)
+        k_trace_finish_fast<<<finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, counters);
+    else
+        k_trace_finish<<<finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, out, bits, counters);
     RTB_CUDA(cudaGetLastError());
     return RT_OK;
 }
@@ -297,6 +310,12 @@ int launch_trace_closest_dev(const SceneView &v, const rt_ray *rays, const uint3
 {
     return launch_trace(v, rays, cap, n_dev, hits, (flags & (RT_TRACE_SHADOW | RT_TRACE_FAST)) | kTraceRecords, nullptr,
                         false, counters, s);
+}
+
+int launch_walk_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_dev, uint32_t cap, rt_hit *hits,
+                    uint32_t *counters, cudaStream_t s)
+{
+    return launch_walk(v, rays, cap, n_dev, hits, RT_TRACE_FAST | kTraceRecords, counters, s);
 }
 
 int launch_trace_visible(const SceneView &v, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags, void *out,
