@@ -8,8 +8,8 @@
 // photon order does not depend on scheduling.
 //
 // The kd-tree is the reference's implicit balanced tree (kdtree.h:78-108): the element at
-// the middle of a range is the node, split on the axis of largest extent, built on the host
-// with the same partial ordering. Queries run one thread per query point on the GPU with a
+// the middle of a range is the node, split on the axis of largest extent, built on the GPU
+// (kdtree.cu), or on the host with the same partial ordering. Queries run one thread per query point on the GPU with a
 // bounded max-heap of the k best candidates in local memory.
 #include <cub/device/device_radix_sort.cuh>
 
@@ -327,6 +327,41 @@ void kd_build(std::vector<KdElem> &e, std::vector<uint8_t> &axis, size_t left, s
     }
 }
 
+// The host build of a map's tree, uploaded to pos and aux.
+int kd_build_host(rt_photon_map *m, DevBuf &pos, DevBuf &aux)
+{
+    cudaStream_t st = m->ctx->stream;
+    const uint64_t n = m->n;
+    std::vector<rt_photon> ph(n);
+    if (n) {
+        RTB_CUDA(cudaMemcpyAsync(ph.data(), m->photons.ptr, n * sizeof(rt_photon), cudaMemcpyDeviceToHost, st));
+        RTB_CUDA(cudaStreamSynchronize(st));
+    }
+    std::vector<KdElem> e(n);
+    for (uint64_t i = 0; i < n; i++) {
+        e[i].p[0] = ph[i].pos[0];
+        e[i].p[1] = ph[i].pos[1];
+        e[i].p[2] = ph[i].pos[2];
+        e[i].shape = ph[i].shape_id;
+        e[i].idx = (uint32_t)i;
+    }
+    std::vector<uint8_t> axis(n, 0);
+    kd_build(e, axis, 0, n, 0);
+    std::vector<float4> np(n);
+    std::vector<int2> na(n);
+    for (uint64_t i = 0; i < n; i++) {
+        uint32_t ax = axis[i];
+        float axf;
+        std::memcpy(&axf, &ax, 4);
+        np[i] = make_float4(e[i].p[0], e[i].p[1], e[i].p[2], axf);
+        na[i] = make_int2(e[i].shape, (int)e[i].idx);
+    }
+    RTB_CHECK(pos.upload(np.data(), n * sizeof(float4), st));
+    RTB_CHECK(aux.upload(na.data(), n * sizeof(int2), st));
+    RTB_CUDA(cudaStreamSynchronize(st));
+    return RT_OK;
+}
+
 }  // namespace
 }  // namespace rtb
 
@@ -392,6 +427,7 @@ int rt_photon_map_from_points(rt_context *ctx, const float *pos, const int32_t *
     rt_photon_map *m = new rt_photon_map();
     m->ctx = ctx;
     m->n = n;
+    m->points = true;
     int st = m->photons.upload(ph.data(), n * sizeof(rt_photon), ctx->stream);
     if (st != RT_OK) {
         delete m;
@@ -407,34 +443,31 @@ int rt_photon_map_build(rt_photon_map *m)
     RTB_CUDA(cudaSetDevice(m->ctx->device));
     cudaStream_t st = m->ctx->stream;
     const uint64_t n = m->n;
-    std::vector<rt_photon> ph(n);
-    if (n) {
-        RTB_CUDA(cudaMemcpyAsync(ph.data(), m->photons.ptr, n * sizeof(rt_photon), cudaMemcpyDeviceToHost, st));
-        RTB_CUDA(cudaStreamSynchronize(st));
-    }
-    std::vector<KdElem> e(n);
-    for (uint64_t i = 0; i < n; i++) {
-        e[i].p[0] = ph[i].pos[0];
-        e[i].p[1] = ph[i].pos[1];
-        e[i].p[2] = ph[i].pos[2];
-        e[i].shape = ph[i].shape_id;
-        e[i].idx = (uint32_t)i;
-    }
-    std::vector<uint8_t> axis(n, 0);
-    kd_build(e, axis, 0, n, 0);
-    std::vector<float4> np(n);
-    std::vector<int2> na(n);
-    for (uint64_t i = 0; i < n; i++) {
-        uint32_t ax = axis[i];
-        float axf;
-        std::memcpy(&axf, &ax, 4);
-        np[i] = make_float4(e[i].p[0], e[i].p[1], e[i].p[2], axf);
-        na[i] = make_int2(e[i].shape, (int)e[i].idx);
-    }
-    RTB_CHECK(m->node_pos.upload(np.data(), n * sizeof(float4), st));
-    RTB_CHECK(m->node_aux.upload(na.data(), n * sizeof(int2), st));
+    std::lock_guard<std::mutex> lk(m->exact_mu);
+    m->exact = m->host_order = false;
+    RTB_CHECK(m->node_pos.reserve(std::max<uint64_t>(n, 1) * sizeof(float4)));
+    RTB_CHECK(m->node_aux.reserve(std::max<uint64_t>(n, 1) * sizeof(int2)));
     RTB_CHECK(m->node_pw.reserve(std::max<uint64_t>(n, 1) * sizeof(float4)));
     RTB_CHECK(m->node_dir.reserve(std::max<uint64_t>(n, 1) * sizeof(float4)));
+    // The host build where the device build gives no valid tree or finds no room for its workspace
+    // (about 100 bytes per photon), and for a point set with equal coordinates, whose queries need
+    // the host's order.
+    uint32_t report = kKdNotFinite;
+    if (n <= kKdDeviceMax) {
+        const int rc = kd_build_device(m->photons.as<rt_photon>(), n, m->node_pos.as<float4>(), m->node_aux.as<int2>(),
+                                       &report, st);
+        if (rc == RT_ERR_OOM) {
+            (void)cudaGetLastError();
+            report = kKdNotFinite;
+        } else if (rc != RT_OK) {
+            return rc;
+        }
+    }
+    if ((report & kKdNotFinite) || (m->points && (report & kKdTies))) {
+        RTB_CHECK(kd_build_host(m, m->node_pos, m->node_aux));
+        report = 0;
+    }
+    m->host_order = report == 0;
     if (n) {
         k_tree_attrs<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(m->node_aux.as<int2>(), m->photons.as<rt_photon>(), n,
                                                                  m->node_pw.as<float4>(), m->node_dir.as<float4>());
@@ -453,8 +486,18 @@ int rt_photon_knn(rt_photon_map *m, const float *q, const int32_t *qs, uint64_t 
     if (k == 0 || k > kKnnMaxK) return fail(RT_ERR_INVALID, "rt_photon_knn: k must be in [1, 128]");
     if (nq == 0) return RT_OK;
     RTB_CUDA(cudaSetDevice(m->ctx->device));
+    const DevBuf *pos = &m->node_pos, *aux = &m->node_aux;
+    {
+        std::lock_guard<std::mutex> lk(m->exact_mu);
+        if (!m->host_order) {
+            if (!m->exact) RTB_CHECK(kd_build_host(m, m->exact_pos, m->exact_aux));
+            m->exact = true;
+            pos = &m->exact_pos;
+            aux = &m->exact_aux;
+        }
+    }
     const uint64_t blocks = (nq + 127) / 128;
-    k_knn<<<(unsigned)blocks, 128, 0, m->ctx->stream>>>(m->node_pos.as<float4>(), m->node_aux.as<int2>(),
+    k_knn<<<(unsigned)blocks, 128, 0, m->ctx->stream>>>(pos->as<float4>(), aux->as<int2>(),
                                                         (uint32_t)m->n, q, qs, nq, k, radius, out_idx, out_dist,
                                                         out_count);
     RTB_CUDA(cudaGetLastError());

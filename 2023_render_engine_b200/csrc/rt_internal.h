@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "../../include/rt_b200.h"
@@ -61,6 +62,13 @@ struct DevBuf {
     template <typename T>
     T *as() const { return static_cast<T *>(ptr); }
 };
+
+// kd-tree of n photons on the GPU (kdtree.cu). report: kKdTies where the tree may differ from the
+// host build's at equal coordinates, kKdNotFinite where it is not valid at all. Returns when done.
+constexpr uint32_t kKdTies = 1u, kKdNotFinite = 2u;
+constexpr uint64_t kKdDeviceMax = 1ull << 28;
+int kd_build_device(const rt_photon *photons, uint64_t n, float4 *node_pos, int2 *node_aux, uint32_t *report,
+                    cudaStream_t st);
 
 // Launch sizes derived from occupancy and per-kernel function attributes are properties of
 // a device, not of the process: each is cached per CUDA device id.
@@ -274,6 +282,13 @@ struct rt_photon_map {
     rtb::DevBuf node_pw;   // float4 per tree slot: power rgb, cos(normal, -direction)
     rtb::DevBuf node_dir;  // float4 per tree slot: arrival direction xyz, 0
     bool built = false;
+    bool points = false;      // rt_photon_map_from_points: made for nearest-neighbour queries
+    bool host_order = false;  // the tree is the host build's, equal coordinates included
+    // the host build's node_pos and node_aux where the tree above is not (made by the first
+    // rt_photon_knn, whose answers at equal distances depend on them)
+    rtb::DevBuf exact_pos, exact_aux;
+    bool exact = false;
+    std::mutex exact_mu;
 };
 
 struct rt_guide {
