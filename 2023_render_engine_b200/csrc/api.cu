@@ -6,6 +6,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "bvh_common.cuh"
 #include "rt_internal.h"
@@ -73,12 +74,73 @@ unsigned device_mem_mib()
     return m;
 }
 
+namespace {
+// Live contexts with a pool, for trim_pools.
+std::mutex g_pools_mu;
+std::vector<rt_context *> g_pools;
+
+void trim_pools()
+{
+    std::lock_guard<std::mutex> lk(g_pools_mu);
+    for (rt_context *c : g_pools) {
+        cudaStreamSynchronize(c->pool_stream);
+        cudaMemPoolTrimTo(c->pool, 0);
+    }
+}
+
+// A context's pool; without one (no support, no memory) its buffers use cudaMalloc.
+void create_pool(rt_context *c)
+{
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = c->device;
+    uint64_t keep = ((uint64_t)device_mem_mib() << 20) / 64;
+    if (cudaStreamCreateWithFlags(&c->pool_stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMemPoolCreate(&c->pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        (void)cudaGetLastError();
+        if (c->pool) cudaMemPoolDestroy(c->pool);
+        c->pool = nullptr;
+        return;
+    }
+    std::lock_guard<std::mutex> lk(g_pools_mu);
+    g_pools.push_back(c);
+}
+
+void destroy_pool(rt_context *c)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_pools_mu);
+        g_pools.erase(std::remove(g_pools.begin(), g_pools.end(), c), g_pools.end());
+    }
+    if (c->pool) cudaMemPoolDestroy(c->pool);  // its memory is released with the last allocation
+    if (c->pool_stream) cudaStreamDestroy(c->pool_stream);
+}
+}  // namespace
+
 int DevBuf::reserve(size_t n)
 {
     if (n <= bytes && ptr) return RT_OK;
     release();
     if (n == 0) return RT_OK;
+    if (ctx && ctx->pool) {
+        cudaError_t e = cudaMallocFromPoolAsync(&ptr, n, ctx->pool, ctx->pool_stream);
+        if (e == cudaSuccess) {
+            pooled = true;
+            bytes = n;
+            const int rc = cuda_status(cudaStreamSynchronize(ctx->pool_stream), "cudaMallocFromPoolAsync");
+            if (rc != RT_OK) release();
+            return rc;
+        }
+        (void)cudaGetLastError();
+    }
     cudaError_t e = cudaMalloc(&ptr, n);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        trim_pools();
+        e = cudaMalloc(&ptr, n);
+    }
     if (e != cudaSuccess) {
         ptr = nullptr;
         return cuda_status(e, "cudaMalloc");
@@ -97,9 +159,16 @@ int DevBuf::upload(const void *src, size_t n, cudaStream_t s)
 
 void DevBuf::release()
 {
-    if (ptr) cudaFree(ptr);
+    if (ptr && pooled) {
+        cudaSetDevice(ctx->device);
+        cudaDeviceSynchronize();
+        cudaFreeAsync(ptr, ctx->pool_stream);
+    } else if (ptr) {
+        cudaFree(ptr);
+    }
     ptr = nullptr;
     bytes = 0;
+    pooled = false;
 }
 
 // Status word written by kernels -> rt_status.
@@ -179,6 +248,7 @@ int rt_context_create(int device, rt_context **out)
         return cuda_status(e, "cudaStreamCreate");
     }
     c->own_stream = true;
+    create_pool(c);
     *out = c;
     return RT_OK;
 }
@@ -188,6 +258,7 @@ int rt_context_destroy(rt_context *ctx)
     if (!ctx) return RT_OK;
     cudaSetDevice(ctx->device);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
+    destroy_pool(ctx);
     delete ctx;
     return RT_OK;
 }
@@ -217,6 +288,11 @@ int rt_scene_create(rt_context *ctx, rt_scene **out)
     if (!ctx || !out) return fail(RT_ERR_INVALID, "rt_scene_create: null argument");
     rt_scene *s = new rt_scene();
     s->ctx = ctx;
+    for (DevBuf *b : {&s->d_nodes, &s->d_tris, &s->d_leafpos, &s->d_ref_boxes, &s->d_ref_sorted, &s->d_ref_pos,
+                      &s->d_spheres, &s->scratch.counters, &s->h2d_rays, &s->d2h_hits, &s->any_hits, &s->d_mats,
+                      &s->d_tri_mat, &s->d_tri_shape, &s->d_tri_nidx, &s->d_normals, &s->d_emit_tri, &s->d_emit_cdf,
+                      &s->d_plights, &s->d_rec_mat, &s->d_tri_transp, &s->d_mat_transp})
+        b->ctx = ctx;
     *out = s;
     return RT_OK;
 }
@@ -242,27 +318,29 @@ int rt_scene_add_mesh(rt_scene *s, const float *xyz, uint32_t nv, const uint32_t
     if (!s || (!xyz && nv) || (!idx && ntri)) return fail(RT_ERR_INVALID, "rt_scene_add_mesh: null argument");
     if (s->merged) return fail(RT_ERR_UNSUPPORTED, "rt_scene_add_mesh: not available on a merged scene");
     if ((normals == nullptr) != (nidx == nullptr)) return fail(RT_ERR_INVALID, "rt_scene_add_mesh: normals need nidx");
-    uint64_t base = s->tri9.size() / 9;
+    const uint64_t base = s->tri9.size() / 9;
     if (base + ntri >= 0x40000000ull) return fail(RT_ERR_CAPACITY, "rt_scene_add_mesh: more than 2^30 triangles");
-    for (uint64_t i = 0; i < 3ull * ntri; i++) {
-        if (idx[i] >= nv) return fail(RT_ERR_INVALID, "rt_scene_add_mesh: vertex index out of range");
-        if (nidx && nidx[i] >= nn) return fail(RT_ERR_INVALID, "rt_scene_add_mesh: normal index out of range");
-    }
-    uint32_t nbase = (uint32_t)(s->normals.size() / 3);
+    const uint64_t n3 = 3ull * ntri;
+    uint32_t vmax = 0, nmax = 0;
+    for (uint64_t i = 0; i < n3; i++) vmax = std::max(vmax, idx[i]);
+    for (uint64_t i = 0; nidx && i < n3; i++) nmax = std::max(nmax, nidx[i]);
+    if (ntri && vmax >= nv) return fail(RT_ERR_INVALID, "rt_scene_add_mesh: vertex index out of range");
+    if (ntri && nidx && nmax >= nn) return fail(RT_ERR_INVALID, "rt_scene_add_mesh: normal index out of range");
+    const uint32_t nbase = (uint32_t)(s->normals.size() / 3);
     if (normals) s->normals.insert(s->normals.end(), normals, normals + 3ull * nn);
-    s->tri9.reserve(s->tri9.size() + 9ull * ntri);
-    for (uint32_t t = 0; t < ntri; t++) {
-        for (int k = 0; k < 3; k++) {
-            const float *p = xyz + 3ull * idx[3ull * t + k];
-            s->tri9.push_back(p[0]);
-            s->tri9.push_back(p[1]);
-            s->tri9.push_back(p[2]);
-            s->tri_normal_idx.push_back(nidx ? (int32_t)(nbase + nidx[3ull * t + k]) : -1);
-        }
-        s->tri_material.push_back(material);
-        s->tri_shape.push_back(shape_id);
-        s->tri_transparent.push_back(transparent ? 1 : 0);
+    s->tri9.resize(s->tri9.size() + 9ull * ntri);
+    float *out = s->tri9.data() + 9 * base;
+    for (uint64_t i = 0; i < n3; i++) {
+        const float *p = xyz + 3ull * idx[i];
+        out[3 * i] = p[0];
+        out[3 * i + 1] = p[1];
+        out[3 * i + 2] = p[2];
     }
+    s->tri_normal_idx.resize(3 * (base + ntri), -1);
+    for (uint64_t i = 0; nidx && i < n3; i++) s->tri_normal_idx[3 * base + i] = (int32_t)(nbase + nidx[i]);
+    s->tri_material.resize(base + ntri, material);
+    s->tri_shape.resize(base + ntri, shape_id);
+    s->tri_transparent.resize(base + ntri, transparent ? 1 : 0);
     if (first_tri) *first_tri = (uint32_t)base;
     s->committed = false;
     return RT_OK;

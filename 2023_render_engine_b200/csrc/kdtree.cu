@@ -9,8 +9,8 @@
 // left / right half") until they fit a block, which finishes its range in shared memory.
 //
 // What bounds it: launches and latency; each level moves some 50 bytes per point. The host's
-// recursion over std::nth_element took 40 ms for 500,000 photons on one core, after a copy of the
-// photons to the host; this build 0.9 ms.
+// recursion over std::nth_element took 40 ms for 413,000 photons on one core, with the copies to the
+// host and back; this build 0.6 ms.
 //
 // Equal coordinates: the tree is the host's, bit for bit, unless a node's coordinate also occurs
 // next to it in its range. Which of the equal elements becomes the node, and on which side the
@@ -258,9 +258,10 @@ unsigned blocks_for(uint64_t n) { return (unsigned)((n + kT - 1) / kT); }
 
 }  // namespace
 
-int kd_build_device(const rt_photon *photons, uint64_t n64, float4 *node_pos, int2 *node_aux, uint32_t *report,
-                    cudaStream_t st)
+int kd_build_device(rt_context *ctx, const rt_photon *photons, uint64_t n64, float4 *node_pos, int2 *node_aux,
+                    uint32_t *report)
 {
+    cudaStream_t st = ctx->stream;
     *report = 0;
     if (n64 == 0) return RT_OK;
     if (n64 > kKdDeviceMax) return fail(RT_ERR_CAPACITY, "kd_build_device: too many points");
@@ -273,7 +274,7 @@ int kd_build_device(const rt_photon *photons, uint64_t n64, float4 *node_pos, in
     uint64_t *none64 = nullptr;
     RTB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, none, none, none, none, (int)n, 0, 32, st));
     if (level) RTB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, none64, none64, (int64_t)n3, st));
-    DevBuf work;
+    DevBuf work(ctx);
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t o = at;

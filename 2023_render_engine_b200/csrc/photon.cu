@@ -327,6 +327,13 @@ void kd_build(std::vector<KdElem> &e, std::vector<uint8_t> &axis, size_t left, s
     }
 }
 
+void map_context(rt_photon_map *m, rt_context *ctx)
+{
+    m->ctx = ctx;
+    for (DevBuf *b : {&m->photons, &m->node_pos, &m->node_aux, &m->node_pw, &m->node_dir, &m->exact_pos, &m->exact_aux})
+        b->ctx = ctx;
+}
+
 // The host build of a map's tree, uploaded to pos and aux.
 int kd_build_host(rt_photon_map *m, DevBuf &pos, DevBuf &aux)
 {
@@ -425,7 +432,7 @@ int rt_photon_map_from_points(rt_context *ctx, const float *pos, const int32_t *
         ph[i].path = (uint32_t)i;
     }
     rt_photon_map *m = new rt_photon_map();
-    m->ctx = ctx;
+    map_context(m, ctx);
     m->n = n;
     m->points = true;
     int st = m->photons.upload(ph.data(), n * sizeof(rt_photon), ctx->stream);
@@ -454,8 +461,8 @@ int rt_photon_map_build(rt_photon_map *m)
     // the host's order.
     uint32_t report = kKdNotFinite;
     if (n <= kKdDeviceMax) {
-        const int rc = kd_build_device(m->photons.as<rt_photon>(), n, m->node_pos.as<float4>(), m->node_aux.as<int2>(),
-                                       &report, st);
+        const int rc = kd_build_device(m->ctx, m->photons.as<rt_photon>(), n, m->node_pos.as<float4>(),
+                                       m->node_aux.as<int2>(), &report);
         if (rc == RT_ERR_OOM) {
             (void)cudaGetLastError();
             report = kKdNotFinite;
@@ -565,7 +572,9 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
     }
     if (!(total > 0)) return fail(RT_ERR_STATE, "rt_photons_trace: lights have no power");
     const uint32_t cap = (uint32_t)n;
-    DevBuf rays[2], beta[2], carry[2], rng[2], hits, sel, perl, dpow, cnt;  // freed on return
+    rt_context *ctx = s->ctx;  // buffers of its pool, freed on return
+    DevBuf rays[2]{DevBuf(ctx), DevBuf(ctx)}, beta[2]{DevBuf(ctx), DevBuf(ctx)}, carry[2]{DevBuf(ctx), DevBuf(ctx)},
+        rng[2]{DevBuf(ctx), DevBuf(ctx)}, hits(ctx), sel(ctx), perl(ctx), dpow(ctx), cnt(ctx);
     for (int b = 0; b < 2; b++) {
         RTB_CHECK(rays[b].reserve(32ull * cap));
         RTB_CHECK(beta[b].reserve(16ull * cap));
@@ -585,7 +594,7 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
     RTB_CUDA(cudaEventCreate(&e1));
     uint64_t stored = 0, rays_traced = 0;
     for (int attempt = 0; attempt < 2; attempt++) {
-        DevBuf store, keys;
+        DevBuf store(ctx), keys(ctx);
         RTB_CHECK(store.reserve(sizeof(rt_photon) * store_cap));
         RTB_CHECK(keys.reserve(8 * store_cap));
         PhotonBuffers pb;
@@ -636,7 +645,7 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
             continue;
         }
         // order by (path, depth)
-        DevBuf keys_out, idx_in, idx_out, tmp, sorted;
+        DevBuf keys_out(ctx), idx_in(ctx), idx_out(ctx), tmp(ctx), sorted(ctx);
         RTB_CHECK(keys_out.reserve(8 * std::max<uint64_t>(stored, 1)));
         RTB_CHECK(idx_in.reserve(4 * std::max<uint64_t>(stored, 1)));
         RTB_CHECK(idx_out.reserve(4 * std::max<uint64_t>(stored, 1)));
@@ -659,7 +668,7 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
         RTB_CUDA(cudaEventRecord(e1, st));
         RTB_CUDA(cudaEventSynchronize(e1));
         m = new rt_photon_map();
-        m->ctx = s->ctx;
+        map_context(m, ctx);
         m->n = stored;
         m->photons = std::move(sorted);
         break;
