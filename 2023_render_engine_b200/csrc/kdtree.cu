@@ -15,7 +15,7 @@
 // Equal coordinates: the tree is the host's, bit for bit, unless a node's coordinate also occurs
 // next to it in its range. Which of the equal elements becomes the node, and on which side the
 // others go, is then a matter of std::nth_element's internals there, and of the elements'
-// indices here; the build reports it (kKdTies).
+// indices here; the build reports it (kKdTies) and counts such nodes.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -88,7 +88,7 @@ __device__ __forceinline__ int kd_axis(const float lo[3], const float hi[3])
 }
 
 // Side of every element of its range: 0 left of the node, 1 the node, 2 right. The nodes get their
-// axis.
+// axis. report: kKdNotFinite, number of nodes with an equal coordinate beside them.
 __global__ void __launch_bounds__(kT) k_kd_side(const float *__restrict__ xyz, const uint32_t *__restrict__ order, uint32_t n,
                                                 int level, uint8_t *__restrict__ side, uint8_t *__restrict__ axis,
                                                 uint32_t *__restrict__ report)
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kT) k_kd_side(const float *__restrict__ xyz, c
         const float *x = xyz + (size_t)ax * n;
         const float c = x[o[m]];
         axis[m] = r - l > 1 ? (uint8_t)ax : 0;
-        if ((m > l && x[o[m - 1]] == c) || (m + 1 < r && x[o[m + 1]] == c)) atomicOr(report, kKdTies);
+        if ((m > l && x[o[m - 1]] == c) || (m + 1 < r && x[o[m + 1]] == c)) atomicAdd(report + 1, 1u);
     }
 }
 
@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(kLocal) k_kd_local(const float *__restrict__ x
     sums[0][t] = id;
     __syncthreads();
     if (on) out[l0 + t] = sums[0][ord[b][0][t]];
-    if (__syncthreads_or(ties) && t == 0) atomicOr(report, kKdTies);
+    const int all = __syncthreads_count(ties);
+    if (all && t == 0) atomicAdd(report + 1, (uint32_t)all);
 }
 
 // The nodes in tree order: position and axis, shape and photon index.
@@ -259,10 +260,10 @@ unsigned blocks_for(uint64_t n) { return (unsigned)((n + kT - 1) / kT); }
 }  // namespace
 
 int kd_build_device(rt_context *ctx, const rt_photon *photons, uint64_t n64, float4 *node_pos, int2 *node_aux,
-                    uint32_t *report)
+                    uint32_t *report, uint32_t *ties)
 {
     cudaStream_t st = ctx->stream;
-    *report = 0;
+    *report = *ties = 0;
     if (n64 == 0) return RT_OK;
     if (n64 > kKdDeviceMax) return fail(RT_ERR_CAPACITY, "kd_build_device: too many points");
     const uint32_t n = (uint32_t)n64;
@@ -284,7 +285,7 @@ int kd_build_device(rt_context *ctx, const rt_photon *photons, uint64_t n64, flo
     const size_t o_xyz = take(4 * n3), o_keys = take(4 * n3), o_keys2 = take(4 * n64), o_ids = take(4 * n64),
                  o_ord = take(4 * n3), o_ord2 = take(4 * n3), o_side = take(n64), o_axis = take(n64),
                  o_flags = take(level ? 8 * n3 : 0), o_sums = take(level ? 8 * n3 : 0),
-                 o_tmp = take(std::max(sort_bytes, scan_bytes)), o_rep = take(4);
+                 o_tmp = take(std::max(sort_bytes, scan_bytes)), o_rep = take(8);
     RTB_CHECK(work.reserve(at));
     char *w = work.as<char>();
     float *xyz = reinterpret_cast<float *>(w + o_xyz);
@@ -293,7 +294,7 @@ int kd_build_device(rt_context *ctx, const rt_photon *photons, uint64_t n64, flo
              *ord2 = reinterpret_cast<uint32_t *>(w + o_ord2), *rep = reinterpret_cast<uint32_t *>(w + o_rep);
     uint8_t *side = reinterpret_cast<uint8_t *>(w + o_side), *axis = reinterpret_cast<uint8_t *>(w + o_axis);
     uint64_t *flags = reinterpret_cast<uint64_t *>(w + o_flags), *sums = reinterpret_cast<uint64_t *>(w + o_sums);
-    RTB_CUDA(cudaMemsetAsync(rep, 0, 4, st));
+    RTB_CUDA(cudaMemsetAsync(rep, 0, 8, st));
     k_kd_keys<<<blocks_for(n), kT, 0, st>>>(photons, n, xyz, keys, ids, rep);
     RTB_CUDA(cudaGetLastError());
     for (int a = 0; a < 3; a++)  // stable: equal coordinates in index order
@@ -312,8 +313,11 @@ int kd_build_device(rt_context *ctx, const rt_photon *photons, uint64_t n64, flo
     k_kd_local<<<1u << level, kLocal, 0, st>>>(xyz, ord, n, level, keys2, ord2, axis, rep);
     k_kd_nodes<<<blocks_for(n), kT, 0, st>>>(photons, ord2, axis, n, node_pos, node_aux);
     RTB_CUDA(cudaGetLastError());
-    RTB_CUDA(cudaMemcpyAsync(report, rep, 4, cudaMemcpyDeviceToHost, st));
+    uint32_t found[2];
+    RTB_CUDA(cudaMemcpyAsync(found, rep, 8, cudaMemcpyDeviceToHost, st));
     RTB_CUDA(cudaStreamSynchronize(st));
+    *report = found[0] | (found[1] ? kKdTies : 0u);
+    *ties = found[1];
     return RT_OK;
 }
 

@@ -9,8 +9,9 @@
 //
 // The kd-tree is the reference's implicit balanced tree (kdtree.h:78-108): the element at
 // the middle of a range is the node, split on the axis of largest extent, built on the GPU
-// (kdtree.cu), or on the host with the same partial ordering. Queries run one thread per query point on the GPU with a
-// bounded max-heap of the k best candidates in local memory.
+// (kdtree.cu), or on the host with the same partial ordering. Nearest-neighbour queries run on eight lanes each
+// (k_knn_group), or on one thread with a bounded max-heap of the k best candidates in local memory
+// (k_knn).
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
@@ -216,10 +217,87 @@ __global__ void __launch_bounds__(128) k_knn(const float4 *__restrict__ node_pos
     out_count[qi] = cnt;
 }
 
-// One warp per query (the render's gather kernel uses the same warp functions).
+// The reference's own query for one thread, its heap in hd / hi (k entries).
+__device__ __noinline__ static uint32_t knn_serial(const float4 *node_pos, const int2 *node_aux, uint32_t n, float qx,
+                                                   float qy, float qz, int32_t sid, uint32_t k, float radius, float *hd,
+                                                   int32_t *hi)
+{
+    const uint32_t cnt = knn_query(node_pos, node_aux, n, qx, qy, qz, sid, k, radius, hd, hi);
+    heap_to_sorted(hd, hi, cnt);
+    return cnt;
+}
+
+// k-nearest queries, kGroup lanes each: group_knn finds the candidates, each lane then ranks its own
+// by counting. Where no two distances are equal that is the only answer; otherwise the order, and at
+// the k-th distance the choice, are those of the reference's heap, which one lane then runs on the
+// host's tree (exact_pos, exact_aux; a few queries in ten thousand on scattered points).
+// 500,000 points, 200,003 queries, k = 50: 3.10 ms one query per thread, 1.35 ms so.
 constexpr int kQueryBlock = 128;
-// Resident blocks per SM of the query kernels (64 registers): k_density 54 / 64 / 79 M queries/s
-// and k_subsurface 4.5 / 4.5 / 5.1 M/s for no bound (80 registers) / 6 / 8, on a 2.1M-photon map.
+__global__ void __launch_bounds__(kQueryBlock) k_knn_group(const float4 *__restrict__ node_pos,
+                                                           const int2 *__restrict__ node_aux,
+                                                           const float4 *__restrict__ exact_pos,
+                                                           const int2 *__restrict__ exact_aux, uint32_t n,
+                                                           const float *__restrict__ queries,
+                                                           const int32_t *__restrict__ qshape, uint64_t nq, uint32_t k,
+                                                           float radius, float radius2, int32_t *__restrict__ out_idx,
+                                                           float *__restrict__ out_dist, uint32_t *__restrict__ out_count)
+{
+    extern __shared__ __align__(16) uint32_t knn_smem[];
+    const KnnGroup g = knn_group(knn_smem + (threadIdx.x >> 5) * 4 * knn_words(k), k);
+    const uint64_t qi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
+    const uint32_t lane = threadIdx.x & (kGroup - 1u), shift = threadIdx.x & 31u & ~(kGroup - 1u);
+    const bool on = qi < nq;
+    const float qx = on ? queries[3 * qi] : 0.f, qy = on ? queries[3 * qi + 1] : 0.f, qz = on ? queries[3 * qi + 2] : 0.f;
+    const int32_t sid = on && qshape ? qshape[qi] : -1;
+    float bound;
+    const uint32_t cnt = group_knn(node_pos, node_aux, n, qx, qy, qz, sid, k, radius2, kKnnSlack, on, g, bound);
+    uint32_t ranks = 0;
+    bool tied = false;
+    for (uint32_t e = lane; e < cnt; e += kGroup) {
+        const float d2 = g.kd[e];
+        tied |= cnt >= k && bound < radius2 && __float_as_int(bound) - __float_as_int(d2) < kRootSteps;
+        g.kd[e] = __fsqrt_rn(d2);
+    }
+    if (lane < 4) g.kd[cnt + lane] = INFINITY;  // the last step of the loop below
+    __syncwarp();
+    for (uint32_t e = lane; e < cnt; e += kGroup) {
+        const float d = g.kd[e];
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < cnt; j += 4) {
+            const float4 x = *reinterpret_cast<const float4 *>(g.kd + j);
+            rank += (x.x < d) + (x.y < d) + (x.z < d) + (x.w < d);
+        }
+        ranks += rank;
+        if (rank < k) {
+            out_idx[qi * k + rank] = __ldg(&node_aux[g.ki[e]].y);
+            if (out_dist) out_dist[qi * k + rank] = d;
+        }
+    }
+    __syncwarp();
+    // equal distances share a rank
+    tied |= group_sum(ranks) != cnt * (cnt - 1) / 2;
+    tied = ((__ballot_sync(kFullMask, tied) >> shift) & 0xFFu) != 0;
+    if (!on) return;
+    const uint32_t found = min(cnt, k);
+    if (lane == 0) {
+        out_count[qi] = found;
+        if (tied) {
+            int32_t *hi = reinterpret_cast<int32_t *>(g.ki);
+            knn_serial(exact_pos, exact_aux, n, qx, qy, qz, sid, k, radius, g.kd, hi);
+            for (uint32_t j = 0; j < found; j++) {
+                out_idx[qi * k + j] = hi[j];
+                if (out_dist) out_dist[qi * k + j] = g.kd[j];
+            }
+        }
+    }
+    for (uint32_t j = found + lane; j < k; j += kGroup) {
+        out_idx[qi * k + j] = -1;
+        if (out_dist) out_dist[qi * k + j] = INFINITY;
+    }
+}
+
+// Resident blocks per SM of the subsurface kernel (64 registers): 4.5 / 4.5 / 5.1 M queries/s for no
+// bound (80 registers) / 6 / 8, on a 2.1M-photon map.
 #ifndef RTB_QUERY_MIN_BLOCKS
 #define RTB_QUERY_MIN_BLOCKS 8
 #endif
@@ -244,20 +322,23 @@ __global__ void k_tree_attrs(const int2 *__restrict__ node_aux, const rt_photon 
 // Scene::combinePhotonContributions (Scene.cu:607-635) per query: the k nearest photons on
 // the same shape within radius, sum of power * lightScattered(-photon direction), divided by
 // pi * (largest neighbour distance)^2.
-__global__ void __launch_bounds__(kQueryBlock, RTB_QUERY_MIN_BLOCKS) k_density(PhotonTree tree, rt_material mat, const float *__restrict__ pts,
-                                                         const float *__restrict__ nrm, const float *__restrict__ wo,
-                                                         const int32_t *__restrict__ shape, uint64_t nq, uint32_t k,
-                                                         float radius, float *__restrict__ out)
+__global__ void __launch_bounds__(kQueryBlock, kGatherBlocks) k_density(PhotonTree tree, rt_material mat,
+                                                                       const float *__restrict__ pts,
+                                                                       const float *__restrict__ nrm,
+                                                                       const float *__restrict__ wo,
+                                                                       const int32_t *__restrict__ shape, uint64_t nq,
+                                                                       uint32_t k, float radius2, float *__restrict__ out)
 {
-    __shared__ PhotonWarpScratch scratch[kQueryBlock / 32];
-    const uint64_t qi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (qi >= nq) return;  // warp-uniform
-    V3 p = v3(pts[3 * qi], pts[3 * qi + 1], pts[3 * qi + 2]);
-    V3 nn = normalize(v3(nrm[3 * qi], nrm[3 * qi + 1], nrm[3 * qi + 2]));
-    V3 w = v3(wo[3 * qi], wo[3 * qi + 1], wo[3 * qi + 2]);
-    V3 c = warp_photon_density(tree, load_bsdf(mat), p, nn, w, shape ? shape[qi] : -1, k, radius, true,
-                               scratch[threadIdx.x >> 5]);
-    if ((threadIdx.x & 31u) == 0) {
+    extern __shared__ __align__(16) uint32_t knn_smem[];
+    const KnnGroup g = knn_group(knn_smem + (threadIdx.x >> 5) * 4 * knn_words(k), k);
+    const uint64_t qi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
+    const bool on = qi < nq;
+    const uint64_t i = on ? qi : nq - 1;
+    V3 p = v3(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
+    V3 nn = normalize(v3(nrm[3 * i], nrm[3 * i + 1], nrm[3 * i + 2]));
+    V3 w = v3(wo[3 * i], wo[3 * i + 1], wo[3 * i + 2]);
+    V3 c = group_photon_density(tree, load_bsdf(mat), p, nn, w, shape ? shape[i] : -1, k, radius2, true, on, g);
+    if (on && (threadIdx.x & (kGroup - 1u)) == 0) {
         out[3 * qi] = c.x;
         out[3 * qi + 1] = c.y;
         out[3 * qi + 2] = c.z;
@@ -459,10 +540,10 @@ int rt_photon_map_build(rt_photon_map *m)
     // The host build where the device build gives no valid tree or finds no room for its workspace
     // (about 100 bytes per photon), and for a point set with equal coordinates, whose queries need
     // the host's order.
-    uint32_t report = kKdNotFinite;
+    uint32_t report = kKdNotFinite, ties = 0;
     if (n <= kKdDeviceMax) {
         const int rc = kd_build_device(m->ctx, m->photons.as<rt_photon>(), n, m->node_pos.as<float4>(),
-                                       m->node_aux.as<int2>(), &report);
+                                       m->node_aux.as<int2>(), &report, &ties);
         if (rc == RT_ERR_OOM) {
             (void)cudaGetLastError();
             report = kKdNotFinite;
@@ -470,6 +551,9 @@ int rt_photon_map_build(rt_photon_map *m)
             return rc;
         }
     }
+    // A query with equal distances is answered a second time, by one lane: not where they are the rule
+    // (lattices).
+    m->scattered = !(report & kKdNotFinite) && ties <= n / 64;
     if ((report & kKdNotFinite) || (m->points && (report & kKdTies))) {
         RTB_CHECK(kd_build_host(m, m->node_pos, m->node_aux));
         report = 0;
@@ -503,10 +587,16 @@ int rt_photon_knn(rt_photon_map *m, const float *q, const int32_t *qs, uint64_t 
             aux = &m->exact_aux;
         }
     }
-    const uint64_t blocks = (nq + 127) / 128;
-    k_knn<<<(unsigned)blocks, 128, 0, m->ctx->stream>>>(pos->as<float4>(), aux->as<int2>(),
-                                                        (uint32_t)m->n, q, qs, nq, k, radius, out_idx, out_dist,
-                                                        out_count);
+    if (m->scattered) {
+        const uint64_t blocks = (nq * kGroup + kQueryBlock - 1) / kQueryBlock;
+        k_knn_group<<<(unsigned)blocks, kQueryBlock, kQueryBlock / kGroup * 4 * knn_words(k), m->ctx->stream>>>(
+            m->node_pos.as<float4>(), m->node_aux.as<int2>(), pos->as<float4>(), aux->as<int2>(), (uint32_t)m->n, q, qs, nq,
+            k, radius, radius_squared(radius), out_idx, out_dist, out_count);
+    } else {
+        const uint64_t blocks = (nq + 127) / 128;
+        k_knn<<<(unsigned)blocks, 128, 0, m->ctx->stream>>>(pos->as<float4>(), aux->as<int2>(), (uint32_t)m->n, q, qs, nq,
+                                                            k, radius, out_idx, out_dist, out_count);
+    }
     RTB_CUDA(cudaGetLastError());
     RTB_CUDA(cudaStreamSynchronize(m->ctx->stream));
     return RT_OK;
@@ -541,9 +631,9 @@ int rt_photon_density(rt_photon_map *m, const rt_material *mat, const float *pts
     if (nq == 0) return RT_OK;
     RTB_CUDA(cudaSetDevice(m->ctx->device));
     if (nq > (1ull << 31) / 32) return fail(RT_ERR_INVALID, "rt_photon_density: nq must be at most 2^26");
-    const uint64_t blocks = (nq * 32 + kQueryBlock - 1) / kQueryBlock;
-    k_density<<<(unsigned)blocks, kQueryBlock, 0, m->ctx->stream>>>(photon_tree(m), *mat, pts, nrm, wo, shape, nq, k,
-                                                                    radius, out_rgb);
+    const uint64_t blocks = (nq * kGroup + kQueryBlock - 1) / kQueryBlock;
+    k_density<<<(unsigned)blocks, kQueryBlock, kQueryBlock / kGroup * 4 * knn_words(k), m->ctx->stream>>>(
+        photon_tree(m), *mat, pts, nrm, wo, shape, nq, k, radius_squared(radius), out_rgb);
     RTB_CUDA(cudaGetLastError());
     RTB_CUDA(cudaStreamSynchronize(m->ctx->stream));
     return RT_OK;

@@ -2,6 +2,10 @@
 // shared by the photon-map entry points (photon.cu) and the renderer (render.cu).
 #pragma once
 
+#include <algorithm>
+#include <cfloat>
+#include <cmath>
+
 #include "surface.cuh"
 
 namespace rtb {
@@ -15,6 +19,13 @@ __device__ __forceinline__ float ref_dist(float qx, float qy, float qz, float4 p
     float dx = __fsub_rn(qx, p.x), dy = __fsub_rn(qy, p.y), dz = __fsub_rn(qz, p.z);
     float s = __fadd_rn(__fadd_rn(__fadd_rn(0.f, __fmul_rn(dx, dx)), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
     return __fsqrt_rn(s);
+}
+
+// The same without the root (0 + r*r is r*r).
+__device__ __forceinline__ float ref_dist2(float qx, float qy, float qz, float4 p)
+{
+    float dx = __fsub_rn(qx, p.x), dy = __fsub_rn(qy, p.y), dz = __fsub_rn(qz, p.z);
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
 }
 
 // nn::KDTree::nearest_neighbors_impl (kdtree.h:111-152) without recursion: photons with
@@ -170,12 +181,11 @@ __device__ __forceinline__ float dipole_eval(const DipoleChannel &c, float r2)
 }
 
 // ------------------------------------------------------- warp-cooperative queries
-// One warp answers one query, with its traversal stack in shared memory. Every lane of the warp
-// must call these functions together. Serial per-node chains of local-memory stack and heap
-// traffic are what bound the one-thread-per-query form: here a warp reads a subtree of at most
-// Scan photons (a contiguous range of the implicit tree) with coalesced loads, keeps k-nearest
-// candidates in a buffer that it narrows to k by a radix select, and reads the photons'
-// attributes in tree order.
+// A warp answers its queries together, with their traversal stacks in shared memory. Every lane of
+// the warp must call these functions together. Serial per-node chains of local-memory stack and
+// heap traffic are what bound the one-thread-per-query form: here a subtree below a given size (a
+// contiguous range of the implicit tree) is read with coalesced loads, k-nearest candidates go to a
+// buffer that is narrowed to about k now and then, and the photons' attributes lie in tree order.
 
 // Device view of a built photon map, all arrays in tree-slot order.
 struct PhotonTree {
@@ -197,21 +207,14 @@ inline PhotonTree photon_tree(const rt_photon_map *m)
     return t;
 }
 
-constexpr uint32_t kKnnScan = 64;      // scanned subtree size of a k-nearest query
-constexpr uint32_t kRadiusScan = 256;  // of a fixed-radius query (no bound to tighten)
-// Stack bound: a popped range is replaced by its two halves, and for n < 2^31 ranges of more
-// than kKnnScan photons lie on at most 25 levels, so the stack holds at most 26 entries.
+constexpr uint32_t kRadiusScan = 256;  // scanned subtree size of a fixed-radius query
+// Stack bound: a popped range is replaced by its two halves, and for n < 2^32 ranges of more
+// than kRadiusScan (or kGroupScan) photons lie on at most 27 levels, so the stack holds at most 28
+// entries.
 constexpr int kWarpStack = 32;
 constexpr unsigned kFullMask = 0xFFFFFFFFu;
 
-// Candidate buffer of a k-nearest query: after a selection it holds k <= kKnnMaxK, and it is
-// selected again before an append could take it past kKnnBuf.
-constexpr uint32_t kKnnBuf = 256;
-static_assert(kKnnBuf >= 2 * kKnnMaxK, "room for k plus one batch of candidates");
-
 struct PhotonWarpScratch {  // per warp, in shared memory
-    float kd[kKnnBuf];     // candidate distances (unordered)
-    uint32_t ki[kKnnBuf];  // and tree slots
     uint32_t sl[kWarpStack], sr[kWarpStack];
     float sd[kWarpStack];
 };
@@ -294,120 +297,270 @@ __device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, flo
     }
 }
 
-// knn_query for a warp: the same neighbour set (the k nearest photons at distance < radius on
-// shape sid, -1: any), up to the order in which photons at exactly equal distances compete
-// for the last place. Candidates (distance below the bound) are appended to a buffer; when it
-// first holds k, and whenever it is nearly full, the k nearest are kept and the bound becomes
-// the k-th distance, as the reference's heap bound does once it holds k. Leaves the neighbours' tree slots
-// unordered in sm.ki; returns their count (all lanes).
-__device__ __forceinline__ uint32_t warp_knn(const PhotonTree &t, float qx, float qy, float qz, int32_t sid, uint32_t k,
-                                             float radius, PhotonWarpScratch &sm)
+// ------------------------------------------------------- k-nearest queries, 8 lanes each
+// A warp answers four k-nearest queries at a time, kGroup lanes each. A whole warp per query was
+// bound by instructions, most of them the same on all lanes (a node step, a selection's counting
+// loop); four queries share them. All 32 lanes run these functions together, converged; a group
+// without a query is idle (on = false). Gathers of a hybrid frame (960x540, 2 samples per pixel,
+// 413,000 photons, k = 50) 8.05 -> 5.45 ms, density of 50,021 points at k = 100 0.56 -> 0.44 ms.
+// Still bound by instructions (0.72 issued per cycle and scheduler): 20 leaves and 44 nodes per
+// query, three selections of about 130 candidates. Leaves of 16 or 64 photons visit 31 or 12 leaves and
+// 62 or 32 nodes, for the same work.
+constexpr uint32_t kGroup = 8;
+constexpr uint32_t kGroupScan = 32;  // subtrees of at most this many photons are read whole
+// Candidates a group may append between two looks at its buffer: a leaf and the nodes above it.
+constexpr uint32_t kGroupBatch = 64;
+static_assert(kGroupScan + 28 <= kGroupBatch, "a descent's candidates");
+// Blocks of 128 threads per SM the density kernels are compiled for (72 registers); their shared
+// memory holds 7 at k = 50, 5 at k = 128.
+constexpr int kGatherBlocks = 7;
+// Candidates a selection may keep beyond k: with some room it ends after two or three counts.
+constexpr uint32_t kKnnSlack = 8;
+
+// Buffer entries of a query, and 32-bit words of shared memory it takes: distances, tree slots,
+// traversal stack; 8 more than a multiple of 32, so that the four groups' accesses fall on
+// different banks.
+__host__ __device__ constexpr uint32_t knn_cap(uint32_t k) { return (k + kKnnSlack + 2 * kGroupBatch + 7) / 8 * 8; }
+__host__ __device__ constexpr uint32_t knn_words(uint32_t k)
 {
-    const uint32_t lane = threadIdx.x & 31u;
+    return (2 * knn_cap(k) + 3 * kWarpStack + 23) / 32 * 32 + 8;
+}
+static_assert(knn_words(50) >= 2 * knn_cap(50) + 3 * kWarpStack && knn_words(50) % 32 == 8, "layout");
+
+struct KnnGroup {
+    float *kd;     // candidates' squared distances (unordered)
+    uint32_t *ki;  // and tree slots
+    uint32_t *sl, *sr;
+    float *sd;
+    uint32_t cap;
+};
+
+// Largest squared distance whose root is below radius (-1: none): the search compares squared
+// distances, and roots are taken of its answers only.
+inline float radius_squared(float radius)
+{
+    if (!(radius > 0.f)) return -1.f;
+    float s = std::min(radius * radius, FLT_MAX);
+    while (s > 0.f && !(std::sqrt(s) < radius)) s = std::nextafter(s, 0.f);
+    while (s < FLT_MAX && std::sqrt(std::nextafter(s, FLT_MAX)) < radius) s = std::nextafter(s, FLT_MAX);
+    return s;
+}
+
+// The calling lane's group in `words`, the shared memory of the warp (4 * knn_words(k)).
+__device__ __forceinline__ KnnGroup knn_group(uint32_t *words, uint32_t k)
+{
+    KnnGroup g;
+    g.cap = knn_cap(k);
+    uint32_t *w = words + ((threadIdx.x & 31u) / kGroup) * knn_words(k);
+    g.kd = reinterpret_cast<float *>(w);
+    g.ki = w + g.cap;
+    g.sl = g.ki + g.cap;
+    g.sr = g.sl + kWarpStack;
+    g.sd = reinterpret_cast<float *>(g.sr + kWarpStack);
+    return g;
+}
+
+template <typename T>
+__device__ __forceinline__ T group_sum(T v)
+{
+#pragma unroll
+    for (uint32_t o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
+    return v;
+}
+__device__ __forceinline__ float group_max(float v)
+{
+#pragma unroll
+    for (uint32_t o = kGroup / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFullMask, v, o));
+    return v;
+}
+
+// Distances that differ by fewer than this many steps of their squares' float representation may
+// be equal.
+constexpr int kRootSteps = 4;
+
+// Keeps the nearest of the groups' candidates where there are more than k + slack: all of those at
+// a squared distance v or less, with v such that there are k to k + slack of them, found by
+// interpolation between counts (photons lie on surfaces: their number grows with the square) and
+// halving on the float bits in turn (the values are not negative, so their bits order like them).
+// Where equal distances leave no such v, exactly k are kept. bound becomes v, or a little more than
+// the largest value where nothing has to go; groups of fewer than k candidates are left alone.
+__device__ __forceinline__ void group_select(const KnnGroup &g, uint32_t k, uint32_t slack, uint32_t &cnt, float &bound)
+{
+    const uint32_t lane = threadIdx.x & (kGroup - 1u), shift = threadIdx.x & 31u & ~(kGroup - 1u);
+    const uint32_t mine = cnt >= k ? cnt : 0u;
+    float mx = 0.f;
+    for (uint32_t j = lane; j < mine; j += kGroup) mx = fmaxf(mx, g.kd[j]);
+    int lo = -1, hi = __float_as_int(group_max(mx)) + 2 * kRootSteps;
+    uint32_t clo = 0, chi = mine;
+    for (uint32_t it = 0;; it++) {
+        const bool more = chi > k + slack && hi - lo > 1;
+        if (!__any_sync(kFullMask, more)) break;
+        int mid = lo + (hi - lo) / 2;
+        if (!(it & 1u)) {
+            const float a = lo < 0 ? 0.f : __int_as_float(lo), b = __int_as_float(hi);
+            const float f = __fdividef((float)(k + slack / 2 - clo), (float)(chi - clo));
+            mid = min(max(__float_as_int(a + (b - a) * f), lo + 1), hi - 1);
+        }
+        uint32_t c = 0;
+        for (uint32_t j = lane; j < mine; j += kGroup) c += __float_as_int(g.kd[j]) <= mid ? 1u : 0u;
+        c = group_sum(c);
+        if (more) {
+            if (c >= k) {
+                hi = mid;
+                chi = c;
+            } else {
+                lo = mid;
+                clo = c;
+            }
+        }
+    }
+    const bool tied = chi > k + slack;  // lo and hi are neighbours
+    if (mine) bound = fminf(bound, __int_as_float(hi));
+    // in place: a kept entry moves down or stays
+    const bool cut = mine > chi || tied;
+    const uint32_t most = __reduce_max_sync(kFullMask, cut ? mine : 0u);
+    const bool ties = __any_sync(kFullMask, tied);
+    uint32_t kept = 0, equal = 0;
+    for (uint32_t j0 = 0; j0 < most; j0 += kGroup) {
+        const uint32_t j = j0 + lane;
+        const bool in = j < mine;
+        const float d = in ? g.kd[j] : 0.f;
+        const uint32_t s = in ? g.ki[j] : 0u;
+        const int key = __float_as_int(d);
+        bool keep = in && key <= hi;
+        if (ties) {
+            const uint32_t eq = (__ballot_sync(kFullMask, in && key == hi) >> shift) & 0xFFu;
+            if (tied && key == hi) keep = keep && clo + equal + __popc(eq & ((1u << lane) - 1u)) < k;
+            equal += __popc(eq);
+        }
+        const uint32_t m = (__ballot_sync(kFullMask, keep) >> shift) & 0xFFu;
+        if (keep) {
+            const uint32_t at = kept + __popc(m & ((1u << lane) - 1u));
+            g.kd[at] = d;
+            g.ki[at] = s;
+        }
+        kept += __popc(m);
+        __syncwarp();
+    }
+    if (cut) cnt = kept;
+}
+
+// The photons nearest to (qx, qy, qz) within the radius (radius2: radius_squared of it) on shape sid
+// (-1: any), as nn::KDTree::nearest_neighbors_impl finds them (kdtree.h:111-152): the near side of
+// a split first, the far side only where the plane is nearer than the search distance, which becomes
+// an upper bound of the k-th distance once k are held. Leaves the candidates unordered in g.kd / g.ki
+// and returns their number: all there are if fewer than k, else the k nearest and up to slack more.
+// bound: every photon within the radius that is not among them has a squared distance above it, or
+// (exactly k kept among equals) one equal to it.
+__device__ __forceinline__ uint32_t group_knn(const float4 *__restrict__ pos, const int2 *__restrict__ aux, uint32_t n,
+                                              float qx, float qy, float qz, int32_t sid, uint32_t k, float radius2,
+                                              uint32_t slack, bool on, const KnnGroup &g, float &bound)
+{
+    const uint32_t lane = threadIdx.x & (kGroup - 1u), shift = threadIdx.x & 31u & ~(kGroup - 1u);
     const uint32_t below = (1u << lane) - 1u;
-    uint32_t cnt = 0, select_at = k;
-    float rcur = radius;
-    // keep the k nearest of cnt > k buffered: the k-th smallest distance v (bitwise search on
-    // the float bits, which order like the values for distances >= 0), then the ones below it
-    // and as many equal to it as fill k
-    auto select = [&]() {
-        uint32_t key[kKnnBuf / 32], slot[kKnnBuf / 32];
-#pragma unroll
-        for (uint32_t i = 0; i < kKnnBuf / 32; i++) {
-            const uint32_t j = lane + 32 * i;
-            key[i] = j < cnt ? __float_as_uint(sm.kd[j]) : 0xFFFFFFFFu;
-            slot[i] = j < cnt ? sm.ki[j] : 0u;
-        }
-        // largest v with fewer than k keys below it (the k-th smallest key), or the first
-        // threshold met with exactly k below it (then those k are the k nearest, no tie)
-        uint32_t v = 0, less = 0;
-        bool exact = false;
-        for (int bit = 30; bit >= 0; bit--) {
-            const uint32_t tv = v | (1u << bit);
-            uint32_t c = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < kKnnBuf / 32; i++) c += key[i] < tv;
-            c = __reduce_add_sync(kFullMask, c);
-            if (c == k) {
-                v = tv;
-                less = k;
-                exact = true;
-                break;
-            }
-            if (c < k) {
-                v = tv;
-                less = c;
-            }
-        }
-        const uint32_t need = k - less;
-        __syncwarp();  // every lane holds its entries before the buffer is rewritten
-        uint32_t blt = 0, beq = 0;
-#pragma unroll
-        for (uint32_t i = 0; i < kKnnBuf / 32; i++) {
-            const bool lt = key[i] < v, eq = key[i] == v;
-            const unsigned mlt = __ballot_sync(kFullMask, lt), meq = __ballot_sync(kFullMask, eq);
-            if (lt) {
-                const uint32_t pos = blt + __popc(mlt & below);
-                sm.kd[pos] = __uint_as_float(key[i]);
-                sm.ki[pos] = slot[i];
-            }
-            if (eq && !exact) {
-                const uint32_t rk = beq + __popc(meq & below);
-                if (rk < need) {
-                    sm.kd[less + rk] = __uint_as_float(key[i]);
-                    sm.ki[less + rk] = slot[i];
+    uint32_t l = 0, r = n, cnt = 0, limit = k;
+    int sp = 0;
+    bool live = on && n > 0;
+    bound = radius2;
+    while (__any_sync(kFullMask, live)) {
+        // down to a leaf
+        for (;;) {
+            const bool down = live && r - l > kGroupScan;
+            if (!__any_sync(kFullMask, down)) break;
+            if (down) {
+                const uint32_t m = (uint32_t)(((uint64_t)l + r) >> 1);
+                const float4 p = __ldg(pos + m);  // one address for the group
+                const float d = ref_dist2(qx, qy, qz, p);
+                if (d <= bound && (sid == -1 || __ldg(&aux[m].x) == sid)) {
+                    if (lane == 0) {
+                        g.kd[cnt] = d;
+                        g.ki[cnt] = m;
+                    }
+                    cnt++;
                 }
+                const uint32_t axis = __float_as_uint(p.w);
+                const float qa = axis == 0 ? qx : (axis == 1 ? qy : qz);
+                const float pa = axis == 0 ? p.x : (axis == 1 ? p.y : p.z);
+                const float diff = __fsub_rn(qa, pa);
+                const float pd = __fmul_rn(diff, diff);  // squared norm(p - pplane) (kdtree.h:138-148)
+                const bool left = qa < pa;
+                if (pd <= bound) {
+                    if (lane == 0) {
+                        g.sl[sp] = left ? m + 1 : l;
+                        g.sr[sp] = left ? r : m;
+                        g.sd[sp] = pd;
+                    }
+                    sp++;
+                }
+                if (left)
+                    r = m;
+                else
+                    l = m + 1;
             }
-            blt += __popc(mlt);
-            beq += __popc(meq);
+        }
+        float4 p[kGroupScan / kGroup];
+#pragma unroll
+        for (uint32_t i = 0; i < kGroupScan / kGroup; i++)
+            if (live && l + lane + kGroup * i < r) p[i] = __ldg(pos + l + lane + kGroup * i);
+#pragma unroll
+        for (uint32_t i = 0; i < kGroupScan / kGroup; i++) {
+            const uint32_t j = l + lane + kGroup * i;
+            const float d = ref_dist2(qx, qy, qz, p[i]);
+            bool c = live && j < r && d <= bound;
+            if (c && sid != -1) c = __ldg(&aux[j].x) == sid;
+            const uint32_t m = (__ballot_sync(kFullMask, c) >> shift) & 0xFFu;
+            if (c) {
+                const uint32_t at = cnt + __popc(m & below);
+                g.kd[at] = d;
+                g.ki[at] = j;
+            }
+            cnt += __popc(m);
         }
         __syncwarp();
-        cnt = k;
-        // the bound: the largest kept distance (v itself unless the search stopped early)
-        float mx = 0.f;
-        for (uint32_t j = lane; j < k; j += 32) mx = fmaxf(mx, sm.kd[j]);
-        rcur = exact ? warp_max(mx) : __uint_as_float(v);
-        select_at = kKnnBuf - 32;
-    };
-    warp_traverse<kKnnScan>(t, qx, qy, qz, sm, [&]() { return rcur; },
-                            [&](bool valid, float dist, int shape, uint32_t slot) {
-                                const bool c = valid && dist < rcur && (sid == -1 || shape == sid);
-                                const unsigned mask = __ballot_sync(kFullMask, c);
-                                if (!mask) return;
-                                if (c) {
-                                    const uint32_t pos = cnt + __popc(mask & below);
-                                    sm.kd[pos] = dist;
-                                    sm.ki[pos] = slot;
-                                }
-                                cnt += __popc(mask);
-                                __syncwarp();
-                                if (cnt >= select_at) select();
-                            });
-    if (cnt > k) select();
-    __syncwarp();
+        // all groups select together: one by itself would take as long
+        if (__any_sync(kFullMask, live && cnt >= limit)) {
+            group_select(g, k, kKnnSlack, cnt, bound);
+            if (cnt >= k) limit = g.cap - kGroupBatch;
+        }
+        if (live) {
+            live = false;
+            while (sp > 0) {
+                sp--;
+                if (g.sd[sp] <= bound) {
+                    l = g.sl[sp];
+                    r = g.sr[sp];
+                    if (r > l) {
+                        live = true;
+                        break;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (__any_sync(kFullMask, cnt > k + slack)) group_select(g, k, slack, cnt, bound);
     return cnt;
 }
 
 // Scene::combinePhotonContributions (Scene.cu:607-635) at point p with shading normal nn and
-// world outgoing direction wo_w, for a warp: sum over the k nearest photons of
+// world outgoing direction wo_w, for a group: sum over the k nearest photons of
 // power * f(wo, -dir)|cos| (SurfaceInteraction::lightScattered, SurfaceInteraction.cu:278-292)
 // / (pi * maxDist^2). The reference weights each photon by |cos| although the photon density
 // already carries the projected-area factor; with compat = false the estimate uses f alone
 // (the radiance estimate of photon mapping). The k terms are summed lane-parallel. Returns the
-// estimate on every lane.
-__device__ __forceinline__ V3 warp_photon_density(const PhotonTree &t, const Bsdf &bs, V3 p, V3 nn, V3 wo_w,
-                                                  int32_t sid, uint32_t k, float radius, bool compat,
-                                                  PhotonWarpScratch &sm)
+// estimate on every lane of the group.
+__device__ __forceinline__ V3 group_photon_density(const PhotonTree &t, const Bsdf &bs, V3 p, V3 nn, V3 wo_w, int32_t sid,
+                                                   uint32_t k, float radius2, bool compat, bool on, const KnnGroup &g)
 {
-    const uint32_t cnt = warp_knn(t, p.x, p.y, p.z, sid, k, radius, sm);
-    if (cnt == 0) return v3(0, 0, 0);
+    float bound;
+    const uint32_t cnt = group_knn(t.pos, t.aux, t.n, p.x, p.y, p.z, sid, k, radius2, 0, on, g, bound);
     V3 tt, b;
     onb(nn, tt, b);
     const V3 wo = v3(dot(wo_w, tt), dot(wo_w, b), dot(wo_w, nn));
     V3 sum = v3(0, 0, 0);
     float maxd = 0.f;
-    for (uint32_t j = threadIdx.x & 31u; j < cnt; j += 32) {
-        const uint32_t s = sm.ki[j];
+    for (uint32_t j = threadIdx.x & (kGroup - 1u); j < cnt; j += kGroup) {
+        const uint32_t s = g.ki[j];
         const float4 pp = __ldg(t.pos + s), pw = __ldg(t.pw + s), pd = __ldg(t.dir + s);
         maxd = fmaxf(maxd, length(v3(pp.x, pp.y, pp.z) - p));
         const V3 w = -v3(pd.x, pd.y, pd.z);
@@ -420,8 +573,10 @@ __device__ __forceinline__ V3 warp_photon_density(const PhotonTree &t, const Bsd
         }
         sum = sum + v3(pw.x, pw.y, pw.z) * f;
     }
-    sum = v3(warp_sum(sum.x), warp_sum(sum.y), warp_sum(sum.z));
-    maxd = warp_max(maxd);
+    __syncwarp();
+    sum = v3(group_sum(sum.x), group_sum(sum.y), group_sum(sum.z));
+    maxd = group_max(maxd);
+    if (cnt == 0) return v3(0, 0, 0);
     return sum * (1.0f / (kPi * maxd * maxd));
 }
 

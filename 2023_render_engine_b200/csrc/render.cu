@@ -55,7 +55,8 @@ struct Buffers {
     rt_ray *srays;
     float4 *scontrib;  // rgb, target index bits (kRetireTarget: retire list)
     float4 *retire;    // L.xyz, pixel index bits
-    float4 *gather;    // photon-map gather requests, 4 float4 each: p+shape, n+material, wo+target, beta
+    float4 *gather;    // photon-map gather requests (push_gather): densities from the front, subsurface
+                       // estimates from the back
     const uint32_t *perm;  // shading order of the wave's queue slots (material sort), or null
     uint32_t cap, scap, gcap;
     bool regen;  // there are more camera samples than queue slots: finished paths make room for them
@@ -69,16 +70,16 @@ constexpr int kCntQueue = 0;          // + 32 b: paths in buffer b
 constexpr int kCntShadow = 64;        // shadow rays of the wave
 constexpr int kCntRetire = 96;        // retired paths of the wave
 constexpr int kCntShadowWork = 128;   // k_shadow's work counter
-constexpr int kCntGather = 160;       // gather requests of the wave
-constexpr int kCntGatherWork = 192;   // k_gather's work counter
-constexpr int kCntSample = 224;       // u64: next camera sample
-constexpr int kCntRays = 256;         // u64: extension rays
-constexpr int kCntShadowRays = 258;   // u64
-constexpr int kCntGathers = 260;      // u64
-constexpr int kCntGuideTimeout = 264; // the guide's tensor-core wait timed out
-constexpr int kCntWaves = 266;        // waves of the device-side loop
-constexpr int kCntCapped = 267;       // its wave cap was reached; k_wave_count: the queues have drained
-constexpr int kCntWords = 288;
+constexpr int kCntGather = 160;       // + 32 kind: gather requests of the wave
+constexpr int kCntGatherWork = 224;   // + 32 kind: k_gather's work counters
+constexpr int kCntSample = 288;       // u64: next camera sample
+constexpr int kCntRays = 320;         // u64: extension rays
+constexpr int kCntShadowRays = 322;   // u64
+constexpr int kCntGathers = 324;      // u64
+constexpr int kCntGuideTimeout = 328; // the guide's tensor-core wait timed out
+constexpr int kCntWaves = 330;        // waves of the device-side loop
+constexpr int kCntCapped = 331;       // its wave cap was reached; k_wave_count: the queues have drained
+constexpr int kCntWords = 352;
 
 struct GuideView {
     const GuideParams *params;  // per queue slot; null while the guide is untrained (BSDF sampling)
@@ -201,27 +202,28 @@ constexpr uint32_t kGatherDensity = 0, kGatherSubsurface = 1;
 
 // Queues a photon-map gather at surface sf, weighted by `weight`, for the path whose radiance
 // lives at `target` (kRetireTarget: the retire list). Five float4: point + shape, normal +
-// material, direction to the previous vertex + target, weight + (kind | guide record << 1),
-// the material's kd at the point (its texture applied).
+// material, direction to the previous vertex + target, weight + guide record, the material's kd at
+// the point (its texture applied). A path queues at most one of each kind per wave, and there is
+// room for two per path.
 // rec: the guide record the estimate also belongs to (kRecNone: none).
 constexpr int kGatherWords = 5;
 __device__ __forceinline__ void push_gather(const Buffers &bf, const Surface &sf, V3 wo_w, V3 weight, uint32_t target,
                                             uint32_t kind, uint32_t rec, V3 kd)
 {
-    const uint32_t gi = append(bf.cnt + kCntGather);
-    if (gi >= bf.gcap) return;
-    float4 *g = bf.gather + (uint64_t)kGatherWords * gi;
+    const uint32_t gi = append(bf.cnt + kCntGather + 32 * kind);
+    if (gi >= bf.gcap / 2) return;
+    float4 *g = bf.gather + (uint64_t)kGatherWords * (kind == kGatherDensity ? gi : bf.gcap - 1 - gi);
     g[0] = make_float4(sf.p.x, sf.p.y, sf.p.z, __int_as_float(sf.shape));
     g[1] = make_float4(sf.n.x, sf.n.y, sf.n.z, __uint_as_float(sf.mat));
     g[2] = make_float4(wo_w.x, wo_w.y, wo_w.z, __uint_as_float(target));
-    g[3] = make_float4(weight.x, weight.y, weight.z, __uint_as_float(kind | (rec << 1)));
+    g[3] = make_float4(weight.x, weight.y, weight.z, __uint_as_float(rec));
     g[4] = make_float4(kd.x, kd.y, kd.z, 0.f);
 }
 
 struct PhotonView {
     PhotonTree tree;
     uint32_t k;
-    float radius;
+    float radius2;  // radius_squared of the search radius
 };
 
 // Material sort: the shading order of a wave. Each block takes chunks of 2^log2 queue slots
@@ -255,7 +257,7 @@ __global__ void __launch_bounds__(kSortBlock) k_material_sort(RenderView rv, Buf
     __shared__ uint32_t wcount[kSortBlock / 32][kSortKeys];
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) bf.cnt[kCntQueue + 32 * (cur ^ 1)] = 0;
-        if (threadIdx.x < 5) bf.cnt[kCntShadow + 32 * threadIdx.x] = 0;
+        if (threadIdx.x < (kCntSample - kCntShadow) / 32) bf.cnt[kCntShadow + 32 * threadIdx.x] = 0;
     }
     const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
     // chunks in a grid-stride loop over the resident blocks (c0 is the same for the whole block)
@@ -717,57 +719,78 @@ __global__ void __launch_bounds__(kB, 12) k_shadow_add(RenderView rv, Buffers bf
 // zero on subsurface materials, Scene.cu:611-612) or the subsurface dipole estimate
 // (Scene::combinePhotonsSubsurface), times the request's weight, added to the path's radiance
 // and, while the guide trains, to the guide record of the vertex before it (as k_shadow does).
-// One warp per request; warps take requests from counter kCntGatherWork until the wave's are done.
+// Warps take the subsurface requests, the longer ones, one by one and then the densities four by
+// four (a group of lanes each) until the wave's are done.
 constexpr int kGatherBlock = 128;
-// Resident blocks per SM k_gather is compiled for (64 registers). Config-4 render at 3840x2160,
-// 4 spp: 538 / 513 / 464 / 467 ms for no bound (118 registers) / 5 / 6 / 8.
-#ifndef RTB_GATHER_MIN_BLOCKS
-#define RTB_GATHER_MIN_BLOCKS 8
-#endif
-__global__ void __launch_bounds__(kGatherBlock, RTB_GATHER_MIN_BLOCKS) k_gather(RenderView rv, Buffers bf, PhotonView pv, int nxt,
-                                                         GuideView gv)
+constexpr int kGatherWarps = kGatherBlock / 32;
+struct GatherRequest {
+    V3 p, n, wo, weight, kd;
+    int32_t shape;
+    uint32_t mat, target, rec;
+};
+__device__ __forceinline__ GatherRequest load_gather(const Buffers &bf, uint32_t kind, uint32_t i)
 {
-    __shared__ PhotonWarpScratch scratch[kGatherBlock / 32];
-    PhotonWarpScratch &sm = scratch[threadIdx.x >> 5];
+    const float4 *g = bf.gather + (uint64_t)kGatherWords * (kind == kGatherDensity ? i : bf.gcap - 1 - i);
+    const float4 a = g[0], b = g[1], c = g[2], d = g[3], k = g[4];
+    return GatherRequest{v3(a.x, a.y, a.z),  v3(b.x, b.y, b.z),    v3(c.x, c.y, c.z),    v3(d.x, d.y, d.z),   v3(k.x, k.y, k.z),
+                         __float_as_int(a.w), __float_as_uint(b.w), __float_as_uint(c.w), __float_as_uint(d.w)};
+}
+__device__ __forceinline__ void add_gather(const Buffers &bf, int nxt, const GuideView &gv, const GatherRequest &q, V3 e)
+{
+    const V3 contrib = q.weight * e;
+    float *dst = (q.target & kRetireTarget) ? reinterpret_cast<float *>(bf.retire + (q.target & ~kRetireTarget))
+                                            : reinterpret_cast<float *>(bf.st1[nxt] + q.target);
+    atomicAdd(dst + 0, contrib.x);
+    atomicAdd(dst + 1, contrib.y);
+    atomicAdd(dst + 2, contrib.z);
+    if (gv.train && q.rec != kRecNone && q.rec < gv.rec_cap) {
+        float4 *r = &gv.recs[q.rec].e;
+        atomicAdd(&r->x, contrib.x);
+        atomicAdd(&r->y, contrib.y);
+        atomicAdd(&r->z, contrib.z);
+    }
+}
+// Shared memory of k_gather: the density groups of its warps, which also hold the subsurface
+// queries' stacks.
+inline uint32_t gather_smem(uint32_t k) { return kGatherBlock / kGroup * 4 * knn_words(k); }
+static_assert(4 * 4 * knn_words(1) >= sizeof(PhotonWarpScratch), "a warp's words hold a stack");
+
+__global__ void __launch_bounds__(kGatherBlock, kGatherBlocks) k_gather(RenderView rv, Buffers bf, PhotonView pv, int nxt,
+                                                                        GuideView gv)
+{
+    extern __shared__ __align__(16) uint32_t gather_words[];
+    uint32_t *words = gather_words + (threadIdx.x >> 5) * 4 * knn_words(pv.k);
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t n = min(bf.cnt[kCntGather], bf.gcap);
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, kCntGathers), (unsigned long long)n);  // stats
+    const uint32_t nd = min(bf.cnt[kCntGather + 32 * kGatherDensity], bf.gcap / 2),
+                   ns = min(bf.cnt[kCntGather + 32 * kGatherSubsurface], bf.gcap / 2);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, kCntGathers), (unsigned long long)nd + ns);  // stats
     const bool compat = (rv.flags & RT_RENDER_COMPAT) != 0;
-    for (;;) {
+    while (ns) {
         uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(bf.cnt + kCntGatherWork, 1u);
+        if (lane == 0) i = atomicAdd(bf.cnt + kCntGatherWork + 32 * kGatherSubsurface, 1u);
         i = __shfl_sync(kFullMask, i, 0);
-        if (i >= n) return;  // warp-uniform
-        const float4 *g = bf.gather + (uint64_t)kGatherWords * i;
-        const float4 a = g[0], b = g[1], c = g[2], d = g[3], k = g[4];
-        const rt_material &m = rv.mats[min(__float_as_uint(b.w), rv.nmats - 1)];
-        const V3 p = v3(a.x, a.y, a.z), nn = v3(b.x, b.y, b.z), wo = v3(c.x, c.y, c.z), kd = v3(k.x, k.y, k.z);
-        const uint32_t kind = __float_as_uint(d.w) & 1u, rec = __float_as_uint(d.w) >> 1;
-        V3 e;
-        if (kind == kGatherSubsurface) {
-            e = warp_photon_subsurface(pv.tree, m, kd, p, nn, wo, __float_as_int(a.w), kSubsurfaceRadius, compat, sm);
-        } else if (m.type == RT_MAT_SUBSURFACE) {
-            e = v3(0, 0, 0);
-        } else {
-            Bsdf bs = load_bsdf(m);
-            bs.color = kd;  // the textured kd the shading point saw
-            e = warp_photon_density(pv.tree, bs, p, nn, wo, __float_as_int(a.w), pv.k, pv.radius, compat, sm);
-        }
-        if (lane == 0) {
-            const V3 contrib = v3(d.x, d.y, d.z) * e;
-            const uint32_t target = __float_as_uint(c.w);
-            float *dst = (target & kRetireTarget) ? reinterpret_cast<float *>(bf.retire + (target & ~kRetireTarget))
-                                                  : reinterpret_cast<float *>(bf.st1[nxt] + target);
-            atomicAdd(dst + 0, contrib.x);
-            atomicAdd(dst + 1, contrib.y);
-            atomicAdd(dst + 2, contrib.z);
-            if (gv.train && rec != kRecNone && rec < gv.rec_cap) {
-                float4 *r = &gv.recs[rec].e;
-                atomicAdd(&r->x, contrib.x);
-                atomicAdd(&r->y, contrib.y);
-                atomicAdd(&r->z, contrib.z);
-            }
-        }
+        if (i >= ns) break;  // warp-uniform
+        const GatherRequest q = load_gather(bf, kGatherSubsurface, i);
+        const V3 e = warp_photon_subsurface(pv.tree, rv.mats[min(q.mat, rv.nmats - 1)], q.kd, q.p, q.n, q.wo, q.shape,
+                                            kSubsurfaceRadius, compat, *reinterpret_cast<PhotonWarpScratch *>(words));
+        if (lane == 0) add_gather(bf, nxt, gv, q, e);
+    }
+    __syncwarp();
+    const KnnGroup g = knn_group(words, pv.k);
+    while (nd) {
+        uint32_t i0 = 0;
+        if (lane == 0) i0 = atomicAdd(bf.cnt + kCntGatherWork + 32 * kGatherDensity, 32u / kGroup);
+        i0 = __shfl_sync(kFullMask, i0, 0);
+        if (i0 >= nd) break;  // warp-uniform
+        const uint32_t i = i0 + lane / kGroup;
+        const GatherRequest q = load_gather(bf, kGatherDensity, min(i, nd - 1));
+        const rt_material &m = rv.mats[min(q.mat, rv.nmats - 1)];
+        const bool on = i < nd && m.type != RT_MAT_SUBSURFACE;
+        Bsdf bs = load_bsdf(m);
+        bs.color = q.kd;  // the textured kd the shading point saw
+        const V3 e = group_photon_density(pv.tree, bs, q.p, q.n, q.wo, q.shape, pv.k, pv.radius2, compat, on, g);
+        if (i < nd && (lane & (kGroup - 1u)) == 0) add_gather(bf, nxt, gv, q, on ? e : v3(0, 0, 0));
+        __syncwarp();
     }
 }
 
@@ -1305,7 +1328,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     if (gathers) {
         pv.tree = photon_tree(s->pmap);
         pv.k = std::min<uint32_t>(std::max<uint32_t>(s->pm_k, 1u), kKnnMaxK);
-        pv.radius = s->pm_radius;
+        pv.radius2 = radius_squared(s->pm_radius);
     }
     bf.cap = cap;
     bf.scap = scap;
@@ -1342,16 +1365,13 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     const unsigned shadow_blocks =
         std::min<unsigned>(resident_grid(SLOT_SHADOW_RESIDENT, k_shadow, kB), (scap + kB - 1) / kB);
     const unsigned add_blocks = std::min<unsigned>((scap + kB - 1) / kB, 16u * device_sm_count());
-    unsigned gather_resident = device_slot(SLOT_GATHER_RESIDENT);  // persistent gather warps: every resident block
-    if (gathers && !gather_resident) {
+    unsigned gather_blocks = 1;  // persistent gather warps: every resident block
+    if (gathers) {
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather, kGatherBlock, 0);
-        gather_resident = device_sm_count() * (unsigned)std::max(per_sm, 1);
-        set_device_slot(SLOT_GATHER_RESIDENT, gather_resident);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather, kGatherBlock, gather_smem(pv.k));
+        gather_blocks = (unsigned)std::min<uint64_t>((uint64_t)device_sm_count() * (unsigned)std::max(per_sm, 1),
+                                                     std::max<uint64_t>(1, (uint64_t)gcap / kGatherWarps));
     }
-    const unsigned gather_blocks =
-        (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(gather_resident, ((uint64_t)gcap * 32 + kGatherBlock - 1) /
-                                                                                kGatherBlock));
     if (gv.params && !(device_slot(SLOT_SMEM_ATTRS) & SMEM_RENDER_INFER)) {
         RTB_CUDA(cudaFuncSetAttribute(k_guide_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem));
         or_device_slot(SLOT_SMEM_ATTRS, SMEM_RENDER_INFER);
@@ -1429,7 +1449,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
             RTB_CUDA(cudaGetLastError());
             RTB_CHECK(mark(k, 5));
             if (gathers) {
-                k_gather<<<gather_blocks, kGatherBlock, 0, st>>>(rv, bf, pv, cur ^ 1, gv);
+                k_gather<<<gather_blocks, kGatherBlock, gather_smem(pv.k), st>>>(rv, bf, pv, cur ^ 1, gv);
                 RTB_CUDA(cudaGetLastError());
             }
             RTB_CHECK(mark(k, 6));

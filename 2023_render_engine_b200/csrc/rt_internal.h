@@ -76,7 +76,7 @@ struct DevBuf {
 constexpr uint32_t kKdTies = 1u, kKdNotFinite = 2u;
 constexpr uint64_t kKdDeviceMax = 1ull << 28;
 int kd_build_device(::rt_context *ctx, const rt_photon *photons, uint64_t n, float4 *node_pos, int2 *node_aux,
-                    uint32_t *report);
+                    uint32_t *report, uint32_t *ties);
 
 // Launch sizes derived from occupancy and per-kernel function attributes are properties of
 // a device, not of the process: each is cached per CUDA device id.
@@ -84,7 +84,6 @@ constexpr int kMaxDevices = 64;
 enum DeviceSlot : int {
     SLOT_TRACE_RESIDENT = 0,   // resident blocks of k_trace_closest (SM count x blocks per SM)
     SLOT_SHADOW_RESIDENT = 1,  // resident blocks of the render's k_shadow
-    SLOT_GATHER_RESIDENT = 2,  // resident blocks of the render's k_gather
     SLOT_SMEM_ATTRS = 3,       // bit mask of kernels whose dynamic shared-memory limit is raised (SMEM_*)
     SLOT_SM_COUNT = 4,         // multiprocessor count
     SLOT_RETIRE_RESIDENT = 5,  // resident blocks of the render's k_retire
@@ -299,6 +298,7 @@ struct rt_photon_map {
     rtb::DevBuf node_dir;  // float4 per tree slot: arrival direction xyz, 0
     bool built = false;
     bool points = false;      // rt_photon_map_from_points: made for nearest-neighbour queries
+    bool scattered = false;   // few nodes tie with another point: queries run on groups of lanes
     bool host_order = false;  // the tree is the host build's, equal coordinates included
     // the host build's node_pos and node_aux where the tree above is not (made by the first
     // rt_photon_knn, whose answers at equal distances depend on them)
