@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_closest(S
     __shared__ TravWarp scratch[kBlock / 32];
     if (n_dev) n = min((uint64_t)*n_dev, n);
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
-    walk_queue<false, false>(
+    walk_queue<false, false, true>(
         v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3, (flags & kTraceVisible) != 0,
         [&](uint32_t i, Walk &W) {
             float4 ra, rb;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_counts(Sc
 {
     __shared__ TravWarp scratch[kBlock / 32];
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
-    walk_queue<ANY, true>(
+    walk_queue<ANY, true, true>(
         v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3, false,
         [&](uint32_t i, Walk &W) {
             float4 ra, rb;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_any(Scene
 {
     __shared__ TravWarp scratch[kBlock / 32];
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
-    walk_queue<true, false>(
+    walk_queue<true, false, true>(
         v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3, false,
         [&](uint32_t i, Walk &W) {
             float4 ra, rb;

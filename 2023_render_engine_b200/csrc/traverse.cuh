@@ -155,7 +155,10 @@ __device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz,
 // warp has lanes, so they mostly take one round, where the serial loop took as many as the lane
 // with the most of them, with a few lanes active in each and a triangle fetch of latency per round.
 // shared_t: the ray's best offset among other lanes (INFINITY: none). Returns whether the walk ended.
-template <bool ANY, bool COUNT>
+// ORDERED: hit children are visited near to far and skipped once the best hit lies before them.
+// Without it (a walk that ends at any hit, whose limit never shrinks) they are visited as they come
+// in the node and the stack holds node indices only, twice as many.
+template <bool ANY, bool COUNT, bool ORDERED>
 __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk &W, bool active, bool unbounded,
                                           float shared_t)
 {
@@ -180,6 +183,12 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
             const uint32_t child_base = n1.x;
             tri_base = n1.y;
             const uint32_t meta_lo = n1.z, meta_hi = n1.w;
+            // the planes the ray meets first and last on each axis, by the sign of its direction:
+            // a selection per node instead of a minimum and a maximum per child and axis
+            const bool fx = W.ix < 0.f, fy = W.iy < 0.f, fz = W.iz < 0.f;
+            const uint32_t nx[2] = {fx ? n3.z : n2.x, fx ? n3.w : n2.y}, hx[2] = {fx ? n2.x : n3.z, fx ? n2.y : n3.w};
+            const uint32_t ny[2] = {fy ? n4.x : n2.z, fy ? n4.y : n2.w}, hy[2] = {fy ? n2.z : n4.x, fy ? n2.w : n4.y};
+            const uint32_t nz[2] = {fz ? n4.z : n3.x, fz ? n4.w : n3.y}, hz[2] = {fz ? n3.x : n4.z, fz ? n3.y : n4.w};
             // per-axis affine map t = q * (s * inv) + (p * inv - o * inv)
             const float ax = sx * W.ix, bx = fmaf(__uint_as_float(n0.x), W.ix, -W.ox * W.ix);
             const float ay = sy * W.iy, by = fmaf(__uint_as_float(n0.y), W.iy, -W.oy * W.iy);
@@ -191,29 +200,38 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
             for (int k = 0; k < 8; k++) {
                 const int b = k & 3;
                 const uint32_t meta = byte_of(k < 4 ? meta_lo : meta_hi, b);
-                const float qlx = (float)byte_of(k < 4 ? n2.x : n2.y, b);
-                const float qly = (float)byte_of(k < 4 ? n2.z : n2.w, b);
-                const float qlz = (float)byte_of(k < 4 ? n3.x : n3.y, b);
-                const float qhx = (float)byte_of(k < 4 ? n3.z : n3.w, b);
-                const float qhy = (float)byte_of(k < 4 ? n4.x : n4.y, b);
-                const float qhz = (float)byte_of(k < 4 ? n4.z : n4.w, b);
-                const float t1x = fmaf(qlx, ax, bx), t2x = fmaf(qhx, ax, bx);
-                const float t1y = fmaf(qly, ay, by), t2y = fmaf(qhy, ay, by);
-                const float t1z = fmaf(qlz, az, bz), t2z = fmaf(qhz, az, bz);
-                const float tn =
-                    fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fmaxf(fminf(t1z, t2z), 0.0f));
-                const float tf =
-                    fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fminf(fmaxf(t1z, t2z), tlimit));
+                float t1x = fmaf((float)byte_of(nx[k >> 2], b), ax, bx), t2x = fmaf((float)byte_of(hx[k >> 2], b), ax, bx);
+                float t1y = fmaf((float)byte_of(ny[k >> 2], b), ay, by), t2y = fmaf((float)byte_of(hy[k >> 2], b), ay, by);
+                float t1z = fmaf((float)byte_of(nz[k >> 2], b), az, bz), t2z = fmaf((float)byte_of(hz[k >> 2], b), az, bz);
+                // a bound that is NaN (of a zero direction component) does not limit the ray; the other
+                // bound of its axis still does in the counts
+                if (COUNT) {
+                    const float lx = fminf(t1x, t2x), ly = fminf(t1y, t2y), lz = fminf(t1z, t2z);
+                    t2x = fmaxf(t1x, t2x), t2y = fmaxf(t1y, t2y), t2z = fmaxf(t1z, t2z);
+                    t1x = lx, t1y = ly, t1z = lz;
+                }
+                const float tn = fmaxf(fmaxf(t1x, t1y), fmaxf(t1z, 0.0f));
+                const float tf = fminf(fminf(t2x, t2y), fminf(t2z, tlimit));
                 const bool hit = (meta != 0xFFu) && (tn <= tf);
                 const bool interior = (imask >> k) & 1u;
-                keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
-                nint += (hit && interior) ? 1u : 0u;
+                if (ORDERED) {
+                    keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
+                    nint += (hit && interior) ? 1u : 0u;
+                } else if (hit && interior) {
+                    if (next != kNoRoot) {
+                        if (W.sp < 2 * kStack)
+                            reinterpret_cast<uint32_t *>(W.st)[W.sp++] = next;
+                        else
+                            W.ok = false, done = true;
+                    }
+                    next = child_base + meta;
+                }
                 if (hit && !interior) {
                     trimask |= ((2u << (meta >> 5)) - 1u) << (meta & 31u);
                     if (COUNT) leafend |= (1u << (meta >> 5)) << (meta & 31u);
                 }
             }
-            if (nint) {
+            if (ORDERED && nint) {
                 sort8(keys);
                 if (W.sp + (int)nint - 1 > kStack) {  // drop the entries beyond the best hit
                     int kept = 0;
@@ -341,6 +359,11 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
         if (!done) {
             if (next != kNoRoot && next_t <= tl) {
                 W.cur = next;
+            } else if (!ORDERED) {
+                if (W.sp > 0)
+                    W.cur = reinterpret_cast<uint32_t *>(W.st)[--W.sp];
+                else
+                    done = true;
             } else {
                 done = true;
 #pragma unroll 1
@@ -377,7 +400,7 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
 // triangle test has no limit (lim only bounds the nodes). COUNT: also counts the triangles a
 // serial walk would test (whole leaves, up to the leaf of the accepted hit under ANY), and every
 // ray keeps its own lane.
-template <bool ANY, bool COUNT, typename Init, typename Finish>
+template <bool ANY, bool COUNT, bool ORDERED, typename Init, typename Finish>
 __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uint32_t n, uint32_t *work,
                                            bool unbounded, Init init, Finish finish)
 {
@@ -415,7 +438,7 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
             if (exhausted) return;
             continue;
         }
-        if (walk_step<ANY, COUNT>(v, sm, W, active, unbounded, INFINITY)) {
+        if (walk_step<ANY, COUNT, ORDERED>(v, sm, W, active, unbounded, INFINITY)) {
             finish(ray, W, W.brec != kNoRec ? sm.bary[lane] : make_float2(0.f, 0.f));
             ray = 0xFFFFFFFFu;
         }
@@ -438,7 +461,10 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
             const uint32_t k = (uint32_t)__popc((give ? givers : idle) & below);
             uint2 e = make_uint2(0u, 0u);
             if (give && k < moves) {
-                e = W.st[--W.sp];
+                if (ORDERED)
+                    e = W.st[--W.sp];
+                else
+                    e.x = reinterpret_cast<uint32_t *>(W.st)[--W.sp];
                 sm.pair[k] = (uint16_t)lane;
             }
             __syncwarp();
@@ -476,7 +502,7 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
         }
         const bool active = ray != 0xFFFFFFFFu;
         const float shared_t = active ? sm.found[W.kz >> 2].x : INFINITY;
-        const bool done = walk_step<ANY, COUNT>(v, sm, W, active, unbounded, shared_t);
+        const bool done = walk_step<ANY, COUNT, ORDERED>(v, sm, W, active, unbounded, shared_t);
         // one ended lane after the other adds what it found to its ray's; the last reports it
         unsigned ended = __ballot_sync(kAllLanes, done);
         while (ended) {
