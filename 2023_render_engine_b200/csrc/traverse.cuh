@@ -215,7 +215,7 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
                 const bool hit = (meta != 0xFFu) && (tn <= tf);
                 const bool interior = (imask >> k) & 1u;
                 if (ORDERED) {
-                    keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | (uint32_t)k) : 0xFFFFFFFFu;
+                    keys[k] = (hit && interior) ? ((__float_as_uint(tn) & ~7u) | meta) : 0xFFFFFFFFu;
                     nint += (hit && interior) ? 1u : 0u;
                 } else if (hit && interior) {
                     if (next != kNoRoot) {
@@ -250,14 +250,11 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
 #pragma unroll
                     for (int j = 7; j >= 1; j--)
                         if (j < (int)nint) {
-                            const uint32_t slot = keys[j] & 7u;
-                            W.st[W.sp] = make_uint2(child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3),
-                                                    keys[j] & ~7u);
+                            W.st[W.sp] = make_uint2(child_base + (keys[j] & 7u), keys[j] & ~7u);
                             W.sp++;
                         }
                 }
-                const uint32_t slot = keys[0] & 7u;
-                next = child_base + byte_of(slot < 4 ? meta_lo : meta_hi, slot & 3);
+                next = child_base + (keys[0] & 7u);
                 next_t = __uint_as_float(keys[0] & ~7u);
             }
         }
