@@ -192,9 +192,9 @@ __global__ void __launch_bounds__(128 * kFbGroups, 1) k_guide_train_tc(const uin
 #pragma unroll
         for (int i = 0; i < 9; i++) q[i] = in_b ? A.q[9 * row + i] : 0.f;
         {
-            __half2 e[72];
-            guide_encode(0, q, A.box, e);
-            guide_encode(1, q, A.box, e);
+            __half2 e[kGuideIn / 2];
+            guide_encode0(q, A.box, e);
+            guide_encode1(q, e + kEncode0 / 2);
 #pragma unroll
             for (int c = 0; c < kGuideIn / 8; c++)
                 *reinterpret_cast<uint4 *>(bufA + tc_chunk(gt, c, kGuideIn / 8)) =

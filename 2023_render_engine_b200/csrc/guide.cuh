@@ -106,42 +106,54 @@ __device__ __forceinline__ float guide_blob(float x, int i)
     return __expf(-0.5f * d * d);
 }
 
-// part 0: position bands (half2 0..35); part 1: direction blobs, normal, zero pad (36..71)
-__device__ __forceinline__ void guide_encode(int part, const float *q, const GuideBox &bx, __half2 *row)
+// The encoding in two parts of whole chunks of 8 features: part 0 the position bands and the first 8
+// blobs (features 0..79), part 1 the other blobs, the normal and the zeros (80..143).
+constexpr int kEncode0 = 80, kEncode1 = kGuideIn - kEncode0;
+
+__device__ __forceinline__ float guide_theta(const float *q)
 {
-    if (part == 0) {
-        const float u[3] = {fminf(fmaxf((q[0] - bx.lo.x) * bx.inv_ext.x, 0.f), 1.f),
-                            fminf(fmaxf((q[1] - bx.lo.y) * bx.inv_ext.y, 0.f), 1.f),
-                            fminf(fmaxf((q[2] - bx.lo.z) * bx.inv_ext.z, 0.f), 1.f)};
-        // band k + 2 doubles the angle of band k: sin 2x = 2 sin x cos x, cos 2x = cos^2 x -
-        // sin^2 x, from sincospi(u) and sincospi(sqrt(2) u); five doublings grow the absolute
-        // error to ~2e-6, far below the FP16 step of the encoded value
+    return acosf(fminf(fmaxf(q[8], -1.f), 1.f)) * (1.f / 3.14159265358979f);
+}
+
+__device__ __forceinline__ void guide_encode0(const float *q, const GuideBox &bx, __half2 *row)
+{
+    const float u[3] = {fminf(fmaxf((q[0] - bx.lo.x) * bx.inv_ext.x, 0.f), 1.f),
+                        fminf(fmaxf((q[1] - bx.lo.y) * bx.inv_ext.y, 0.f), 1.f),
+                        fminf(fmaxf((q[2] - bx.lo.z) * bx.inv_ext.z, 0.f), 1.f)};
+    // band k + 2 doubles the angle of band k: sin 2x = 2 sin x cos x, cos 2x = cos^2 x -
+    // sin^2 x, from sincospi(u) and sincospi(sqrt(2) u); five doublings grow the absolute
+    // error to ~2e-6, far below the FP16 step of the encoded value
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            float s0, c0, s1, c1;
-            sincospif(u[a], &s0, &c0);
-            sincospif(u[a] * 1.41421356f, &s1, &c1);
+    for (int a = 0; a < 3; a++) {
+        float s0, c0, s1, c1;
+        sincospif(u[a], &s0, &c0);
+        sincospif(u[a] * 1.41421356f, &s1, &c1);
 #pragma unroll
-            for (int k = 0; k < 12; k += 2) {
-                row[a * 12 + k] = __floats2half2_rn(s0, c0);
-                row[a * 12 + k + 1] = __floats2half2_rn(s1, c1);
-                const float s0n = 2.f * s0 * c0, c0n = fmaf(c0, c0, -s0 * s0);
-                const float s1n = 2.f * s1 * c1, c1n = fmaf(c1, c1, -s1 * s1);
-                s0 = s0n, c0 = c0n, s1 = s1n, c1 = c1n;
-            }
+        for (int k = 0; k < 12; k += 2) {
+            row[a * 12 + k] = __floats2half2_rn(s0, c0);
+            row[a * 12 + k + 1] = __floats2half2_rn(s1, c1);
+            const float s0n = 2.f * s0 * c0, c0n = fmaf(c0, c0, -s0 * s0);
+            const float s1n = 2.f * s1 * c1, c1n = fmaf(c1, c1, -s1 * s1);
+            s0 = s0n, c0 = c0n, s1 = s1n, c1 = c1n;
         }
-    } else {
-        const float th = acosf(fminf(fmaxf(q[8], -1.f), 1.f)) * (1.f / 3.14159265358979f);
-        const float ph = atan2f(q[7], q[6]) * (1.f / 6.28318530717959f) + 0.5f;
-#pragma unroll
-        for (int i = 0; i < 16; i++) row[36 + i] = __floats2half2_rn(guide_blob(th, 2 * i), guide_blob(th, 2 * i + 1));
-#pragma unroll
-        for (int i = 0; i < 16; i++) row[52 + i] = __floats2half2_rn(guide_blob(ph, 2 * i), guide_blob(ph, 2 * i + 1));
-        row[68] = __floats2half2_rn(q[3], q[4]);
-        row[69] = __floats2half2_rn(q[5], 0.f);
-        row[70] = __floats2half2_rn(0.f, 0.f);
-        row[71] = __floats2half2_rn(0.f, 0.f);
     }
+    const float th = guide_theta(q);
+#pragma unroll
+    for (int i = 0; i < 4; i++) row[36 + i] = __floats2half2_rn(guide_blob(th, 2 * i), guide_blob(th, 2 * i + 1));
+}
+
+__device__ __forceinline__ void guide_encode1(const float *q, __half2 *row)
+{
+    const float th = guide_theta(q);
+    const float ph = atan2f(q[7], q[6]) * (1.f / 6.28318530717959f) + 0.5f;
+#pragma unroll
+    for (int i = 4; i < 16; i++) row[i - 4] = __floats2half2_rn(guide_blob(th, 2 * i), guide_blob(th, 2 * i + 1));
+#pragma unroll
+    for (int i = 0; i < 16; i++) row[12 + i] = __floats2half2_rn(guide_blob(ph, 2 * i), guide_blob(ph, 2 * i + 1));
+    row[28] = __floats2half2_rn(q[3], q[4]);
+    row[29] = __floats2half2_rn(q[5], 0.f);
+    row[30] = __floats2half2_rn(0.f, 0.f);
+    row[31] = __floats2half2_rn(0.f, 0.f);
 }
 
 // ------------------------------------------------------------------ vMF mixture
@@ -392,22 +404,23 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
 // [8c, 8c + 8) of an operand with KC chunks per row sit at byte (r / 8) * KC * 128 + c * 128 +
 // (r % 8) * 16.
 constexpr int kInferRows = 128;
-constexpr int kInferGroups = 4;
+constexpr int kInferGroups = 6;
 constexpr int kInferWarps = 4 * kInferGroups;
 // byte offset of layer l's weight operand (W_l^T: guide_out(l) rows of guide_in(l) halves)
 __host__ __device__ constexpr int tc_w(int l) { return l == 0 ? 0 : tc_w(l - 1) + guide_out(l - 1) * guide_in(l - 1) * 2; }
 constexpr int kTcBias = tc_w(kGuideLayers);                                 // 304 FP32 biases
 constexpr int kTcA = 50432;                                                 // activation tiles
-constexpr int kTcATile = kInferRows * kGuideIn * 2;                         // 128 x 144 halves
+constexpr int kTcATile = kInferRows * kEncode0 * 2;                         // 128 x 80 halves
 constexpr int kTcBar = kTcA + kInferGroups * kTcATile;                      // mbarriers, TMEM base
 constexpr int kInferSmem = kTcBar + 8 * kInferGroups + 16;
 constexpr int kTmemColsPerGroup = 64;
-constexpr int kTmemCols = kTmemColsPerGroup * kInferGroups;  // a power of 2 in [32, 512]
+constexpr int kTmemCols = 512;  // a power of 2 in [32, 512]
 constexpr uint32_t kUmmaWaitPolls = 1u << 22;
 static_assert(tc_w(1) == 18432 && tc_w(4) == 43008 && kTcBias == 49152, "operand sizes");
 static_assert(kTcBias + 4 * (4 * 64 + 48) <= kTcA && kTcA % 128 == 0 && kTcBar % 8 == 0, "shared layout");
 static_assert(kInferSmem <= 227 * 1024, "shared memory per CTA");
-static_assert(kTmemCols == 256, "TMEM allocation");
+static_assert(kTmemColsPerGroup * kInferGroups <= kTmemCols, "TMEM allocation");
+static_assert(kEncode0 % 16 == 0 && kEncode1 % 16 == 0 && kEncode1 <= kEncode0 && 64 <= kEncode0, "operand tile");
 
 // byte offset of row r, chunk c (8 halves) in an operand of kc chunks per row
 __host__ __device__ constexpr uint32_t tc_chunk(uint32_t r, uint32_t c, uint32_t kc)
@@ -477,6 +490,16 @@ __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBo
     unsigned char *A = sm + kTcA + grp * kTcATile;
     uint32_t phase = 0;
     bool failed = false;
+    // the K = 16 steps [s0, s1) of layer l, from an operand tile of kca chunks per row that starts at
+    // step s0
+    auto issue = [&](int l, uint32_t kca, int s0, int s1) {
+        const uint32_t idesc = umma_idesc_f16(kInferRows, guide_out(l)), kc = guide_in(l) / 8;
+        const uint32_t a0 = smem_u32(A), b0 = smem_u32(sm + tc_w(l));
+        for (int s = s0; s < s1; s++)
+            umma_f16(tmem, umma_desc(a0 + 256u * (s - s0), 128u, 128u * kca), umma_desc(b0 + 256u * s, 128u, 128u * kc),
+                     idesc, s > 0 ? 1u : 0u);
+        umma_commit(bar);
+    };
     const uint32_t stride = gridDim.x * kInferGroups;
     for (uint32_t tile = blockIdx.x * kInferGroups + grp; !failed && (uint64_t)tile * kInferRows < n; tile += stride) {
         const uint32_t row = tile * kInferRows + gt;
@@ -485,13 +508,11 @@ __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBo
         float q[9];
         const bool valid = row < n && src(row, q);
         if (valid) {
-            __half2 e[72];
-            guide_encode(0, q, box, e);
-            guide_encode(1, q, box, e);
+            __half2 e[kEncode0 / 2];
+            guide_encode0(q, box, e);
 #pragma unroll
-            for (int c = 0; c < kGuideIn / 8; c++)
-                *reinterpret_cast<uint4 *>(A + tc_chunk(gt, c, kGuideIn / 8)) =
-                    *reinterpret_cast<const uint4 *>(&e[4 * c]);
+            for (int c = 0; c < kEncode0 / 8; c++)
+                *reinterpret_cast<uint4 *>(A + tc_chunk(gt, c, kEncode0 / 8)) = *reinterpret_cast<const uint4 *>(&e[4 * c]);
         }
         fence_async_smem();
         tc_fence_before();
@@ -499,17 +520,31 @@ __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBo
             if (row < n) sink(row, false, q);
             continue;
         }
+        // the first part's product runs while the second part is computed
+        if (gt == 0) {
+            tc_fence_after();
+            issue(0, kEncode0 / 8, 0, kEncode0 / 16);
+        }
+        {
+            __half2 e[kEncode1 / 2];
+            if (valid) guide_encode1(q, e);
+            failed = !__all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, kUmmaWaitPolls));
+            phase ^= 1u;
+            tc_fence_after();
+            if (valid && !failed)
+#pragma unroll
+                for (int c = 0; c < kEncode1 / 8; c++)
+                    *reinterpret_cast<uint4 *>(A + tc_chunk(gt, c, kEncode1 / 8)) =
+                        *reinterpret_cast<const uint4 *>(&e[4 * c]);
+        }
+        fence_async_smem();
+        tc_fence_before();
+        failed = group_sync_or(bar_id, failed);
 #pragma unroll 1
         for (int l = 0; l < kGuideLayers && !failed; l++) {
-            const int kc = guide_in(l) / 8;
             if (gt == 0) {
                 tc_fence_after();
-                const uint32_t idesc = umma_idesc_f16(kInferRows, guide_out(l));
-                const uint32_t a0 = smem_u32(A), b0 = smem_u32(sm + tc_w(l));
-                for (int s = 0; s < kc / 2; s++)
-                    umma_f16(tmem, umma_desc(a0 + 256u * s, 128u, 128u * kc), umma_desc(b0 + 256u * s, 128u, 128u * kc),
-                             idesc, s > 0 ? 1u : 0u);
-                umma_commit(bar);
+                issue(l, l == 0 ? kEncode1 / 8 : guide_in(l) / 8, l == 0 ? kEncode0 / 16 : 0, guide_in(l) / 16);
             }
             // warp-uniform, as the tcgen05.ld below is .sync.aligned
             const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, kUmmaWaitPolls));
