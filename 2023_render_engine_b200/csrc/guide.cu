@@ -6,8 +6,8 @@
 //   k_guide_train_tc  per 128-row tile: encode, forward, loss gradient per row, backward
 //                     through the 5 layers; writes every layer's input and output gradient
 //                     feature-major, so the weight gradient is a contraction over rows
-//   k_guide_wgrad_tc  dW_l = X_l^T G_l per chunk of rows (FP32 partials), all layers at once
-//   k_guide_bias_grad db_l = sum G_l per chunk of rows
+//   k_guide_wgrad_tc  dW_l = X_l^T G_l and db_l = 1^T G_l per chunk of rows (FP32 partials), all layers
+//                     at once
 //   k_guide_reduce    sum of the chunk partials in a fixed order (deterministic gradient)
 //   k_guide_adam      Adam on the FP32 master weights; refreshes the FP16 image
 #include <cuda_fp16.h>
@@ -27,12 +27,6 @@ namespace {
 constexpr int kWsumBlocks = 128;
 constexpr float kAdamB1 = 0.9f, kAdamB2 = 0.99f, kAdamEps = 1e-8f;
 
-__device__ __forceinline__ uint32_t pack_h2(__half a, __half b)
-{
-    __half2 h = __halves2half2(a, b);
-    return *reinterpret_cast<uint32_t *>(&h);
-}
-
 struct TrainArgs {
     const float *q, *dir, *pdf, *w;
     uint64_t B, Bpad;
@@ -45,16 +39,20 @@ struct TrainArgs {
 // ------------------------------------------------------------------ training on tcgen05
 //
 // k_guide_train_tc: the forward and backward passes of 128-row tiles on the 5th-generation tensor
-// cores, two independent 128-thread groups per CTA sharing one copy of the weights in shared
-// memory. Per layer one thread issues tcgen05.mma (M = 128 rows, FP16 operands in K-major core
+// cores, two independent 256-thread groups per CTA sharing one copy of the weights in shared
+// memory, two threads per row (of a layer's columns, lobes or encoded features each takes a half).
+// Per layer one thread issues tcgen05.mma (M = 128 rows, FP16 operands in K-major core
 // matrices, FP32 accumulator in the group's 64 TMEM columns) and commits to the group's
-// mbarrier; every thread then reads its own row back (tcgen05.ld), applies bias and ReLU (forward)
-// or the ReLU mask (backward) and writes the next operand. The forward operand is W_l^T (the
-// inference staging); the backward operand is W_l itself, restaged once per CTA. Each thread
-// keeps its row's ReLU signs as bit masks, so only two operand buffers per group are needed.
-// Every layer input X_l and output gradient G_l is also written feature-major (planes of Bp rows)
-// for the weight gradient.
+// mbarrier; the threads then read their rows back (tcgen05.ld), apply bias and ReLU (forward)
+// or the ReLU mask (backward) and write the next operand. The forward operand is W_l^T (the
+// inference staging); the backward operand is W_l itself, transposed from it once per CTA. Each
+// thread keeps its half row's ReLU signs as a bit mask, so only two operand buffers per group are
+// needed. Every layer input X_l and output gradient G_l is also written feature-major (planes of Bp
+// rows) for the weight gradient, transposed by ldmatrix.
+// The usual batch, two tiles per SM, is one chain of steps per tile and bound by latency: 37,888 rows
+// took 99 us with one thread per row and transpositions half by half, 46 us so.
 constexpr int kFbGroups = 2;
+constexpr int kFbThreads = 256;  // of a group
 constexpr int kFbWb = 50432;  // backward weights W_1..W_4 (64 rows of out_l halves), 8 KB slots
 __host__ __device__ constexpr int fb_wb(int l) { return kFbWb + (l - 1) * 8192; }
 constexpr int kFbGroup0 = kFbWb + 4 * 8192;
@@ -80,32 +78,30 @@ __device__ __forceinline__ void fb_mma(uint32_t tmem, uint32_t a0, uint32_t kca,
 }
 
 // The group's 128-row operand tile (kc chunks of 8 halves per row, core-matrix layout) to the
-// feature-major planes dst[f * Bp + row0 + r] for features f < nfeat: each 16-byte store holds
-// one feature of 8 consecutive rows (read from the 8 rows of one core matrix).
-__device__ __forceinline__ void tile_to_planes(const unsigned char *tile, int kc, int nfeat, __half *dst, uint64_t Bp,
-                                               uint64_t row0, int gt)
+// feature-major planes dst[f * Bp + row0 + r] for features f < nfeat: a warp transposes four core
+// matrices at a time, one chunk of 32 rows.
+__device__ __forceinline__ void tile_to_planes(uint32_t tile, int kc, int nfeat, __half *dst, uint64_t Bp, uint64_t row0,
+                                               int gt)
 {
-    for (int i = gt; i < nfeat * 16; i += 128) {
-        const int f = i >> 4, rg = i & 15;  // feature, group of 8 rows
-        const unsigned char *src = tile + tc_chunk((uint32_t)(8 * rg), (uint32_t)(f >> 3), (uint32_t)kc) + 2 * (f & 7);
+    const int lane = gt & 31;
+    for (int i = gt >> 5; i < nfeat / 2; i += kFbThreads / 32) {
+        const int c = i >> 2, rg = 4 * (i & 3);  // chunk, first of four groups of 8 rows
         uint32_t w[4];
+        ldmatrix4_trans(tile + (uint32_t)((rg + (lane >> 3)) * kc * 128 + c * 128 + (lane & 7) * 16), w);
+        uint32_t *p = reinterpret_cast<uint32_t *>(dst + (uint64_t)(8 * c + (lane >> 2)) * Bp + row0 + 8 * rg) + (lane & 3);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const __half lo = *reinterpret_cast<const __half *>(src + 32 * j);
-            const __half hi = *reinterpret_cast<const __half *>(src + 32 * j + 16);
-            w[j] = pack_h2(lo, hi);
-        }
-        *reinterpret_cast<uint4 *>(dst + (uint64_t)f * Bp + row0 + 8 * rg) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int j = 0; j < 4; j++) p[4 * j] = w[j];
     }
 }
 
-__global__ void __launch_bounds__(128 * kFbGroups, 1) k_guide_train_tc(const uint4 *img, TrainArgs A)
+__global__ void __launch_bounds__(kFbThreads * kFbGroups, 1) k_guide_train_tc(const uint4 *img, TrainArgs A)
 {
     extern __shared__ __align__(128) unsigned char fb_smem[];
     unsigned char *sm = fb_smem;
     __shared__ double wsum;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int grp = tid >> 7, gt = tid & 127;
+    const int grp = tid / kFbThreads, gt = tid % kFbThreads;
+    const int tr = gt & 127, half = gt >> 7;  // the thread's row of the tile, and which half of it
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm + kFbBar) + grp;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + kFbBar + 8 * kFbGroups);
     const unsigned char *ib = reinterpret_cast<const unsigned char *>(img);
@@ -121,22 +117,17 @@ __global__ void __launch_bounds__(128 * kFbGroups, 1) k_guide_train_tc(const uin
     }
     for (int i = tid; i < (4 * 64 + 48) / 4; i += blockDim.x)
         reinterpret_cast<uint4 *>(sm + kTcBias)[i] = reinterpret_cast<const uint4 *>(ib + kGuideImgBias)[i];
-    // backward weights W_l (l = 1..4): row i (input), chunk c = outputs 8c .. 8c + 7
-    const __half *ih = reinterpret_cast<const __half *>(img);
-#pragma unroll 1
-    for (int l = 1; l < kGuideLayers; l++) {
-        const int kc = guide_out(l) / 8;
-        for (int i = tid; i < 64 * kc; i += blockDim.x) {
-            const int r = i / kc, c = i - r * kc;
-            uint32_t w[4];
+    // backward weights W_l (l = 1..4), rows of inputs: each core matrix is one of W_l^T transposed
+    __syncthreads();
+    for (int i = warp; i < 3 * 16 + 12; i += blockDim.x / 32) {
+        const int l = i < 48 ? 1 + i / 16 : 4, kco = guide_out(l) / 8;
+        const int core = 4 * (i < 48 ? i % 16 : i - 48);  // of W_l^T: output group * 8 + input group
+        uint32_t w[4];
+        ldmatrix4_trans(smem_u32(sm + tc_w(l) + (core + (lane >> 3)) * 128 + (lane & 7) * 16), w);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const __half lo = ih[guide_iw(l) + (8 * c + 2 * j) * guide_stride(l) + r];
-                const __half hi = ih[guide_iw(l) + (8 * c + 2 * j + 1) * guide_stride(l) + r];
-                w[j] = pack_h2(lo, hi);
-            }
-            *reinterpret_cast<uint4 *>(sm + fb_wb(l) + tc_chunk(r, c, kc)) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<uint32_t *>(sm + fb_wb(l) + (((core + j) & 7) * kco + ((core + j) >> 3)) * 128 + 4 * lane) =
+                w[j];
     }
     if (tid < 32) {
         double sw = 0.0;
@@ -169,142 +160,160 @@ __global__ void __launch_bounds__(128 * kFbGroups, 1) k_guide_train_tc(const uin
         const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, kUmmaWaitPolls));
         phase ^= 1u;
         tc_fence_after();
-        return !group_sync_or(bar_id, !ok);
+        return !group_sync_or<kFbThreads>(bar_id, !ok);
     };
     // the operand just written becomes visible to the tensor core; thread 0 of the group issues,
     // then the group copies the operand to its feature-major planes while the MMA runs
-    auto issue = [&](uint32_t a0, uint32_t kca, uint32_t b0, uint32_t kcb, int ksteps, int n, const unsigned char *tile,
-                     int nfeat, __half *planes, uint64_t row0) {
+    auto issue = [&](uint32_t a0, uint32_t kca, uint32_t b0, uint32_t kcb, int ksteps, int n, int nfeat, __half *planes,
+                     uint64_t row0) {
         fence_async_smem();
         tc_fence_before();
-        group_sync_or(bar_id, false);
+        group_sync_or<kFbThreads>(bar_id, false);
         if (gt == 0) {
             tc_fence_after();
             fb_mma(tmem, a0, kca, b0, kcb, ksteps, n, bar);
         }
-        tile_to_planes(tile, (int)kca, nfeat, planes, Bp, row0, gt);
+        __syncwarp();
+        tile_to_planes(a0, (int)kca, nfeat, planes, Bp, row0, gt);
     };
     const uint32_t stride = gridDim.x * kFbGroups;
     for (uint64_t tile = (uint64_t)blockIdx.x * kFbGroups + grp; !failed && tile * 128 < Bp; tile += stride) {
-        const uint64_t row = tile * 128 + gt;
-        const bool in_b = row < A.B, in_p = row < Bp;
+        const uint64_t row = tile * 128 + tr;
+        const bool in_b = row < A.B;
         float q[9];
 #pragma unroll
         for (int i = 0; i < 9; i++) q[i] = in_b ? A.q[9 * row + i] : 0.f;
         {
-            __half2 e[kGuideIn / 2];
-            guide_encode0(q, A.box, e);
-            guide_encode1(q, e + kEncode0 / 2);
+            __half2 e[kEncode0 / 2];
+            if (half == 0)
+                guide_encode0(q, A.box, e);
+            else
+                guide_encode1(q, e);
 #pragma unroll
-            for (int c = 0; c < kGuideIn / 8; c++)
-                *reinterpret_cast<uint4 *>(bufA + tc_chunk(gt, c, kGuideIn / 8)) =
-                    *reinterpret_cast<const uint4 *>(&e[4 * c]);
+            for (int c = 0; c < kEncode0 / 8; c++)
+                if (half == 0 || c < kEncode1 / 8)
+                    *reinterpret_cast<uint4 *>(bufA + tc_chunk(tr, half * (kEncode0 / 8) + c, kGuideIn / 8)) =
+                        *reinterpret_cast<const uint4 *>(&e[4 * c]);
         }
         const uint64_t row0 = tile * 128;
         // forward: X_0 (A) -> X_1 (B) -> X_2 (A) -> X_3 (B) -> X_4 (A) -> outputs
-        uint32_t mask[4][2];
-#pragma unroll 1
-        for (int l = 0; l < kGuideLayers - 1 && !failed; l++) {
+        uint32_t mask[kGuideLayers - 1];  // ReLU signs of the thread's 32 columns
+#pragma unroll
+        for (int l = 0; l < kGuideLayers - 1; l++) {
             const uint32_t src = (l & 1) ? aB : aA;
             unsigned char *dst = (l & 1) ? bufA : bufB;
-            issue(src, guide_in(l) / 8, smem_u32(sm + tc_w(l)), guide_in(l) / 8, guide_in(l) / 16, 64,
-                  (l & 1) ? bufB : bufA, guide_in(l), A.xt + (uint64_t)guide_xoff(l) * Bp, row0);
+            issue(src, guide_in(l) / 8, smem_u32(sm + tc_w(l)), guide_in(l) / 8, guide_in(l) / 16, 64, guide_in(l),
+                  A.xt + (uint64_t)guide_xoff(l) * Bp, row0);
             if (!wait_mma()) {
                 failed = true;
                 break;
             }
-            const float *b = bias + guide_ib(l);
-            uint32_t m0 = 0, m1 = 0;
+            const float *b = bias + guide_ib(l) + 32 * half;
+            uint32_t m = 0;
 #pragma unroll
-            for (int h = 0; h < 4; h++) {
+            for (int h = 0; h < 2; h++) {
                 float v[16];
-                tmem_ld16(tlane + 16u * h, v);
+                tmem_ld16(tlane + 32u * half + 16u * h, v);
                 uint32_t w[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
                     w[j] = relu_half2(v[2 * j] + b[16 * h + 2 * j], v[2 * j + 1] + b[16 * h + 2 * j + 1]);
                     const __half2 hv = *reinterpret_cast<const __half2 *>(&w[j]);
                     const uint32_t bits = (__low2float(hv) > 0.f ? 1u : 0u) | (__high2float(hv) > 0.f ? 2u : 0u);
-                    const int f = 16 * h + 2 * j;
-                    if (f < 32)
-                        m0 |= bits << f;
-                    else
-                        m1 |= bits << (f - 32);
+                    m |= bits << (16 * h + 2 * j);
                 }
-                *reinterpret_cast<uint4 *>(dst + tc_chunk(gt, 2 * h, 8)) = make_uint4(w[0], w[1], w[2], w[3]);
-                *reinterpret_cast<uint4 *>(dst + tc_chunk(gt, 2 * h + 1, 8)) = make_uint4(w[4], w[5], w[6], w[7]);
+                *reinterpret_cast<uint4 *>(dst + tc_chunk(tr, 4 * half + 2 * h, 8)) = make_uint4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<uint4 *>(dst + tc_chunk(tr, 4 * half + 2 * h + 1, 8)) =
+                    make_uint4(w[4], w[5], w[6], w[7]);
             }
-            mask[l][0] = m0;
-            mask[l][1] = m1;
+            mask[l] = m;
         }
         if (failed) break;
-        issue(aA, 8, smem_u32(sm + tc_w(4)), 8, 4, kGuideOut, bufA, kGuideHidden, A.xt + (uint64_t)guide_xoff(4) * Bp,
-              row0);
+        issue(aA, 8, smem_u32(sm + tc_w(4)), 8, 4, kGuideOut, kGuideHidden, A.xt + (uint64_t)guide_xoff(4) * Bp, row0);
         if (!wait_mma()) {
             failed = true;
             break;
         }
         {
-            float o[kGuideOut];
-#pragma unroll
-            for (int h = 0; h < kGuideOut / 16; h++) tmem_ld16(tlane + 16u * h, o + 16 * h);
+            float o[16], oa[16];  // the thread's lobes; outputs 32..47 (alpha first)
+            tmem_ld16(tlane + 16u * half, o);
+            tmem_ld16(tlane + 32u, oa);
             const float *b = bias + guide_ib(4);
 #pragma unroll
-            for (int j = 0; j < kGuideOut; j++) o[j] += b[j];
-            float dout[kGuideOut];
+            for (int j = 0; j < 16; j++) o[j] += b[16 * half + j];
+            GuideLossLobes L[kLossLobes];
+            float wt = 0.f, pdfb = 0.f;
+            V3 wi = v3(0.f, 0.f, 1.f);
             if (in_b) {
-                const float wt = fminf(A.w[row] * winv, kGuideWeightClip);
-                const V3 wi = v3(A.dir[3 * row], A.dir[3 * row + 1], A.dir[3 * row + 2]);
-                lsum += guide_loss_grad(o, wi, A.pdf[row], wt, dout);
+                wt = fminf(A.w[row] * winv, kGuideWeightClip);
+                wi = v3(A.dir[3 * row], A.dir[3 * row + 1], A.dir[3 * row + 2]);
+                pdfb = A.pdf[row];
+            }
+            const GuideLossPart mine = guide_loss_lobes(o, wi, L);
+            // X_4, in buffer A, has been read by the product and copied to its planes
+            float4 *part = reinterpret_cast<float4 *>(bufA);
+            part[2 * tr + half] = make_float4(mine.lmax, mine.lsum, mine.vmax, mine.vsum);
+            group_sync_or<kFbThreads>(bar_id, false);
+            const float4 p0 = part[2 * tr], p1 = part[2 * tr + 1];
+            float dout[24], loss;
+            const float log_v = guide_loss_finish(o, wi, wt, L, GuideLossPart{p0.x, p0.y, p0.z, p0.w},
+                                                  GuideLossPart{p1.x, p1.y, p1.z, p1.w}, dout, &loss);
+            // outputs 32..39 to the first half, 40..47 to the second
+#pragma unroll
+            for (int j = 16; j < 24; j++) dout[j] = 0.f;
+            if (half == 0) dout[16] = guide_loss_alpha(oa[0] + b[32], log_v, pdfb, wt);
+            if (in_b) {
+                if (half == 0) lsum += loss;
             } else {
 #pragma unroll
-                for (int j = 0; j < kGuideOut; j++) dout[j] = 0.f;
-            }
-            uint32_t w[kGuideOut / 2];
-#pragma unroll
-            for (int j = 0; j < kGuideOut / 2; j++) {
-                const __half2 hv =
-                    __floats2half2_rn(dout[2 * j] * (1.f / kGuideGradScale), dout[2 * j + 1] * (1.f / kGuideGradScale));
-                w[j] = *reinterpret_cast<const uint32_t *>(&hv);
+                for (int j = 0; j < 24; j++) dout[j] = 0.f;
             }
 #pragma unroll
-            for (int c = 0; c < kGuideOut / 8; c++)
-                *reinterpret_cast<uint4 *>(bufB + tc_chunk(gt, c, kGuideOut / 8)) =
-                    make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+            for (int c = 0; c < 3; c++) {
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const __half2 hv = __floats2half2_rn(dout[8 * c + 2 * j] * (1.f / kGuideGradScale),
+                                                         dout[8 * c + 2 * j + 1] * (1.f / kGuideGradScale));
+                    w[j] = *reinterpret_cast<const uint32_t *>(&hv);
+                }
+                *reinterpret_cast<uint4 *>(bufB + tc_chunk(tr, c < 2 ? 2 * half + c : 4 + half, kGuideOut / 8)) =
+                    make_uint4(w[0], w[1], w[2], w[3]);
+            }
         }
         // backward: G_4 (B) -> G_3 (A) -> G_2 (B) -> G_1 (A) -> G_0 (planes only)
-#pragma unroll 1
-        for (int l = kGuideLayers - 1; l >= 1 && !failed; l--) {
+#pragma unroll
+        for (int l = kGuideLayers - 1; l >= 1; l--) {
             const uint32_t src = (l & 1) ? aA : aB;  // l = 4: G_4 in B; 3: G_3 in A; ...
             unsigned char *dst = (l & 1) ? bufB : bufA;
             const int kco = guide_out(l) / 8;
-            issue(src, kco, smem_u32(sm + fb_wb(l)), kco, guide_out(l) / 16, 64, (l & 1) ? bufA : bufB, guide_out(l),
+            issue(src, kco, smem_u32(sm + fb_wb(l)), kco, guide_out(l) / 16, 64, guide_out(l),
                   A.gt + (uint64_t)guide_goff(l) * Bp, row0);
             if (!wait_mma()) {
                 failed = true;
                 break;
             }
-            const uint32_t m0 = mask[l - 1][0], m1 = mask[l - 1][1];
+            const uint32_t m = mask[l - 1];
 #pragma unroll
-            for (int h = 0; h < 4; h++) {
+            for (int h = 0; h < 2; h++) {
                 float v[16];
-                tmem_ld16(tlane + 16u * h, v);
+                tmem_ld16(tlane + 32u * half + 16u * h, v);
                 uint32_t w[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    const int f = 16 * h + 2 * j;
-                    const uint32_t bits = f < 32 ? (m0 >> f) : (m1 >> (f - 32));
+                    const uint32_t bits = m >> (16 * h + 2 * j);
                     const __half2 hv = __floats2half2_rn((bits & 1u) ? v[2 * j] : 0.f, (bits & 2u) ? v[2 * j + 1] : 0.f);
                     w[j] = *reinterpret_cast<const uint32_t *>(&hv);
                 }
-                *reinterpret_cast<uint4 *>(dst + tc_chunk(gt, 2 * h, 8)) = make_uint4(w[0], w[1], w[2], w[3]);
-                *reinterpret_cast<uint4 *>(dst + tc_chunk(gt, 2 * h + 1, 8)) = make_uint4(w[4], w[5], w[6], w[7]);
-            }
-            if (l == 1) {  // G_0 feeds no further product: only its planes
-                group_sync_or(bar_id, false);
-                tile_to_planes(dst, 8, kGuideHidden, A.gt, Bp, row0, gt);
+                *reinterpret_cast<uint4 *>(dst + tc_chunk(tr, 4 * half + 2 * h, 8)) = make_uint4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<uint4 *>(dst + tc_chunk(tr, 4 * half + 2 * h + 1, 8)) =
+                    make_uint4(w[4], w[5], w[6], w[7]);
             }
         }
+        if (failed) break;
+        // G_0 feeds no further product: only its planes
+        group_sync_or<kFbThreads>(bar_id, false);
+        tile_to_planes(aB, 8, kGuideHidden, A.gt, Bp, row0, gt);
     }
     if (failed) {
         if (gt == 0) atomicOr(reinterpret_cast<uint32_t *>(A.scal) + 2, 2u);  // tensor-core wait ran out
@@ -325,10 +334,13 @@ __global__ void __launch_bounds__(128 * kFbGroups, 1) k_guide_train_tc(const uin
 // k_guide_wgrad_tc: dW_l^T = G_l^T X_l over a chunk of rows, all five layers, on tcgen05. The
 // feature-major planes are K-major operands with the rows as K: A = G_l^T (M = 128 lanes, the
 // out_l valid ones first; the rest of the tile is the next layer's rows or unused bytes, whose
-// products land in TMEM lanes nobody reads), B = X_l^T (N = in_l). Stages of 64 rows are loaded
-// into one of two shared-memory buffers while the tensor core works on the other; the five
-// accumulators (144 + 4 x 64 TMEM columns) stay in TMEM for the whole chunk, which then writes
-// its FP32 partial dW in the master layout.
+// products land in TMEM lanes nobody reads), B = X_l^T (N = in_l) and a row of ones, whose product is
+// the bias gradient: the last of the input's zero features, and 16 more rows for the other layers.
+// Stages of 64 rows are copied (cp.async) into one of two shared-memory buffers while the tensor core
+// works on the other; the five accumulators (144 + 4 x 80 TMEM columns) stay in TMEM for the whole
+// chunk, which then writes its FP32 partial gradients in the master layout.
+// A chunk of the usual batch (37,888 rows) has four stages, and loading them bounds it: 35 us with 128
+// threads that loaded and stored 16 bytes at a time, 23 us so; the bias gradient was 15 us by itself.
 // rows per CTA: a multiple of 64 chosen per step so the chunks about cover the SMs once
 __host__ __device__ inline uint64_t wgrad_chunk(uint64_t Bp, uint32_t sms)
 {
@@ -336,17 +348,33 @@ __host__ __device__ inline uint64_t wgrad_chunk(uint64_t Bp, uint32_t sms)
     return c < 256 ? 256 : c;
 }
 constexpr int kWgStageA = 5 * 8192 + 8192;         // G^T tiles: layer l at l * 8 KB (64 valid rows)
-constexpr int kWgStageB = 18 * 1024 + 4 * 8192;    // X^T tiles: layer 0 (144 rows), layers 1-4 (64)
+constexpr int kWgStageB = 18 * 1024 + 4 * 10240;   // X^T tiles: layer 0 (144 rows), layers 1-4 (80)
+constexpr int kWgThreads = 256;
 constexpr int kWgStage = kWgStageA + kWgStageB;
 constexpr int kWgBar = 2 * kWgStage;
 constexpr int kWgSmem = kWgBar + 16 + 16;
 constexpr int kWgTmemCols = 512;
 static_assert(kWgSmem <= 227 * 1024, "weight-gradient shared memory");
-__host__ __device__ constexpr int wg_b(int l) { return kWgStageA + (l == 0 ? 0 : 18 * 1024 + (l - 1) * 8192); }
-__host__ __device__ constexpr int wg_col(int l) { return l == 0 ? 0 : kGuideIn + (l - 1) * 64; }
+__host__ __device__ constexpr int wg_b(int l) { return kWgStageA + (l == 0 ? 0 : 18 * 1024 + (l - 1) * 10240); }
+__host__ __device__ constexpr int wg_n(int l) { return l == 0 ? kGuideIn : 80; }  // the ones: row wg_ones(l)
+__host__ __device__ constexpr int wg_ones(int l) { return l == 0 ? kGuideIn - 1 : kGuideHidden; }
+__host__ __device__ constexpr int wg_col(int l) { return l == 0 ? 0 : kGuideIn + (l - 1) * 80; }
+static_assert(wg_col(4) + wg_n(4) <= kWgTmemCols, "weight-gradient TMEM");
 
-__global__ void __launch_bounds__(128, 1) k_guide_wgrad_tc(const __half *xt, const __half *gt, uint64_t Bp,
-                                                           uint64_t chunk, float *partial, float *scal)
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all but the latest `pending` groups of copies have arrived
+template <int pending>
+__device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(pending) : "memory");
+}
+
+__global__ void __launch_bounds__(kWgThreads, 1) k_guide_wgrad_tc(const __half *xt, const __half *gt, uint64_t Bp,
+                                                                  uint64_t chunk, float *partial, float *scal)
 {
     extern __shared__ __align__(128) unsigned char wg_smem[];
     unsigned char *sm = wg_smem;
@@ -362,73 +390,99 @@ __global__ void __launch_bounds__(128, 1) k_guide_wgrad_tc(const __half *xt, con
     }
     __syncwarp();
     if (warp == 0) tmem_alloc(tslot, kWgTmemCols);
+    // stage s to its buffer: G^T, 304 features x 8 chunks of 8 rows; X^T: 400 features x 8 chunks, without
+    // the row of ones
+    auto load = [&](int s) {
+        const uint32_t buf = smem_u32(sm + (s & 1) * kWgStage);
+        const uint64_t rs = r0 + 64ull * s;
+        // eight lanes take eight features, one row of a core matrix each: their stores fill 128 bytes
+        for (int i = tid; i < kGuideGFeatures * 8; i += kWgThreads) {
+            const int f = 8 * (i >> 6) + (i & 7), c = (i >> 3) & 7;
+            const int l = f < 4 * kGuideHidden ? f / kGuideHidden : 4, fl = f - guide_goff(l);
+            copy16_async(buf + l * 8192 + tc_chunk(fl, c, 8), gt + (uint64_t)f * Bp + rs + 8 * c);
+        }
+        for (int i = tid; i < kGuideXFeatures * 8; i += kWgThreads) {
+            const int f = 8 * (i >> 6) + (i & 7), c = (i >> 3) & 7;
+            const int l = f < kGuideIn ? 0 : 1 + (f - kGuideIn) / kGuideHidden, fl = f - guide_xoff(l);
+            if (f != wg_ones(0)) copy16_async(buf + wg_b(l) + tc_chunk(fl, c, 8), xt + (uint64_t)f * Bp + rs + 8 * c);
+        }
+    };
+    for (int s = 0; s < 2; s++) {
+        if (s < nstages) load(s);
+        copy_commit();
+        // rows of ones: feature 143 of layer 0, rows 64..79 of the others
+        const uint32_t one2 = 0x3C003C00u;
+        for (int i = tid; i < (1 + 4 * 16) * 8; i += kWgThreads) {
+            const int r = i >> 3, c = i & 7;
+            const int l = r == 0 ? 0 : 1 + (r - 1) / 16;
+            *reinterpret_cast<uint4 *>(sm + s * kWgStage + wg_b(l) +
+                                       tc_chunk(r == 0 ? wg_ones(0) : kGuideHidden + (r - 1) % 16, c, 8)) =
+                make_uint4(one2, one2, one2, one2);
+        }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
     uint32_t phase[2] = {0u, 0u};
     bool failed = false;
-    for (int s = 0; s < nstages && !failed; s++) {
+    for (int s = 0; s < nstages; s++) {
         const int b = s & 1;
-        unsigned char *buf = sm + b * kWgStage;
-        if (s >= 2) {  // the MMAs of stage s - 2 read this buffer
-            const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar + b, phase[b], kUmmaWaitPolls));
-            phase[b] ^= 1u;
-            failed = __syncthreads_or(!ok) != 0;
-            if (failed) break;
-        }
-        const uint64_t rs = r0 + 64ull * s;
-        // G^T: 304 features x 8 chunks of 8 rows; X^T: 400 features x 8 chunks
-        for (int i = tid; i < kGuideGFeatures * 8; i += 128) {
-            const int f = i >> 3, c = i & 7;
-            const int l = f < 4 * kGuideHidden ? f / kGuideHidden : 4, fl = f - guide_goff(l);
-            *reinterpret_cast<uint4 *>(buf + l * 8192 + tc_chunk(fl, c, 8)) =
-                __ldg(reinterpret_cast<const uint4 *>(gt + (uint64_t)f * Bp + rs) + c);
-        }
-        for (int i = tid; i < kGuideXFeatures * 8; i += 128) {
-            const int f = i >> 3, c = i & 7;
-            const int l = f < kGuideIn ? 0 : 1 + (f - kGuideIn) / kGuideHidden, fl = f - guide_xoff(l);
-            *reinterpret_cast<uint4 *>(buf + wg_b(l) + tc_chunk(fl, c, 8)) =
-                __ldg(reinterpret_cast<const uint4 *>(xt + (uint64_t)f * Bp + rs) + c);
-        }
+        copy_wait<1>();
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t base = smem_u32(buf);
+            const uint32_t base = smem_u32(sm + b * kWgStage);
 #pragma unroll 1
             for (int l = 0; l < kGuideLayers; l++) {
-                const uint32_t idesc = umma_idesc_f16(128, guide_in(l));
+                const uint32_t idesc = umma_idesc_f16(128, wg_n(l));
                 for (int k = 0; k < 4; k++)
                     umma_f16(tmem + (uint32_t)wg_col(l), umma_desc(base + l * 8192 + 256u * k, 128u, 1024u),
                              umma_desc(base + wg_b(l) + 256u * k, 128u, 1024u), idesc, (s > 0 || k > 0) ? 1u : 0u);
             }
             umma_commit(bar + b);
         }
+        __syncwarp();
+        // stage s + 2 takes this buffer once the products have read it
+        if (s + 2 < nstages) {
+            const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar + b, phase[b], kUmmaWaitPolls));
+            phase[b] ^= 1u;
+            failed = __syncthreads_or(!ok) != 0;
+            if (failed) break;
+            load(s + 2);
+        }
+        copy_commit();
     }
+    copy_wait<0>();
     // the last batch of each buffer
     for (int b = 0; b < 2 && !failed; b++) {
-        const int last = nstages - 1 - ((nstages - 1 - b) & 1);  // latest stage that used buffer b
-        if (last < 0 || last < nstages - 2) continue;
+        if (b >= nstages) continue;
         const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar + b, phase[b], kUmmaWaitPolls));
         phase[b] ^= 1u;
         failed = __syncthreads_or(!ok) != 0;
     }
     tc_fence_after();
     float *part = partial + (uint64_t)blockIdx.x * kGuideParamCount;
-    if (!failed && warp < 2) {  // TMEM lanes 0..63: the output features
-        const int o = 32 * warp + (tid & 31);
-        const uint32_t tl = tmem + ((uint32_t)(32 * warp) << 16);
-#pragma unroll 1
+    if (!failed && (warp & 2) == 0) {  // TMEM lanes 0..63: the output features; two warps each
+        const int o = 32 * (warp & 1) + (tid & 31);
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 1)) << 16);
+#pragma unroll
         for (int l = 0; l < kGuideLayers; l++) {
-            const int nin = guide_in(l), out = guide_out(l);
-            for (int c0 = 0; c0 < nin; c0 += 16) {
+            const int out = guide_out(l);
+            float *w = part + guide_pw(l) + o;
+#pragma unroll 1
+            for (int c0 = 16 * (warp >> 2); c0 < wg_n(l); c0 += 32) {
                 float v[16];
                 tmem_ld16(tl + (uint32_t)(wg_col(l) + c0), v);
-                if (o < out)
+                if (o >= out) continue;
+                // the ones are the first column of their 16 for l > 0 and the last for l = 0
+                if (c0 == wg_ones(l) / 16 * 16) part[guide_pb(l) + o] = v[wg_ones(l) % 16];
+                if (l > 0 && c0 == wg_ones(l)) continue;
+                if (l == 0 && c0 == wg_ones(0) / 16 * 16) v[wg_ones(0) % 16] = 0.f;
 #pragma unroll
-                    for (int j = 0; j < 16; j++) part[guide_pw(l) + (c0 + j) * out + o] = v[j];
+                for (int j = 0; j < 16; j++) w[(c0 + j) * out] = v[j];
             }
         }
     }
@@ -442,34 +496,6 @@ __global__ void __launch_bounds__(128, 1) k_guide_wgrad_tc(const __half *xt, con
     if (warp == 0) {
         __syncwarp();
         tmem_dealloc(tmem, kWgTmemCols);
-    }
-}
-
-// db_l = sum of G_l over the chunk's rows (feature-major planes), one warp per 8 features
-__global__ void __launch_bounds__(256) k_guide_bias_grad(const __half *gt, uint64_t Bp, uint64_t chunk, float *partial)
-{
-    const uint64_t r0 = (uint64_t)blockIdx.x * chunk;
-    const uint64_t r1 = r0 + chunk < Bp ? r0 + chunk : Bp;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *part = partial + (uint64_t)blockIdx.x * kGuideParamCount;
-    for (int f = blockIdx.y * 64 + warp; f < kGuideGFeatures && f < (int)blockIdx.y * 64 + 64; f += 8) {
-        const uint4 *g4 = reinterpret_cast<const uint4 *>(gt + (uint64_t)f * Bp + r0);
-        float s = 0.f;
-        for (uint64_t i = lane; i < (r1 - r0) / 8; i += 32) {
-            const uint4 v = __ldg(g4 + i);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&w[k]));
-                s += h.x + h.y;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-            const int l = f < 4 * kGuideHidden ? f / kGuideHidden : 4;
-            part[guide_pb(l) + (f - guide_goff(l))] = s;
-        }
     }
 }
 
@@ -707,13 +733,10 @@ int guide_train(rt_guide *g, const float *q, const float *dir, const float *pdf,
     const uint64_t tiles = Bp / 128;
     const unsigned grid =
         (unsigned)std::min<uint64_t>((tiles + kFbGroups - 1) / kFbGroups, (uint64_t)std::max(g->ctx->sm_count, 1));
-    k_guide_train_tc<<<grid, 128 * kFbGroups, kFbSmem, st>>>(g->img.as<uint4>(), a);
+    k_guide_train_tc<<<grid, kFbThreads * kFbGroups, kFbSmem, st>>>(g->img.as<uint4>(), a);
     RTB_CUDA(cudaGetLastError());
-    k_guide_wgrad_tc<<<nchunks, 128, kWgSmem, st>>>(g->xt.as<__half>(), g->gt.as<__half>(), Bp, chunk,
+    k_guide_wgrad_tc<<<nchunks, kWgThreads, kWgSmem, st>>>(g->xt.as<__half>(), g->gt.as<__half>(), Bp, chunk,
                                                     g->partial.as<float>(), scal);
-    RTB_CUDA(cudaGetLastError());
-    k_guide_bias_grad<<<dim3(nchunks, (kGuideGFeatures + 63) / 64), 256, 0, st>>>(g->gt.as<__half>(), Bp, chunk,
-                                                                              g->partial.as<float>());
     RTB_CUDA(cudaGetLastError());
     const unsigned pblocks = (kGuideParamCount + 255) / 256;
     k_guide_reduce<<<pblocks, 256, 0, st>>>(g->partial.as<float>(), nchunks, kGuideGradScale / (float)B,

@@ -231,66 +231,90 @@ __device__ __forceinline__ V3 guide_sample(const GuideParams &P, float u0, float
 //   loss = -wt * log V(wi) + wt^2 * qc / q,   q = alpha * Vc + (1 - alpha) * pdf_bsdf,
 // V the vMF mixture; Vc and qc are V and q held constant (the second term trains alpha only;
 // its value is wt^2). log V is a log-sum-exp over the lobes, so samples far from every lobe
-// keep a gradient.
-// dout[0..47] receives the gradient (clamped to +-kGuideGradClamp; 0 for the unused outputs).
-__device__ __forceinline__ float guide_loss_grad(const float *o, V3 wi, float pdfb, float wt, float *dout)
+// keep a gradient. Two threads share a row, half the lobes each: both compute their lobes'
+// terms (guide_loss_lobes), exchange the four numbers of GuideLossPart and finish with their sum.
+constexpr int kLossLobes = kGuideLobes / 2;
+
+struct GuideLossPart {
+    float lmax, lsum;  // of the lobes' weight logits: largest, sum of exp(logit - largest)
+    float vmax, vsum;  // of their log densities (without the softmax's normalisation): the same
+};
+
+struct GuideLossLobes {
+    float th, ph, sk;      // sigmoids of the angles and of log kappa
+    float st, ct, sp, cp;  // of the angles
+    float k, cj, lv;       // kappa, cosine to wi, log density before the softmax's normalisation
+};
+
+// o: the 4 raw outputs of each of the thread's lobes
+__device__ __forceinline__ GuideLossPart guide_loss_lobes(const float *o, V3 wi, GuideLossLobes *L)
 {
-    float lmax = o[3];
+    GuideLossPart p{-INFINITY, 0.f, -INFINITY, 0.f};
 #pragma unroll
-    for (int j = 1; j < kGuideLobes; j++) lmax = fmaxf(lmax, o[4 * j + 3]);
-    float se = 0.f;
-#pragma unroll
-    for (int j = 0; j < kGuideLobes; j++) se += expf(o[4 * j + 3] - lmax);
-    const float lse_l = lmax + logf(se);
-    float ls[kGuideLobes], kap[kGuideLobes], cj[kGuideLobes];
-    float lsmax = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < kGuideLobes; j++) {
-        const float th = 3.14159265358979f * guide_sigmoid(o[4 * j]);
-        const float ph = 6.28318530717959f * guide_sigmoid(o[4 * j + 1]);
-        const float lk = kGuideLogKappaMin + kGuideLogKappaSpan * guide_sigmoid(o[4 * j + 2]);
-        kap[j] = expf(lk);
-        float st, ct, sp, cp;
-        sincosf(th, &st, &ct);
-        sincosf(ph, &sp, &cp);
-        cj[j] = st * cp * wi.x + st * sp * wi.y + ct * wi.z;
-        // log(lam_j * norm_j * exp(kappa_j (c_j - 1)))
-        ls[j] = (o[4 * j + 3] - lse_l) + lk - 1.83787706640935f - logf(-expm1f(-2.f * kap[j])) +
-                kap[j] * (cj[j] - 1.f);
-        lsmax = fmaxf(lsmax, ls[j]);
+    for (int j = 0; j < kLossLobes; j++) {
+        GuideLossLobes &l = L[j];
+        l.th = guide_sigmoid(o[4 * j]);
+        l.ph = guide_sigmoid(o[4 * j + 1]);
+        l.sk = guide_sigmoid(o[4 * j + 2]);
+        const float lk = kGuideLogKappaMin + kGuideLogKappaSpan * l.sk;
+        l.k = expf(lk);
+        sincosf(3.14159265358979f * l.th, &l.st, &l.ct);
+        sincosf(6.28318530717959f * l.ph, &l.sp, &l.cp);
+        l.cj = l.st * l.cp * wi.x + l.st * l.sp * wi.y + l.ct * wi.z;
+        // log(norm_j * exp(kappa_j (c_j - 1))) + logit_j
+        l.lv = o[4 * j + 3] + lk - 1.83787706640935f - logf(-expm1f(-2.f * l.k)) + l.k * (l.cj - 1.f);
+        p.lmax = fmaxf(p.lmax, o[4 * j + 3]);
+        p.vmax = fmaxf(p.vmax, l.lv);
     }
-    float sv = 0.f;
 #pragma unroll
-    for (int j = 0; j < kGuideLobes; j++) sv += expf(ls[j] - lsmax);
-    const float logV = lsmax + logf(sv);
-    const float V = expf(logV);
-    const float sa = guide_sigmoid(o[32]);
+    for (int j = 0; j < kLossLobes; j++) {
+        p.lsum += expf(o[4 * j + 3] - p.lmax);
+        p.vsum += expf(L[j].lv - p.vmax);
+    }
+    return p;
+}
+
+__device__ __forceinline__ float guide_clamp_grad(float g)
+{
+    return fminf(fmaxf(g, -kGuideGradClamp), kGuideGradClamp);
+}
+
+// p, q: the parts of the first and the second half of the lobes. dout receives the gradient with
+// respect to o (clamped to +-kGuideGradClamp), *loss the sample's loss; returns log V.
+__device__ __forceinline__ float guide_loss_finish(const float *o, V3 wi, float wt, const GuideLossLobes *L,
+                                                   const GuideLossPart &p, const GuideLossPart &q, float *dout,
+                                                   float *loss)
+{
+    const float lmax = fmaxf(p.lmax, q.lmax), vmax = fmaxf(p.vmax, q.vmax);
+    const float lse = lmax + logf(p.lsum * expf(p.lmax - lmax) + q.lsum * expf(q.lmax - lmax));
+    const float lsv = vmax + logf(p.vsum * expf(p.vmax - vmax) + q.vsum * expf(q.vmax - vmax));
+#pragma unroll
+    for (int j = 0; j < kLossLobes; j++) {
+        const GuideLossLobes &l = L[j];
+        const float r = expf(l.lv - lsv);  // share of lobe j in V(wi)
+        const float lam = expf(o[4 * j + 3] - lse);
+        const float dth = r * l.k * (l.ct * l.cp * wi.x + l.ct * l.sp * wi.y - l.st * wi.z) * 3.14159265358979f * l.th *
+                          (1.f - l.th);
+        const float dph = r * l.k * (-l.st * l.sp * wi.x + l.st * l.cp * wi.y) * 6.28318530717959f * l.ph * (1.f - l.ph);
+        const float dk = r * (1.f - 2.f * l.k / expm1f(2.f * l.k) + l.k * (l.cj - 1.f)) * kGuideLogKappaSpan * l.sk *
+                         (1.f - l.sk);
+        dout[4 * j + 0] = guide_clamp_grad(-wt * dth);
+        dout[4 * j + 1] = guide_clamp_grad(-wt * dph);
+        dout[4 * j + 2] = guide_clamp_grad(-wt * dk);
+        dout[4 * j + 3] = guide_clamp_grad(-wt * (r - lam));
+    }
+    const float log_v = lsv - lse;
+    *loss = -wt * log_v + wt * wt;
+    return log_v;
+}
+
+// gradient with respect to the raw alpha output
+__device__ __forceinline__ float guide_loss_alpha(float o, float log_v, float pdfb, float wt)
+{
+    const float v = expf(log_v), sa = guide_sigmoid(o);
     const float alpha = kGuideAlphaMin + kGuideAlphaSpan * sa;
-    const float q = fmaxf(alpha * V + (1.f - alpha) * pdfb, 1e-30f);
-    auto clampg = [](float g) { return fminf(fmaxf(g, -kGuideGradClamp), kGuideGradClamp); };
-#pragma unroll
-    for (int j = 0; j < kGuideLobes; j++) {
-        const float sth = guide_sigmoid(o[4 * j]), sph = guide_sigmoid(o[4 * j + 1]);
-        const float th = 3.14159265358979f * sth, ph = 6.28318530717959f * sph;
-        float st, ct, sp, cp;
-        sincosf(th, &st, &ct);
-        sincosf(ph, &sp, &cp);
-        const float r = expf(ls[j] - logV);  // share of lobe j in V(wi)
-        const float k = kap[j];
-        const float lam = expf(o[4 * j + 3] - lse_l);
-        const float dth = r * k * (ct * cp * wi.x + ct * sp * wi.y - st * wi.z) * 3.14159265358979f * sth * (1.f - sth);
-        const float dph = r * k * (-st * sp * wi.x + st * cp * wi.y) * 6.28318530717959f * sph * (1.f - sph);
-        const float sk = guide_sigmoid(o[4 * j + 2]);
-        const float dk = r * (1.f - 2.f * k / expm1f(2.f * k) + k * (cj[j] - 1.f)) * kGuideLogKappaSpan * sk * (1.f - sk);
-        dout[4 * j + 0] = clampg(-wt * dth);
-        dout[4 * j + 1] = clampg(-wt * dph);
-        dout[4 * j + 2] = clampg(-wt * dk);
-        dout[4 * j + 3] = clampg(-wt * (r - lam));
-    }
-    dout[32] = clampg(-wt * wt * (V - pdfb) / q * kGuideAlphaSpan * sa * (1.f - sa));
-#pragma unroll
-    for (int i = 33; i < kGuideOut; i++) dout[i] = 0.f;
-    return -wt * logV + wt * wt;
+    const float q = fmaxf(alpha * v + (1.f - alpha) * pdfb, 1e-30f);
+    return guide_clamp_grad(-wt * wt * (v - pdfb) / q * kGuideAlphaSpan * sa * (1.f - sa));
 }
 
 // ------------------------------------------------------------------ tcgen05 (UMMA) primitives
@@ -392,6 +416,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// four 8x8 matrices of halves in shared memory, transposed: lane t provides the address of row t % 8
+// of matrix t / 8 and receives, of each matrix, rows 2 (t % 4) and the next of column t / 4
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t addr, uint32_t r[4])
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
 // ------------------------------------------------------------------ batched inference
 
 // Tiles of 128 rows run through the network on the tensor cores: per layer, tcgen05.mma
@@ -399,7 +433,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
 // one thread, then the 128 threads of the tile read their own row back from TMEM for bias,
 // ReLU and the FP16 store of the next layer's operand. A CTA holds one copy of the weights
 // and kInferGroups independent 128-thread groups, each with its own activation tile, TMEM
-// columns, mbarrier and named barrier, so 16 warps per SM hide each other's latency.
+// columns, mbarrier and named barrier, so 24 warps per SM hide each other's latency: bound by
+// the instructions of encoding and decoding (3,500 per row) at 60% of the issue rate. Sampling and
+// density of 1,000,003 rows: 479 / 450 / 429 us for 4 groups (the encoding in one operand) / 5 / 6.
 // Operands are K-major without swizzle, in core matrices of 8 rows x 8 halves: row r, halves
 // [8c, 8c + 8) of an operand with KC chunks per row sit at byte (r / 8) * KC * 128 + c * 128 +
 // (r % 8) * 16.
@@ -434,15 +470,16 @@ __device__ __forceinline__ uint32_t relu_half2(float a, float b)
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// barrier of the 128 threads of a group (named barrier `id`); returns whether any of them
+// barrier of the `threads` threads of a group (named barrier `id`); returns whether any of them
 // passed `v`
+template <int threads = 128>
 __device__ __forceinline__ bool group_sync_or(uint32_t id, bool v)
 {
     uint32_t r;
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, %2, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, %2, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(r)
-        : "r"((uint32_t)v), "r"(id)
+        : "r"((uint32_t)v), "r"(id), "n"(threads)
         : "memory");
     return r != 0;
 }
