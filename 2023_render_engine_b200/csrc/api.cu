@@ -249,6 +249,10 @@ int rt_context_create(int device, rt_context **out)
     }
     c->own_stream = true;
     create_pool(c);
+    if (cudaHostAlloc(&c->status_page, 4096, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->status_page = nullptr;
+    }
     *out = c;
     return RT_OK;
 }
@@ -259,6 +263,7 @@ int rt_context_destroy(rt_context *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     destroy_pool(ctx);
+    if (ctx->status_page) cudaFreeHost(ctx->status_page);
     delete ctx;
     return RT_OK;
 }
@@ -289,10 +294,19 @@ int rt_scene_create(rt_context *ctx, rt_scene **out)
     rt_scene *s = new rt_scene();
     s->ctx = ctx;
     for (DevBuf *b : {&s->d_nodes, &s->d_tris, &s->d_leafpos, &s->d_ref_boxes, &s->d_ref_sorted, &s->d_ref_pos,
-                      &s->d_spheres, &s->scratch.counters, &s->h2d_rays, &s->d2h_hits, &s->any_hits, &s->d_mats,
+                      &s->d_spheres, &s->scratch.counters, &s->scratch.call, &s->h2d_rays, &s->d2h_hits, &s->any_hits,
+                      &s->d_mats,
                       &s->d_tri_mat, &s->d_tri_shape, &s->d_tri_nidx, &s->d_normals, &s->d_emit_tri, &s->d_emit_cdf,
                       &s->d_plights, &s->d_rec_mat, &s->d_tri_transp, &s->d_mat_transp})
         b->ctx = ctx;
+    {
+        std::lock_guard<std::mutex> lk(ctx->status_mu);
+        if (ctx->status_page && ctx->status_free) {
+            const int slot = __builtin_ctzll(ctx->status_free);
+            ctx->status_free &= ctx->status_free - 1;
+            s->scratch.status = ctx->status_page + 16 * slot;
+        }
+    }
     *out = s;
     return RT_OK;
 }
@@ -307,6 +321,10 @@ int rt_scene_destroy(rt_scene *s)
                       &s->d_tri_mat, &s->d_tri_shape, &s->d_tri_nidx, &s->d_normals, &s->d_emit_tri, &s->d_emit_cdf, &s->d_plights, &s->d_rec_mat})
         b->release();
     s->rscratch.release();
+    if (s->scratch.status) {
+        std::lock_guard<std::mutex> lk(s->ctx->status_mu);
+        s->ctx->status_free |= 1ull << ((s->scratch.status - s->ctx->status_page) / 16);
+    }
     delete s;
     return RT_OK;
 }
@@ -444,6 +462,7 @@ int rt_scene_commit(rt_scene *s)
     s->render_dirty = true;
     RTB_CHECK(s->d_spheres.upload(s->spheres.data(), s->spheres.size() * sizeof(SphereRecord), st));
     RTB_CHECK(s->scratch.counters.reserve(64));
+    RTB_CHECK(s->scratch.call.reserve(64));
     RTB_CHECK(refresh_transparency(s));
     RTB_CUDA(cudaStreamSynchronize(st));
     s->build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -484,6 +503,27 @@ int rt_scene_stats_get(rt_scene *s, rt_scene_stats *out)
     return RT_OK;
 }
 
+// The counters of a trace call; end_call waits for it and reads them.
+static TraceCall begin_call(rt_scene *s)
+{
+    const TraceCall c{s->scratch.call.as<uint32_t>(), s->scratch.status, s->scratch.clean};
+    s->scratch.clean = false;  // until the call has ended well
+    return c;
+}
+
+static int end_call(rt_scene *s, uint32_t counts[3])
+{
+    cudaStream_t st = s->ctx->stream;
+    if (!s->scratch.status) RTB_CUDA(cudaMemcpyAsync(counts, s->scratch.call.ptr, 12, cudaMemcpyDeviceToHost, st));
+    RTB_CUDA(cudaStreamSynchronize(st));
+    if (s->scratch.status) {
+        const volatile uint32_t *w = s->scratch.status;
+        for (int k = 0; k < 3; k++) counts[k] = w[k];
+        s->scratch.clean = true;
+    }
+    return RT_OK;
+}
+
 static int trace_common(rt_scene *s, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags)
 {
     if (!s) return fail(RT_ERR_INVALID, "rt_trace_closest: null scene");
@@ -494,8 +534,7 @@ static int trace_common(rt_scene *s, const rt_ray *rays, uint64_t n, rt_hit *hit
     if ((reinterpret_cast<uintptr_t>(rays) | reinterpret_cast<uintptr_t>(hits)) & 15u)
         return fail(RT_ERR_INVALID, "rt_trace_closest: buffers must be 16-byte aligned");
     RTB_CUDA(cudaSetDevice(s->ctx->device));
-    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, s->scratch.counters.as<uint32_t>(),
-                                   s->ctx->stream));
+    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, begin_call(s), s->ctx->stream));
     return RT_OK;
 }
 
@@ -504,9 +543,8 @@ static int finish_trace(rt_scene *s, uint64_t n)
     s->last_rays = n;
     s->last_fallback = 0;
     if (n == 0) return RT_OK;  // nothing launched: the counters still hold an earlier call's
-    uint32_t c[4] = {0, 0, 0, 0};
-    RTB_CUDA(cudaMemcpyAsync(c, s->scratch.counters.ptr, sizeof(c), cudaMemcpyDeviceToHost, s->ctx->stream));
-    RTB_CUDA(cudaStreamSynchronize(s->ctx->stream));
+    uint32_t c[3];
+    RTB_CHECK(end_call(s, c));
     s->last_fallback = c[0];
     return check_device_status(c[1]);
 }
@@ -549,16 +587,15 @@ static int trace_any_common(rt_scene *s, const rt_ray *rays, uint64_t n, void *o
     if (flags & RT_TRACE_FAST) {
         if (bits) RTB_CHECK(s->any_hits.reserve(n));
         RTB_CHECK(launch_trace_any(s->view(), rays, n, bits ? s->any_hits.as<uint8_t>() : static_cast<uint8_t *>(out),
-                                   out, bits, flags, s->scratch.counters.as<uint32_t>(), st));
+                                   out, bits, flags, begin_call(s), st));
     } else {
         // the reference's decision: its closest hit along the unbounded ray, then t <= tmax
         RTB_CHECK(s->any_hits.reserve(n * sizeof(rt_hit)));
         RTB_CHECK(launch_trace_visible(s->view(), rays, n, s->any_hits.as<rt_hit>(), flags, out, bits,
-                                       s->scratch.counters.as<uint32_t>(), st));
+                                       begin_call(s), st));
     }
-    uint32_t c[4] = {0, 0, 0, 0};
-    RTB_CUDA(cudaMemcpyAsync(c, s->scratch.counters.ptr, sizeof(c), cudaMemcpyDeviceToHost, s->ctx->stream));
-    RTB_CUDA(cudaStreamSynchronize(s->ctx->stream));
+    uint32_t c[3];
+    RTB_CHECK(end_call(s, c));
     return check_device_status(c[1]);
 }
 

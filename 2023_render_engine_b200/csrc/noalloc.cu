@@ -69,7 +69,7 @@ extern "C" int rt_trace_closest_noalloc(rt_scene *s, const rt_ray *rays, uint64_
     uint32_t *counters = nullptr;  // cleared by the launch before the kernels run
     RTB_CHECK(scratch_for(s->ctx->device, &counters));
     cudaStream_t st = s->ctx->stream;
-    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, counters, st));
+    RTB_CHECK(launch_trace_closest(s->view(), rays, n, hits, flags, TraceCall{counters, nullptr, false}, st));
     uint32_t c[4] = {0, 0, 0, 0};
     RTB_CUDA(cudaMemcpyAsync(c, counters, sizeof(c), cudaMemcpyDeviceToHost, st));
     RTB_CUDA(cudaStreamSynchronize(st));

@@ -206,7 +206,17 @@ void build_ref_tree(const float *tri9, uint32_t n, RefTreeHost &out);
 // ---------------------------------------------------------------- kernels
 
 struct TraceScratch {
-    DevBuf counters;  // [0] rays that needed the reference tree, [1] status word, [2] replays, [3] work counter
+    DevBuf counters;  // of the renderer's and the photon passes' traces
+    // Of the trace calls: [0] rays that needed the reference tree, [1] status word, [2] replays, [3] work
+    // counter, [4] blocks that have ended. The last block leaves the first three in `status` and
+    // all of them clear.
+    DevBuf call;
+    uint32_t *status = nullptr;  // pinned host memory (rt_context::status_page); null: none was left
+    bool clean = false;          // `call` is known to be clear
+};
+struct TraceCall {
+    uint32_t *counters, *status;
+    bool clean;
 };
 
 // Internal trace flags (above the public RT_TRACE_* bits).
@@ -218,7 +228,7 @@ constexpr uint32_t kTraceRecords = 0x40000000u;
 // kTraceIds: the walk itself writes triangle ids (set by the launcher when nothing else is left to do).
 constexpr uint32_t kTraceIds = 0x20000000u;
 int launch_trace_closest(const SceneView &v, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags,
-                         uint32_t *counters, cudaStream_t s);
+                         const TraceCall &c, cudaStream_t s);
 // Same with the ray count read on the device (queues built by other kernels); cap bounds it. The
 // hits are the renderer's form (kTraceRecords).
 int launch_trace_closest_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_dev, uint32_t cap, rt_hit *hits,
@@ -231,13 +241,13 @@ int launch_walk_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_de
 // than the ray's tmax. One byte per ray, or (bits) bit i % 32 of word i / 32 (the last word's bits
 // past n are 0). hits: n entries of scratch.
 int launch_trace_visible(const SceneView &v, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags, void *out,
-                         bool bits, uint32_t *counters, cudaStream_t s);
+                         bool bits, const TraceCall &c, cudaStream_t s);
 int launch_trace_counts(const SceneView &v, const rt_ray *rays, uint64_t n, uint32_t flags, bool anyhit,
                         uint32_t *counts, uint32_t *counters, cudaStream_t s);
 // Any-hit occlusion of n rays, in the same two forms. walk_out: n bytes of scratch (`out` itself
 // may serve for the byte form).
 int launch_trace_any(const SceneView &v, const rt_ray *rays, uint64_t n, uint8_t *walk_out, void *out, bool bits,
-                     uint32_t flags, uint32_t *counters, cudaStream_t s);
+                     uint32_t flags, const TraceCall &c, cudaStream_t s);
 
 // Wavefront buffers of rt_render (grown on demand, kept between calls).
 struct RenderScratch {
@@ -286,6 +296,11 @@ struct rt_context {
     // the pool is idle whichever streams its users ran on.
     cudaMemPool_t pool = nullptr;
     cudaStream_t pool_stream = nullptr;
+    // 64 slots of 64 bytes in pinned host memory, one per scene while there are some: a trace call's
+    // counters arrive there with its last kernel instead of by a copy of their own
+    uint32_t *status_page = nullptr;
+    uint64_t status_free = ~0ull;
+    std::mutex status_mu;
 };
 
 struct rt_photon_map {

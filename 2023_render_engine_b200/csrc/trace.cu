@@ -27,10 +27,76 @@ namespace {
 
 constexpr int kBlock = 128;
 
-// Scene index a ray carries in its last word (merged scenes only; 0 otherwise).
-__device__ __forceinline__ uint32_t ray_scene(const SceneView &v, const rt_ray *rays, uint64_t i)
+// What the exact walk leaves to do for a ray (ra, rb) with hit hv: the proof or the replay of the
+// reference's answer (see the file comment), its id or record, and the analytic shapes.
+__device__ __forceinline__ float4 finish_exact(const SceneView &v, float4 ra, float4 rb, uint32_t flags, float4 hv,
+                                               uint32_t *counters)
 {
-    return v.subs ? __float_as_uint(__ldg(reinterpret_cast<const float *>(rays) + 8 * i + 7)) : 0u;
+    const bool visible = (flags & kTraceVisible) != 0, shadow = (flags & RT_TRACE_SHADOW) != 0;
+    float t = hv.x, b1 = hv.z, b2 = hv.w;
+    int32_t rec = __float_as_int(hv.y), prim = rec;
+    bool replay = rec == kHitReplay;
+    const float tri_max = visible ? INFINITY : ra.w;
+    if (rec >= 0 && !replay) {
+        const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
+        const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+        prim = (int32_t)__float_as_uint(b.w);
+        const float ix = fdiv(1.0f, rb.x), iy = fdiv(1.0f, rb.y), iz = fdiv(1.0f, rb.z);
+        const float lx = fminf(fminf(a.x, b.x), c.x), ly = fminf(fminf(a.y, b.y), c.y),
+                    lz = fminf(fminf(a.z, b.z), c.z);
+        const float hx = fmaxf(fmaxf(a.x, b.x), c.x), hy = fmaxf(fmaxf(a.y, b.y), c.y),
+                    hz = fmaxf(fmaxf(a.z, b.z), c.z);
+        if (!(tri_max == INFINITY) || rb.x == 0.f || rb.y == 0.f || rb.z == 0.f ||
+            !ref_box_test(lx, ly, lz, hx, hy, hz, ra.x, ra.y, ra.z, ix, iy, iz, tri_max)) {
+            // walk the winner's ancestors in the reference tree (the root is never
+            // box-tested)
+            atomicAdd(counters, 1u);
+            uint32_t j = v.ref_pos[prim];
+            const uint32_t m = v.ntri, root = 2 * m - 2;
+            while (m > 1) {
+                const uint32_t q = m + j / 2;
+                if (q >= root) break;
+                const float2 *bx = v.ref_boxes + 3 * (size_t)q;
+                const float2 b0 = __ldg(bx), b1v = __ldg(bx + 1), b2v = __ldg(bx + 2);
+                if (!ref_box_test(b0.x, b0.y, b1v.x, b1v.y, b2v.x, b2v.y, ra.x, ra.y, ra.z, ix, iy, iz,
+                                  tri_max)) {
+                    replay = true;
+                    break;
+                }
+                j = q;
+            }
+        }
+    }
+    if (replay) {
+        const WatertightRay w = make_watertight(ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max);
+        bool overflow = false;
+        prim = replay_reference(v, w, fdiv(1.0f, rb.x), fdiv(1.0f, rb.y), fdiv(1.0f, rb.z), shadow, t, b1,
+                                b2, overflow);
+        if (overflow) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
+        atomicAdd(counters + 2, 1u);
+    }
+    if (prim < 0) t = INFINITY;
+    if ((flags & kTraceRecords) && prim >= 0) prim = (int32_t)v.leafpos[prim];
+    if (v.nspheres)
+        intersect_spheres(v, v.subs ? __float_as_uint(rb.w) : 0u, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max, shadow, t,
+                          prim, b1, b2);
+    return make_float4(t, __int_as_float(prim), b1, b2);
+}
+
+// The call's counters for the host: the last block to end writes them to `status` (pinned host memory;
+// null: the host copies them itself) and clears them for the next call. Every thread of the block calls it.
+__device__ __forceinline__ void publish_status(uint32_t *counters, uint32_t *status)
+{
+    if (!status) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(counters + 4, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    volatile uint32_t *c = counters, *out = status;
+    for (int k = 0; k < 3; k++) out[k] = c[k];
+    for (int k = 0; k < 5; k++) c[k] = 0;
+    __threadfence_system();
 }
 
 // Persistent closest-hit kernel: warps fetch rays from counters[3] until all n are done.
@@ -43,15 +109,12 @@ __device__ __forceinline__ uint32_t ray_scene(const SceneView &v, const rt_ray *
 // cannot change the decision, as a hit at t <= tmax is the nearest of all, and without one the
 // reference's offset is above tmax too unless a blocked triangle (b) lies within tmax, which
 // the walk sees and leaves to the replay.
-__global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_closest(SceneView v, const rt_ray *__restrict__ rays, uint64_t n,
-                                                          const uint32_t *__restrict__ n_dev, rt_hit *__restrict__ hits,
-                                                          uint32_t flags, uint32_t *__restrict__ counters)
+__device__ __forceinline__ uint2 walk_closest(const SceneView &v, TravWarp &scratch, const rt_ray *rays, uint64_t n,
+                                              rt_hit *hits, uint32_t flags, uint32_t *counters)
 {
-    __shared__ TravWarp scratch[kBlock / 32];
-    if (n_dev) n = min((uint64_t)*n_dev, n);
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
-    walk_queue<false, false, true>(
-        v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3, (flags & kTraceVisible) != 0,
+    return walk_queue<false, false, true>(
+        v, scratch, (uint32_t)n, counters + 3, (flags & kTraceVisible) != 0,
         [&](uint32_t i, Walk &W) {
             float4 ra, rb;
             load_ray(rays, i, ra, rb);
@@ -78,6 +141,41 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_closest(S
             }
             reinterpret_cast<float4 *>(hits)[i] = make_float4(W.bt, __int_as_float(rec), bary.x, bary.y);
         });
+}
+
+__global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_closest(SceneView v, const rt_ray *__restrict__ rays,
+                                                                               uint64_t n,
+                                                                               const uint32_t *__restrict__ n_dev,
+                                                                               rt_hit *__restrict__ hits, uint32_t flags,
+                                                                               uint32_t *__restrict__ counters)
+{
+    __shared__ TravWarp scratch[kBlock / 32];
+    if (n_dev) n = min((uint64_t)*n_dev, n);
+    walk_closest(v, scratch[threadIdx.x >> 5], rays, n, hits, flags, counters);
+}
+
+// A queue of at most 32 rays per resident warp in one launch: each warp takes one range of it, and
+// finishes the rays of that range itself once they have all ended. 997 rays of a Cornell box took
+// a memset, two kernels and a copy of the counters, 40 us a call; 29 us so.
+__global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_small(SceneView v, const rt_ray *__restrict__ rays,
+                                                                             uint64_t n, rt_hit *hits, uint32_t flags,
+                                                                             uint32_t *counters, uint32_t *status)
+{
+    __shared__ TravWarp scratch[kBlock / 32];
+    const uint2 mine = walk_closest(v, scratch[threadIdx.x >> 5], rays, n, hits, flags, counters);
+    __syncwarp();
+    if ((threadIdx.x & 31u) < mine.y) {
+        const uint32_t i = mine.x + (threadIdx.x & 31u);
+        float4 *h = reinterpret_cast<float4 *>(hits) + i;
+        if (flags & RT_TRACE_FAST) {
+            *h = finish_fast(v, rays, i, flags, *h, counters);
+        } else {
+            float4 ra, rb;
+            load_ray(rays, i, ra, rb);
+            *h = finish_exact(v, ra, rb, flags, *h, counters);
+        }
+    }
+    publish_status(counters, status);
 }
 
 // Traversal work per ray (rt_trace_counts): the persistent walk of k_trace_closest without its
@@ -114,69 +212,22 @@ __global__ void __launch_bounds__(kBlock, 8) k_trace_finish(SceneView v, const r
                                                             const uint32_t *__restrict__ n_dev,
                                                             rt_hit *__restrict__ hits, uint32_t flags,
                                                             void *__restrict__ out, bool bits,
-                                                            uint32_t *__restrict__ counters)
+                                                            uint32_t *counters, uint32_t *status)
 {
     if (n_dev) n = min((uint64_t)*n_dev, n);
-    const bool visible = (flags & kTraceVisible) != 0, shadow = (flags & RT_TRACE_SHADOW) != 0;
+    const bool visible = (flags & kTraceVisible) != 0;
     // whole warps stay in the loop (the bit mask is gathered with a ballot)
     for (uint64_t i0 = (uint64_t)blockIdx.x * kBlock; i0 < n; i0 += (uint64_t)gridDim.x * kBlock) {
         const uint64_t i = i0 + threadIdx.x;
         bool occ = false;
         if (i < n) {
-            const float4 hv = reinterpret_cast<const float4 *>(hits)[i];
             float4 ra, rb;
             load_ray(rays, i, ra, rb);
-            float t = hv.x, b1 = hv.z, b2 = hv.w;
-            int32_t rec = __float_as_int(hv.y), prim = rec;
-            bool replay = rec == kHitReplay;
-            const float tri_max = visible ? INFINITY : ra.w;
-            if (rec >= 0 && !replay) {
-                const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
-                const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-                prim = (int32_t)__float_as_uint(b.w);
-                const float ix = fdiv(1.0f, rb.x), iy = fdiv(1.0f, rb.y), iz = fdiv(1.0f, rb.z);
-                const float lx = fminf(fminf(a.x, b.x), c.x), ly = fminf(fminf(a.y, b.y), c.y),
-                            lz = fminf(fminf(a.z, b.z), c.z);
-                const float hx = fmaxf(fmaxf(a.x, b.x), c.x), hy = fmaxf(fmaxf(a.y, b.y), c.y),
-                            hz = fmaxf(fmaxf(a.z, b.z), c.z);
-                if (!(tri_max == INFINITY) || rb.x == 0.f || rb.y == 0.f || rb.z == 0.f ||
-                    !ref_box_test(lx, ly, lz, hx, hy, hz, ra.x, ra.y, ra.z, ix, iy, iz, tri_max)) {
-                    // walk the winner's ancestors in the reference tree (the root is never
-                    // box-tested)
-                    atomicAdd(counters, 1u);
-                    uint32_t j = v.ref_pos[prim];
-                    const uint32_t m = v.ntri, root = 2 * m - 2;
-                    while (m > 1) {
-                        const uint32_t q = m + j / 2;
-                        if (q >= root) break;
-                        const float2 *bx = v.ref_boxes + 3 * (size_t)q;
-                        const float2 b0 = __ldg(bx), b1v = __ldg(bx + 1), b2v = __ldg(bx + 2);
-                        if (!ref_box_test(b0.x, b0.y, b1v.x, b1v.y, b2v.x, b2v.y, ra.x, ra.y, ra.z, ix, iy, iz,
-                                          tri_max)) {
-                            replay = true;
-                            break;
-                        }
-                        j = q;
-                    }
-                }
-            }
-            if (replay) {
-                const WatertightRay w = make_watertight(ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max);
-                bool overflow = false;
-                prim = replay_reference(v, w, fdiv(1.0f, rb.x), fdiv(1.0f, rb.y), fdiv(1.0f, rb.z), shadow, t, b1,
-                                        b2, overflow);
-                if (overflow) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
-                atomicAdd(counters + 2, 1u);
-            }
-            if (prim < 0) t = INFINITY;
-            if ((flags & kTraceRecords) && prim >= 0) prim = (int32_t)v.leafpos[prim];
-            if (v.nspheres)
-                intersect_spheres(v, ray_scene(v, rays, i), ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tri_max, shadow, t,
-                                  prim, b1, b2);
+            const float4 h = finish_exact(v, ra, rb, flags, reinterpret_cast<const float4 *>(hits)[i], counters);
             if (visible)
-                occ = prim != RT_PRIM_NONE && t <= ra.w;
+                occ = __float_as_int(h.y) != RT_PRIM_NONE && h.x <= ra.w;
             else
-                reinterpret_cast<float4 *>(hits)[i] = make_float4(t, __int_as_float(prim), b1, b2);
+                reinterpret_cast<float4 *>(hits)[i] = h;
         }
         if (visible) {
             if (bits) {
@@ -187,6 +238,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_trace_finish(SceneView v, const r
             }
         }
     }
+    publish_status(counters, status);
 }
 
 // The same in fast mode (finish_fast). With nothing to do for most rays it only looks at those whose
@@ -194,21 +246,23 @@ __global__ void __launch_bounds__(kBlock, 8) k_trace_finish(SceneView v, const r
 __global__ void __launch_bounds__(kBlock, 12) k_trace_finish_fast(SceneView v, const rt_ray *__restrict__ rays, uint64_t n,
                                                                   const uint32_t *__restrict__ n_dev,
                                                                   rt_hit *__restrict__ hits, uint32_t flags,
-                                                                  uint32_t *__restrict__ counters)
+                                                                  uint32_t *counters, uint32_t *status)
 {
     if (n_dev) n = min((uint64_t)*n_dev, n);
-    if (!v.nspheres && *(volatile uint32_t *)counters == 0u) return;
+    if (!v.nspheres && *(volatile uint32_t *)counters == 0u) n = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kBlock) {
         float4 *h = reinterpret_cast<float4 *>(hits) + i;
         *h = finish_fast(v, rays, i, flags, *h, counters);
     }
+    publish_status(counters, status);
 }
 
 // Any hit before tmax (RT_TRACE_FAST occlusion): the walk writes one byte per ray, k_any_finish
 // adds the analytic shapes and packs the bits.
 __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_any(SceneView v, const rt_ray *__restrict__ rays,
                                                                           uint64_t n, uint8_t *__restrict__ occluded,
-                                                                          uint32_t flags, uint32_t *__restrict__ counters)
+                                                                          uint32_t flags, uint32_t *counters,
+                                                                          uint32_t *status)
 {
     __shared__ TravWarp scratch[kBlock / 32];
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
@@ -223,6 +277,7 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_any(Scene
             if (!W.ok) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
             occluded[i] = (W.brec != kNoRec && W.bt < W.lim) ? 1 : 0;
         });
+    publish_status(counters, status);
 }
 
 template <bool BITS>
@@ -280,36 +335,54 @@ static int launch_walk(const SceneView &v, const rt_ray *rays, uint64_t n, const
     return RT_OK;
 }
 
+// Fast, triangles only, ids wanted: the walk writes the ids itself; what is left are the rays whose walk
+// could not finish, and their replays give ids.
+static uint32_t walk_flags(const SceneView &v, uint32_t flags)
+{
+    return (flags & RT_TRACE_FAST) && !v.nspheres && !(flags & kTraceRecords) ? flags | kTraceIds : flags;
+}
+
+// Clears a call's counters unless the last call left them clear.
+static int begin_call(const TraceCall &c, cudaStream_t s)
+{
+    if (!c.clean) RTB_CUDA(cudaMemsetAsync(c.counters, 0, 5 * sizeof(uint32_t), s));
+    return RT_OK;
+}
+
 // The walk and what it leaves to do.
 static int launch_trace(const SceneView &v, const rt_ray *rays, uint64_t n, const uint32_t *n_dev, rt_hit *hits,
-                        uint32_t flags, void *out, bool bits, uint32_t *counters, cudaStream_t s)
+                        uint32_t flags, void *out, bool bits, const TraceCall &c, cudaStream_t s)
 {
     if (n == 0) return RT_OK;
-    // fast, triangles only, ids wanted: the walk writes the ids itself and nothing is left to finish
-    if ((flags & RT_TRACE_FAST) && !v.nspheres && !(flags & kTraceRecords)) flags |= kTraceIds;
-    RTB_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(uint32_t), s));
-    RTB_CHECK(launch_walk(v, rays, n, n_dev, hits, flags, counters, s));
+    flags = walk_flags(v, flags);
+    RTB_CHECK(begin_call(c, s));
     const unsigned finish = (unsigned)std::min<uint64_t>((n + kBlock - 1) / kBlock, 16ull * device_sm_count());
+    RTB_CHECK(launch_walk(v, rays, n, n_dev, hits, flags, c.counters, s));
     if (flags & RT_TRACE_FAST)
-        k_trace_finish_fast<<<finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, counters);
+        k_trace_finish_fast<<<finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, c.counters, c.status);
     else
-        k_trace_finish<<<finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, out, bits, counters);
+        k_trace_finish<<<finish, kBlock, 0, s>>>(v, rays, n, n_dev, hits, flags, out, bits, c.counters, c.status);
     RTB_CUDA(cudaGetLastError());
     return RT_OK;
 }
 
 int launch_trace_closest(const SceneView &v, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags,
-                         uint32_t *counters, cudaStream_t s)
+                         const TraceCall &c, cudaStream_t s)
 {
-    return launch_trace(v, rays, n, nullptr, hits, flags & (RT_TRACE_SHADOW | RT_TRACE_FAST), nullptr, false, counters,
-                        s);
+    flags &= RT_TRACE_SHADOW | RT_TRACE_FAST;
+    const uint64_t blocks = walk_blocks(n);
+    if (n == 0 || n > 32ull * blocks * (kBlock / 32)) return launch_trace(v, rays, n, nullptr, hits, flags, nullptr, false, c, s);
+    RTB_CHECK(begin_call(c, s));
+    k_trace_small<<<(unsigned)blocks, kBlock, 0, s>>>(v, rays, n, hits, walk_flags(v, flags), c.counters, c.status);
+    RTB_CUDA(cudaGetLastError());
+    return RT_OK;
 }
 
 int launch_trace_closest_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_dev, uint32_t cap, rt_hit *hits,
                              uint32_t flags, uint32_t *counters, cudaStream_t s)
 {
     return launch_trace(v, rays, cap, n_dev, hits, (flags & (RT_TRACE_SHADOW | RT_TRACE_FAST)) | kTraceRecords, nullptr,
-                        false, counters, s);
+                        false, TraceCall{counters, nullptr, false}, s);
 }
 
 int launch_walk_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_dev, uint32_t cap, rt_hit *hits,
@@ -319,9 +392,9 @@ int launch_walk_dev(const SceneView &v, const rt_ray *rays, const uint32_t *n_de
 }
 
 int launch_trace_visible(const SceneView &v, const rt_ray *rays, uint64_t n, rt_hit *hits, uint32_t flags, void *out,
-                         bool bits, uint32_t *counters, cudaStream_t s)
+                         bool bits, const TraceCall &c, cudaStream_t s)
 {
-    return launch_trace(v, rays, n, nullptr, hits, (flags & RT_TRACE_SHADOW) | kTraceVisible, out, bits, counters, s);
+    return launch_trace(v, rays, n, nullptr, hits, (flags & RT_TRACE_SHADOW) | kTraceVisible, out, bits, c, s);
 }
 
 int launch_trace_counts(const SceneView &v, const rt_ray *rays, uint64_t n, uint32_t flags, bool anyhit,
@@ -337,12 +410,12 @@ int launch_trace_counts(const SceneView &v, const rt_ray *rays, uint64_t n, uint
 }
 
 int launch_trace_any(const SceneView &v, const rt_ray *rays, uint64_t n, uint8_t *walk_out, void *out, bool bits,
-                     uint32_t flags, uint32_t *counters, cudaStream_t s)
+                     uint32_t flags, const TraceCall &c, cudaStream_t s)
 {
     if (n == 0) return RT_OK;
-    RTB_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(uint32_t), s));
+    RTB_CHECK(begin_call(c, s));
     const uint64_t blocks = walk_blocks(n);
-    k_trace_any<<<(unsigned)blocks, kBlock, 0, s>>>(v, rays, n, walk_out, flags, counters);
+    k_trace_any<<<(unsigned)blocks, kBlock, 0, s>>>(v, rays, n, walk_out, flags, c.counters, c.status);
     RTB_CUDA(cudaGetLastError());
     if (bits || v.nspheres) {
         const uint64_t all = (n + kBlock - 1) / kBlock;

@@ -394,11 +394,12 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
 //
 // init(i, W) prepares ray i (walk_init); finish(i, W, bary) consumes its result. ANY: the walk
 // ends at the first accepted hit in triangle order (in the node that has one). unbounded: the
-// triangle test has no limit (lim only bounds the nodes). COUNT: also counts the triangles a
+// triangle test has no limit (lim only bounds the nodes). Returns the warp's rays where each warp
+// takes one range of the queue ([x, x + y), y = 0 otherwise). COUNT: also counts the triangles a
 // serial walk would test (whole leaves, up to the leaf of the accepted hit under ANY), and every
 // ray keeps its own lane.
 template <bool ANY, bool COUNT, bool ORDERED, typename Init, typename Finish>
-__device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uint32_t n, uint32_t *work,
+__device__ __forceinline__ uint2 walk_queue(const SceneView &v, TravWarp &sm, uint32_t n, uint32_t *work,
                                            bool unbounded, Init init, Finish finish)
 {
     const unsigned lane = threadIdx.x & 31u;
@@ -408,6 +409,7 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
     const bool single = !COUNT && (uint64_t)quota * warps >= n;
     uint32_t ray = 0xFFFFFFFFu;
     bool exhausted = false;
+    uint2 taken = make_uint2(0u, 0u);
     Walk W;
     for (;;) {
         const unsigned idle = __ballot_sync(kAllLanes, ray == 0xFFFFFFFFu);
@@ -418,6 +420,7 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
             if (lane == 0) base = atomicAdd(work, want);
             base = __shfl_sync(kAllLanes, base, 0);
             exhausted = single || base + want >= n;
+            if (single && base < n) taken = make_uint2(base, min(want, n - base));
             const uint32_t rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
             if (ray == 0xFFFFFFFFu && rank < want && base + rank < n) {
                 ray = base + rank;
@@ -432,7 +435,7 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
         }
         const bool active = ray != 0xFFFFFFFFu;
         if (!__any_sync(kAllLanes, active)) {
-            if (exhausted) return;
+            if (exhausted) return taken;
             continue;
         }
         if (walk_step<ANY, COUNT, ORDERED>(v, sm, W, active, unbounded, INFINITY)) {
@@ -440,7 +443,7 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
             ray = 0xFFFFFFFFu;
         }
     }
-    if (COUNT) return;
+    if (COUNT) return taken;
     // the queue is empty: the warp's last rays, with all its lanes
     sm.lanes[lane] = 1;
     sm.found[lane] = make_float4(INFINITY, __uint_as_float(kNoRec), 0.f, 0.f);
@@ -448,7 +451,7 @@ __device__ __forceinline__ void walk_queue(const SceneView &v, TravWarp &sm, uin
     __syncwarp();
     for (;;) {
         const unsigned idle = __ballot_sync(kAllLanes, ray == 0xFFFFFFFFu);
-        if (idle == kAllLanes) return;
+        if (idle == kAllLanes) return taken;
         // idle lane k takes the top entry of the k-th lane that has one
         const bool give = ray != 0xFFFFFFFFu && W.sp > 0;
         const unsigned givers = __ballot_sync(kAllLanes, give);
