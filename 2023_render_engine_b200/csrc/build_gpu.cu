@@ -11,7 +11,8 @@
 //      traversal order from the subtree leaf counts, top down;
 //   3. PLOC: per round, each cluster's nearest neighbour in the window, the mutual pairs merged
 //      by the lower index, new nodes numbered and survivors compacted by one prefix sum
-//      (merges in the low word, survivors in the high word);
+//      (merges in the low word, survivors in the high word); the rounds of the last kPlocTail
+//      clusters, most of them, in one block;
 //   4. depth-first numbering (subtree sizes in creation order, range starts in reverse) and
 //      the SAH leaf rule;
 //   5. collapse to 8-wide nodes one breadth-first level at a time: a prefix sum over the
@@ -141,6 +142,12 @@ __global__ void k_ref_rank(const uint32_t *__restrict__ sorted, const uint32_t *
 
 // ----------------------------------------------------------------------------------- PLOC
 
+__global__ void k_fill(uint32_t *__restrict__ v, uint64_t n, uint32_t x)
+{
+    const uint64_t i = (uint64_t)blockIdx.x * kT + threadIdx.x;
+    if (i < n) v[i] = x;
+}
+
 __global__ void k_ploc_leaves(const float *__restrict__ tri, const uint32_t *__restrict__ sorted, uint32_t n,
                               float margin, BBox *__restrict__ bx, uint32_t *__restrict__ cl)
 {
@@ -164,14 +171,14 @@ __global__ void k_ploc_flags(const uint32_t *__restrict__ nn, uint32_t m, uint64
     const uint32_t i = blockIdx.x * kT + threadIdx.x;
     if (i >= m) return;
     const uint32_t j = nn[i];
-    const bool mutual = nn[j] == i;
+    const bool mutual = j < m && nn[j] == i;  // no neighbour where no area is finite
     flags[i] = (uint64_t)(mutual && i < j) | ((uint64_t)(!mutual || i < j) << 32);
 }
 
 __global__ void k_ploc_merge(BBox *__restrict__ bx, const uint32_t *__restrict__ cl, const uint32_t *__restrict__ nn,
                              uint32_t m, const uint64_t *__restrict__ flags, const uint64_t *__restrict__ pos,
                              uint32_t made, uint32_t *__restrict__ c0, uint32_t *__restrict__ c1,
-                             uint32_t *__restrict__ next, uint64_t *__restrict__ totals)
+                             uint32_t *__restrict__ size, uint32_t *__restrict__ next, uint64_t *__restrict__ totals)
 {
     const uint32_t i = blockIdx.x * kT + threadIdx.x;
     if (i >= m) return;
@@ -184,25 +191,150 @@ __global__ void k_ploc_merge(BBox *__restrict__ bx, const uint32_t *__restrict__
         BBox u = bx[a];
         bbox_grow(u, bx[b]);
         bx[k] = u;  // a new node: no thread of this merge pass reads it
+        size[k] = size[a] + size[b];
     }
     if (f >> 32) next[(uint32_t)(pp >> 32)] = (f & 1u) ? k : cl[i];
     if (i == m - 1) *totals = pp + f;
 }
 
+// The rounds from m <= kPlocTail clusters down to one, the same merges and numbers, by one block. A
+// round takes five launches and a read of its totals, 45 us, whatever its size: 36 of the 53 rounds of
+// a 328,000-triangle mesh have this few clusters, 1.6 ms, 0.19 ms so. Its line: what fits shared
+// memory at four clusters per thread.
+constexpr uint32_t kPlocTail = 4096;
+constexpr uint32_t kTailItems = kPlocTail / 1024;
+struct PlocTail {
+    uint32_t made, root, rounds, left;  // nodes made in all, the last cluster, rounds, clusters left (1)
+};
+constexpr uint32_t kTailSmem = kPlocTail * (6 * 4 + 4 + 2);
+
+// batches[r]: nodes made after round r
+__global__ void __launch_bounds__(1024) k_ploc_tail(BBox *bx, const uint32_t *__restrict__ cl, uint32_t m, uint32_t made,
+                                                    uint32_t *__restrict__ c0, uint32_t *__restrict__ c1,
+                                                    uint32_t *size, uint32_t *__restrict__ batches,
+                                                    PlocTail *__restrict__ out)
+{
+    extern __shared__ float tail_smem[];
+    float(*box)[kPlocTail] = reinterpret_cast<float(*)[kPlocTail]>(tail_smem);
+    uint32_t *id = reinterpret_cast<uint32_t *>(tail_smem + 6 * kPlocTail);
+    uint16_t *nn = reinterpret_cast<uint16_t *>(id + kPlocTail);
+    __shared__ uint32_t wsum[32], total;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    auto box_of = [&](int64_t j) {
+        BBox b;
+        for (int c = 0; c < 3; c++) {
+            b.lo[c] = box[c][j];
+            b.hi[c] = box[3 + c][j];
+        }
+        return b;
+    };
+    for (uint32_t i = t; i < m; i += 1024) {
+        const BBox b = bx[cl[i]];
+        id[i] = cl[i];
+        for (int c = 0; c < 3; c++) {
+            box[c][i] = b.lo[c];
+            box[3 + c][i] = b.hi[c];
+        }
+    }
+    uint32_t rounds = 0;
+    for (;;) {
+        __syncthreads();
+        if (m <= 1 || rounds >= kPlocTail) break;
+        for (uint32_t i = t; i < m; i += 1024) nn[i] = (uint16_t)ploc_nearest(i, m, kPlocRadius, box_of);
+        __syncthreads();
+        // the thread's clusters, in order: new nodes (low half) and survivors before them
+        uint32_t mine = 0, flag[kTailItems];
+#pragma unroll
+        for (uint32_t q = 0; q < kTailItems; q++) {
+            const uint32_t i = kTailItems * t + q;
+            flag[q] = 0;
+            if (i < m) {
+                const uint32_t j = nn[i];
+                const bool mutual = j < m && nn[j] == i;  // no neighbour where no area is finite
+                flag[q] = (mutual && i < j ? 1u : 0u) | (!mutual || i < j ? 1u << 16 : 0u);
+            }
+            mine += flag[q];
+        }
+        uint32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            const uint32_t v = wsum[lane];
+            uint32_t w = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+                if (lane >= (uint32_t)o) w += y;
+            }
+            wsum[lane] = w - v;
+            if (lane == 31) total = w;
+        }
+        __syncthreads();
+        uint32_t before = incl - mine + wsum[warp];
+        uint32_t nid[kTailItems], to[kTailItems];
+        BBox nb[kTailItems];
+#pragma unroll
+        for (uint32_t q = 0; q < kTailItems; q++) {
+            const uint32_t i = kTailItems * t + q;
+            to[q] = before >> 16;
+            if (flag[q]) {
+                nid[q] = id[i];
+                nb[q] = box_of(i);
+                if (flag[q] & 1u) {
+                    const uint32_t k = made + (before & 0xFFFFu), j = nn[i], a = id[i], b = id[j];
+                    c0[k] = a;
+                    c1[k] = b;
+                    bbox_grow(nb[q], box_of(j));
+                    bx[k] = nb[q];
+                    size[k] = size[a] + size[b];
+                    nid[q] = k;
+                }
+            }
+            before += flag[q];
+        }
+        const uint32_t merges = total & 0xFFFFu, keep = total >> 16;
+        __syncthreads();  // the old clusters have been read
+#pragma unroll
+        for (uint32_t q = 0; q < kTailItems; q++)
+            if (flag[q] >> 16) {
+                id[to[q]] = nid[q];
+                for (int c = 0; c < 3; c++) {
+                    box[c][to[q]] = nb[q].lo[c];
+                    box[3 + c][to[q]] = nb[q].hi[c];
+                }
+            }
+        if (merges == 0) break;  // uniform; the host reports it
+        made += merges;
+        m = keep;
+        if (t == 0) batches[rounds] = made;
+        rounds++;
+    }
+    if (t == 0) *out = PlocTail{made, id[0], rounds, m};
+}
+
+// k_first over the rounds of k_ploc_tail, the last first
+__global__ void __launch_bounds__(1024) k_first_tail(const uint32_t *__restrict__ c0, const uint32_t *__restrict__ c1,
+                                                     const uint32_t *__restrict__ size,
+                                                     const uint32_t *__restrict__ batches, uint32_t made0, uint32_t rounds,
+                                                     uint32_t *first)
+{
+    for (uint32_t r = rounds; r > 0; r--) {
+        const uint32_t b = r > 1 ? batches[r - 2] : made0, e = batches[r - 1];
+        for (uint32_t k = b + threadIdx.x; k < e; k += 1024) {
+            const uint32_t f = first[k];
+            first[c0[k]] = f;
+            first[c1[k]] = f + size[c0[k]];
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------- depth-first numbering, leaves
-
-__global__ void k_fill(uint32_t *__restrict__ v, uint64_t n, uint32_t x)
-{
-    const uint64_t i = (uint64_t)blockIdx.x * kT + threadIdx.x;
-    if (i < n) v[i] = x;
-}
-
-__global__ void k_sizes(const uint32_t *__restrict__ c0, const uint32_t *__restrict__ c1, uint32_t b, uint32_t e,
-                        uint32_t *__restrict__ size)
-{
-    const uint32_t k = b + blockIdx.x * kT + threadIdx.x;
-    if (k < e) size[k] = size[c0[k]] + size[c1[k]];
-}
 
 __global__ void k_first(const uint32_t *__restrict__ c0, const uint32_t *__restrict__ c1,
                         const uint32_t *__restrict__ size, uint32_t b, uint32_t e, uint32_t *__restrict__ first)
@@ -401,8 +533,10 @@ int build_scene_device(rt_scene *s, float margin_out[1])
     uint32_t *c0 = buf<uint32_t>(d_c0, n, rc), *c1 = buf<uint32_t>(d_c1, n, rc), *cl = buf<uint32_t>(d_cl, n, rc),
              *cl2 = buf<uint32_t>(d_cl2, n, rc), *nn = buf<uint32_t>(d_nn, n, rc);
     uint64_t *flags = buf<uint64_t>(d_flags, n, rc), *pos = buf<uint64_t>(d_pos, n, rc),
-             *tot = buf<uint64_t>(d_tot, 2, rc);
+             *tot = buf<uint64_t>(d_tot, 4 + kPlocTail / 2, rc);  // a round's totals; k_ploc_tail's, its batches
+    uint32_t *size = buf<uint32_t>(d_size, nb, rc);
     RTB_CHECK(rc);
+    k_fill<<<blocks_for(nb), kT, 0, st>>>(size, nb, 1u);  // of leaves; nodes get theirs when they are made
     k_ploc_leaves<<<blocks_for(n), kT, 0, st>>>(tri, sorted, n, margin, bx, cl);
     tmp_bytes = 0;
     RTB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, flags, pos, (int)n, st));
@@ -410,12 +544,12 @@ int build_scene_device(rt_scene *s, float margin_out[1])
     RTB_CHECK(rc);
     std::vector<uint32_t> batches{0};  // internal nodes made per round: [batches[t], batches[t + 1])
     uint32_t m = n, made = 0;
-    for (uint32_t round = 0; m > 1; round++) {
+    for (uint32_t round = 0; m > kPlocTail; round++) {
         if (round > n) return fail(RT_ERR_TIMEOUT, "build_scene_device: clustering made no progress");
         k_ploc_nn<<<blocks_for(m), kT, 0, st>>>(bx, cl, m, kPlocRadius, nn);
         k_ploc_flags<<<blocks_for(m), kT, 0, st>>>(nn, m, flags);
         RTB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flags, pos, (int)m, st));
-        k_ploc_merge<<<blocks_for(m), kT, 0, st>>>(bx, cl, nn, m, flags, pos, made, c0, c1, cl2, tot);
+        k_ploc_merge<<<blocks_for(m), kT, 0, st>>>(bx, cl, nn, m, flags, pos, made, c0, c1, size, cl2, tot);
         RTB_CUDA(cudaGetLastError());
         uint64_t t = 0;
         RTB_CUDA(cudaMemcpyAsync(&t, tot, 8, cudaMemcpyDeviceToHost, st));
@@ -427,27 +561,31 @@ int build_scene_device(rt_scene *s, float margin_out[1])
         m = keep;
         std::swap(cl, cl2);
     }
-    uint32_t root = 0;
-    RTB_CUDA(cudaMemcpyAsync(&root, cl, 4, cudaMemcpyDeviceToHost, st));
+    if (!(device_slot(SLOT_SMEM_ATTRS) & SMEM_PLOC_TAIL)) {
+        RTB_CUDA(cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
+        or_device_slot(SLOT_SMEM_ATTRS, SMEM_PLOC_TAIL);
+    }
+    PlocTail *tail = reinterpret_cast<PlocTail *>(tot + 2);
+    uint32_t *tail_batches = reinterpret_cast<uint32_t *>(tot + 4);
+    k_ploc_tail<<<1, 1024, kTailSmem, st>>>(bx, cl, m, made, c0, c1, size, tail_batches, tail);
+    RTB_CUDA(cudaGetLastError());
+    PlocTail tl{};
+    RTB_CUDA(cudaMemcpyAsync(&tl, tail, sizeof(tl), cudaMemcpyDeviceToHost, st));
+    RTB_CUDA(cudaStreamSynchronize(st));
+    if (tl.left != 1 || tl.made != n - 1) return fail(RT_ERR_TIMEOUT, "build_scene_device: clustering stalled");
+    const uint32_t root = tl.root;
 
     // 4. depth-first numbering and leaves
-    uint32_t *size = buf<uint32_t>(d_size, nb, rc), *first = buf<uint32_t>(d_first, nb, rc),
-             *ids = buf<uint32_t>(d_ids, n, rc);
+    uint32_t *first = buf<uint32_t>(d_first, nb, rc), *ids = buf<uint32_t>(d_ids, n, rc);
     uint8_t *leaf = buf<uint8_t>(d_leaf, nb, rc);
     RTB_CHECK(rc);
     RTB_CUDA(cudaMemsetAsync(ids, 0, 4ull * n, st));
-    {
-        k_fill<<<blocks_for(nb), kT, 0, st>>>(size, nb, 1u);  // leaf sizes; internal sizes overwritten below
-        RTB_CUDA(cudaMemsetAsync(first, 0, 4ull * nb, st));
-        for (size_t t = 0; t + 1 < batches.size(); t++)
-            k_sizes<<<blocks_for(batches[t + 1] - batches[t]), kT, 0, st>>>(c0, c1, batches[t], batches[t + 1],
-                                                                            size);
-        for (size_t t = batches.size() - 1; t > 0; t--)
-            k_first<<<blocks_for(batches[t] - batches[t - 1]), kT, 0, st>>>(c0, c1, size, batches[t - 1],
-                                                                             batches[t], first);
-        k_leaf_setup<<<blocks_for(n), kT, 0, st>>>(sorted, first, bx, c0, c1, size, n, ids, leaf);
-        RTB_CUDA(cudaGetLastError());
-    }
+    RTB_CUDA(cudaMemsetAsync(first, 0, 4ull * nb, st));
+    k_first_tail<<<1, 1024, 0, st>>>(c0, c1, size, tail_batches, made, tl.rounds, first);
+    for (size_t t = batches.size() - 1; t > 0; t--)
+        k_first<<<blocks_for(batches[t] - batches[t - 1]), kT, 0, st>>>(c0, c1, size, batches[t - 1], batches[t], first);
+    k_leaf_setup<<<blocks_for(n), kT, 0, st>>>(sorted, first, bx, c0, c1, size, n, ids, leaf);
+    RTB_CUDA(cudaGetLastError());
 
     // 5. collapse, level by level
     Bvh8Node *nodes = buf<Bvh8Node>(d_wide, n, rc);  // room for the most nodes n triangles can need

@@ -91,7 +91,7 @@ enum DeviceSlot : int {
     SLOT_MEM_MIB = 7,          // device memory, MiB
     SLOT_COUNT = 8
 };
-enum SmemAttr : unsigned { SMEM_RENDER_INFER = 1u, SMEM_GUIDE_TRAIN = 2u, SMEM_GUIDE_EVAL = 4u };
+enum SmemAttr : unsigned { SMEM_RENDER_INFER = 1u, SMEM_GUIDE_TRAIN = 2u, SMEM_GUIDE_EVAL = 4u, SMEM_PLOC_TAIL = 8u };
 // Value of `slot` for the current device; 0 until set_device_slot stored one.
 unsigned device_slot(DeviceSlot slot);
 void set_device_slot(DeviceSlot slot, unsigned value);
