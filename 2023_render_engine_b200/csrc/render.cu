@@ -237,6 +237,7 @@ struct PhotonView {
 constexpr int kSortBlock = 256;
 constexpr int kSortKeys = 16;  // 0: miss, 1 + rt_material_type
 constexpr uint32_t kSortMaxLog2 = 13;
+constexpr uint32_t kSortMinLog2 = 8;  // kSortBlock slots
 __device__ __forceinline__ uint32_t shade_key(const RenderView &rv, int32_t prim)
 {
     if (prim < 0) return 0;
@@ -259,7 +260,10 @@ __global__ void __launch_bounds__(kSortBlock) k_material_sort(RenderView rv, Buf
         if (threadIdx.x == 0) bf.cnt[kCntQueue + 32 * (cur ^ 1)] = 0;
         if (threadIdx.x < (kCntSample - kCntShadow) / 32) bf.cnt[kCntShadow + 32 * threadIdx.x] = 0;
     }
+    if (finish) prefetch_shapes(rv.sv);
     const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
+    // a wave that leaves blocks idle is sorted in smaller chunks, down to one slot per thread
+    while (log2 > kSortMinLog2 && n <= gridDim.x << (log2 - 1)) log2--;
     // chunks in a grid-stride loop over the resident blocks (c0 is the same for the whole block)
     for (uint32_t c0 = blockIdx.x << log2; c0 < n; c0 += gridDim.x << log2) {
         const uint32_t len = min(1u << log2, n - c0);
@@ -683,6 +687,7 @@ __global__ void __launch_bounds__(kB, RTB_TRAV_MIN_BLOCKS) k_shadow(RenderView r
 __global__ void __launch_bounds__(kB, 12) k_shadow_add(RenderView rv, Buffers bf, int nxt, GuideView gv)
 {
     const uint32_t n = min(bf.cnt[kCntShadow], bf.scap);
+    if (blockIdx.x * blockDim.x < n) prefetch_shapes(rv.sv);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 c = bf.scontrib[i];
         const uint32_t target = __float_as_uint(c.w);
@@ -1337,7 +1342,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     // material sort of the shading order, chunks of 2^sort_log2 queue slots (0: off)
     const uint32_t sort_log2 = s->sort_log2 ? std::min<uint32_t>(std::max<uint32_t>(s->sort_log2, 5u), kSortMaxLog2) : 0u;
     const unsigned sort_blocks =
-        sort_log2 ? std::min((unsigned)((cap + (1u << sort_log2) - 1) >> sort_log2),
+        sort_log2 ? std::min((unsigned)(cap >> std::min(sort_log2, kSortMinLog2)) + 1u,
                              resident_grid(SLOT_SORT_RESIDENT, k_material_sort, kSortBlock))
                   : 0u;
     if (sort_log2) RTB_CHECK(rs.perm.reserve(4ull * cap));

@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_trace_finish(SceneView v, const r
                                                             uint32_t *counters, uint32_t *status)
 {
     if (n_dev) n = min((uint64_t)*n_dev, n);
+    prefetch_shapes(v);
     const bool visible = (flags & kTraceVisible) != 0;
     // whole warps stay in the loop (the bit mask is gathered with a ballot)
     for (uint64_t i0 = (uint64_t)blockIdx.x * kBlock; i0 < n; i0 += (uint64_t)gridDim.x * kBlock) {
@@ -250,6 +251,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_trace_finish_fast(SceneView v, c
 {
     if (n_dev) n = min((uint64_t)*n_dev, n);
     if (!v.nspheres && *(volatile uint32_t *)counters == 0u) n = 0;
+    if ((uint64_t)blockIdx.x * kBlock < n) prefetch_shapes(v);
     for (uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kBlock) {
         float4 *h = reinterpret_cast<float4 *>(hits) + i;
         *h = finish_fast(v, rays, i, flags, *h, counters);

@@ -547,6 +547,15 @@ __device__ __noinline__ static bool shape_test(const SphereRecord *sr, float ox,
     return ok;
 }
 
+// The shapes' records into the L1 cache, which every kernel finds empty: the loop over the shapes reads
+// record after record, each a trip to the L2 otherwise.
+__device__ __forceinline__ void prefetch_shapes(const SceneView &v)
+{
+    const uint32_t lines = (min(v.nspheres, 256u) * (uint32_t)sizeof(SphereRecord) + 127u) / 128u;
+    for (uint32_t i = threadIdx.x; i < lines; i += blockDim.x)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char *>(v.spheres) + 128u * i));
+}
+
 // Scene::intersects' loop over the analytic shapes (Scene.cu:141-146) of scene `sub`.
 __device__ __forceinline__ void intersect_spheres(const SceneView &v, uint32_t sub, float ox, float oy, float oz,
                                                   float dx, float dy, float dz, float tmax, bool shadow, float &t,
