@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "photon_query.cuh"
+#include "traverse.cuh"
 
 namespace rtb {
 namespace {
@@ -38,8 +39,9 @@ struct PhotonBuffers {
     unsigned long long *keys;  // (path << 8) | depth
     uint32_t store_cap;
     uint32_t cap;
-    // [0],[1] queue sizes, [2] stored count, [3] status
-    uint32_t *cnt;
+    uint32_t *queued;     // paths at each depth
+    uint32_t *stored;     // photons stored
+    uint32_t *trace_cnt;  // the walk's counters
 };
 
 __device__ __forceinline__ Pcg photon_rng(uint64_t path, uint32_t seed)
@@ -98,89 +100,95 @@ __global__ void k_emit(RenderView rv, uint64_t n, uint32_t seed, const float *po
     pb.rng[0][q] = make_uint4((uint32_t)r.state, (uint32_t)(r.state >> 32), 0u, 0u);
 }
 
-__global__ void __launch_bounds__(kPB) k_photon_shade(RenderView rv, PhotonBuffers pb, int cur, uint32_t max_depth,
-                                                      uint32_t rr_depth, uint32_t seed, uint32_t flags)
+// One bounce of the paths at `depth0`, whose hits the walk left (finish_fast). The paths that continue
+// are the next depth's.
+__global__ void __launch_bounds__(kPB) k_photon_shade(RenderView rv, PhotonBuffers pb, uint32_t depth0,
+                                                      uint32_t max_depth, uint32_t rr_depth, uint32_t seed, uint32_t flags)
 {
-    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n = min(pb.cnt[cur], pb.cap);
-    if (q >= n) return;
-    const int nxt = cur ^ 1;
+    const uint32_t n = min(pb.queued[depth0], pb.cap);
+    const int cur = depth0 & 1, nxt = cur ^ 1;
     const bool compat = (flags & RT_RENDER_COMPAT) != 0;
-    float4 hv = reinterpret_cast<const float4 *>(pb.hits)[q];
-    rt_hit h{hv.x, __float_as_int(hv.y), hv.z, hv.w};
-    if (h.prim < 0) return;  // escaped
-    float4 r0 = reinterpret_cast<const float4 *>(pb.rays[cur])[2 * q];
-    float4 r1 = reinterpret_cast<const float4 *>(pb.rays[cur])[2 * q + 1];
-    float4 b4 = pb.beta[cur][q], c4 = pb.carry[cur][q];
-    uint4 s4 = pb.rng[cur][q];
-    V3 o = v3(r0.x, r0.y, r0.z), d = v3(r1.x, r1.y, r1.z);
-    V3 beta = v3(b4.x, b4.y, b4.z), carry = v3(c4.x, c4.y, c4.z);
-    const uint32_t path = __float_as_uint(c4.w);
-    const uint32_t depth = s4.w;
-    Pcg rng;
-    rng.state = ((uint64_t)s4.y << 32) | s4.x;
-    rng.inc = ((((uint64_t)0xFFFFFFFFu << 32) | (seed ^ 0x9E3779B9u)) << 1u) | 1u;
-    Surface sf = surface_at(rv, h, o, d, compat);
-    const rt_material &m = rv.mats[min(sf.mat, rv.nmats - 1)];
-    Bsdf bs = load_bsdf(m);
-    const bool scattering = is_scattering(bs);  // from the material's own kd
-    if (m.texture) {
-        const float2 uv = surface_uv(rv, h, sf);
-        texture_bsdf(bs, tex_color(rv, m.texture - 1u, uv.x, uv.y));
-    }
-    if (scattering) {  // samplePhotonIntersections (photonDispersion.cu:40-54)
-        uint32_t slot = append(pb.cnt + 2);
-        if (slot < pb.store_cap) {
-            V3 pw = carry * beta;
-            rt_photon ph;
-            ph.pos[0] = sf.p.x;
-            ph.pos[1] = sf.p.y;
-            ph.pos[2] = sf.p.z;
-            ph.shape_id = sf.shape;
-            ph.dir[0] = d.x;
-            ph.dir[1] = d.y;
-            ph.dir[2] = d.z;
-            ph.path = path;
-            ph.power[0] = pw.x;
-            ph.power[1] = pw.y;
-            ph.power[2] = pw.z;
-            ph.depth = depth;
-            ph.normal[0] = sf.n.x;
-            ph.normal[1] = sf.n.y;
-            ph.normal[2] = sf.n.z;
-            ph.reserved = 0.f;
-            pb.store[slot] = ph;
-            pb.keys[slot] = ((unsigned long long)path << 8) | depth;
+    // the next walk's work counter; this depth's walk is over, and none of the replays below use it
+    if (blockIdx.x == 0 && threadIdx.x == 0) pb.trace_cnt[3] = 0;
+    if (blockIdx.x * blockDim.x < n) prefetch_shapes(rv.sv);
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        const float4 hv = finish_fast(rv.sv, pb.rays[cur], q, RT_TRACE_FAST | kTraceRecords,
+                                      reinterpret_cast<const float4 *>(pb.hits)[q], pb.trace_cnt);
+        rt_hit h{hv.x, __float_as_int(hv.y), hv.z, hv.w};
+        if (h.prim < 0) continue;  // escaped
+        float4 r0 = reinterpret_cast<const float4 *>(pb.rays[cur])[2 * q];
+        float4 r1 = reinterpret_cast<const float4 *>(pb.rays[cur])[2 * q + 1];
+        float4 b4 = pb.beta[cur][q], c4 = pb.carry[cur][q];
+        uint4 s4 = pb.rng[cur][q];
+        V3 o = v3(r0.x, r0.y, r0.z), d = v3(r1.x, r1.y, r1.z);
+        V3 beta = v3(b4.x, b4.y, b4.z), carry = v3(c4.x, c4.y, c4.z);
+        const uint32_t path = __float_as_uint(c4.w);
+        const uint32_t depth = s4.w;
+        Pcg rng;
+        rng.state = ((uint64_t)s4.y << 32) | s4.x;
+        rng.inc = ((((uint64_t)0xFFFFFFFFu << 32) | (seed ^ 0x9E3779B9u)) << 1u) | 1u;
+        Surface sf = surface_at(rv, h, o, d, compat);
+        const rt_material &m = rv.mats[min(sf.mat, rv.nmats - 1)];
+        Bsdf bs = load_bsdf(m);
+        const bool scattering = is_scattering(bs);  // from the material's own kd
+        if (m.texture) {
+            const float2 uv = surface_uv(rv, h, sf);
+            texture_bsdf(bs, tex_color(rv, m.texture - 1u, uv.x, uv.y));
         }
+        if (scattering) {  // samplePhotonIntersections (photonDispersion.cu:40-54)
+            uint32_t slot = append(pb.stored);
+            if (slot < pb.store_cap) {
+                V3 pw = carry * beta;
+                rt_photon ph;
+                ph.pos[0] = sf.p.x;
+                ph.pos[1] = sf.p.y;
+                ph.pos[2] = sf.p.z;
+                ph.shape_id = sf.shape;
+                ph.dir[0] = d.x;
+                ph.dir[1] = d.y;
+                ph.dir[2] = d.z;
+                ph.path = path;
+                ph.power[0] = pw.x;
+                ph.power[1] = pw.y;
+                ph.power[2] = pw.z;
+                ph.depth = depth;
+                ph.normal[0] = sf.n.x;
+                ph.normal[1] = sf.n.y;
+                ph.normal[2] = sf.n.z;
+                ph.reserved = 0.f;
+                pb.store[slot] = ph;
+                pb.keys[slot] = ((unsigned long long)path << 8) | depth;
+            }
+        }
+        V3 t, bv;
+        onb(sf.n, t, bv);
+        V3 wow = -d;
+        V3 wo = v3(dot(wow, t), dot(wow, bv), dot(wow, sf.n));
+        V3 Le = (bs.type == RT_MAT_LIGHT) ? bs.color * m.intensity : v3(0, 0, 0);
+        V3 wi;
+        float pdf;
+        bool delta;
+        V3 f = bsdf_sample(bs, wo, rng, compat, wi, pdf, delta);
+        carry = carry + beta * Le;  // photonDispersion.cu:64-65
+        beta = beta * f;
+        bool finished = is_black(f);
+        if (!finished && scattering && depth > rr_depth) {  // finishStep (pathTracing.cu:91-102)
+            float qrr = fmaxf(0.05f, 1.f - luminance(beta));
+            if (pcg_float(rng) < qrr)
+                finished = true;
+            else
+                beta = beta * (1.f / (1.f - qrr));
+        }
+        if (finished || depth + 1 >= max_depth) continue;
+        V3 wiw = t * wi.x + bv * wi.y + sf.n * wi.z;
+        V3 no = spawn_origin(sf.p, sf.n, sf.perr, wiw);
+        uint32_t qn = append(pb.queued + depth0 + 1);
+        reinterpret_cast<float4 *>(pb.rays[nxt])[2 * qn] = make_float4(no.x, no.y, no.z, INFINITY);
+        reinterpret_cast<float4 *>(pb.rays[nxt])[2 * qn + 1] = make_float4(wiw.x, wiw.y, wiw.z, 0.f);
+        pb.beta[nxt][qn] = make_float4(beta.x, beta.y, beta.z, 0.f);
+        pb.carry[nxt][qn] = make_float4(carry.x, carry.y, carry.z, __uint_as_float(path));
+        pb.rng[nxt][qn] = make_uint4((uint32_t)rng.state, (uint32_t)(rng.state >> 32), 0u, depth + 1);
     }
-    V3 t, bv;
-    onb(sf.n, t, bv);
-    V3 wow = -d;
-    V3 wo = v3(dot(wow, t), dot(wow, bv), dot(wow, sf.n));
-    V3 Le = (bs.type == RT_MAT_LIGHT) ? bs.color * m.intensity : v3(0, 0, 0);
-    V3 wi;
-    float pdf;
-    bool delta;
-    V3 f = bsdf_sample(bs, wo, rng, compat, wi, pdf, delta);
-    carry = carry + beta * Le;  // photonDispersion.cu:64-65
-    beta = beta * f;
-    bool finished = is_black(f);
-    if (!finished && scattering && depth > rr_depth) {  // finishStep (pathTracing.cu:91-102)
-        float qrr = fmaxf(0.05f, 1.f - luminance(beta));
-        if (pcg_float(rng) < qrr)
-            finished = true;
-        else
-            beta = beta * (1.f / (1.f - qrr));
-    }
-    if (finished || depth + 1 >= max_depth) return;
-    V3 wiw = t * wi.x + bv * wi.y + sf.n * wi.z;
-    V3 no = spawn_origin(sf.p, sf.n, sf.perr, wiw);
-    uint32_t qn = append(pb.cnt + nxt);
-    reinterpret_cast<float4 *>(pb.rays[nxt])[2 * qn] = make_float4(no.x, no.y, no.z, INFINITY);
-    reinterpret_cast<float4 *>(pb.rays[nxt])[2 * qn + 1] = make_float4(wiw.x, wiw.y, wiw.z, 0.f);
-    pb.beta[nxt][qn] = make_float4(beta.x, beta.y, beta.z, 0.f);
-    pb.carry[nxt][qn] = make_float4(carry.x, carry.y, carry.z, __uint_as_float(path));
-    pb.rng[nxt][qn] = make_uint4((uint32_t)rng.state, (uint32_t)(rng.state >> 32), 0u, depth + 1);
 }
 
 __global__ void k_gather_photons(const rt_photon *src, const uint32_t *order, uint64_t n, rt_photon *dst)
@@ -675,7 +683,9 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
     RTB_CHECK(sel.reserve(4ull * cap));
     RTB_CHECK(perl.reserve(8ull * nl));
     RTB_CHECK(dpow.upload(power.data(), 4ull * nl, st));
-    RTB_CHECK(cnt.reserve(64));
+    // paths at each depth (max_depth <= 255), photons stored
+    constexpr uint32_t kStored = 256, kCounts = 257;
+    RTB_CHECK(cnt.reserve(4 * kCounts));
     RTB_CHECK(s->scratch.counters.reserve(64));
     uint64_t store_cap = std::max<uint64_t>(4 * n, 1024);
     rt_photon_map *m = nullptr;
@@ -699,9 +709,12 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
         pb.keys = keys.as<unsigned long long>();
         pb.store_cap = (uint32_t)std::min<uint64_t>(store_cap, 0xFFFFFFFFull);
         pb.cap = cap;
-        pb.cnt = cnt.as<uint32_t>();
+        pb.queued = cnt.as<uint32_t>();
+        pb.stored = pb.queued + kStored;
+        pb.trace_cnt = s->scratch.counters.as<uint32_t>();
         RTB_CUDA(cudaEventRecord(e0, st));
-        RTB_CUDA(cudaMemsetAsync(cnt.ptr, 0, 64, st));
+        RTB_CUDA(cudaMemsetAsync(cnt.ptr, 0, 4 * kCounts, st));
+        RTB_CUDA(cudaMemsetAsync(pb.trace_cnt, 0, 16, st));
         RTB_CUDA(cudaMemsetAsync(perl.ptr, 0, 8ull * nl, st));
         const unsigned blocks = (unsigned)((n + kPB - 1) / kPB);
         k_select<<<blocks, kPB, 0, st>>>(rv, n, seed, dpow.as<float>(), total, sel.as<uint32_t>(),
@@ -711,25 +724,23 @@ int rt_photons_trace(rt_scene *s, uint64_t n, uint32_t max_depth, uint32_t rr_de
         RTB_CUDA(cudaGetLastError());
         uint32_t n0 = (uint32_t)n;
         RTB_CUDA(cudaMemcpyAsync(cnt.ptr, &n0, 4, cudaMemcpyHostToDevice, st));
-        int cur = 0;
-        rays_traced = 0;
+        // Two launches a depth: a depth without paths costs less than asking for their number, which
+        // the host does every kDepths depths (a copy, a wait and a gap of 20 us).
+        constexpr uint32_t kDepths = 16;
+        const unsigned shade_blocks = std::min<unsigned>(cap / kPB + 1, 16u * device_sm_count());
+        uint32_t hc[kCounts];
         for (uint32_t depth = 0; depth < max_depth; depth++) {
-            RTB_CHECK(launch_trace_closest_dev(rv.sv, pb.rays[cur], pb.cnt + cur, cap, pb.hits, RT_TRACE_FAST,
-                                               s->scratch.counters.as<uint32_t>(), st));
-            RTB_CUDA(cudaMemsetAsync(pb.cnt + (cur ^ 1), 0, 4, st));
-            k_photon_shade<<<cap / kPB + 1, kPB, 0, st>>>(rv, pb, cur, max_depth, rr_depth, seed, flags);
+            RTB_CHECK(launch_walk_dev(rv.sv, pb.rays[depth & 1], pb.queued + depth, cap, pb.hits, pb.trace_cnt, st));
+            k_photon_shade<<<shade_blocks, kPB, 0, st>>>(rv, pb, depth, max_depth, rr_depth, seed, flags);
             RTB_CUDA(cudaGetLastError());
-            uint32_t hc[4];
-            RTB_CUDA(cudaMemcpyAsync(hc, cnt.ptr, 16, cudaMemcpyDeviceToHost, st));
+            if ((depth + 1) % kDepths && depth + 1 < max_depth) continue;
+            RTB_CUDA(cudaMemcpyAsync(hc, cnt.ptr, sizeof(hc), cudaMemcpyDeviceToHost, st));
             RTB_CUDA(cudaStreamSynchronize(st));
-            rays_traced += hc[cur];
-            cur ^= 1;
-            if (hc[cur] == 0) break;
+            if (hc[depth + 1] == 0) break;
         }
-        uint32_t hc[4];
-        RTB_CUDA(cudaMemcpyAsync(hc, cnt.ptr, 16, cudaMemcpyDeviceToHost, st));
-        RTB_CUDA(cudaStreamSynchronize(st));
-        stored = hc[2];
+        rays_traced = 0;
+        for (uint32_t depth = 0; depth < max_depth; depth++) rays_traced += hc[depth];
+        stored = hc[kStored];
         if (stored > store_cap) {  // deterministic: retrace with room for every photon
             store_cap = stored;
             continue;
