@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kQueryBlock, RTB_QUERY_MIN_BLOCKS) k_subsurfac
                                                             const float *__restrict__ nrm,
                                                             const float *__restrict__ wo,
                                                             const int32_t *__restrict__ shape, uint64_t nq,
-                                                            float radius, int compat, float *__restrict__ out)
+                                                            float radius2, int compat, float *__restrict__ out)
 {
     __shared__ PhotonWarpScratch scratch[kQueryBlock / 32];
     const uint64_t qi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kQueryBlock, RTB_QUERY_MIN_BLOCKS) k_subsurfac
     const V3 nn = v3(nrm[3 * qi], nrm[3 * qi + 1], nrm[3 * qi + 2]);
     const V3 w = v3(wo[3 * qi], wo[3 * qi + 1], wo[3 * qi + 2]);
     const V3 c = warp_photon_subsurface(tree, mat, v3(mat.color[0], mat.color[1], mat.color[2]), p, nn, w,
-                                        shape ? shape[qi] : -1, radius, compat != 0, scratch[threadIdx.x >> 5]);
+                                        shape ? shape[qi] : -1, radius2, compat != 0, scratch[threadIdx.x >> 5]);
     if ((threadIdx.x & 31u) == 0) {
         out[3 * qi] = c.x;
         out[3 * qi + 1] = c.y;
@@ -622,7 +622,8 @@ int rt_photon_subsurface(rt_photon_map *m, const rt_material *mat, const float *
     if (nq > (1ull << 31) / 32) return fail(RT_ERR_INVALID, "rt_photon_subsurface: nq must be at most 2^26");
     const uint64_t blocks = (nq * 32 + kQueryBlock - 1) / kQueryBlock;
     k_subsurface<<<(unsigned)blocks, kQueryBlock, 0, m->ctx->stream>>>(photon_tree(m), *mat, pts, nrm, wo, shape, nq,
-                                                                       radius, (flags & RT_RENDER_COMPAT) ? 1 : 0,
+                                                                       radius_squared(radius),
+                                                                       (flags & RT_RENDER_COMPAT) ? 1 : 0,
                                                                        out_rgb);
     RTB_CUDA(cudaGetLastError());
     RTB_CUDA(cudaStreamSynchronize(m->ctx->stream));

@@ -180,6 +180,17 @@ __device__ __forceinline__ float dipole_eval(const DipoleChannel &c, float r2)
     return c1 * rd * c.omf * c.alpha;
 }
 
+// Largest squared distance whose root is below radius (-1: none): the search compares squared
+// distances, and roots are taken of its answers only.
+inline float radius_squared(float radius)
+{
+    if (!(radius > 0.f)) return -1.f;
+    float s = std::min(radius * radius, FLT_MAX);
+    while (s > 0.f && !(std::sqrt(s) < radius)) s = std::nextafter(s, 0.f);
+    while (s < FLT_MAX && std::sqrt(std::nextafter(s, FLT_MAX)) < radius) s = std::nextafter(s, FLT_MAX);
+    return s;
+}
+
 // ------------------------------------------------------- warp-cooperative queries
 // A warp answers its queries together, with their traversal stacks in shared memory. Every lane of
 // the warp must call these functions together. Serial per-node chains of local-memory stack and
@@ -217,6 +228,8 @@ constexpr unsigned kFullMask = 0xFFFFFFFFu;
 struct PhotonWarpScratch {  // per warp, in shared memory
     uint32_t sl[kWarpStack], sr[kWarpStack];
     float sd[kWarpStack];
+    float d2[64];  // squared distances and
+    uint32_t slot[64];  // tree slots of photons found and not yet added
 };
 
 __device__ __forceinline__ float warp_sum(float v)
@@ -234,12 +247,12 @@ __device__ __forceinline__ float warp_max(float v)
 // The pruned traversal of knn_query (kdtree.h:111-152) for a warp: the same depth-first,
 // near-side-first order with the same pruning (a far side is skipped when its split plane is
 // not nearer than the bound), decided warp-uniformly with the stack in shared memory. A range
-// of at most Scan photons is read 32 photons per load instead of node by node. bound() is the
-// current search distance (warp-uniform); visit(valid, dist, shape, slot) is offered up to 32
+// of at most Scan photons is read 32 photons per load instead of node by node. radius2 is the squared
+// search distance (radius_squared); visit(valid, squared distance, shape, slot) is offered up to 32
 // photons, one per lane (an internal node's photon on lane 0).
-template <uint32_t Scan, class Bound, class Visit>
-__device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, float qy, float qz, PhotonWarpScratch &sm,
-                                              Bound &&bound, Visit &&visit)
+template <uint32_t Scan, class Visit>
+__device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, float qy, float qz, float radius2,
+                                              PhotonWarpScratch &sm, Visit &&visit)
 {
     const uint32_t lane = threadIdx.x & 31u;
     int sp = 1;
@@ -254,7 +267,7 @@ __device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, flo
         const uint32_t l = sm.sl[sp], r = sm.sr[sp];
         const float pd = sm.sd[sp];
         __syncwarp();  // every lane has read the entry before lane 0 reuses it
-        if (!(pd < bound()) || r <= l) continue;
+        if (!(pd <= radius2) || r <= l) continue;
         if (r - l <= Scan) {
             for (uint32_t base = l; base < r; base += 64) {  // two loads in flight per lane
                 const uint32_t j0 = base + lane, j1 = base + 32 + lane;
@@ -268,19 +281,19 @@ __device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, flo
                     p1 = __ldg(t.pos + j1);
                     s1 = __ldg(&t.aux[j1].x);
                 }
-                visit(j0 < r, j0 < r ? ref_dist(qx, qy, qz, p0) : INFINITY, s0, j0);
-                if (base + 32 < r) visit(j1 < r, j1 < r ? ref_dist(qx, qy, qz, p1) : INFINITY, s1, j1);
+                visit(j0 < r, j0 < r ? ref_dist2(qx, qy, qz, p0) : INFINITY, s0, j0);
+                if (base + 32 < r) visit(j1 < r, j1 < r ? ref_dist2(qx, qy, qz, p1) : INFINITY, s1, j1);
             }
             continue;
         }
         const uint32_t m = (l + r) >> 1;
         const float4 p = __ldg(t.pos + m);  // one address for the warp
-        visit(lane == 0, ref_dist(qx, qy, qz, p), __ldg(&t.aux[m].x), m);
+        visit(lane == 0, ref_dist2(qx, qy, qz, p), __ldg(&t.aux[m].x), m);
         const uint32_t axis = __float_as_uint(p.w);
         const float qa = axis == 0 ? qx : (axis == 1 ? qy : qz);
         const float pa = axis == 0 ? p.x : (axis == 1 ? p.y : p.z);
         const float diff = __fsub_rn(qa, pa);
-        const float pd2 = __fsqrt_rn(__fmul_rn(diff, diff));  // norm(p - pplane) (kdtree.h:138-148)
+        const float pd2 = __fmul_rn(diff, diff);  // squared norm(p - pplane) (kdtree.h:138-148)
         if (sp + 2 <= kWarpStack) {  // holds for n < 2^31 (kWarpStack)
             if (lane == 0) {
                 if (qa < pa) {
@@ -334,17 +347,6 @@ struct KnnGroup {
     float *sd;
     uint32_t cap;
 };
-
-// Largest squared distance whose root is below radius (-1: none): the search compares squared
-// distances, and roots are taken of its answers only.
-inline float radius_squared(float radius)
-{
-    if (!(radius > 0.f)) return -1.f;
-    float s = std::min(radius * radius, FLT_MAX);
-    while (s > 0.f && !(std::sqrt(s) < radius)) s = std::nextafter(s, 0.f);
-    while (s < FLT_MAX && std::sqrt(std::nextafter(s, FLT_MAX)) < radius) s = std::nextafter(s, FLT_MAX);
-    return s;
-}
 
 // The calling lane's group in `words`, the shared memory of the warp (4 * knn_words(k)).
 __device__ __forceinline__ KnnGroup knn_group(uint32_t *words, uint32_t k)
@@ -590,7 +592,7 @@ __device__ __forceinline__ V3 group_photon_density(const PhotonTree &t, const Bs
 // divides 0 by 0 (a NaN sample, which the film drops); `compat` keeps that, otherwise 0. The
 // terms are summed lane-parallel. Returns the estimate on every lane.
 __device__ __forceinline__ V3 warp_photon_subsurface(const PhotonTree &t, const rt_material &m, V3 kd, V3 p, V3 nn,
-                                                     V3 wo_w, int32_t sid, float radius, bool compat,
+                                                     V3 wo_w, int32_t sid, float radius2, bool compat,
                                                      PhotonWarpScratch &sm)
 {
     const float eta = m.ior, g = m.roughness[1];
@@ -599,25 +601,42 @@ __device__ __forceinline__ V3 warp_photon_subsurface(const PhotonTree &t, const 
     const DipoleChannel d0 = dipole_setup(m.eta[0], m.extra[0], g, eta), d1 = dipole_setup(m.eta[1], m.extra[1], g, eta),
                         d2 = dipole_setup(m.eta[2], m.extra[2], g, eta);
     V3 sum = v3(0, 0, 0);
-    float maxd = 0.f;
-    uint32_t cnt = 0;
-    auto add = [&](uint32_t s, float r) {  // r: the photon's distance, as the search measured it
-        const float4 pw = __ldg(t.pw + s);
-        maxd = fmaxf(maxd, r);
+    float maxd2 = 0.f;
+    uint32_t cnt = 0, held = 0;
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    auto add = [&](uint32_t e) {  // entry e of the photons found
+        const float4 pw = __ldg(t.pw + sm.slot[e]);
+        const float r2 = sm.d2[e];
+        maxd2 = fmaxf(maxd2, r2);
         const float sc = kInvPi * (1.f - fresnel_dielectric_ref(pw.w, 1.f, eta)) * ft_o;
-        const float r2 = r * r;
         const V3 rd = v3(dipole_eval(d0, r2), dipole_eval(d1, r2), dipole_eval(d2, r2));
         sum = sum + rd * sc * v3(pw.x, pw.y, pw.z) * kd;
     };
-    warp_traverse<kRadiusScan>(t, p.x, p.y, p.z, sm, [&]() { return radius; },
-                               [&](bool valid, float dist, int shape, uint32_t s) {
-                                   const bool ok = valid && dist < radius && (sid == -1 || shape == sid);
-                                   cnt += __popc(__ballot_sync(kFullMask, ok));
-                                   if (ok) add(s, dist);
-                               });
+    // photons within the radius are collected and added 32 at a time: where they were found, most of the
+    // lanes waited for the few whose photons lay within it
+    warp_traverse<kRadiusScan>(t, p.x, p.y, p.z, radius2, sm, [&](bool valid, float dist2, int shape, uint32_t s) {
+        const bool ok = valid && dist2 <= radius2 && (sid == -1 || shape == sid);
+        const unsigned found = __ballot_sync(kFullMask, ok);
+        if (!found) return;
+        if (ok) {
+            const uint32_t at = held + __popc(found & below);
+            sm.d2[at] = dist2;
+            sm.slot[at] = s;
+        }
+        cnt += __popc(found);
+        held += __popc(found);
+        __syncwarp();
+        if (held >= 32) {
+            held -= 32;
+            add(held + lane);
+            __syncwarp();
+        }
+    });
+    if (lane < held) add(lane);
+    __syncwarp();
     if (cnt == 0) return compat ? v3(NAN, NAN, NAN) : v3(0, 0, 0);
     sum = v3(warp_sum(sum.x), warp_sum(sum.y), warp_sum(sum.z));
-    maxd = warp_max(maxd);
+    const float maxd = __fsqrt_rn(warp_max(maxd2));
     return sum * (1.f / (2.f * kPi * maxd * maxd));
 }
 

@@ -224,6 +224,7 @@ struct PhotonView {
     PhotonTree tree;
     uint32_t k;
     float radius2;  // radius_squared of the search radius
+    float subsurface_radius2;
 };
 
 // Material sort: the shading order of a wave. Each block takes chunks of 2^log2 queue slots
@@ -777,7 +778,7 @@ __global__ void __launch_bounds__(kGatherBlock, kGatherBlocks) k_gather(RenderVi
         if (i >= ns) break;  // warp-uniform
         const GatherRequest q = load_gather(bf, kGatherSubsurface, i);
         const V3 e = warp_photon_subsurface(pv.tree, rv.mats[min(q.mat, rv.nmats - 1)], q.kd, q.p, q.n, q.wo, q.shape,
-                                            kSubsurfaceRadius, compat, *reinterpret_cast<PhotonWarpScratch *>(words));
+                                            pv.subsurface_radius2, compat, *reinterpret_cast<PhotonWarpScratch *>(words));
         if (lane == 0) add_gather(bf, nxt, gv, q, e);
     }
     __syncwarp();
@@ -1334,6 +1335,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         pv.tree = photon_tree(s->pmap);
         pv.k = std::min<uint32_t>(std::max<uint32_t>(s->pm_k, 1u), kKnnMaxK);
         pv.radius2 = radius_squared(s->pm_radius);
+        pv.subsurface_radius2 = radius_squared(kSubsurfaceRadius);
     }
     bf.cap = cap;
     bf.scap = scap;
