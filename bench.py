@@ -644,7 +644,7 @@ def run_ours(args):
     # ---- scene commit: device vs host build of the same structures
     scene_build = measure_scene_build(core, N, ctx, v, f) if world == 1 else None
     if scene_build is not None and ref_cuda is not None:
-        scene_build["reference_ms"] = ref_cuda["build_ms"]
+        scene_build["reference_ms"] = ref_cuda.get("build_ms")  # absent without the reference harness
 
     ms, ms_e2e, ms_trace = max_over_ranks([ms, ms_e2e, ms_trace], world)
     if rank == 0:
