@@ -145,10 +145,13 @@ def build_scene(core, ctx, S):
 
 
 def cpu_reference_rate(v, f, o, d, threads):
-    """Reference traversal (oracle/_ref) over the sample; returns (Mrays/s, seconds)."""
+    """Reference traversal (oracle/_ref) over the sample; returns (Mrays/s, seconds), None without it."""
     from oracle import bindings
 
-    R = bindings.RefOracle()
+    try:
+        R = bindings.RefOracle()
+    except FileNotFoundError:
+        return None
     b = R.bvh(v, f)
     t0 = time.perf_counter()
     b.intersect(o, d, threads=threads)
@@ -712,11 +715,13 @@ def run_ours(args):
                               f"1 spp, depth 12 ({rays_ref} rays in {r['render_s']:.1f} s; BVH built and traversed "
                               f"by its own code on the host cores)"}
             ns = args.cpu_sample
-            val, dt = cpu_reference_rate(v, f, o[:ns], d[:ns], threads)
-            line["cpu_baseline_traversal"] = {
-                "value": val, "unit": "Mrays/s", "cores": threads, "kind": "reference",
-                "sample": f"first {ns} rays of the BVH-stress ray set through the reference's BVH::intersectRay "
-                          f"({dt:.1f} s); traversal only", "ours": trace_rate}
+            rate_cpu = cpu_reference_rate(v, f, o[:ns], d[:ns], threads)
+            if rate_cpu:
+                val, dt = rate_cpu
+                line["cpu_baseline_traversal"] = {
+                    "value": val, "unit": "Mrays/s", "cores": threads, "kind": "reference",
+                    "sample": f"first {ns} rays of the BVH-stress ray set through the reference's BVH::intersectRay "
+                              f"({dt:.1f} s); traversal only", "ours": trace_rate}
         print(json.dumps(line), flush=True)
     if world > 1:
         torch.distributed.destroy_process_group()
