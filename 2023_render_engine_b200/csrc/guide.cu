@@ -31,7 +31,7 @@ struct TrainArgs {
     const float *q, *dir, *pdf, *w;
     uint64_t B, Bpad;
     __half *xt, *gt;
-    float *scal;          // [1] loss sum (accumulated)
+    float *scal;          // [2] flags (uint); as double [2]: the loss sum
     const double *wpart;  // kWsumBlocks partial sums of the weights
     GuideBox box;
 };
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kFbThreads * kFbGroups, 1) k_guide_train_tc(co
     const float wmean = A.B ? (float)(wsum / (double)A.B) : 0.f;
     const float winv = wmean > 0.f ? 1.f / wmean : 0.f;
     const uint64_t Bp = A.Bpad;
-    float lsum = 0.f;
+    double lsum = 0.0;  // summed in 64 bits: a sum over the batch in 32 loses what the rows keep
     uint32_t phase = 0;
     bool failed = false;
     // waits for this group's MMA batch; false (for the whole group) when a wait ran out
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kFbThreads * kFbGroups, 1) k_guide_train_tc(co
             for (int j = 16; j < 24; j++) dout[j] = 0.f;
             if (half == 0) dout[16] = guide_loss_alpha(oa[0] + b[32], log_v, pdfb, wt);
             if (in_b) {
-                if (half == 0) lsum += loss;
+                if (half == 0) lsum += (double)loss;
             } else {
 #pragma unroll
                 for (int j = 0; j < 24; j++) dout[j] = 0.f;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kFbThreads * kFbGroups, 1) k_guide_train_tc(co
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if (lane == 0 && lsum != 0.f) atomicAdd(A.scal + 1, lsum);
+    if (lane == 0 && lsum != 0.0) atomicAdd(reinterpret_cast<double *>(A.scal) + 2, lsum);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(256) k_guide_wsum(const float *w, uint64_t B, 
         for (int i = 0; i < 8; i++) t += red[i];
         part[blockIdx.x] = t;
         if (blockIdx.x == 0) {
-            scal[1] = 0.f;
+            reinterpret_cast<double *>(scal)[2] = 0.0;
             reinterpret_cast<uint32_t *>(scal)[2] = 0u;
         }
     }
@@ -580,10 +580,19 @@ struct QuerySrc {
 
 struct RawSink {
     float *out;
+    bool aligned;  // to 16 bytes: a row of 48 values in 12 stores instead of 48
     __device__ void operator()(uint32_t row, bool valid, const float *o) const
     {
         if (!valid) return;
-        for (int i = 0; i < kGuideOut; i++) out[(uint64_t)row * kGuideOut + i] = o[i];
+        float *dst = out + (uint64_t)row * kGuideOut;
+        if (aligned) {
+#pragma unroll
+            for (int i = 0; i < kGuideOut / 4; i++)
+                reinterpret_cast<float4 *>(dst)[i] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < kGuideOut; i++) dst[i] = o[i];
+        }
     }
 };
 
@@ -755,13 +764,13 @@ int guide_train(rt_guide *g, const float *q, const float *dir, const float *pdf,
         RTB_CUDA(cudaGetLastError());
     }
     if (loss_out || grad_host) {
-        RTB_CUDA(cudaMemcpyAsync(g->host_scal, scal, 16, cudaMemcpyDeviceToHost, st));
+        RTB_CUDA(cudaMemcpyAsync(g->host_scal, scal, 32, cudaMemcpyDeviceToHost, st));
         if (grad_host)
             RTB_CUDA(cudaMemcpyAsync(grad_host, g->grad.ptr, 4ull * kGuideParamCount, cudaMemcpyDeviceToHost, st));
         RTB_CUDA(cudaStreamSynchronize(st));
         if (static_cast<const uint32_t *>(g->host_scal)[2] & 2u)
             return fail(RT_ERR_TIMEOUT, "guide training: a tensor-core completion wait timed out");
-        if (loss_out) *loss_out = static_cast<const float *>(g->host_scal)[1] / (float)B;
+        if (loss_out) *loss_out = (float)(static_cast<const double *>(g->host_scal)[2] / (double)B);
     }
     return RT_OK;
 }
@@ -923,7 +932,7 @@ int rt_guide_eval(rt_guide *g, const float *queries, uint64_t B, float *out)
     if (!queries || !out) return fail(RT_ERR_INVALID, "rt_guide_eval: null buffer");
     RTB_CHECK(guide_eval_begin(g));
     k_guide_eval<RawSink><<<infer_grid(g, B), kInferWarps * 32, kInferSmem, g->ctx->stream>>>(
-        g->img.as<uint4>(), guide_box(g), (uint32_t)B, QuerySrc{queries}, RawSink{out}, g->werr.as<uint32_t>());
+        g->img.as<uint4>(), guide_box(g), (uint32_t)B, QuerySrc{queries}, RawSink{out, (reinterpret_cast<uintptr_t>(out) & 15u) == 0}, g->werr.as<uint32_t>());
     RTB_CUDA(cudaGetLastError());
     return guide_eval_end(g, "rt_guide_eval");
 }

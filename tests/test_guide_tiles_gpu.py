@@ -39,3 +39,25 @@ def test_gradient_of_ragged_batches(core, gpu_ctx, B):
             assert np.linalg.norm(grad[a:b] - ref[a:b]) <= 0.1 * np.linalg.norm(ref[a:b]), (l, a)
     assert np.array_equal(grad, g.train_step(*args, apply=False, want_grad=True)[1])
     g.close()
+
+
+def test_raw_outputs_at_any_alignment(core, gpu_ctx):
+    """Rows are written 16 bytes at a time where the buffer allows it: the same values one float on."""
+    import ctypes
+    import torch
+
+    N = importlib.import_module("2023_render_engine_b200._native")
+    rng = np.random.default_rng(2)
+    B = 1001
+    unit = lambda v: v / np.linalg.norm(v, axis=-1, keepdims=True)
+    q = np.concatenate([rng.uniform(LO, HI, (B, 3)), unit(rng.normal(size=(B, 3))), unit(rng.normal(size=(B, 3)))],
+                       1).astype(np.float32)
+    g = core.Guide(gpu_ctx, LO, HI, learning_rate=1e-2, seed=7)
+    qd = torch.from_numpy(q.reshape(-1)).cuda()
+    want = g.eval(qd).reshape(-1)
+    for shift in (1, 2, 3):
+        out = torch.full((B * N.GUIDE_OUTPUTS + 8,), -7.0, device="cuda")
+        N.check(N.lib().rt_guide_eval(g.handle, qd.data_ptr(), B, ctypes.c_void_p(out.data_ptr() + 4 * shift)))
+        assert torch.equal(out[shift:shift + want.numel()], want)
+        assert (out[:shift] == -7.0).all() and (out[shift + want.numel():] == -7.0).all()
+    g.close()
