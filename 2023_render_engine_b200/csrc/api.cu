@@ -160,8 +160,7 @@ int DevBuf::upload(const void *src, size_t n, cudaStream_t s)
 void DevBuf::release()
 {
     if (ptr && pooled) {
-        cudaSetDevice(ctx->device);
-        cudaDeviceSynchronize();
+        cudaStreamSynchronize(ctx->stream);
         cudaFreeAsync(ptr, ctx->pool_stream);
     } else if (ptr) {
         cudaFree(ptr);

@@ -292,8 +292,9 @@ struct rt_context {
     // pages: 13 of the 17 ms of a photon pass, and 6 of the 17 ms of loading a 328,000-triangle mesh.
     // The pool keeps up to 1/64 of the device's memory between calls; it is given back with the
     // context, or when an allocation finds no memory. Allocations and frees go through a stream of
-    // their own, and a free waits for the device first, as cudaFree does, so that memory in
-    // the pool is idle whichever streams its users ran on.
+    // their own, and a free waits for the context's stream first (a call that returns has left
+    // no work behind on an earlier one), so that memory in the pool is idle. Waiting for the whole
+    // device instead would break another thread's stream capture.
     cudaMemPool_t pool = nullptr;
     cudaStream_t pool_stream = nullptr;
     // 64 slots of 64 bytes in pinned host memory, one per scene while there are some: a trace call's
@@ -330,7 +331,7 @@ struct rt_guide {
     // parameters: FP32 master, Adam moments, last gradient, FP16 shared-memory image
     rtb::DevBuf master, adam_m, adam_v, grad, img;
     // training scratch: transposed activations / gradients, per-chunk weight-gradient
-    // partials, scalars ([0] weight mean, [1] loss sum, [2] non-finite flag)
+    // partials, scalars (flags, loss sum, partial sums of the weights)
     rtb::DevBuf xt, gt, partial, scal;
     rtb::DevBuf tq, tdir, tpdf, tw;  // batch drawn from the records
     // path-tracer side: decoded mixture per queue slot, training records, the list of records
