@@ -239,7 +239,7 @@ __device__ __noinline__ static uint32_t knn_serial(const float4 *node_pos, const
 // by counting. Where no two distances are equal that is the only answer; otherwise the order, and at
 // the k-th distance the choice, are those of the reference's heap, which one lane then runs on the
 // host's tree (exact_pos, exact_aux; a few queries in ten thousand on scattered points).
-// 500,000 points, 200,003 queries, k = 50: 3.10 ms one query per thread, 1.35 ms so.
+// 500,000 points, 200,003 queries, k = 50: 3.10 ms one query per thread, 1.30 ms so.
 constexpr int kQueryBlock = 128;
 __global__ void __launch_bounds__(kQueryBlock) k_knn_group(const float4 *__restrict__ node_pos,
                                                            const int2 *__restrict__ node_aux,
