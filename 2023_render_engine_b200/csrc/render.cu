@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kB, RTB_TRAV_MIN_BLOCKS) k_shadow(RenderView r
     const uint32_t n = min(bf.cnt[kCntShadow], bf.scap);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(cnt64(bf.cnt, kCntShadowRays), (unsigned long long)n);  // stats
     walk_queue<true, false, false>(
-        rv.sv, scratch[threadIdx.x >> 5], n, bf.cnt + kCntShadowWork, false,
+        rv.sv, scratch[threadIdx.x >> 5], n, bf.cnt + kCntShadowWork,
         [&](uint32_t i, Walk &W) {
             const float4 r0 = reinterpret_cast<const float4 *>(bf.srays)[2 * i];
             const float4 r1 = reinterpret_cast<const float4 *>(bf.srays)[2 * i + 1];

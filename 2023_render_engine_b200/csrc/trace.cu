@@ -104,22 +104,22 @@ __device__ __forceinline__ void publish_status(uint32_t *counters, uint32_t *sta
 // A merged scene (rt_scene_merge) has no reference-order tree: a ray whose walk ran out of
 // stack keeps the hit found so far there (status word set).
 //
-// kTraceVisible: the call wants Scene::isVisible's decision, hit and offset <= the ray's tmax,
-// for the unbounded ray. Nodes beyond tmax are skipped all the same: a triangle hit beyond tmax
-// cannot change the decision, as a hit at t <= tmax is the nearest of all, and without one the
-// reference's offset is above tmax too unless a blocked triangle (b) lies within tmax, which
-// the walk sees and leaves to the replay.
+// kTraceVisible: the call wants Scene::isVisible's decision, hit and offset <= the ray's tmax, for the
+// unbounded ray, and the walk is unbounded too. Skipping nodes that the ray enters beyond tmax would
+// lose occluders: an entry distance is rounded by some 1e-7 of the origin's distance, which from a few
+// hundred scene sizes away is more than the boxes' margin, and at grazing incidence the offset itself
+// may lie before the entry (a barycentric mean of the vertices' offsets, not a point of the ray).
 __device__ __forceinline__ uint2 walk_closest(const SceneView &v, TravWarp &scratch, const rt_ray *rays, uint64_t n,
                                               rt_hit *hits, uint32_t flags, uint32_t *counters)
 {
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
     return walk_queue<false, false, true>(
-        v, scratch, (uint32_t)n, counters + 3, (flags & kTraceVisible) != 0,
+        v, scratch, (uint32_t)n, counters + 3,
         [&](uint32_t i, Walk &W) {
             float4 ra, rb;
             load_ray(rays, i, ra, rb);
             const uint32_t root = scene_root(v, v.subs ? __float_as_uint(rb.w) : 0u);
-            walk_init(W, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w, root, shadow);
+            walk_init(W, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, (flags & kTraceVisible) ? INFINITY : ra.w, root, shadow);
         },
         [&](uint32_t i, Walk &W, float2 bary) {
             int32_t rec = (int32_t)W.brec;
@@ -128,10 +128,7 @@ __device__ __forceinline__ uint2 walk_closest(const SceneView &v, TravWarp &scra
                 replay = v.subs == nullptr;
                 if (v.subs) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
             } else if (!(flags & RT_TRACE_FAST)) {
-                if (flags & kTraceVisible)
-                    replay = W.minblock < (W.bt <= W.lim ? W.bt : INFINITY);
-                else
-                    replay = rec >= 0 && W.minblock < W.bt;
+                replay = rec >= 0 && W.minblock < W.bt;
             }
             if (replay) {
                 rec = kHitReplay;
@@ -190,7 +187,7 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_counts(Sc
     __shared__ TravWarp scratch[kBlock / 32];
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
     walk_queue<ANY, true, true>(
-        v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3, false,
+        v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3,
         [&](uint32_t i, Walk &W) {
             float4 ra, rb;
             load_ray(rays, i, ra, rb);
@@ -269,7 +266,7 @@ __global__ void __launch_bounds__(kBlock, RTB_TRAV_MIN_BLOCKS) k_trace_any(Scene
     __shared__ TravWarp scratch[kBlock / 32];
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
     walk_queue<true, false, true>(
-        v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3, false,
+        v, scratch[threadIdx.x >> 5], (uint32_t)n, counters + 3,
         [&](uint32_t i, Walk &W) {
             float4 ra, rb;
             load_ray(rays, i, ra, rb);

@@ -120,7 +120,7 @@ __device__ __forceinline__ void scene_spheres(const SceneView &v, uint32_t sub, 
 }
 
 // root: the BVH8 node the walk starts at (kNoRoot: the scene has no triangles; the walk is
-// skipped). lim: the ray's limit (the walk's; the triangle test's too unless it is unbounded).
+// skipped). lim: the ray's limit.
 __device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz, float dx, float dy, float dz,
                                           float lim, uint32_t root, bool shadow)
 {
@@ -159,8 +159,7 @@ __device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz,
 // Without it (a walk that ends at any hit, whose limit never shrinks) they are visited as they come
 // in the node and the stack holds node indices only, twice as many.
 template <bool ANY, bool COUNT, bool ORDERED>
-__device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk &W, bool active, bool unbounded,
-                                          float shared_t)
+__device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk &W, bool active, float shared_t)
 {
     const unsigned lane = threadIdx.x & 31u;
     // visit a node: its eight quantized child boxes; the triangles of the hit leaves as a
@@ -292,9 +291,8 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
             w.Sx = __shfl_sync(kAllLanes, W.Sx, src);
             w.Sy = __shfl_sync(kAllLanes, W.Sy, src);
             w.Sz = __shfl_sync(kAllLanes, W.Sz, src);
-            const float lim = __shfl_sync(kAllLanes, W.lim, src);
             const uint32_t axis_base = __shfl_sync(kAllLanes, (tri_base << 2) | (W.kz & 3u), src);
-            w.tmax = unbounded ? INFINITY : lim;
+            w.tmax = __shfl_sync(kAllLanes, W.lim, src);
             w.kz = (int)(axis_base & 3u);
             w.kx = w.kz == 2 ? 0 : w.kz + 1;
             w.ky = w.kx == 2 ? 0 : w.kx + 1;
@@ -393,14 +391,13 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
 // there are idle lanes to help from the start.
 //
 // init(i, W) prepares ray i (walk_init); finish(i, W, bary) consumes its result. ANY: the walk
-// ends at the first accepted hit in triangle order (in the node that has one). unbounded: the
-// triangle test has no limit (lim only bounds the nodes). Returns the warp's rays where each warp
-// takes one range of the queue ([x, x + y), y = 0 otherwise). COUNT: also counts the triangles a
+// ends at the first accepted hit in triangle order (in the node that has one). Returns the warp's
+// rays where each warp takes one range of the queue ([x, x + y), y = 0 otherwise). COUNT: also counts the triangles a
 // serial walk would test (whole leaves, up to the leaf of the accepted hit under ANY), and every
 // ray keeps its own lane.
 template <bool ANY, bool COUNT, bool ORDERED, typename Init, typename Finish>
 __device__ __forceinline__ uint2 walk_queue(const SceneView &v, TravWarp &sm, uint32_t n, uint32_t *work,
-                                           bool unbounded, Init init, Finish finish)
+                                           Init init, Finish finish)
 {
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t warps = gridDim.x * (blockDim.x / 32u);
@@ -438,7 +435,7 @@ __device__ __forceinline__ uint2 walk_queue(const SceneView &v, TravWarp &sm, ui
             if (exhausted) return taken;
             continue;
         }
-        if (walk_step<ANY, COUNT, ORDERED>(v, sm, W, active, unbounded, INFINITY)) {
+        if (walk_step<ANY, COUNT, ORDERED>(v, sm, W, active, INFINITY)) {
             finish(ray, W, W.brec != kNoRec ? sm.bary[lane] : make_float2(0.f, 0.f));
             ray = 0xFFFFFFFFu;
         }
@@ -502,7 +499,7 @@ __device__ __forceinline__ uint2 walk_queue(const SceneView &v, TravWarp &sm, ui
         }
         const bool active = ray != 0xFFFFFFFFu;
         const float shared_t = active ? sm.found[W.kz >> 2].x : INFINITY;
-        const bool done = walk_step<ANY, COUNT, ORDERED>(v, sm, W, active, unbounded, shared_t);
+        const bool done = walk_step<ANY, COUNT, ORDERED>(v, sm, W, active, shared_t);
         // one ended lane after the other adds what it found to its ray's; the last reports it
         unsigned ended = __ballot_sync(kAllLanes, done);
         while (ended) {
