@@ -343,6 +343,7 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
                     break;
                 }
             }
+            if (COUNT && ANY) __syncwarp();  // the owners have read their pairs (above) before the next round's
         }
         if (COUNT && ANY) W.tested += W.brec != kNoRec ? before : mytris;
         __syncwarp();
