@@ -215,6 +215,16 @@ uint64_t rt_scene::device_bytes() const
            d_spheres.bytes + scratch.counters.bytes + d_tri_transp.bytes + d_mat_transp.bytes;
 }
 
+void context_release(rt_context *ctx)
+{
+    if (!ctx || --ctx->refs) return;
+    cudaSetDevice(ctx->device);
+    if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
+    destroy_pool(ctx);
+    if (ctx->status_page) cudaFreeHost(ctx->status_page);
+    delete ctx;
+}
+
 extern "C" {
 
 int rt_abi_version(void) { return RT_B200_ABI_VERSION; }
@@ -258,12 +268,7 @@ int rt_context_create(int device, rt_context **out)
 
 int rt_context_destroy(rt_context *ctx)
 {
-    if (!ctx) return RT_OK;
-    cudaSetDevice(ctx->device);
-    if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
-    destroy_pool(ctx);
-    if (ctx->status_page) cudaFreeHost(ctx->status_page);
-    delete ctx;
+    context_release(ctx);
     return RT_OK;
 }
 

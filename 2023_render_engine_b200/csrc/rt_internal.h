@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -302,10 +303,33 @@ struct rt_context {
     uint32_t *status_page = nullptr;
     uint64_t status_free = ~0ull;
     std::mutex status_mu;
+    // rt_context_create's own and one per scene, photon map and guide (ContextRef). They free their
+    // memory through the context's streams, and a host may let go of them in any order (a garbage
+    // collector does).
+    std::atomic<uint32_t> refs{1};
+};
+void context_release(rt_context *ctx);  // the last reference ends the context
+
+// An object's reference to its context. Its first member, so that it goes last.
+struct ContextRef {
+    rt_context *ctx = nullptr;
+    ContextRef() = default;
+    ContextRef(const ContextRef &) = delete;
+    ContextRef &operator=(const ContextRef &) = delete;
+    ContextRef &operator=(rt_context *c)
+    {
+        if (c) c->refs++;
+        context_release(ctx);
+        ctx = c;
+        return *this;
+    }
+    ~ContextRef() { context_release(ctx); }
+    rt_context *operator->() const { return ctx; }
+    operator rt_context *() const { return ctx; }
 };
 
 struct rt_photon_map {
-    rt_context *ctx = nullptr;
+    ContextRef ctx;
     uint64_t n = 0;
     rtb::DevBuf photons;   // rt_photon[n], (path, depth) order
     rtb::DevBuf node_pos;  // float4 per tree slot: xyz, split axis (uint bits)
@@ -324,7 +348,7 @@ struct rt_photon_map {
 };
 
 struct rt_guide {
-    rt_context *ctx = nullptr;
+    ContextRef ctx;
     rt_guide_opts opts{};
     uint64_t step = 0;     // Adam steps taken
     bool trained = false;  // parameters came from training or the caller: rendering samples the guide
@@ -344,7 +368,7 @@ struct rt_guide {
 };
 
 struct rt_scene {
-    rt_context *ctx = nullptr;
+    ContextRef ctx;
     // host copies of what was added
     std::vector<float> tri9;           // 9 floats per triangle
     std::vector<uint32_t> tri_material;

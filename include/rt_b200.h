@@ -53,6 +53,8 @@ RT_API int rt_last_error(char *buf, size_t len);
 /* Selects the device (replaces the bare cudaSetDevice(argv[2]) of the reference
  * mains, cornellBoxGuion.cu:35-49) and creates the context's stream. */
 RT_API int rt_context_create(int device, rt_context **out);
+/* Scenes, photon maps and guides made in the context keep what they need of it, and may be
+ * destroyed after it; its stream and memory go with the last of them. */
 RT_API int rt_context_destroy(rt_context *ctx);
 /* Use a caller-owned cudaStream_t (passed as void*) instead of the internal one. */
 RT_API int rt_context_set_stream(rt_context *ctx, void *cuda_stream);
