@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -205,14 +206,18 @@ __global__ void k_iota(uint32_t *v, uint64_t n)
 
 // ------------------------------------------------------------------- kNN
 
+// Mark in a query's count: it has equal distances and waits for the reference's heap (k is at most 128).
+constexpr uint32_t kKnnTied = 0x80000000u;
+
+// One thread per query, the reference's own heap. tied_only: only for the queries that k_knn_group marked.
 __global__ void __launch_bounds__(128) k_knn(const float4 *__restrict__ node_pos, const int2 *__restrict__ node_aux,
                                              uint32_t n, const float *__restrict__ queries,
                                              const int32_t *__restrict__ qshape, uint64_t nq, uint32_t k,
-                                             float radius, int32_t *__restrict__ out_idx,
+                                             float radius, bool tied_only, int32_t *__restrict__ out_idx,
                                              float *__restrict__ out_dist, uint32_t *__restrict__ out_count)
 {
     const uint64_t qi = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (qi >= nq) return;
+    if (qi >= nq || (tied_only && !(out_count[qi] & kKnnTied))) return;
     float hd[kKnnMaxK];
     int32_t hi[kKnnMaxK];
     const uint32_t cnt = knn_query(node_pos, node_aux, n, queries[3 * qi], queries[3 * qi + 1], queries[3 * qi + 2],
@@ -238,7 +243,8 @@ __device__ __noinline__ static uint32_t knn_serial(const float4 *node_pos, const
 // k-nearest queries, kGroup lanes each: group_knn finds the candidates, each lane then ranks its own
 // by counting. Where no two distances are equal that is the only answer; otherwise the order, and at
 // the k-th distance the choice, are those of the reference's heap, which one lane then runs on the
-// host's tree (exact_pos, exact_aux; a few queries in ten thousand on scattered points).
+// host's tree (exact_pos, exact_aux; a few queries in ten thousand on scattered points). Without that
+// tree (exact_pos null) the query is marked in its count, and *any_tied set.
 // 500,000 points, 200,003 queries, k = 50: 3.10 ms one query per thread, 1.30 ms so.
 constexpr int kQueryBlock = 128;
 __global__ void __launch_bounds__(kQueryBlock) k_knn_group(const float4 *__restrict__ node_pos,
@@ -248,7 +254,8 @@ __global__ void __launch_bounds__(kQueryBlock) k_knn_group(const float4 *__restr
                                                            const float *__restrict__ queries,
                                                            const int32_t *__restrict__ qshape, uint64_t nq, uint32_t k,
                                                            float radius, float radius2, int32_t *__restrict__ out_idx,
-                                                           float *__restrict__ out_dist, uint32_t *__restrict__ out_count)
+                                                           float *__restrict__ out_dist, uint32_t *__restrict__ out_count,
+                                                           uint32_t *any_tied)
 {
     extern __shared__ __align__(16) uint32_t knn_smem[];
     const KnnGroup g = knn_group(knn_smem + (threadIdx.x >> 5) * 4 * knn_words(k), k);
@@ -288,8 +295,11 @@ __global__ void __launch_bounds__(kQueryBlock) k_knn_group(const float4 *__restr
     if (!on) return;
     const uint32_t found = min(cnt, k);
     if (lane == 0) {
-        out_count[qi] = found;
-        if (tied) {
+        const bool wait = tied && !exact_pos;
+        out_count[qi] = found | (wait ? kKnnTied : 0u);
+        if (wait) {
+            *any_tied = 1;
+        } else if (tied) {
             int32_t *hi = reinterpret_cast<int32_t *>(g.ki);
             knn_serial(exact_pos, exact_aux, n, qx, qy, qz, sid, k, radius, g.kd, hi);
             for (uint32_t j = 0; j < found; j++) {
@@ -419,13 +429,12 @@ void kd_build(std::vector<KdElem> &e, std::vector<uint8_t> &axis, size_t left, s
 void map_context(rt_photon_map *m, rt_context *ctx)
 {
     m->ctx = ctx;
-    for (DevBuf *b : {&m->photons, &m->node_pos, &m->node_aux, &m->node_pw, &m->node_dir, &m->exact_pos, &m->exact_aux})
+    for (DevBuf *b : {&m->photons, &m->node_pos, &m->node_aux, &m->node_pw, &m->node_dir, &m->exact_pos, &m->exact_aux, &m->any_tied})
         b->ctx = ctx;
 }
 
 // The host build of a map's tree, uploaded to pos and aux.
-int kd_build_host(rt_photon_map *m, DevBuf &pos, DevBuf &aux)
-{
+int kd_build_host(rt_photon_map *m, DevBuf &pos, DevBuf &aux) try {
     cudaStream_t st = m->ctx->stream;
     const uint64_t n = m->n;
     std::vector<rt_photon> ph(n);
@@ -455,6 +464,17 @@ int kd_build_host(rt_photon_map *m, DevBuf &pos, DevBuf &aux)
     RTB_CHECK(pos.upload(np.data(), n * sizeof(float4), st));
     RTB_CHECK(aux.upload(na.data(), n * sizeof(int2), st));
     RTB_CUDA(cudaStreamSynchronize(st));
+    return RT_OK;
+} catch (const std::bad_alloc &) {
+    return fail(RT_ERR_OOM, "photon map: no host memory for the tree");
+}
+
+// That tree, where the map's own is not it: built when a query first needs it.
+int exact_tree(rt_photon_map *m)
+{
+    std::lock_guard<std::mutex> lk(m->exact_mu);
+    if (!m->exact) RTB_CHECK(kd_build_host(m, m->exact_pos, m->exact_aux));
+    m->exact = true;
     return RT_OK;
 }
 
@@ -541,6 +561,8 @@ int rt_photon_map_build(rt_photon_map *m)
     const uint64_t n = m->n;
     std::lock_guard<std::mutex> lk(m->exact_mu);
     m->exact = m->host_order = false;
+    RTB_CHECK(m->any_tied.reserve(4));
+    RTB_CUDA(cudaMemsetAsync(m->any_tied.ptr, 0, 4, st));
     RTB_CHECK(m->node_pos.reserve(std::max<uint64_t>(n, 1) * sizeof(float4)));
     RTB_CHECK(m->node_aux.reserve(std::max<uint64_t>(n, 1) * sizeof(int2)));
     RTB_CHECK(m->node_pw.reserve(std::max<uint64_t>(n, 1) * sizeof(float4)));
@@ -585,29 +607,35 @@ int rt_photon_knn(rt_photon_map *m, const float *q, const int32_t *qs, uint64_t 
     if (k == 0 || k > kKnnMaxK) return fail(RT_ERR_INVALID, "rt_photon_knn: k must be in [1, 128]");
     if (nq == 0) return RT_OK;
     RTB_CUDA(cudaSetDevice(m->ctx->device));
-    const DevBuf *pos = &m->node_pos, *aux = &m->node_aux;
-    {
+    cudaStream_t st = m->ctx->stream;
+    const uint32_t n = (uint32_t)m->n;
+    bool exact = m->host_order;  // the host's tree is there
+    if (!exact) {
+        if (!m->scattered) RTB_CHECK(exact_tree(m));
         std::lock_guard<std::mutex> lk(m->exact_mu);
-        if (!m->host_order) {
-            if (!m->exact) RTB_CHECK(kd_build_host(m, m->exact_pos, m->exact_aux));
-            m->exact = true;
-            pos = &m->exact_pos;
-            aux = &m->exact_aux;
-        }
+        exact = m->exact;
     }
-    if (m->scattered) {
-        const uint64_t blocks = (nq * kGroup + kQueryBlock - 1) / kQueryBlock;
-        k_knn_group<<<(unsigned)blocks, kQueryBlock, kQueryBlock / kGroup * 4 * knn_words(k), m->ctx->stream>>>(
-            m->node_pos.as<float4>(), m->node_aux.as<int2>(), pos->as<float4>(), aux->as<int2>(), (uint32_t)m->n, q, qs, nq,
-            k, radius, radius_squared(radius), out_idx, out_dist, out_count);
-    } else {
-        const uint64_t blocks = (nq + 127) / 128;
-        k_knn<<<(unsigned)blocks, 128, 0, m->ctx->stream>>>(pos->as<float4>(), aux->as<int2>(), (uint32_t)m->n, q, qs, nq,
-                                                            k, radius, out_idx, out_dist, out_count);
-    }
+    const DevBuf &pos = m->host_order ? m->node_pos : m->exact_pos, &aux = m->host_order ? m->node_aux : m->exact_aux;
+    auto by_thread = [&](bool tied_only) -> int {
+        k_knn<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(pos.as<float4>(), aux.as<int2>(), n, q, qs, nq, k, radius,
+                                                            tied_only, out_idx, out_dist, out_count);
+        RTB_CUDA(cudaGetLastError());
+        RTB_CUDA(cudaStreamSynchronize(st));
+        return RT_OK;
+    };
+    if (!m->scattered) return by_thread(false);
+    const uint64_t blocks = (nq * kGroup + kQueryBlock - 1) / kQueryBlock;
+    k_knn_group<<<(unsigned)blocks, kQueryBlock, kQueryBlock / kGroup * 4 * knn_words(k), st>>>(
+        m->node_pos.as<float4>(), m->node_aux.as<int2>(), exact ? pos.as<float4>() : nullptr, exact ? aux.as<int2>() : nullptr,
+        n, q, qs, nq, k, radius, radius_squared(radius), out_idx, out_dist, out_count, m->any_tied.as<uint32_t>());
     RTB_CUDA(cudaGetLastError());
-    RTB_CUDA(cudaStreamSynchronize(m->ctx->stream));
-    return RT_OK;
+    // set once and for all by the first query with equal distances: from then on the host's tree is there
+    uint32_t any_tied = 0;
+    if (!exact) RTB_CUDA(cudaMemcpyAsync(&any_tied, m->any_tied.ptr, 4, cudaMemcpyDeviceToHost, st));
+    RTB_CUDA(cudaStreamSynchronize(st));
+    if (!any_tied) return RT_OK;
+    RTB_CHECK(exact_tree(m));
+    return by_thread(true);
 }
 
 int rt_photon_subsurface(rt_photon_map *m, const rt_material *mat, const float *pts, const float *nrm, const float *wo,

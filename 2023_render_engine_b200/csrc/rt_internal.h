@@ -340,9 +340,9 @@ struct rt_photon_map {
     bool points = false;      // rt_photon_map_from_points: made for nearest-neighbour queries
     bool scattered = false;   // few nodes tie with another point: queries run on groups of lanes
     bool host_order = false;  // the tree is the host build's, equal coordinates included
-    // the host build's node_pos and node_aux where the tree above is not (made by the first
-    // rt_photon_knn, whose answers at equal distances depend on them)
-    rtb::DevBuf exact_pos, exact_aux;
+    // the host build's node_pos and node_aux where the tree above is not: made when rt_photon_knn first
+    // meets equal distances, whose order depends on them (any_tied: it has)
+    rtb::DevBuf exact_pos, exact_aux, any_tied;
     bool exact = false;
     std::mutex exact_mu;
 };
