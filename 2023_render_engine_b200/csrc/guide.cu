@@ -579,6 +579,7 @@ struct QuerySrc {
 };
 
 struct RawSink {
+    static constexpr int slot = 0;  // of its kernels in SMEM_GUIDE_EVAL
     float *out;
     bool aligned;  // to 16 bytes: a row of 48 values in 12 stores instead of 48
     __device__ void operator()(uint32_t row, bool valid, const float *o) const
@@ -597,6 +598,7 @@ struct RawSink {
 };
 
 struct PdfSink {
+    static constexpr int slot = 1;  // of its kernels in SMEM_GUIDE_EVAL
     const float *dir, *pdfb;
     float *out;
     __device__ void operator()(uint32_t row, bool valid, const float *o) const
@@ -610,6 +612,7 @@ struct PdfSink {
 };
 
 struct SampleSink {
+    static constexpr int slot = 2;  // of its kernels in SMEM_GUIDE_EVAL
     const float *u;
     float *dirs, *pdf;
     __device__ void operator()(uint32_t row, bool valid, const float *o) const
@@ -625,11 +628,11 @@ struct SampleSink {
     }
 };
 
-template <class Sink>
-__global__ void __launch_bounds__(kInferWarps * 32, 1) k_guide_eval(const uint4 *img, GuideBox box, uint32_t n,
-                                                                  QuerySrc src, Sink sink, uint32_t *werr)
+template <bool WHOLE, class Sink>
+__global__ void __launch_bounds__(InferShape<WHOLE>::threads, 1) k_guide_eval(const uint4 *img, GuideBox box, uint32_t n,
+                                                                              QuerySrc src, Sink sink, uint32_t *werr)
 {
-    guide_infer_rows(img, box, n, src, sink, werr);
+    guide_infer_rows<WHOLE>(img, box, n, src, sink, werr);
 }
 
 // ------------------------------------------------------------------ training samples
@@ -890,22 +893,36 @@ static int guide_eval_common(rt_guide *g, uint64_t B, const char *who)
     if (!g) return fail(RT_ERR_INVALID, std::string(who) + ": null guide");
     if (B >= (1ull << 31)) return fail(RT_ERR_INVALID, std::string(who) + ": batch too large");
     RTB_CUDA(cudaSetDevice(g->ctx->device));
-    if (!(device_slot(SLOT_SMEM_ATTRS) & SMEM_GUIDE_EVAL)) {
-        RTB_CUDA(cudaFuncSetAttribute(k_guide_eval<RawSink>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem));
-        RTB_CUDA(cudaFuncSetAttribute(k_guide_eval<PdfSink>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem));
-        RTB_CUDA(
-            cudaFuncSetAttribute(k_guide_eval<SampleSink>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem));
-        or_device_slot(SLOT_SMEM_ATTRS, SMEM_GUIDE_EVAL);
-    }
     return RT_OK;
 }
 
-static unsigned infer_grid(rt_guide *g, uint64_t B)
+}  // extern "C"
+
+template <bool WHOLE, class Sink>
+static int launch_eval(rt_guide *g, const float *queries, uint64_t B, const Sink &sink)
 {
+    using Shape = InferShape<WHOLE>;
+    const unsigned attr = SMEM_GUIDE_EVAL << (2 * Sink::slot + WHOLE);
+    if (!(device_slot(SLOT_SMEM_ATTRS) & attr)) {
+        RTB_CUDA(cudaFuncSetAttribute(k_guide_eval<WHOLE, Sink>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::smem));
+        or_device_slot(SLOT_SMEM_ATTRS, attr);
+    }
     const uint64_t tiles = (B + kInferRows - 1) / kInferRows;
-    return (unsigned)std::max<uint64_t>(
-        1, std::min<uint64_t>((tiles + kInferGroups - 1) / kInferGroups, (uint64_t)std::max(g->ctx->sm_count, 1)));
+    const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)std::max(g->ctx->sm_count, 1));
+    k_guide_eval<WHOLE><<<grid, Shape::threads, Shape::smem, g->ctx->stream>>>(
+        g->img.as<uint4>(), guide_box(g), (uint32_t)B, QuerySrc{queries}, sink, g->werr.as<uint32_t>());
+    return cuda_status(cudaGetLastError(), "k_guide_eval");
 }
+
+// B > 0 rows
+template <class Sink>
+static int eval(rt_guide *g, const float *queries, uint64_t B, const Sink &sink)
+{
+    return infer_whole(B, (uint64_t)std::max(g->ctx->sm_count, 1)) ? launch_eval<true>(g, queries, B, sink)
+                                                                   : launch_eval<false>(g, queries, B, sink);
+}
+
+extern "C" {
 
 // zeroes the tensor-core wait flag before an evaluation launch
 static int guide_eval_begin(rt_guide *g)
@@ -931,9 +948,7 @@ int rt_guide_eval(rt_guide *g, const float *queries, uint64_t B, float *out)
     if (B == 0) return RT_OK;
     if (!queries || !out) return fail(RT_ERR_INVALID, "rt_guide_eval: null buffer");
     RTB_CHECK(guide_eval_begin(g));
-    k_guide_eval<RawSink><<<infer_grid(g, B), kInferWarps * 32, kInferSmem, g->ctx->stream>>>(
-        g->img.as<uint4>(), guide_box(g), (uint32_t)B, QuerySrc{queries}, RawSink{out, (reinterpret_cast<uintptr_t>(out) & 15u) == 0}, g->werr.as<uint32_t>());
-    RTB_CUDA(cudaGetLastError());
+    RTB_CHECK(eval(g, queries, B, RawSink{out, (reinterpret_cast<uintptr_t>(out) & 15u) == 0}));
     return guide_eval_end(g, "rt_guide_eval");
 }
 
@@ -943,9 +958,7 @@ int rt_guide_pdf(rt_guide *g, const float *queries, const float *dirs, const flo
     if (B == 0) return RT_OK;
     if (!queries || !dirs || !bsdf_pdf || !out) return fail(RT_ERR_INVALID, "rt_guide_pdf: null buffer");
     RTB_CHECK(guide_eval_begin(g));
-    k_guide_eval<PdfSink><<<infer_grid(g, B), kInferWarps * 32, kInferSmem, g->ctx->stream>>>(
-        g->img.as<uint4>(), guide_box(g), (uint32_t)B, QuerySrc{queries}, PdfSink{dirs, bsdf_pdf, out}, g->werr.as<uint32_t>());
-    RTB_CUDA(cudaGetLastError());
+    RTB_CHECK(eval(g, queries, B, PdfSink{dirs, bsdf_pdf, out}));
     return guide_eval_end(g, "rt_guide_pdf");
 }
 
@@ -955,9 +968,7 @@ int rt_guide_sample(rt_guide *g, const float *queries, const float *u3, uint64_t
     if (B == 0) return RT_OK;
     if (!queries || !u3 || !out_dirs || !out_pdf) return fail(RT_ERR_INVALID, "rt_guide_sample: null buffer");
     RTB_CHECK(guide_eval_begin(g));
-    k_guide_eval<SampleSink><<<infer_grid(g, B), kInferWarps * 32, kInferSmem, g->ctx->stream>>>(
-        g->img.as<uint4>(), guide_box(g), (uint32_t)B, QuerySrc{queries}, SampleSink{u3, out_dirs, out_pdf}, g->werr.as<uint32_t>());
-    RTB_CUDA(cudaGetLastError());
+    RTB_CHECK(eval(g, queries, B, SampleSink{u3, out_dirs, out_pdf}));
     return guide_eval_end(g, "rt_guide_sample");
 }
 

@@ -432,30 +432,37 @@ __device__ __forceinline__ void ldmatrix4_trans(uint32_t addr, uint32_t r[4])
 // (M = 128, FP16 operands from shared memory, FP32 accumulator in 64 TMEM columns) issued by
 // one thread, then the 128 threads of the tile read their own row back from TMEM for bias,
 // ReLU and the FP16 store of the next layer's operand. A CTA holds one copy of the weights
-// and kInferGroups independent 128-thread groups, each with its own activation tile, TMEM
+// and InferShape::groups independent 128-thread groups, each with its own activation tile, TMEM
 // columns, mbarrier and named barrier, so 24 warps per SM hide each other's latency: bound by
 // the instructions of encoding and decoding (3,500 per row) at 60% of the issue rate. Sampling and
 // density of 1,000,003 rows: 479 / 450 / 429 us for 4 groups (the encoding in one operand) / 5 / 6.
+// Six operands fit only in two parts of the encoding, which costs each tile a round trip to the tensor
+// core more. Where four whole operands need no more rounds (infer_whole), they are taken: the two
+// calls for 1,000 / 37,888 / 150,000 rows take 91 / 92 / 125 us, against 96 / 100 / 129 us with six;
+// 1,000,003 rows 464 against 435. Tiles go to different SMs first; six to an SM, 1,000 rows took 112 us.
 // Operands are K-major without swizzle, in core matrices of 8 rows x 8 halves: row r, halves
 // [8c, 8c + 8) of an operand with KC chunks per row sit at byte (r / 8) * KC * 128 + c * 128 +
 // (r % 8) * 16.
 constexpr int kInferRows = 128;
-constexpr int kInferGroups = 6;
-constexpr int kInferWarps = 4 * kInferGroups;
 // byte offset of layer l's weight operand (W_l^T: guide_out(l) rows of guide_in(l) halves)
 __host__ __device__ constexpr int tc_w(int l) { return l == 0 ? 0 : tc_w(l - 1) + guide_out(l - 1) * guide_in(l - 1) * 2; }
 constexpr int kTcBias = tc_w(kGuideLayers);                                 // 304 FP32 biases
 constexpr int kTcA = 50432;                                                 // activation tiles
-constexpr int kTcATile = kInferRows * kEncode0 * 2;                         // 128 x 80 halves
-constexpr int kTcBar = kTcA + kInferGroups * kTcATile;                      // mbarriers, TMEM base
-constexpr int kInferSmem = kTcBar + 8 * kInferGroups + 16;
 constexpr int kTmemColsPerGroup = 64;
-constexpr int kTmemCols = 512;  // a power of 2 in [32, 512]
+// WHOLE: the encoding is one operand; otherwise it goes to the tensor core in two parts.
+template <bool WHOLE>
+struct InferShape {
+    static constexpr int groups = WHOLE ? 4 : 6, threads = 128 * groups;
+    static constexpr int tile = kInferRows * (WHOLE ? kGuideIn : kEncode0) * 2;  // bytes of an activation tile
+    static constexpr int bar = kTcA + groups * tile;                              // mbarriers, TMEM base
+    static constexpr int smem = bar + 8 * groups + 16;
+    static constexpr int tmem_cols = WHOLE ? 256 : 512;  // a power of 2 in [32, 512]
+    static_assert(smem <= 227 * 1024 && bar % 8 == 0, "shared memory per CTA");
+    static_assert(kTmemColsPerGroup * groups <= tmem_cols, "TMEM allocation");
+};
 constexpr uint32_t kUmmaWaitPolls = 1u << 22;
 static_assert(tc_w(1) == 18432 && tc_w(4) == 43008 && kTcBias == 49152, "operand sizes");
-static_assert(kTcBias + 4 * (4 * 64 + 48) <= kTcA && kTcA % 128 == 0 && kTcBar % 8 == 0, "shared layout");
-static_assert(kInferSmem <= 227 * 1024, "shared memory per CTA");
-static_assert(kTmemColsPerGroup * kInferGroups <= kTmemCols, "TMEM allocation");
+static_assert(kTcBias + 4 * (4 * 64 + 48) <= kTcA && kTcA % 128 == 0, "shared layout");
 static_assert(kEncode0 % 16 == 0 && kEncode1 % 16 == 0 && kEncode1 <= kEncode0 && 64 <= kEncode0, "operand tile");
 
 // byte offset of row r, chunk c (8 halves) in an operand of kc chunks per row
@@ -484,22 +491,31 @@ __device__ __forceinline__ bool group_sync_or(uint32_t id, bool v)
     return r != 0;
 }
 
+// Whether n rows on `sms` SMs take no more rounds of four whole operands than of six in two parts: up to
+// 4 tiles on an SM, and 7 or 8.
+inline bool infer_whole(uint64_t n, uint64_t sms)
+{
+    const uint64_t each = ((n + kInferRows - 1) / kInferRows + sms - 1) / sms;
+    return (each + 3) / 4 <= (each + 5) / 6;
+}
+
 // Forward pass over rows [0, n): src(row, q) fills the 9-float query and says whether the row
 // is guided; sink(row, valid, out) receives the 48 raw outputs (biases added; meaningless
 // where valid is false). Persistent CTAs
-// of kInferWarps warps and kInferSmem bytes of dynamic shared memory, one per SM; the weight
+// of InferShape<WHOLE>'s threads and dynamic shared memory, one per SM; the weight
 // image is staged once per CTA. A tensor-core wait that runs out of polls sets *werr
 // (nullable) and ends the group; the CTA frees its TMEM on exit.
-template <class Src, class Sink>
+template <bool WHOLE, class Src, class Sink>
 __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBox &box, uint32_t n, Src &src,
                                                  Sink &sink, uint32_t *werr)
 {
+    using Shape = InferShape<WHOLE>;
     extern __shared__ __align__(128) unsigned char guide_smem[];
     unsigned char *sm = guide_smem;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int grp = tid >> 7, gt = tid & 127;  // group, thread within the group
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + kTcBar) + grp;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + kTcBar + 8 * kInferGroups);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + Shape::bar) + grp;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(sm + Shape::bar + 8 * Shape::groups);
     // weights: image rows (W_l^T, stride guide_stride(l) halves) to core-matrix chunks
     const unsigned char *ib = reinterpret_cast<const unsigned char *>(img);
 #pragma unroll 1
@@ -515,7 +531,7 @@ __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBo
         reinterpret_cast<uint4 *>(sm + kTcBias)[i] = reinterpret_cast<const uint4 *>(ib + kGuideImgBias)[i];
     if (gt == 0) mbar_init(bar, 1);
     __syncwarp();
-    if (warp == 0) tmem_alloc(tslot, kTmemCols);
+    if (warp == 0) tmem_alloc(tslot, Shape::tmem_cols);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -524,7 +540,8 @@ __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBo
     const uint32_t tlane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);    // this warp's 32 lanes
     const uint32_t bar_id = 1u + (uint32_t)grp;                           // 0 is __syncthreads
     const float *bias = reinterpret_cast<const float *>(sm + kTcBias);
-    unsigned char *A = sm + kTcA + grp * kTcATile;
+    const uint32_t tiles = n / kInferRows + (n % kInferRows != 0);
+    unsigned char *A = sm + kTcA + grp * Shape::tile;
     uint32_t phase = 0;
     bool failed = false;
     // the K = 16 steps [s0, s1) of layer l, from an operand tile of kca chunks per row that starts at
@@ -537,51 +554,63 @@ __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBo
                      idesc, s > 0 ? 1u : 0u);
         umma_commit(bar);
     };
-    const uint32_t stride = gridDim.x * kInferGroups;
-    for (uint32_t tile = blockIdx.x * kInferGroups + grp; !failed && (uint64_t)tile * kInferRows < n; tile += stride) {
+    // tiles across the SMs first, so that few of them share one
+    for (uint32_t tile = blockIdx.x + gridDim.x * grp; !failed && tile < tiles; tile += gridDim.x * Shape::groups) {
         const uint32_t row = tile * kInferRows + gt;
         // rows that are not guided keep whatever their operand row holds: a row of the
         // product depends on its own operand row only, and their outputs are not used
         float q[9];
         const bool valid = row < n && src(row, q);
+        bool any = true;  // of the tile's rows is guided
         if (valid) {
             __half2 e[kEncode0 / 2];
             guide_encode0(q, box, e);
 #pragma unroll
             for (int c = 0; c < kEncode0 / 8; c++)
-                *reinterpret_cast<uint4 *>(A + tc_chunk(gt, c, kEncode0 / 8)) = *reinterpret_cast<const uint4 *>(&e[4 * c]);
+                *reinterpret_cast<uint4 *>(A + tc_chunk(gt, c, (WHOLE ? kGuideIn : kEncode0) / 8)) =
+                    *reinterpret_cast<const uint4 *>(&e[4 * c]);
         }
-        fence_async_smem();
-        tc_fence_before();
-        if (!group_sync_or(bar_id, valid)) {  // no guided row in the tile: no network pass
+        if (!WHOLE) {  // the first part's product runs while the second part is computed
+            fence_async_smem();
+            tc_fence_before();
+            any = group_sync_or(bar_id, valid);
+            if (any && gt == 0) {
+                tc_fence_after();
+                issue(0, kEncode0 / 8, 0, kEncode0 / 16);
+            }
+        }
+        if (any) {
+            __half2 e[kEncode1 / 2];
+            if (valid) guide_encode1(q, e);
+            bool ok = true;
+            if (!WHOLE) {
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, kUmmaWaitPolls));
+                phase ^= 1u;
+                tc_fence_after();
+            }
+            if (valid && ok)
+#pragma unroll
+                for (int c = 0; c < kEncode1 / 8; c++)
+                    *reinterpret_cast<uint4 *>(
+                        A + (WHOLE ? tc_chunk(gt, kEncode0 / 8 + c, kGuideIn / 8) : tc_chunk(gt, c, kEncode1 / 8))) =
+                        *reinterpret_cast<const uint4 *>(&e[4 * c]);
+            fence_async_smem();
+            tc_fence_before();
+            const bool r = group_sync_or(bar_id, WHOLE ? valid : !ok);
+            if (WHOLE)
+                any = r;
+            else
+                failed = r;
+        }
+        if (!any) {  // no network pass
             if (row < n) sink(row, false, q);
             continue;
         }
-        // the first part's product runs while the second part is computed
-        if (gt == 0) {
-            tc_fence_after();
-            issue(0, kEncode0 / 8, 0, kEncode0 / 16);
-        }
-        {
-            __half2 e[kEncode1 / 2];
-            if (valid) guide_encode1(q, e);
-            failed = !__all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, kUmmaWaitPolls));
-            phase ^= 1u;
-            tc_fence_after();
-            if (valid && !failed)
-#pragma unroll
-                for (int c = 0; c < kEncode1 / 8; c++)
-                    *reinterpret_cast<uint4 *>(A + tc_chunk(gt, c, kEncode1 / 8)) =
-                        *reinterpret_cast<const uint4 *>(&e[4 * c]);
-        }
-        fence_async_smem();
-        tc_fence_before();
-        failed = group_sync_or(bar_id, failed);
 #pragma unroll 1
         for (int l = 0; l < kGuideLayers && !failed; l++) {
             if (gt == 0) {
                 tc_fence_after();
-                issue(l, l == 0 ? kEncode1 / 8 : guide_in(l) / 8, l == 0 ? kEncode0 / 16 : 0, guide_in(l) / 16);
+                issue(l, l == 0 && !WHOLE ? kEncode1 / 8 : guide_in(l) / 8, l == 0 && !WHOLE ? kEncode0 / 16 : 0, guide_in(l) / 16);
             }
             // warp-uniform, as the tcgen05.ld below is .sync.aligned
             const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar, phase, kUmmaWaitPolls));
@@ -623,7 +652,7 @@ __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBo
     tc_fence_after();
     if (warp == 0) {
         __syncwarp();
-        tmem_dealloc(*tslot, kTmemCols);
+        tmem_dealloc(*tslot, Shape::tmem_cols);
     }
 }
 

@@ -857,8 +857,10 @@ __global__ void __launch_bounds__(kB) k_retire(Buffers bf, float *sum, uint32_t 
 
 // Guide network at the wave's hits (queue slots of buffer `cur`); writes the decoded mixture
 // per slot, alpha = 0 where the vertex is not guided.
-__global__ void __launch_bounds__(kInferWarps * 32, 1) k_guide_infer(RenderView rv, Buffers bf, int cur, const uint4 *img,
-                                                                   GuideBox box, GuideParams *params, uint32_t max_depth)
+template <bool WHOLE>
+__global__ void __launch_bounds__(InferShape<WHOLE>::threads, 1) k_guide_infer(RenderView rv, Buffers bf, int cur,
+                                                                               const uint4 *img, GuideBox box,
+                                                                               GuideParams *params, uint32_t max_depth)
 {
     // kCntGuideTimeout: set when a tensor-core completion wait ran out (checked after every wave group)
     const uint32_t n = min(bf.cnt[kCntQueue + 32 * cur], bf.cap);
@@ -893,7 +895,7 @@ __global__ void __launch_bounds__(kInferWarps * 32, 1) k_guide_infer(RenderView 
         guide_decode(o, P);
         params[q] = P;
     };
-    guide_infer_rows(img, box, n, src, sink, bf.cnt + kCntGuideTimeout);
+    guide_infer_rows<WHOLE>(img, box, n, src, sink, bf.cnt + kCntGuideTimeout);
 }
 
 __global__ void k_texture_lookup(RenderView rv, uint32_t id, const float *uv, uint64_t n, float *rgb)
@@ -1379,11 +1381,17 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
         gather_blocks = (unsigned)std::min<uint64_t>((uint64_t)device_sm_count() * (unsigned)std::max(per_sm, 1),
                                                      std::max<uint64_t>(1, (uint64_t)gcap / kGatherWarps));
     }
-    if (gv.params && !(device_slot(SLOT_SMEM_ATTRS) & SMEM_RENDER_INFER)) {
-        RTB_CUDA(cudaFuncSetAttribute(k_guide_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem));
-        or_device_slot(SLOT_SMEM_ATTRS, SMEM_RENDER_INFER);
+    // by the capacity: the waves' sizes are known on the device only
+    const bool infer_in_one = infer_whole(cap, (uint64_t)std::max(1, s->ctx->sm_count));
+    auto infer_kernel = infer_in_one ? k_guide_infer<true> : k_guide_infer<false>;
+    const int infer_threads = infer_in_one ? InferShape<true>::threads : InferShape<false>::threads;
+    const int infer_smem = infer_in_one ? InferShape<true>::smem : InferShape<false>::smem;
+    const unsigned infer_attr = SMEM_RENDER_INFER << (infer_in_one ? 1 : 0);
+    if (gv.params && !(device_slot(SLOT_SMEM_ATTRS) & infer_attr)) {
+        RTB_CUDA(cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, infer_smem));
+        or_device_slot(SLOT_SMEM_ATTRS, infer_attr);
     }
-    const unsigned infer_blocks = (unsigned)std::max(1, s->ctx->sm_count);  // one CTA of 4 tile groups per SM
+    const unsigned infer_blocks = (unsigned)std::max(1, s->ctx->sm_count);  // one CTA per SM
     const GuideBox gbox = guided ? guide_box(guide) : GuideBox{};
     k_start<<<blocks, kB, 0, st>>>(rv, bf);
     RTB_CUDA(cudaGetLastError());
@@ -1423,7 +1431,7 @@ int render_views(rt_scene *s, const rt_view *views, uint32_t nviews, uint32_t fl
     auto wave_group = [&]() -> int {
         int cur = 0;
         auto infer = [&]() -> int {
-            k_guide_infer<<<infer_blocks, kInferWarps * 32, kInferSmem, st>>>(
+            infer_kernel<<<infer_blocks, infer_threads, infer_smem, st>>>(
                 rv, bf, cur, guide->img.as<uint4>(), gbox, guide->params.as<GuideParams>(), gv.max_depth);
             RTB_CUDA(cudaGetLastError());
             return RT_OK;

@@ -92,7 +92,12 @@ enum DeviceSlot : int {
     SLOT_MEM_MIB = 7,          // device memory, MiB
     SLOT_COUNT = 8
 };
-enum SmemAttr : unsigned { SMEM_RENDER_INFER = 1u, SMEM_GUIDE_TRAIN = 2u, SMEM_GUIDE_EVAL = 4u, SMEM_PLOC_TAIL = 8u };
+enum SmemAttr : unsigned {
+    SMEM_RENDER_INFER = 1u,  // two kernels: bits 0 and 1
+    SMEM_GUIDE_TRAIN = 4u,
+    SMEM_PLOC_TAIL = 8u,
+    SMEM_GUIDE_EVAL = 16u,  // six: bits 4 to 9
+};
 // Value of `slot` for the current device; 0 until set_device_slot stored one.
 unsigned device_slot(DeviceSlot slot);
 void set_device_slot(DeviceSlot slot, unsigned value);
