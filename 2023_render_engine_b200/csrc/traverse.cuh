@@ -147,6 +147,40 @@ __device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz,
     W.tested = 0;
 }
 
+// The triangles of a node's hit leaves for one lane, one after the other: what walk_step does with
+// SERIAL, and what its pairs give.
+template <bool ANY>
+__device__ __forceinline__ void lane_triangles(const SceneView &v, TravWarp &sm, Walk &W, uint32_t tri_base, uint32_t trimask)
+{
+    WatertightRay w;
+    w.ox = W.ox, w.oy = W.oy, w.oz = W.oz;
+    w.Sx = W.Sx, w.Sy = W.Sy, w.Sz = W.Sz;
+    w.tmax = W.lim;
+    w.kz = (int)(W.kz & 3u);
+    w.kx = w.kz == 2 ? 0 : w.kz + 1;
+    w.ky = w.kx == 2 ? 0 : w.kx + 1;
+#pragma unroll 1
+    while (trimask) {
+        const uint32_t rec = tri_base + (uint32_t)__ffs(trimask) - 1u;
+        trimask &= trimask - 1u;
+        const float4 *p = reinterpret_cast<const float4 *>(v.tris + rec);
+        const float4 a = ld_scene(p), b = ld_scene(p + 1), c = ld_scene(p + 2);
+        TriHit h;
+        if (!watertight_test(w, a, b, c, h)) continue;
+        if (W.shadow && (__float_as_uint(c.w) & 1u)) continue;
+        if (h.t > W.bt) continue;
+        if (h.t == W.bt && W.brec != kNoRec && __float_as_uint(a.w) < __float_as_uint(__ldg(&v.tris[W.brec].v0.w))) continue;
+        if (h.t <= watertight_delta_t(h)) {
+            W.minblock = fminf(W.minblock, h.t);
+            continue;
+        }
+        W.bt = h.t;
+        W.brec = rec;
+        sm.bary[threadIdx.x & 31u] = make_float2(fmul(h.e1, h.invDet), fmul(h.e2, h.invDet));
+        if (ANY) return;
+    }
+}
+
 // One step of a warp's walks: each active lane visits its next node, then the warp tests the
 // triangles of the leaves its lanes hit, one (ray, triangle) pair per lane: the pairs are numbered
 // by a prefix sum over the lanes, each lane reads its pair's ray from the owner by shuffles, and the
@@ -158,7 +192,8 @@ __device__ __forceinline__ void walk_init(Walk &W, float ox, float oy, float oz,
 // ORDERED: hit children are visited near to far and skipped once the best hit lies before them.
 // Without it (a walk that ends at any hit, whose limit never shrinks) they are visited as they come
 // in the node and the stack holds node indices only, twice as many.
-template <bool ANY, bool COUNT, bool ORDERED>
+// SERIAL: every lane tests its own triangles.
+template <bool ANY, bool COUNT, bool ORDERED, bool SERIAL = false>
 __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk &W, bool active, float shared_t)
 {
     const unsigned lane = threadIdx.x & 31u;
@@ -260,7 +295,10 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
     }
     // the triangles of the whole warp, 32 pairs a round
     const uint32_t mytris = (uint32_t)__popc(trimask);
-    if (__any_sync(kAllLanes, trimask != 0)) {
+    if (SERIAL) {
+        lane_triangles<ANY>(v, sm, W, tri_base, trimask);
+        __syncwarp();
+    } else if (__any_sync(kAllLanes, trimask != 0)) {
         uint32_t incl = mytris;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -534,13 +572,20 @@ __device__ __forceinline__ uint2 walk_queue(const SceneView &v, TravWarp &sm, ui
     }
 }
 
-// The exact test of one analytic shape, out of line: a ray comes here for the few shapes it may hit.
+// The exact test of one analytic shape. A plane hit reports its object-space (x, y); 0 for spheres.
+__device__ __forceinline__ bool shape_hit(const SphereRecord &sr, float ox, float oy, float oz, float dx, float dy,
+                                          float dz, float tmax, float &t, float &u, float &v)
+{
+    u = v = 0.f;
+    return (sr.flags & kShapePlane) ? plane_test(sr.w2o, ox, oy, oz, dx, dy, dz, tmax, t, u, v)
+                                    : sphere_test(sr.w2o, sr.radius, ox, oy, oz, dx, dy, dz, tmax, t);
+}
+// Out of line, where a ray comes for the few shapes it may hit.
 __device__ __noinline__ static bool shape_test(const SphereRecord *sr, float ox, float oy, float oz, float dx, float dy,
                                                float dz, float tmax, float3 *hit)
 {
-    float t, u = 0.f, v = 0.f;
-    const bool ok = (sr->flags & kShapePlane) ? plane_test(sr->w2o, ox, oy, oz, dx, dy, dz, tmax, t, u, v)
-                                              : sphere_test(sr->w2o, sr->radius, ox, oy, oz, dx, dy, dz, tmax, t);
+    float t, u, v;
+    const bool ok = shape_hit(*sr, ox, oy, oz, dx, dy, dz, tmax, t, u, v);
     if (ok) *hit = make_float3(t, u, v);
     return ok;
 }
@@ -554,7 +599,9 @@ __device__ __forceinline__ void prefetch_shapes(const SceneView &v)
         asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char *>(v.spheres) + 128u * i));
 }
 
-// Scene::intersects' loop over the analytic shapes (Scene.cu:141-146) of scene `sub`.
+// Scene::intersects' loop over the analytic shapes (Scene.cu:141-146) of scene `sub`. FEW: of few shapes
+// some ray of a warp comes near each, so that the test for those it passes by a margin saves nothing.
+template <bool FEW = false>
 __device__ __forceinline__ void intersect_spheres(const SceneView &v, uint32_t sub, float ox, float oy, float oz,
                                                   float dx, float dy, float dz, float tmax, bool shadow, float &t,
                                                   int32_t &prim, float &b1, float &b2)
@@ -562,14 +609,21 @@ __device__ __forceinline__ void intersect_spheres(const SceneView &v, uint32_t s
     uint32_t s0, ns;
     scene_spheres(v, sub, s0, ns);
     for (uint32_t s = s0; s < s0 + ns; s++) {
-        const SphereRecord *sr = v.spheres + s;
-        const float4 *m = reinterpret_cast<const float4 *>(sr->w2o);
-        const float4 tail = __ldg(reinterpret_cast<const float4 *>(&sr->radius));  // radius, material, shape id, flags
-        const uint32_t flags = __float_as_uint(tail.w);
-        if (shadow && (flags & 1u)) continue;
-        if ((flags & kShapeAffine) && sphere_missed(m, tail.x, ox, oy, oz, dx, dy, dz)) continue;
-        float3 hit;  // offset; a plane hit reports its object-space (x, y); 0 for spheres
-        if (shape_test(sr, ox, oy, oz, dx, dy, dz, tmax, &hit) && hit.x < t) {
+        float3 hit;  // offset, and of a plane the object-space (x, y)
+        if (FEW) {
+            const SphereRecord &sr = v.spheres[s];
+            if (shadow && (sr.flags & 1u)) continue;
+            if (!shape_hit(sr, ox, oy, oz, dx, dy, dz, tmax, hit.x, hit.y, hit.z)) continue;
+        } else {
+            const SphereRecord *sr = v.spheres + s;
+            const float4 *m = reinterpret_cast<const float4 *>(sr->w2o);
+            const float4 tail = __ldg(reinterpret_cast<const float4 *>(&sr->radius));  // radius, material, shape id, flags
+            const uint32_t flags = __float_as_uint(tail.w);
+            if (shadow && (flags & 1u)) continue;
+            if ((flags & kShapeAffine) && sphere_missed(m, tail.x, ox, oy, oz, dx, dy, dz)) continue;
+            if (!shape_test(sr, ox, oy, oz, dx, dy, dz, tmax, &hit)) continue;
+        }
+        if (hit.x < t) {
             t = hit.x;
             prim = RT_PRIM_SHAPE | (int32_t)s;
             b1 = hit.y;
@@ -633,34 +687,53 @@ __device__ __noinline__ static int32_t replay_reference(const SceneView &v, cons
 // rt_hit::prim between the walk and the end of a trace: a triangle record, -1, or
 constexpr int32_t kHitReplay = 0x7FFFFFFE;  // the reference traversal decides
 
-// What a fast-mode walk (RT_TRACE_FAST) leaves to do for ray i: the replay of a walk that ran out of
-// stack, the triangle's id unless the caller wants records or the walk wrote ids, and the
-// analytic shapes. Returns the ray's hit.
-__device__ __forceinline__ float4 finish_fast(const SceneView &v, const rt_ray *rays, uint64_t i, uint32_t flags,
-                                              float4 hv, uint32_t *counters)
+// The reference traversal's hit of a ray: offset, triangle id or -1, b1, b2. Out of line, values in and
+// out, so that the few rays that need it cost the others no memory.
+__device__ __noinline__ static float4 replay_hit(const SceneView &v, float4 ra, float4 rb, float tmax, bool shadow,
+                                                 uint32_t *counters)
 {
+    const WatertightRay w = make_watertight(ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, tmax);
+    bool overflow = false;
+    float t, b1 = 0.f, b2 = 0.f;
+    const int32_t prim =
+        replay_reference(v, w, fdiv(1.0f, rb.x), fdiv(1.0f, rb.y), fdiv(1.0f, rb.z), shadow, t, b1, b2, overflow);
+    if (overflow) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
+    atomicAdd(counters + 2, 1u);
+    return make_float4(t, __int_as_float(prim), b1, b2);
+}
+
+// What a fast-mode walk (RT_TRACE_FAST) leaves to do for a ray (ra, rb): the replay of a walk that ran
+// out of stack, the triangle's id unless the caller wants records or the walk wrote ids, and the
+// analytic shapes. Returns the ray's hit.
+template <bool FEW = false>
+__device__ __forceinline__ float4 finish_fast(const SceneView &v, float4 ra, float4 rb, uint32_t flags, float4 hv,
+                                              uint32_t *counters)
+{
+    const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
+    if (__float_as_int(hv.y) == kHitReplay) {
+        hv = replay_hit(v, ra, rb, ra.w, shadow, counters);
+        if ((flags & kTraceRecords) && __float_as_int(hv.y) >= 0) hv.y = __uint_as_float(v.leafpos[__float_as_int(hv.y)]);
+    } else if (__float_as_int(hv.y) >= 0 && !(flags & (kTraceRecords | kTraceIds))) {
+        hv.y = __ldg(&v.tris[__float_as_int(hv.y)].v1.w);
+    }
     float t = hv.x, b1 = hv.z, b2 = hv.w;
     int32_t prim = __float_as_int(hv.y);
-    const bool replay = prim == kHitReplay, shadow = (flags & RT_TRACE_SHADOW) != 0;
-    if (!v.nspheres && !replay) return hv;
-    float4 ra, rb;
-    load_ray(rays, i, ra, rb);
-    if (replay) {
-        const WatertightRay w = make_watertight(ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w);
-        bool overflow = false;
-        prim = replay_reference(v, w, fdiv(1.0f, rb.x), fdiv(1.0f, rb.y), fdiv(1.0f, rb.z), shadow, t, b1, b2, overflow);
-        if (overflow) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
-        atomicAdd(counters + 2, 1u);
-        if ((flags & kTraceRecords) && prim >= 0) prim = (int32_t)v.leafpos[prim];
-    } else if (prim >= 0 && !(flags & (kTraceRecords | kTraceIds))) {
-        prim = (int32_t)__float_as_uint(__ldg(&v.tris[prim].v1.w));
-    }
     if (prim < 0) t = INFINITY;
     // the ray's last word is its scene in a merged scene
     if (v.nspheres)
-        intersect_spheres(v, v.subs ? __float_as_uint(rb.w) : 0u, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w, shadow, t, prim,
-                          b1, b2);
+        intersect_spheres<FEW>(v, v.subs ? __float_as_uint(rb.w) : 0u, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w, shadow, t,
+                               prim, b1, b2);
     return make_float4(t, __int_as_float(prim), b1, b2);
+}
+
+// The same for ray i, which is read only where there is something to do.
+__device__ __forceinline__ float4 finish_fast(const SceneView &v, const rt_ray *rays, uint64_t i, uint32_t flags,
+                                              float4 hv, uint32_t *counters)
+{
+    if (!v.nspheres && __float_as_int(hv.y) != kHitReplay) return hv;
+    float4 ra, rb;
+    load_ray(rays, i, ra, rb);
+    return finish_fast(v, ra, rb, flags, hv, counters);
 }
 
 }  // namespace rtb
