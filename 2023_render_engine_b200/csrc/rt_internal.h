@@ -260,7 +260,8 @@ struct RenderScratch {
     DevBuf rays[2], st0[2], st1[2], st2[2], hits, srays, scontrib, retire, cnt, gather;
     DevBuf views, view_sample0, view_pixel0;  // the render's views and their prefix sums
     DevBuf perm;  // shading order of the wave (material sort)
-    void *host_cnt = nullptr;  // pinned
+    void *host_cnt = nullptr;  // pinned: a copy of the counters, two words of k_wave_count
+    cudaEvent_t look[2] = {};  // after the kernel that writes them
     double stage_ms[RT_RENDER_STAGES] = {};  // last render's per-stage time (RT_RENDER_STAGE_TIMES)
     void release();
 };
