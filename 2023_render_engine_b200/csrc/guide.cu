@@ -6,7 +6,7 @@
 //   k_guide_train_tc  per 128-row tile: encode, forward, loss gradient per row, backward
 //                     through the 5 layers; writes every layer's input and output gradient
 //                     feature-major, so the weight gradient is a contraction over rows
-//   k_guide_wgrad_tc  dW_l = X_l^T G_l and db_l = 1^T G_l per chunk of rows (FP32 partials), all layers
+//   k_guide_wgrad_tc  dW_l = X_l^T G_l and db_l = sum G_l per chunk of rows (FP32 partials), all layers
 //                     at once
 //   k_guide_reduce    sum of the chunk partials in a fixed order (deterministic gradient)
 //   k_guide_adam      Adam on the FP32 master weights; refreshes the FP16 image
@@ -334,13 +334,14 @@ __global__ void __launch_bounds__(kFbThreads * kFbGroups, 1) k_guide_train_tc(co
 // k_guide_wgrad_tc: dW_l^T = G_l^T X_l over a chunk of rows, all five layers, on tcgen05. The
 // feature-major planes are K-major operands with the rows as K: A = G_l^T (M = 128 lanes, the
 // out_l valid ones first; the rest of the tile is the next layer's rows or unused bytes, whose
-// products land in TMEM lanes nobody reads), B = X_l^T (N = in_l) and a row of ones, whose product is
-// the bias gradient: the last of the input's zero features, and 16 more rows for the other layers.
+// products land in TMEM lanes nobody reads), B = X_l^T (N = in_l).
 // Stages of 64 rows are copied (cp.async) into one of two shared-memory buffers while the tensor core
-// works on the other; the five accumulators (144 + 4 x 80 TMEM columns) stay in TMEM for the whole
-// chunk, which then writes its FP32 partial gradients in the master layout.
+// works on the other; the five accumulators (144 + 4 x 64 TMEM columns) stay in TMEM for the whole
+// chunk, which then writes its FP32 partial gradients in the master layout. The bias gradient is summed
+// by the threads, in FP32, while the tensor core has the stage (as a product with a row of ones it rounds
+// worse: 7e-7 of its norm at 262,144 rows).
 // A chunk of the usual batch (37,888 rows) has four stages, and loading them bounds it: 35 us with 128
-// threads that loaded and stored 16 bytes at a time, 23 us so; the bias gradient was 15 us by itself.
+// threads that loaded and stored 16 bytes at a time, 26 us so, the sums included (15 us by themselves).
 // rows per CTA: a multiple of 64 chosen per step so the chunks about cover the SMs once
 __host__ __device__ inline uint64_t wgrad_chunk(uint64_t Bp, uint32_t sms)
 {
@@ -348,18 +349,32 @@ __host__ __device__ inline uint64_t wgrad_chunk(uint64_t Bp, uint32_t sms)
     return c < 256 ? 256 : c;
 }
 constexpr int kWgStageA = 5 * 8192 + 8192;         // G^T tiles: layer l at l * 8 KB (64 valid rows)
-constexpr int kWgStageB = 18 * 1024 + 4 * 10240;   // X^T tiles: layer 0 (144 rows), layers 1-4 (80)
+constexpr int kWgStageB = 18 * 1024 + 4 * 8192;    // X^T tiles: layer 0 (144 rows), layers 1-4 (64)
 constexpr int kWgThreads = 256;
 constexpr int kWgStage = kWgStageA + kWgStageB;
 constexpr int kWgBar = 2 * kWgStage;
 constexpr int kWgSmem = kWgBar + 16 + 16;
 constexpr int kWgTmemCols = 512;
 static_assert(kWgSmem <= 227 * 1024, "weight-gradient shared memory");
-__host__ __device__ constexpr int wg_b(int l) { return kWgStageA + (l == 0 ? 0 : 18 * 1024 + (l - 1) * 10240); }
-__host__ __device__ constexpr int wg_n(int l) { return l == 0 ? kGuideIn : 80; }  // the ones: row wg_ones(l)
-__host__ __device__ constexpr int wg_ones(int l) { return l == 0 ? kGuideIn - 1 : kGuideHidden; }
-__host__ __device__ constexpr int wg_col(int l) { return l == 0 ? 0 : kGuideIn + (l - 1) * 80; }
-static_assert(wg_col(4) + wg_n(4) <= kWgTmemCols, "weight-gradient TMEM");
+__host__ __device__ constexpr int wg_b(int l) { return kWgStageA + (l == 0 ? 0 : 18 * 1024 + (l - 1) * 8192); }
+__host__ __device__ constexpr int wg_col(int l) { return l == 0 ? 0 : kGuideIn + (l - 1) * 64; }
+static_assert(wg_col(4) + 64 <= kWgTmemCols, "weight-gradient TMEM");
+// (feature, 8 rows) pairs of a stage per thread
+constexpr int kWgBiasPairs = (kGuideGFeatures * 8 + kWgThreads - 1) / kWgThreads;
+static_assert(8 * kGuideGFeatures * 4 <= kWgStage, "room for the bias partials");
+
+// sum of 8 halves, pairwise
+__device__ __forceinline__ float sum_halves(uint4 v)
+{
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    float s[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&w[k]));
+        s[k] = h.x + h.y;
+    }
+    return (s[0] + s[1]) + (s[2] + s[3]);
+}
 
 __device__ __forceinline__ void copy16_async(uint32_t dst, const void *src)
 {
@@ -390,8 +405,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_guide_wgrad_tc(const __half *
     }
     __syncwarp();
     if (warp == 0) tmem_alloc(tslot, kWgTmemCols);
-    // stage s to its buffer: G^T, 304 features x 8 chunks of 8 rows; X^T: 400 features x 8 chunks, without
-    // the row of ones
+    // stage s to its buffer: G^T, 304 features x 8 chunks of 8 rows; X^T: 400 features x 8 chunks
     auto load = [&](int s) {
         const uint32_t buf = smem_u32(sm + (s & 1) * kWgStage);
         const uint64_t rs = r0 + 64ull * s;
@@ -404,21 +418,12 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_guide_wgrad_tc(const __half *
         for (int i = tid; i < kGuideXFeatures * 8; i += kWgThreads) {
             const int f = 8 * (i >> 6) + (i & 7), c = (i >> 3) & 7;
             const int l = f < kGuideIn ? 0 : 1 + (f - kGuideIn) / kGuideHidden, fl = f - guide_xoff(l);
-            if (f != wg_ones(0)) copy16_async(buf + wg_b(l) + tc_chunk(fl, c, 8), xt + (uint64_t)f * Bp + rs + 8 * c);
+            copy16_async(buf + wg_b(l) + tc_chunk(fl, c, 8), xt + (uint64_t)f * Bp + rs + 8 * c);
         }
     };
     for (int s = 0; s < 2; s++) {
         if (s < nstages) load(s);
         copy_commit();
-        // rows of ones: feature 143 of layer 0, rows 64..79 of the others
-        const uint32_t one2 = 0x3C003C00u;
-        for (int i = tid; i < (1 + 4 * 16) * 8; i += kWgThreads) {
-            const int r = i >> 3, c = i & 7;
-            const int l = r == 0 ? 0 : 1 + (r - 1) / 16;
-            *reinterpret_cast<uint4 *>(sm + s * kWgStage + wg_b(l) +
-                                       tc_chunk(r == 0 ? wg_ones(0) : kGuideHidden + (r - 1) % 16, c, 8)) =
-                make_uint4(one2, one2, one2, one2);
-        }
     }
     tc_fence_before();
     __syncthreads();
@@ -426,6 +431,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_guide_wgrad_tc(const __half *
     const uint32_t tmem = *tslot;
     uint32_t phase[2] = {0u, 0u};
     bool failed = false;
+    float bias[kWgBiasPairs] = {};
     for (int s = 0; s < nstages; s++) {
         const int b = s & 1;
         copy_wait<1>();
@@ -437,7 +443,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_guide_wgrad_tc(const __half *
             const uint32_t base = smem_u32(sm + b * kWgStage);
 #pragma unroll 1
             for (int l = 0; l < kGuideLayers; l++) {
-                const uint32_t idesc = umma_idesc_f16(128, wg_n(l));
+                const uint32_t idesc = umma_idesc_f16(128, guide_in(l));
                 for (int k = 0; k < 4; k++)
                     umma_f16(tmem + (uint32_t)wg_col(l), umma_desc(base + l * 8192 + 256u * k, 128u, 1024u),
                              umma_desc(base + wg_b(l) + 256u * k, 128u, 1024u), idesc, (s > 0 || k > 0) ? 1u : 0u);
@@ -445,7 +451,15 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_guide_wgrad_tc(const __half *
             umma_commit(bar + b);
         }
         __syncwarp();
-        // stage s + 2 takes this buffer once the products have read it
+#pragma unroll
+        for (int k = 0; k < kWgBiasPairs; k++) {  // the pairs of load()
+            const int i = tid + k * kWgThreads, f = 8 * (i >> 6) + (i & 7), c = (i >> 3) & 7;
+            const int l = f < 4 * kGuideHidden ? f / kGuideHidden : 4;
+            if (f < kGuideGFeatures)
+                bias[k] += sum_halves(*reinterpret_cast<const uint4 *>(sm + b * kWgStage + l * 8192 +
+                                                                       tc_chunk(f - guide_goff(l), c, 8)));
+        }
+        // stage s + 2 takes this buffer once the products and the sums have read it
         if (s + 2 < nstages) {
             const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar + b, phase[b], kUmmaWaitPolls));
             phase[b] ^= 1u;
@@ -473,17 +487,31 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_guide_wgrad_tc(const __half *
             const int out = guide_out(l);
             float *w = part + guide_pw(l) + o;
 #pragma unroll 1
-            for (int c0 = 16 * (warp >> 2); c0 < wg_n(l); c0 += 32) {
+            for (int c0 = 16 * (warp >> 2); c0 < guide_in(l); c0 += 32) {
                 float v[16];
+                __syncwarp();
                 tmem_ld16(tl + (uint32_t)(wg_col(l) + c0), v);
-                if (o >= out) continue;
-                // the ones are the first column of their 16 for l > 0 and the last for l = 0
-                if (c0 == wg_ones(l) / 16 * 16) part[guide_pb(l) + o] = v[wg_ones(l) % 16];
-                if (l > 0 && c0 == wg_ones(l)) continue;
-                if (l == 0 && c0 == wg_ones(0) / 16 * 16) v[wg_ones(0) % 16] = 0.f;
+                if (o < out) {
 #pragma unroll
-                for (int j = 0; j < 16; j++) w[(c0 + j) * out] = v[j];
+                    for (int j = 0; j < 16; j++) w[(c0 + j) * out] = v[j];
+                }
             }
+        }
+    }
+    if (!failed) {  // the products have read the stages: their memory takes the bias partials
+        float *red = reinterpret_cast<float *>(sm);
+#pragma unroll
+        for (int k = 0; k < kWgBiasPairs; k++) {
+            const int i = tid + k * kWgThreads, f = 8 * (i >> 6) + (i & 7), c = (i >> 3) & 7;
+            if (f < kGuideGFeatures) red[c * kGuideGFeatures + f] = bias[k];
+        }
+        __syncthreads();
+        for (int f = tid; f < kGuideGFeatures; f += kWgThreads) {
+            const int l = f < 4 * kGuideHidden ? f / kGuideHidden : 4;
+            float p[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) p[c] = red[c * kGuideGFeatures + f];
+            part[guide_pb(l) + f - guide_goff(l)] = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
         }
     }
     if (failed) {
