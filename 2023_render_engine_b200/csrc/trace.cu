@@ -218,8 +218,7 @@ __global__ void __launch_bounds__(kBlock, kTinyBlocks) k_trace_tiny(SceneView v,
     TravWarp &sm = scratch[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
-    flags = (flags & RT_TRACE_SHADOW) | (KIND == kTinyFast ? RT_TRACE_FAST : 0u) |
-            (KIND == kTinyVisible ? kTraceVisible : 0u);  // the rest is known here
+    flags = (flags & RT_TRACE_SHADOW) | (KIND == kTinyVisible ? kTraceVisible : 0u);  // the rest is known here
     prefetch_shapes(v);
     for (;;) {
         uint32_t base = 0;
@@ -248,8 +247,13 @@ __global__ void __launch_bounds__(kBlock, kTinyBlocks) k_trace_tiny(SceneView v,
                     atomicAdd(counters, 1u);
                 }
                 float4 h = make_float4(W.bt, __int_as_float(rec), bary.x, bary.y);
-                h = KIND == kTinyFast ? finish_fast<true>(v, ra, rb, flags, h, counters)
-                                      : finish_exact<true>(v, ra, rb, flags, h, counters);
+                if (KIND == kTinyFast) {
+                    if (rec >= 0) rec = (int32_t)__float_as_uint(__ldg(&v.tris[rec].v1.w));
+                    intersect_spheres<true>(v, 0u, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w, shadow, h.x, rec, h.z, h.w);
+                    h.y = __int_as_float(rec);
+                } else {
+                    h = finish_exact<true>(v, ra, rb, flags, h, counters);
+                }
                 if (KIND == kTinyVisible)
                     occ = visible_hit(h, ra);
                 else

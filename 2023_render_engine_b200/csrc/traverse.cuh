@@ -702,38 +702,34 @@ __device__ __noinline__ static float4 replay_hit(const SceneView &v, float4 ra, 
     return make_float4(t, __int_as_float(prim), b1, b2);
 }
 
-// What a fast-mode walk (RT_TRACE_FAST) leaves to do for a ray (ra, rb): the replay of a walk that ran
-// out of stack, the triangle's id unless the caller wants records or the walk wrote ids, and the
+// What a fast-mode walk (RT_TRACE_FAST) leaves to do for ray i: the replay of a walk that ran out of
+// stack, the triangle's id unless the caller wants records or the walk wrote ids, and the
 // analytic shapes. Returns the ray's hit.
-template <bool FEW = false>
-__device__ __forceinline__ float4 finish_fast(const SceneView &v, float4 ra, float4 rb, uint32_t flags, float4 hv,
-                                              uint32_t *counters)
-{
-    const bool shadow = (flags & RT_TRACE_SHADOW) != 0;
-    if (__float_as_int(hv.y) == kHitReplay) {
-        hv = replay_hit(v, ra, rb, ra.w, shadow, counters);
-        if ((flags & kTraceRecords) && __float_as_int(hv.y) >= 0) hv.y = __uint_as_float(v.leafpos[__float_as_int(hv.y)]);
-    } else if (__float_as_int(hv.y) >= 0 && !(flags & (kTraceRecords | kTraceIds))) {
-        hv.y = __ldg(&v.tris[__float_as_int(hv.y)].v1.w);
-    }
-    float t = hv.x, b1 = hv.z, b2 = hv.w;
-    int32_t prim = __float_as_int(hv.y);
-    if (prim < 0) t = INFINITY;
-    // the ray's last word is its scene in a merged scene
-    if (v.nspheres)
-        intersect_spheres<FEW>(v, v.subs ? __float_as_uint(rb.w) : 0u, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w, shadow, t,
-                               prim, b1, b2);
-    return make_float4(t, __int_as_float(prim), b1, b2);
-}
-
-// The same for ray i, which is read only where there is something to do.
 __device__ __forceinline__ float4 finish_fast(const SceneView &v, const rt_ray *rays, uint64_t i, uint32_t flags,
                                               float4 hv, uint32_t *counters)
 {
-    if (!v.nspheres && __float_as_int(hv.y) != kHitReplay) return hv;
+    float t = hv.x, b1 = hv.z, b2 = hv.w;
+    int32_t prim = __float_as_int(hv.y);
+    const bool replay = prim == kHitReplay, shadow = (flags & RT_TRACE_SHADOW) != 0;
+    if (!v.nspheres && !replay) return hv;
     float4 ra, rb;
     load_ray(rays, i, ra, rb);
-    return finish_fast(v, ra, rb, flags, hv, counters);
+    if (replay) {
+        const WatertightRay w = make_watertight(ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w);
+        bool overflow = false;
+        prim = replay_reference(v, w, fdiv(1.0f, rb.x), fdiv(1.0f, rb.y), fdiv(1.0f, rb.z), shadow, t, b1, b2, overflow);
+        if (overflow) atomicCAS(counters + 1, 0u, (uint32_t)DEV_STACK_OVERFLOW);
+        atomicAdd(counters + 2, 1u);
+        if ((flags & kTraceRecords) && prim >= 0) prim = (int32_t)v.leafpos[prim];
+    } else if (prim >= 0 && !(flags & (kTraceRecords | kTraceIds))) {
+        prim = (int32_t)__float_as_uint(__ldg(&v.tris[prim].v1.w));
+    }
+    if (prim < 0) t = INFINITY;
+    // the ray's last word is its scene in a merged scene
+    if (v.nspheres)
+        intersect_spheres(v, v.subs ? __float_as_uint(rb.w) : 0u, ra.x, ra.y, ra.z, rb.x, rb.y, rb.z, ra.w, shadow, t, prim,
+                          b1, b2);
+    return make_float4(t, __int_as_float(prim), b1, b2);
 }
 
 }  // namespace rtb
