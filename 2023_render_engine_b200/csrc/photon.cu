@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kQueryBlock) k_knn_group(const float4 *__restr
     }
     __syncwarp();
     // equal distances share a rank
-    tied |= group_sum(ranks) != cnt * (cnt - 1) / 2;
+    tied |= group_sum<kGroup>(ranks) != cnt * (cnt - 1) / 2;
     tied = ((__ballot_sync(kFullMask, tied) >> shift) & 0xFFu) != 0;
     if (!on) return;
     const uint32_t found = min(cnt, k);
@@ -343,10 +343,23 @@ __global__ void k_tree_attrs(const int2 *__restrict__ node_aux, const rt_photon 
 }
 
 
+// Lanes per query of k_density, of n photons: a query's own time counts where there are few, the instructions
+// all of them take where there are many, and their buffers' shared memory at large k. us by 32 / 16 / 8
+// lanes, 830,000 photons: 1,000 queries of 50 151 / 181 / 218, 12,000 of 50 220 / 239 / 291, 20,000 of 50
+// 278 / 268 / 299, 50,000 of 50 541 / 461 / 453, of 128 681 / 628 / 709; 20,000 photons: 4,000 of 50
+// 63 / 62 / 75, 8,000 of 50 89 / 75 / 79, 12,000 of 50 115 / 98 / 85, of 128 150 / 142 / 171.
+inline uint32_t density_lanes(uint64_t n, uint32_t k, uint64_t nq)
+{
+    const bool large = n >= 1u << 17;  // beyond the L1 caches
+    if (nq <= (large ? 14000u : 6000u)) return 32;
+    return k > 110 || (k > 85 && nq > 14000 && nq < 20000) || nq <= (large ? 40000u : 10000u) ? 16 : kGroup;
+}
+
 // Scene::combinePhotonContributions (Scene.cu:607-635) per query: the k nearest photons on
 // the same shape within radius, sum of power * lightScattered(-photon direction), divided by
 // pi * (largest neighbour distance)^2.
-__global__ void __launch_bounds__(kQueryBlock, kGatherBlocks) k_density(PhotonTree tree, rt_material mat,
+template <uint32_t G>
+__global__ void __launch_bounds__(kQueryBlock, G == 32 ? 8 : kGatherBlocks) k_density(PhotonTree tree, rt_material mat,
                                                                        const float *__restrict__ pts,
                                                                        const float *__restrict__ nrm,
                                                                        const float *__restrict__ wo,
@@ -354,15 +367,21 @@ __global__ void __launch_bounds__(kQueryBlock, kGatherBlocks) k_density(PhotonTr
                                                                        uint32_t k, float radius2, float *__restrict__ out)
 {
     extern __shared__ __align__(16) uint32_t knn_smem[];
-    const KnnGroup g = knn_group(knn_smem + (threadIdx.x >> 5) * 4 * knn_words(k), k);
-    const uint64_t qi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
+    const uint64_t qi = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
     const bool on = qi < nq;
     const uint64_t i = on ? qi : nq - 1;
     V3 p = v3(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
     V3 nn = normalize(v3(nrm[3 * i], nrm[3 * i + 1], nrm[3 * i + 2]));
     V3 w = v3(wo[3 * i], wo[3 * i + 1], wo[3 * i + 2]);
-    V3 c = group_photon_density(tree, load_bsdf(mat), p, nn, w, shape ? shape[i] : -1, k, radius2, true, on, g);
-    if (on && (threadIdx.x & (kGroup - 1u)) == 0) {
+    const int32_t sid = shape ? shape[i] : -1;
+    V3 c;
+    if (G == 32)
+        c = warp_photon_density(tree, load_bsdf(mat), p, nn, w, sid, k, radius2, true,
+                                reinterpret_cast<KnnWarpScratch *>(knn_smem)[threadIdx.x >> 5]);
+    else
+        c = group_photon_density<G>(tree, load_bsdf(mat), p, nn, w, sid, k, radius2, true, on,
+                                    knn_group<G>(knn_smem + (threadIdx.x >> 5) * (32 / G) * knn_words(k), k));
+    if (on && (threadIdx.x & (G - 1u)) == 0) {
         out[3 * qi] = c.x;
         out[3 * qi + 1] = c.y;
         out[3 * qi + 2] = c.z;
@@ -674,9 +693,18 @@ int rt_photon_density(rt_photon_map *m, const rt_material *mat, const float *pts
     if (nq == 0) return RT_OK;
     RTB_CUDA(cudaSetDevice(m->ctx->device));
     if (nq > (1ull << 31) / 32) return fail(RT_ERR_INVALID, "rt_photon_density: nq must be at most 2^26");
-    const uint64_t blocks = (nq * kGroup + kQueryBlock - 1) / kQueryBlock;
-    k_density<<<(unsigned)blocks, kQueryBlock, kQueryBlock / kGroup * 4 * knn_words(k), m->ctx->stream>>>(
-        photon_tree(m), *mat, pts, nrm, wo, shape, nq, k, radius_squared(radius), out_rgb);
+    auto launch = [&](auto kernel, uint32_t lanes) {
+        const uint64_t blocks = (nq * lanes + kQueryBlock - 1) / kQueryBlock;
+        const size_t smem = lanes == 32 ? kQueryBlock / 32 * sizeof(KnnWarpScratch)
+                                        : kQueryBlock / lanes * 4 * (size_t)knn_words(k);
+        kernel<<<(unsigned)blocks, kQueryBlock, smem, m->ctx->stream>>>(photon_tree(m), *mat, pts, nrm, wo, shape, nq, k,
+                                                                       radius_squared(radius), out_rgb);
+    };
+    switch (density_lanes(m->n, k, nq)) {
+    case 32: launch(k_density<32>, 32); break;
+    case 16: launch(k_density<16>, 16); break;
+    default: launch(k_density<kGroup>, kGroup);
+    }
     RTB_CUDA(cudaGetLastError());
     RTB_CUDA(cudaStreamSynchronize(m->ctx->stream));
     return RT_OK;

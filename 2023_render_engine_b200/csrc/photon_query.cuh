@@ -247,12 +247,12 @@ __device__ __forceinline__ float warp_max(float v)
 // The pruned traversal of knn_query (kdtree.h:111-152) for a warp: the same depth-first,
 // near-side-first order with the same pruning (a far side is skipped when its split plane is
 // not nearer than the bound), decided warp-uniformly with the stack in shared memory. A range
-// of at most Scan photons is read 32 photons per load instead of node by node. radius2 is the squared
-// search distance (radius_squared); visit(valid, squared distance, shape, slot) is offered up to 32
+// of at most Scan photons is read 32 photons per load instead of node by node. bound() is the squared
+// search distance (warp-uniform); visit(valid, squared distance, shape, slot) is offered up to 32
 // photons, one per lane (an internal node's photon on lane 0).
-template <uint32_t Scan, class Visit>
-__device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, float qy, float qz, float radius2,
-                                              PhotonWarpScratch &sm, Visit &&visit)
+template <uint32_t Scan, class Scratch, class Bound, class Visit>
+__device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, float qy, float qz, Scratch &sm,
+                                              Bound &&bound, Visit &&visit)
 {
     const uint32_t lane = threadIdx.x & 31u;
     int sp = 1;
@@ -267,7 +267,7 @@ __device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, flo
         const uint32_t l = sm.sl[sp], r = sm.sr[sp];
         const float pd = sm.sd[sp];
         __syncwarp();  // every lane has read the entry before lane 0 reuses it
-        if (!(pd <= radius2) || r <= l) continue;
+        if (!(pd <= bound()) || r <= l) continue;
         if (r - l <= Scan) {
             for (uint32_t base = l; base < r; base += 64) {  // two loads in flight per lane
                 const uint32_t j0 = base + lane, j1 = base + 32 + lane;
@@ -310,6 +310,116 @@ __device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, flo
     }
 }
 
+// ------------------------------------------------------- k-nearest queries, a warp each
+// For few queries (density_lanes), where a query's own time counts: a whole warp scans and selects for it.
+// 500 / 4,000 estimates of 50 among 830,000 photons: 108 / 160 us, with 8 lanes each 176 / 263.
+constexpr uint32_t kKnnScan = 64;  // scanned subtree size
+// Candidate buffer: after a selection it holds k <= kKnnMaxK, and it is selected again before an append
+// could take it past kKnnBuf.
+constexpr uint32_t kKnnBuf = 256;
+static_assert(kKnnBuf >= 2 * kKnnMaxK, "room for k plus one batch of candidates");
+
+struct KnnWarpScratch {  // per warp, in shared memory
+    float kd[kKnnBuf];     // candidates' squared distances (unordered)
+    uint32_t ki[kKnnBuf];  // and tree slots
+    uint32_t sl[kWarpStack], sr[kWarpStack];
+    float sd[kWarpStack];
+};
+
+// The k nearest photons within the radius (radius2: radius_squared of it) on shape sid (-1: any), up to
+// the order in which photons at exactly equal distances compete for the last place. Candidates are
+// appended to a buffer; when it first holds k, and whenever it is nearly full, the k nearest are kept and
+// the bound becomes the k-th distance, as the reference's heap bound does once it holds k. Leaves the
+// neighbours' tree slots unordered in sm.ki; returns their count (all lanes).
+__device__ __forceinline__ uint32_t warp_knn(const PhotonTree &t, float qx, float qy, float qz, int32_t sid, uint32_t k,
+                                             float radius2, KnnWarpScratch &sm)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t cnt = 0, select_at = k;
+    // photons nearer than this (squared): all within the radius at first
+    float rcur = radius2 < 0.f ? -1.f : __int_as_float(__float_as_int(radius2) + 1);
+    // keep the k nearest of cnt > k buffered: the k-th smallest distance v (bitwise search on
+    // the float bits, which order like the values for distances >= 0), then the ones below it
+    // and as many equal to it as fill k
+    auto select = [&]() {
+        uint32_t key[kKnnBuf / 32], slot[kKnnBuf / 32];
+#pragma unroll
+        for (uint32_t i = 0; i < kKnnBuf / 32; i++) {
+            const uint32_t j = lane + 32 * i;
+            key[i] = j < cnt ? __float_as_uint(sm.kd[j]) : 0xFFFFFFFFu;
+            slot[i] = j < cnt ? sm.ki[j] : 0u;
+        }
+        // largest v with fewer than k keys below it (the k-th smallest key), or the first
+        // threshold met with exactly k below it (then those k are the k nearest, no tie)
+        uint32_t v = 0, less = 0;
+        bool exact = false;
+        for (int bit = 30; bit >= 0; bit--) {
+            const uint32_t tv = v | (1u << bit);
+            uint32_t c = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < kKnnBuf / 32; i++) c += key[i] < tv;
+            c = __reduce_add_sync(kFullMask, c);
+            if (c == k) {
+                v = tv;
+                less = k;
+                exact = true;
+                break;
+            }
+            if (c < k) {
+                v = tv;
+                less = c;
+            }
+        }
+        const uint32_t need = k - less;
+        __syncwarp();  // every lane holds its entries before the buffer is rewritten
+        uint32_t blt = 0, beq = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < kKnnBuf / 32; i++) {
+            const bool lt = key[i] < v, eq = key[i] == v;
+            const unsigned mlt = __ballot_sync(kFullMask, lt), meq = __ballot_sync(kFullMask, eq);
+            if (lt) {
+                const uint32_t pos = blt + __popc(mlt & below);
+                sm.kd[pos] = __uint_as_float(key[i]);
+                sm.ki[pos] = slot[i];
+            }
+            if (eq && !exact) {
+                const uint32_t rk = beq + __popc(meq & below);
+                if (rk < need) {
+                    sm.kd[less + rk] = __uint_as_float(key[i]);
+                    sm.ki[less + rk] = slot[i];
+                }
+            }
+            blt += __popc(mlt);
+            beq += __popc(meq);
+        }
+        __syncwarp();
+        cnt = k;
+        // the bound: the largest kept distance (v itself unless the search stopped early)
+        float mx = 0.f;
+        for (uint32_t j = lane; j < k; j += 32) mx = fmaxf(mx, sm.kd[j]);
+        rcur = exact ? warp_max(mx) : __uint_as_float(v);
+        select_at = kKnnBuf - 32;
+    };
+    warp_traverse<kKnnScan>(t, qx, qy, qz, sm, [&]() { return rcur; },
+                            [&](bool valid, float dist2, int shape, uint32_t slot) {
+                                const bool c = valid && dist2 < rcur && (sid == -1 || shape == sid);
+                                const unsigned mask = __ballot_sync(kFullMask, c);
+                                if (!mask) return;
+                                if (c) {
+                                    const uint32_t pos = cnt + __popc(mask & below);
+                                    sm.kd[pos] = dist2;
+                                    sm.ki[pos] = slot;
+                                }
+                                cnt += __popc(mask);
+                                __syncwarp();
+                                if (cnt >= select_at) select();
+                            });
+    if (cnt > k) select();
+    __syncwarp();
+    return cnt;
+}
+
 // ------------------------------------------------------- k-nearest queries, 8 lanes each
 // A warp answers four k-nearest queries at a time, kGroup lanes each. A whole warp per query was
 // bound by instructions, most of them the same on all lanes (a node step, a selection's counting
@@ -320,6 +430,12 @@ __device__ __forceinline__ void warp_traverse(const PhotonTree &t, float qx, flo
 // query, three selections of about 130 candidates. Leaves of 16 or 64 photons visit 31 or 12 leaves and
 // 62 or 32 nodes, for the same work.
 constexpr uint32_t kGroup = 8;
+// Lanes of a group's ballot.
+template <uint32_t G>
+__device__ __forceinline__ uint32_t group_mask()
+{
+    return 0xFFFFFFFFu >> (32u - G);
+}
 constexpr uint32_t kGroupScan = 32;  // subtrees of at most this many photons are read whole
 // Candidates a group may append between two looks at its buffer: a leaf and the nodes above it.
 constexpr uint32_t kGroupBatch = 64;
@@ -353,12 +469,13 @@ struct KnnGroup {
     uint32_t cap;
 };
 
-// The calling lane's group in `words`, the shared memory of the warp (4 * knn_words(k)).
+// The calling lane's group of G lanes in `words`, the shared memory of the warp (32 / G * knn_words(k)).
+template <uint32_t G = kGroup>
 __device__ __forceinline__ KnnGroup knn_group(uint32_t *words, uint32_t k)
 {
     KnnGroup g;
     g.cap = knn_cap(k);
-    uint32_t *w = words + ((threadIdx.x & 31u) / kGroup) * knn_words(k);
+    uint32_t *w = words + ((threadIdx.x & 31u) / G) * knn_words(k);
     g.kd = reinterpret_cast<float *>(w);
     g.ki = w + g.cap;
     g.sl = g.ki + g.cap;
@@ -367,17 +484,18 @@ __device__ __forceinline__ KnnGroup knn_group(uint32_t *words, uint32_t k)
     return g;
 }
 
-template <typename T>
+template <uint32_t G, typename T>
 __device__ __forceinline__ T group_sum(T v)
 {
 #pragma unroll
-    for (uint32_t o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
+    for (uint32_t o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
     return v;
 }
+template <uint32_t G>
 __device__ __forceinline__ float group_max(float v)
 {
 #pragma unroll
-    for (uint32_t o = kGroup / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFullMask, v, o));
+    for (uint32_t o = G / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFullMask, v, o));
     return v;
 }
 
@@ -391,13 +509,14 @@ constexpr int kRootSteps = 4;
 // halving on the float bits in turn (the values are not negative, so their bits order like them).
 // Where equal distances leave no such v, exactly k are kept. bound becomes v, or a little more than
 // the largest value where nothing has to go; groups of fewer than k candidates are left alone.
+template <uint32_t G>
 __device__ __forceinline__ void group_select(const KnnGroup &g, uint32_t k, uint32_t slack, uint32_t &cnt, float &bound)
 {
-    const uint32_t lane = threadIdx.x & (kGroup - 1u), shift = threadIdx.x & 31u & ~(kGroup - 1u);
+    const uint32_t lane = threadIdx.x & (G - 1u), shift = threadIdx.x & 31u & ~(G - 1u);
     const uint32_t mine = cnt >= k ? cnt : 0u;
     float mx = 0.f;
-    for (uint32_t j = lane; j < mine; j += kGroup) mx = fmaxf(mx, g.kd[j]);
-    int lo = -1, hi = __float_as_int(group_max(mx)) + 2 * kRootSteps;
+    for (uint32_t j = lane; j < mine; j += G) mx = fmaxf(mx, g.kd[j]);
+    int lo = -1, hi = __float_as_int(group_max<G>(mx)) + 2 * kRootSteps;
     uint32_t clo = 0, chi = mine;
     for (uint32_t it = 0;; it++) {
         const bool more = chi > k + slack && hi - lo > 1;
@@ -409,8 +528,8 @@ __device__ __forceinline__ void group_select(const KnnGroup &g, uint32_t k, uint
             mid = min(max(__float_as_int(a + (b - a) * f), lo + 1), hi - 1);
         }
         uint32_t c = 0;
-        for (uint32_t j = lane; j < mine; j += kGroup) c += __float_as_int(g.kd[j]) <= mid ? 1u : 0u;
-        c = group_sum(c);
+        for (uint32_t j = lane; j < mine; j += G) c += __float_as_int(g.kd[j]) <= mid ? 1u : 0u;
+        c = group_sum<G>(c);
         if (more) {
             if (c >= k) {
                 hi = mid;
@@ -428,7 +547,7 @@ __device__ __forceinline__ void group_select(const KnnGroup &g, uint32_t k, uint
     const uint32_t most = __reduce_max_sync(kFullMask, cut ? mine : 0u);
     const bool ties = __any_sync(kFullMask, tied);
     uint32_t kept = 0, equal = 0;
-    for (uint32_t j0 = 0; j0 < most; j0 += kGroup) {
+    for (uint32_t j0 = 0; j0 < most; j0 += G) {
         const uint32_t j = j0 + lane;
         const bool in = j < mine;
         const float d = in ? g.kd[j] : 0.f;
@@ -436,11 +555,11 @@ __device__ __forceinline__ void group_select(const KnnGroup &g, uint32_t k, uint
         const int key = __float_as_int(d);
         bool keep = in && key <= hi;
         if (ties) {
-            const uint32_t eq = (__ballot_sync(kFullMask, in && key == hi) >> shift) & 0xFFu;
+            const uint32_t eq = (__ballot_sync(kFullMask, in && key == hi) >> shift) & group_mask<G>();
             if (tied && key == hi) keep = keep && clo + equal + __popc(eq & ((1u << lane) - 1u)) < k;
             equal += __popc(eq);
         }
-        const uint32_t m = (__ballot_sync(kFullMask, keep) >> shift) & 0xFFu;
+        const uint32_t m = (__ballot_sync(kFullMask, keep) >> shift) & group_mask<G>();
         if (keep) {
             const uint32_t at = kept + __popc(m & ((1u << lane) - 1u));
             g.kd[at] = d;
@@ -459,11 +578,12 @@ __device__ __forceinline__ void group_select(const KnnGroup &g, uint32_t k, uint
 // and returns their number: all there are if fewer than k, else the k nearest and up to slack more.
 // bound: every photon within the radius that is not among them has a squared distance above it, or
 // (exactly k kept among equals) one equal to it.
+template <uint32_t G = kGroup>
 __device__ __forceinline__ uint32_t group_knn(const float4 *__restrict__ pos, const int2 *__restrict__ aux, uint32_t n,
                                               float qx, float qy, float qz, int32_t sid, uint32_t k, float radius2,
                                               uint32_t slack, bool on, const KnnGroup &g, float &bound)
 {
-    const uint32_t lane = threadIdx.x & (kGroup - 1u), shift = threadIdx.x & 31u & ~(kGroup - 1u);
+    const uint32_t lane = threadIdx.x & (G - 1u), shift = threadIdx.x & 31u & ~(G - 1u);
     const uint32_t below = (1u << lane) - 1u;
     uint32_t l = 0, r = n, cnt = 0, limit = k;
     int sp = 0;
@@ -505,17 +625,17 @@ __device__ __forceinline__ uint32_t group_knn(const float4 *__restrict__ pos, co
                     l = m + 1;
             }
         }
-        float4 p[kGroupScan / kGroup];
+        float4 p[kGroupScan / G];
 #pragma unroll
-        for (uint32_t i = 0; i < kGroupScan / kGroup; i++)
-            if (live && l + lane + kGroup * i < r) p[i] = __ldg(pos + l + lane + kGroup * i);
+        for (uint32_t i = 0; i < kGroupScan / G; i++)
+            if (live && l + lane + G * i < r) p[i] = __ldg(pos + l + lane + G * i);
 #pragma unroll
-        for (uint32_t i = 0; i < kGroupScan / kGroup; i++) {
-            const uint32_t j = l + lane + kGroup * i;
+        for (uint32_t i = 0; i < kGroupScan / G; i++) {
+            const uint32_t j = l + lane + G * i;
             const float d = ref_dist2(qx, qy, qz, p[i]);
             bool c = live && j < r && d <= bound;
             if (c && sid != -1) c = __ldg(&aux[j].x) == sid;
-            const uint32_t m = (__ballot_sync(kFullMask, c) >> shift) & 0xFFu;
+            const uint32_t m = (__ballot_sync(kFullMask, c) >> shift) & group_mask<G>();
             if (c) {
                 const uint32_t at = cnt + __popc(m & below);
                 g.kd[at] = d;
@@ -526,7 +646,7 @@ __device__ __forceinline__ uint32_t group_knn(const float4 *__restrict__ pos, co
         __syncwarp();
         // all groups select together: one by itself would take as long
         if (__any_sync(kFullMask, live && cnt >= limit)) {
-            group_select(g, k, kKnnSlack, cnt, bound);
+            group_select<G>(g, k, kKnnSlack, cnt, bound);
             if (cnt >= k) limit = g.cap - kGroupBatch;
         }
         if (live) {
@@ -545,7 +665,7 @@ __device__ __forceinline__ uint32_t group_knn(const float4 *__restrict__ pos, co
         }
         __syncwarp();
     }
-    if (__any_sync(kFullMask, cnt > k + slack)) group_select(g, k, slack, cnt, bound);
+    if (__any_sync(kFullMask, cnt > k + slack)) group_select<G>(g, k, slack, cnt, bound);
     return cnt;
 }
 
@@ -554,20 +674,19 @@ __device__ __forceinline__ uint32_t group_knn(const float4 *__restrict__ pos, co
 // power * f(wo, -dir)|cos| (SurfaceInteraction::lightScattered, SurfaceInteraction.cu:278-292)
 // / (pi * maxDist^2). The reference weights each photon by |cos| although the photon density
 // already carries the projected-area factor; with compat = false the estimate uses f alone
-// (the radiance estimate of photon mapping). The k terms are summed lane-parallel. Returns the
-// estimate on every lane of the group.
-__device__ __forceinline__ V3 group_photon_density(const PhotonTree &t, const Bsdf &bs, V3 p, V3 nn, V3 wo_w, int32_t sid,
-                                                   uint32_t k, float radius2, bool compat, bool on, const KnnGroup &g)
+// (the radiance estimate of photon mapping). The cnt terms (tree slots) are summed lane-parallel. Returns
+// the estimate on every lane of the group.
+template <uint32_t G>
+__device__ __forceinline__ V3 photon_density(const PhotonTree &t, const Bsdf &bs, V3 p, V3 nn, V3 wo_w, bool compat,
+                                             const uint32_t *slots, uint32_t cnt)
 {
-    float bound;
-    const uint32_t cnt = group_knn(t.pos, t.aux, t.n, p.x, p.y, p.z, sid, k, radius2, 0, on, g, bound);
     V3 tt, b;
     onb(nn, tt, b);
     const V3 wo = v3(dot(wo_w, tt), dot(wo_w, b), dot(wo_w, nn));
     V3 sum = v3(0, 0, 0);
     float maxd = 0.f;
-    for (uint32_t j = threadIdx.x & (kGroup - 1u); j < cnt; j += kGroup) {
-        const uint32_t s = g.ki[j];
+    for (uint32_t j = threadIdx.x & (G - 1u); j < cnt; j += G) {
+        const uint32_t s = slots[j];
         const float4 pp = __ldg(t.pos + s), pw = __ldg(t.pw + s), pd = __ldg(t.dir + s);
         maxd = fmaxf(maxd, length(v3(pp.x, pp.y, pp.z) - p));
         const V3 w = -v3(pd.x, pd.y, pd.z);
@@ -581,10 +700,26 @@ __device__ __forceinline__ V3 group_photon_density(const PhotonTree &t, const Bs
         sum = sum + v3(pw.x, pw.y, pw.z) * f;
     }
     __syncwarp();
-    sum = v3(group_sum(sum.x), group_sum(sum.y), group_sum(sum.z));
-    maxd = group_max(maxd);
+    sum = v3(group_sum<G>(sum.x), group_sum<G>(sum.y), group_sum<G>(sum.z));
+    maxd = group_max<G>(maxd);
     if (cnt == 0) return v3(0, 0, 0);
     return sum * (1.0f / (kPi * maxd * maxd));
+}
+
+// The estimate of a group of G lanes (on = false: none), and of a whole warp.
+template <uint32_t G = kGroup>
+__device__ __forceinline__ V3 group_photon_density(const PhotonTree &t, const Bsdf &bs, V3 p, V3 nn, V3 wo_w, int32_t sid,
+                                                   uint32_t k, float radius2, bool compat, bool on, const KnnGroup &g)
+{
+    float bound;
+    const uint32_t cnt = group_knn<G>(t.pos, t.aux, t.n, p.x, p.y, p.z, sid, k, radius2, 0, on, g, bound);
+    return photon_density<G>(t, bs, p, nn, wo_w, compat, g.ki, cnt);
+}
+__device__ __forceinline__ V3 warp_photon_density(const PhotonTree &t, const Bsdf &bs, V3 p, V3 nn, V3 wo_w, int32_t sid,
+                                                  uint32_t k, float radius2, bool compat, KnnWarpScratch &sm)
+{
+    const uint32_t cnt = warp_knn(t, p.x, p.y, p.z, sid, k, radius2, sm);
+    return photon_density<32>(t, bs, p, nn, wo_w, compat, sm.ki, cnt);
 }
 
 // Scene::combinePhotonsSubsurface (Scene.cu:667-701) at point p (shading normal nn, direction
@@ -619,7 +754,8 @@ __device__ __forceinline__ V3 warp_photon_subsurface(const PhotonTree &t, const 
     };
     // photons within the radius are collected and added 32 at a time: where they were found, most of the
     // lanes waited for the few whose photons lay within it
-    warp_traverse<kRadiusScan>(t, p.x, p.y, p.z, radius2, sm, [&](bool valid, float dist2, int shape, uint32_t s) {
+    warp_traverse<kRadiusScan>(t, p.x, p.y, p.z, sm, [&]() { return radius2; },
+                               [&](bool valid, float dist2, int shape, uint32_t s) {
         const bool ok = valid && dist2 <= radius2 && (sid == -1 || shape == sid);
         const unsigned found = __ballot_sync(kFullMask, ok);
         if (!found) return;
