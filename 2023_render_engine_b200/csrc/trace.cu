@@ -70,7 +70,8 @@ __device__ __forceinline__ float4 finish_exact(const SceneView &v, float4 ra, fl
     }
     if (replay) {
         const float4 r = replay_hit(v, ra, rb, tri_max, shadow, counters);
-        t = r.x, prim = __float_as_int(r.y), b1 = r.z, b2 = r.w;
+        t = r.x, prim = __float_as_int(r.y);
+        if (prim >= 0) b1 = r.z, b2 = r.w;  // a ray the replay finds to miss keeps those of its walk
     }
     if (prim < 0) t = INFINITY;
     if ((flags & kTraceRecords) && prim >= 0) prim = (int32_t)v.leafpos[prim];
