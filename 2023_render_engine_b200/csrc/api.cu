@@ -104,6 +104,7 @@ void create_pool(rt_context *c)
         c->pool = nullptr;
         return;
     }
+    c->pool_keep = keep;
     std::lock_guard<std::mutex> lk(g_pools_mu);
     g_pools.push_back(c);
 }
@@ -124,7 +125,9 @@ int DevBuf::reserve(size_t n)
     if (n <= bytes && ptr) return RT_OK;
     release();
     if (n == 0) return RT_OK;
-    if (ctx && ctx->pool) {
+    uint64_t used = 0;
+    if (ctx && ctx->pool && cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+        used + n <= ctx->pool_keep) {
         cudaError_t e = cudaMallocFromPoolAsync(&ptr, n, ctx->pool, ctx->pool_stream);
         if (e == cudaSuccess) {
             pooled = true;

@@ -297,13 +297,17 @@ struct rt_context {
     rtb::DevBuf build[32];
     // Memory of scenes, photon maps and photon passes. cudaMalloc and cudaFree map and unmap
     // pages: 13 of the 17 ms of a photon pass, and 6 of the 17 ms of loading a 328,000-triangle mesh.
-    // The pool keeps up to 1/64 of the device's memory between calls; it is given back with the
-    // context, or when an allocation finds no memory. Allocations and frees go through a stream of
+    // The pool holds up to 1/64 of the device's memory (2.9 GB), kept between calls; it is given back
+    // with the context, or when an allocation finds no memory. A buffer that would take it beyond
+    // that comes from cudaMalloc: the pool gives back what it may not keep, and mapping that again costs
+    // more than cudaMalloc does (tracing 20 million photons: 97-117 ms all from the pool, 22 now, 54
+    // with cudaMalloc alone; 5 million, which fit: 4.0 against 24). Allocations and frees go through a stream of
     // their own, and a free waits for the context's stream first (a call that returns has left
     // no work behind on an earlier one), so that memory in the pool is idle. Waiting for the whole
     // device instead would break another thread's stream capture.
     cudaMemPool_t pool = nullptr;
     cudaStream_t pool_stream = nullptr;
+    uint64_t pool_keep = 0;
     // 64 slots of 64 bytes in pinned host memory, one per scene while there are some: a trace call's
     // counters arrive there with its last kernel instead of by a copy of their own
     uint32_t *status_page = nullptr;
