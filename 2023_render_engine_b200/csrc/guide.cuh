@@ -501,9 +501,8 @@ inline bool infer_whole(uint64_t n, uint64_t sms)
 
 // Forward pass over rows [0, n): src(row, q) fills the 9-float query and says whether the row
 // is guided; sink(row, valid, out) receives the 48 raw outputs (biases added; meaningless
-// where valid is false). Persistent CTAs
-// of InferShape<WHOLE>'s threads and dynamic shared memory, one per SM; the weight
-// image is staged once per CTA. A tensor-core wait that runs out of polls sets *werr
+// where valid is false). Persistent CTAs of InferShape<WHOLE>'s threads and dynamic shared memory,
+// one per SM; the weight image is staged once per CTA. A tensor-core wait that runs out of polls sets *werr
 // (nullable) and ends the group; the CTA frees its TMEM on exit.
 template <bool WHOLE, class Src, class Sink>
 __device__ __forceinline__ void guide_infer_rows(const uint4 *img, const GuideBox &box, uint32_t n, Src &src,

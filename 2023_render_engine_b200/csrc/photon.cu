@@ -9,9 +9,9 @@
 //
 // The kd-tree is the reference's implicit balanced tree (kdtree.h:78-108): the element at
 // the middle of a range is the node, split on the axis of largest extent, built on the GPU
-// (kdtree.cu), or on the host with the same partial ordering. Nearest-neighbour queries run on eight lanes each
-// (k_knn_group), or on one thread with a bounded max-heap of the k best candidates in local memory
-// (k_knn).
+// (kdtree.cu), or on the host with the same partial ordering. Nearest-neighbour queries run on eight
+// lanes each (k_knn_group), or on one thread with a bounded max-heap of the k best candidates in local
+// memory (k_knn: few neighbours of many queries, and queries with equal distances).
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>

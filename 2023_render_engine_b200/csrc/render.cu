@@ -13,7 +13,7 @@
 //             path they belong to
 //   retire  - finished paths add their radiance to the film (NaN/Inf samples dropped)
 // Path state moves with the queue (double-buffered SoA), so every stage reads and writes
-// its arrays with coalesced 16-byte accesses; queue appends are warp-aggregated.
+// its arrays with coalesced 16-byte accesses; a block takes its queue slots with one atomic a queue.
 //
 // Guided mode (RT_RENDER_GUIDE) adds an inference kernel between extend and shade: the
 // guide network maps each hit to a vMF mixture, and shade samples it or the BSDF (one-sample

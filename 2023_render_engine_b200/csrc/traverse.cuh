@@ -431,9 +431,9 @@ __device__ __forceinline__ bool walk_step(const SceneView &v, TravWarp &sm, Walk
 //
 // init(i, W) prepares ray i (walk_init); finish(i, W, bary) consumes its result. ANY: the walk
 // ends at the first accepted hit in triangle order (in the node that has one). Returns the warp's
-// rays where each warp takes one range of the queue ([x, x + y), y = 0 otherwise). COUNT: also counts the triangles a
-// serial walk would test (whole leaves, up to the leaf of the accepted hit under ANY), and every
-// ray keeps its own lane.
+// rays where each warp takes one range of the queue ([x, x + y), y = 0 otherwise). COUNT: also
+// counts the triangles a serial walk would test (whole leaves, up to the leaf of the accepted hit
+// under ANY), and every ray keeps its own lane.
 template <bool ANY, bool COUNT, bool ORDERED, typename Init, typename Finish>
 __device__ __forceinline__ uint2 walk_queue(const SceneView &v, TravWarp &sm, uint32_t n, uint32_t *work,
                                            Init init, Finish finish)

@@ -44,11 +44,11 @@ WORKLOAD = ("BVH-stress render: 1920x1080, 64 spp, max depth 12, RR after depth 
 TRACE_WORKLOAD = "closest hit of 2^{} seeded rays (origins uniform in [-1,1]^3, directions uniform), reference-exact ids"
 NRAYS = 1 << 24
 ALG_BYTES_PER_RAY = 48  # 32 B ray in + 16 B hit out (queue level)
-# DRAM bytes (read + write) of one k_trace_closest launch of the 2^24-ray call: the mean of the
-# four 2^24-ray launches of one ncu capture of this file's render command (1 pass, --cache-control
-# none; profiles/k_trace_closest_bvh_stress.md), taken at commit 39de656 of the traversal. A
-# change to traverse.cuh or trace.cu that alters k_trace_closest needs a new capture.
-TRACE_TRAFFIC_BYTES_2_24 = 2_479_014_720 + 1_033_936_064
+# DRAM bytes (read + write) of the two kernels of one 2^24-ray call (k_trace_closest, k_trace_finish): the
+# mean of the four exact calls of one ncu capture of this file's render command (1 pass,
+# --cache-control none; profiles/k_trace_closest_bvh_stress.md), taken at commit 37db333 of the
+# traversal. A change to traverse.cuh or trace.cu that alters either kernel needs a new capture.
+TRACE_TRAFFIC_BYTES_2_24 = (1_896_722_688 + 441_973_888) + (1_102_157_504 + 299_362_624)
 
 
 def dist_env():
@@ -676,23 +676,24 @@ def run_ours(args):
             "trace": {"workload": TRACE_WORKLOAD.format(NRAYS.bit_length() - 1), "value": trace_rate, "unit": "Mrays/s", "ms_per_step": ms_trace,
                       "exact_fallback_rays": int(fallback),
                       "fast_value": NRAYS * world / (ms_trace_fast / 1000) / 1e6, "fast_ms_per_step": ms_trace_fast},
-            # per frame: 6 kernels a wave (closest hit, its replay, material sort, shade, shadow,
-            # retire), the wave check of each 4-wave group and the first camera rays
+            # per frame: 6 kernels a wave (closest-hit walk, material sort, shade, shadow rays, their
+            # contributions, retire), the wave check of each 4-wave group and the first camera rays
             "gpu_launches": args.steps * (int(st_last["waves"]) * 6 + (int(st_last["waves"]) + 3) // 4 + 1),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak,
                          "traffic": (TRACE_TRAFFIC_BYTES_2_24 / (ms_trace / 1000) / 1e9) if NRAYS == 1 << 24 else None,
                          "traffic_bytes_per_launch": TRACE_TRAFFIC_BYTES_2_24 if NRAYS == 1 << 24 else None,
-                         "kernel": "k_trace_closest (2^24-ray closest-hit call, 48 B/ray queue-level bytes)",
+                         "kernel": "k_trace_closest and k_trace_finish (2^24-ray closest-hit call, 48 B/ray queue-level bytes)",
                          # what the walk itself reads (nodes x 80 B + triangle records x 48 B per ray, counted
                          # by rt_trace_counts), over the same launch time: mostly L1 and L2 hits
                          "walk": ({"bytes_per_ray": trav_work["config 1 (BVH stress)"]["bytes_per_ray"]["mean"],
                                    "gbs": trav_work["config 1 (BVH stress)"]["walk_gbs"],
                                    "frac_of_hbm_peak": trav_work["config 1 (BVH stress)"]["walk_gbs"] / peak}
                                   if trav_work else None),
-                         "note": f"peak {peak_kind}; traffic (GB/s over the same launch time) from the ncu capture "
-                                 "of the full launch: 4.4x the algorithmic bytes, the scene re-read past L2 and the "
-                                 "traversal stacks in local memory; see profiles/"},
+                         "note": f"peak {peak_kind}; traffic (GB/s over the same call time) from the ncu capture "
+                                 "of the full call: 4.6x the algorithmic bytes, the rays and hits read again by the "
+                                 "finishing kernel, the scene re-read past L2 and the traversal stacks in local "
+                                 "memory; see profiles/"},
             "clocks": clk.summary(),
             "traversal_work": trav_work,
             "guiding": guiding,
